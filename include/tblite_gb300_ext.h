@@ -96,13 +96,12 @@ void tblite_gb300_set_batch_streams(int count);
 /* smallest orbital count of a closed shell that takes the spectral projection in the batch (the
  * autotuner's threshold); a value <= 0 only queries.  Returns the previous value. */
 int tblite_gb300_set_projection_threshold(int nao);
-/* tridiagonalisation of batch buckets of at most 156 orbitals: 1 (default) the one-CTA kernel
- * with the full matrix in shared memory, 0 the packed lower-triangle kernel (a cluster of one or
- * two CTAs; two thirds of the FMAs) */
+/* tridiagonalisation of batch molecules that fit one CTA's shared memory (about 160 orbitals): 1
+ * (default) one CTA per molecule, 0 at least a cluster of two */
 void tblite_gb300_set_small_tridiag(int full_storage);
-/* schedule of the batched tridiagonalisation: 2 (default) clusters wide enough that two CTAs
- * share an SM (one computes while the other waits at a cluster barrier), 1 the narrowest
- * cluster whose CTAs fit the shared memory of one SM each */
+/* schedule of the batched tridiagonalisation: 2 (default) clusters wider than the matrix needs
+ * while the batch has few molecules (half of the SMs to spare), 1 the narrowest cluster whose
+ * CTAs hold the matrix */
 void tblite_gb300_set_tridiag_ctas_per_sm(int count);
 
 /* enable (1) or disable (0) event timing for subsequent single points (process wide) */

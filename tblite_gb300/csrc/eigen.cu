@@ -3,8 +3,8 @@
 //
 //   once per geometry   S = L L^T (Cholesky), X = L^-T                      (linalg.cu)
 //   every iteration     A = X^T F X            two triangle-aware GEMMs
-//                       A = Q T Q^T            Householder tridiagonalisation, one cooperative
-//                                              kernel, two grid barriers per column
+//                       A = Q T Q^T            Householder tridiagonalisation (tridiag.cu up to
+//                                              512 orbitals, the kernels here above)
 //                       T y = y e              all eigenvalues by Sturm-count bisection
 //   after Fermi filling eigenvectors only for the occupied orbitals: inverse iteration on T,
 //                       clusters of close eigenvalues re-orthonormalised + Rayleigh-Ritz,
@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <stdexcept>
@@ -41,6 +42,7 @@ struct EigenSolver {
   cudaStream_t stream = nullptr;
   double *L = nullptr, *X = nullptr, *A = nullptr, *T1 = nullptr;
   double *d = nullptr, *e = nullptr, *tau = nullptr, *w = nullptr, *pv = nullptr, *scal = nullptr;
+  long long* xch = nullptr;  // exchange of the grid-wide tridiagonalisation
   double *lu = nullptr;   // inverse iteration scratch [5][n][n]
   double *tw = nullptr;   // eigenvalue scratch: e^2 [n] (double), d and e^2 [n] (float)
   double *Y = nullptr;    // eigenvectors of T, column-major [k][n]
@@ -191,120 +193,169 @@ __global__ void __launch_bounds__(256) k_tridiag(int n, double* A, double* d, do
   if (n == 1 && gwarp == 0 && lane == 0) d[0] = A[0];
 }
 
-constexpr size_t TRIDIAG_SMEM_MAX = 200 * 1024;
+constexpr size_t TRIDIAG_SMEM_MAX = 220 * 1024;
+constexpr int TRIDIAG_ROWS = 8;  // rows per thread of the vector steps: n <= 2048
+constexpr size_t tridiag_smem_doubles(int n, int nb) {
+  return ((size_t)(n + nb - 1) / nb + 3) * n;
+}
 
 // Shared-memory resident variant for n where every block can hold its columns: global column j
-// lives in block j % nb (slot j / nb) for the whole reduction, so the symmetric matrix-vector
-// product, the rank-2 update and the next reflector read and write shared memory only; just the
-// reflector v and the product p travel through L2.  Two grid barriers per column.
-template <class Sync>
-__device__ __forceinline__ void tridiag_smem_body(int n, double* A, double* d, double* e, double* tau,
-                                                  double* vbuf, double* pbuf, int nb, int b,
-                                                  Sync sync) {
-  // columns owned round-robin by the nb cooperating blocks; sync() is their common barrier
+// lives in block j % nb (slot j / nb) for the whole reduction.  One grid barrier per column: p = t A v
+// (each block's own entries) and the next pivot column before its last update (from its owner)
+// travel through L2; K, w, the pivot column after the update and its reflector are formed by every
+// block for itself, and the update of the owned columns and their products with the next reflector
+// are one pass.  FP64 with the same operations in the same order as the two-barrier form before it,
+// so the results are the same bit for bit; the sums over the warps and the scalars are left to one
+// warp, because an FP64 instruction takes its scheduler 64 cycles whatever the lanes do.
+__global__ void __launch_bounds__(256) k_tridiag_smem(int n, double* A, double* d, double* e,
+                                                      double* tau, double* buf) {
+  cg::grid_group grid = cg::this_grid();
   extern __shared__ double sm[];
-
+  const int nb = (int)gridDim.x, b = (int)blockIdx.x;
   const int ncpb = (n + nb - 1) / nb;
-  double* scol = sm;                    // [ncpb][n]
-  double* sv = sm + (size_t)ncpb * n;   // [n]  reflector of the current step
-  double* sp = sv + n;                  // [n]  p of the current step
-  __shared__ double red[32];
-  __shared__ double sK;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-  // load owned columns
+  double* scol = sm;                   // [ncpb][n]
+  double* sv = sm + (size_t)ncpb * n;  // [n]  reflector of the current step
+  double* sn = sv + n;                 // [n]  pivot column, then the next reflector
+  double* sp = sn + n;                 // [n]  w of the current step
+  __shared__ double red[8];
+  __shared__ double sK, s_t, s_sc;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwb = blockDim.x >> 5;
   for (int s = 0; s < ncpb; ++s) {
     const int j = b + s * nb;
     if (j >= n) break;
-    for (int r = threadIdx.x; r < n; r += blockDim.x) scol[(size_t)s * n + r] = A[r + (size_t)j * n];
+    for (int r = tid; r < n; r += blockDim.x) scol[(size_t)s * n + r] = A[r + (size_t)j * n];
   }
-  __syncthreads();
-  // owner of column i builds reflector i from its shared copy and publishes it
-  auto reflector = [&](int i) {
-    double* col = scol + (size_t)(i / nb) * n;
-    const double alpha = col[i + 1];
-    double s = 0.0;
-    for (int r = i + 2 + threadIdx.x; r < n; r += blockDim.x) s += col[r] * col[r];
-    s = block_sum256(s, red);
-    double t = 0.0, beta = alpha;
-    if (s > 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + s), alpha);
-      t = (beta - alpha) / beta;
-    }
-    const double sc = s > 0.0 ? 1.0 / (alpha - beta) : 0.0;
-    for (int r = i + 2 + threadIdx.x; r < n; r += blockDim.x) {
-      const double v = col[r] * sc;
-      col[r] = v;
-      vbuf[r] = v;
-      A[r + (size_t)i * n] = v;
-    }
-    if (threadIdx.x == 0) {
-      vbuf[i + 1] = 1.0;
-      tau[i] = t;
-      e[i] = beta;
-      d[i] = col[i];
-    }
-  };
-  if (n > 1 && b == 0) reflector(0);
-  if (n == 1 && b == 0 && threadIdx.x == 0) d[0] = scol[0];
-  sync();
-  for (int i = 0; i < n - 1; ++i) {
-    const int m = n - i - 1;
-    const double t = tau[i];
-    // copy v (rows i+1..n-1) into shared memory
-    for (int r = i + 1 + threadIdx.x; r < n; r += blockDim.x) sv[r] = vbuf[r];
-    __syncthreads();
-    // p_j = t * A(i+1:n, j) . v for owned columns j > i
-    for (int s = wid; s < ncpb; s += nwb) {
-      const int j = b + s * nb;
-      if (j <= i || j >= n) continue;
-      const double* col = scol + (size_t)s * n;
-      double acc = 0.0;
-      for (int r = i + 1 + lane; r < n; r += 32) acc += col[r] * sv[r];
-      acc = wred(acc) * t;
-      if (lane == 0) {
-        pbuf[j] = acc;
-        pbuf[n + j] = acc * sv[j];
+  for (int r = tid; r < n; r += blockDim.x) sn[r] = A[r];
+  grid.sync();  // column 0 has been read everywhere before its owner writes the reflector there
+  double t = 0.0;
+  for (int i = -1; i < n - 1; ++i) {
+    const double* in = buf + (size_t)(i & 1) * 3 * n;
+    double* out = buf + (size_t)((i + 1) & 1) * 3 * n;
+    if (i >= 0) {
+      // K = -1/2 t (p . v), same order in every block; w = p + K v once per row
+      double pr[TRIDIAG_ROWS], qr[TRIDIAG_ROWS], cr[TRIDIAG_ROWS];
+#pragma unroll
+      for (int k = 0; k < TRIDIAG_ROWS; ++k) {
+        const int r = i + 1 + tid + k * 256;
+        const bool on = r < n;
+        pr[k] = on ? __ldcg(in + r) : 0.0;
+        qr[k] = on ? __ldcg(in + n + r) : 0.0;
+        cr[k] = on ? __ldcg(in + 2 * n + r) : 0.0;
       }
+      if (t != 0.0) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < TRIDIAG_ROWS; ++k)
+          if (i + 1 + tid + k * 256 < n) s += qr[k];
+        s = wred(s);
+        if (lane == 0) red[wid] = s;
+        __syncthreads();
+        if (wid == 0) {
+          double a = 0.0;
+          for (int k = 0; k < nwb; ++k) a += red[k];
+          if (lane == 0) sK = -0.5 * t * a;
+        }
+        __syncthreads();
+        const double K = sK;
+#pragma unroll
+        for (int k = 0; k < TRIDIAG_ROWS; ++k) {
+          const int r = i + 1 + tid + k * 256;
+          if (r < n) {
+            pr[k] = fma(K, sv[r], pr[k]);
+            sp[r] = pr[k];
+          }
+        }
+        __syncthreads();
+        const double vc = sv[i + 1], wc = sp[i + 1];
+#pragma unroll
+        for (int k = 0; k < TRIDIAG_ROWS; ++k) {
+          const int r = i + 1 + tid + k * 256;
+          if (r < n) cr[k] = fma(-sv[r], wc, fma(-pr[k], vc, cr[k]));
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < TRIDIAG_ROWS; ++k) {
+        const int r = i + 1 + tid + k * 256;
+        if (r < n) sn[r] = cr[k];
+      }
+      __syncthreads();
     }
-    sync();
-    // K = -1/2 t (p . v), same order in every block
+    const bool own = (i + 1) % nb == b;
+    if (own && tid == 0) d[i + 1] = sn[i + 1];
+    if (i + 1 == n - 1) break;
+    // reflector of column i + 1
     {
       double s = 0.0;
-      for (int r = i + 1 + threadIdx.x; r < n; r += blockDim.x) {
-        sp[r] = pbuf[r];
-        s += pbuf[n + r];
-      }
-      s = block_sum256(s, red);
-      if (threadIdx.x == 0) sK = -0.5 * t * s;
+      for (int r = i + 3 + tid; r < n; r += blockDim.x) s += sn[r] * sn[r];
+      s = wred(s);
+      if (lane == 0) red[wid] = s;
       __syncthreads();
-    }
-    const double K = sK;
-    if (t != 0.0) {
-      // w = p + K v once per row, then two FMAs per element: A -= v w^T + w v^T
-      for (int r = i + 1 + threadIdx.x; r < n; r += blockDim.x) sp[r] = fma(K, sv[r], sp[r]);
-      __syncthreads();
-      for (int s = 0; s < ncpb; ++s) {
-        const int j = b + s * nb;
-        if (j <= i || j >= n) continue;
-        double* col = scol + (size_t)s * n;
-        const double vc = sv[j], wc = sp[j];
-        for (int r = i + 1 + threadIdx.x; r < n; r += blockDim.x)
-          col[r] = fma(-sv[r], wc, fma(-sp[r], vc, col[r]));
+      if (wid == 0) {
+        s = 0.0;
+        for (int k = 0; k < nwb; ++k) s += red[k];
+        const double alpha = sn[i + 2];
+        double tn = 0.0, beta = alpha;
+        if (s > 0.0) {
+          beta = -copysign(sqrt(alpha * alpha + s), alpha);
+          tn = (beta - alpha) / beta;
+        }
+        const double sc = s > 0.0 ? 1.0 / (alpha - beta) : 0.0;
+        if (lane == 0) {
+          s_t = tn;
+          s_sc = sc;
+          if (own) {
+            tau[i + 1] = tn;
+            e[i + 1] = beta;
+          }
+        }
       }
+      __syncthreads();
+      const double sc = s_sc;
+      for (int r = i + 3 + tid; r < n; r += blockDim.x) {
+        const double v = sn[r] * sc;
+        sn[r] = v;
+        if (own) A[r + (size_t)(i + 1) * n] = v;
+      }
+      if (tid == 0) sn[i + 2] = 1.0;
     }
+    const double tn = s_t;
     __syncthreads();
-    if ((i + 1) % nb == b) {
-      if (i + 1 < n - 1) reflector(i + 1);
-      else if (threadIdx.x == 0) d[n - 1] = scol[(size_t)((n - 1) / nb) * n + (n - 1)];
+    // owned columns j >= i + 2: A -= v w^T + w v^T (two FMAs per element), then
+    // p_j = t A(i+2:n, j) . v with the next reflector; the next pivot column goes out too
+    const int r0 = i + 2;
+    for (int s = wid; s < ncpb; s += nwb) {
+      const int j = b + s * nb;
+      if (j < r0 || j >= n) continue;
+      double* col = scol + (size_t)s * n;
+      const bool piv = j == r0;
+      double acc = 0.0;
+      if (t != 0.0) {
+        const double vc = sv[j], wc = sp[j];
+#pragma unroll 4
+        for (int r = r0 + lane; r < n; r += 32) {
+          const double c = fma(-sv[r], wc, fma(-sp[r], vc, col[r]));
+          col[r] = c;
+          acc += c * sn[r];
+          if (piv) __stcg(out + 2 * n + r, c);
+        }
+      } else {
+        for (int r = r0 + lane; r < n; r += 32) {
+          acc += col[r] * sn[r];
+          if (piv) __stcg(out + 2 * n + r, col[r]);
+        }
+      }
+      acc = wred(acc) * tn;
+      if (lane == 0) {
+        __stcg(out + j, acc);
+        __stcg(out + n + j, acc * sn[j]);
+      }
     }
-    sync();
+    t = tn;
+    double* x = sv;
+    sv = sn;
+    sn = x;
+    grid.sync();
   }
-}
-__global__ void __launch_bounds__(256) k_tridiag_smem(int n, double* A, double* d, double* e,
-                                                      double* tau, double* vbuf, double* pbuf) {
-  cg::grid_group grid = cg::this_grid();
-  tridiag_smem_body(n, A, d, e, tau, vbuf, pbuf, (int)gridDim.x, (int)blockIdx.x,
-                    [&] { grid.sync(); });
 }
 
 // ------------------------------------------------------------------------------------------
@@ -979,8 +1030,9 @@ EigenSolver* eigen_create(int n, cudaStream_t s) {
   ck(cudaMalloc(&e->e, sizeof(double) * (n + 1)), "e");
   ck(cudaMalloc(&e->tau, sizeof(double) * (n + 1)), "tau");
   ck(cudaMalloc(&e->w, sizeof(double) * (n + 1)), "w");
-  ck(cudaMalloc(&e->pv, sizeof(double) * 4 * (n + 1)), "pv");
+  ck(cudaMalloc(&e->pv, sizeof(double) * 6 * (n + 1)), "pv");
   ck(cudaMalloc(&e->tw, sizeof(double) * 2 * (n + 1)), "tw");
+  ck(cudaMalloc(&e->xch, sizeof(long long) * tridiag_exchange_words(n)), "xch");
   ck(cudaMalloc(&e->scal, sizeof(double) * 8), "scal");
   ck(cudaMalloc(&e->status, sizeof(int)), "status");
   ck(cudaMalloc(&e->gstatus, sizeof(int)), "gstatus");
@@ -1007,6 +1059,7 @@ void eigen_destroy(EigenSolver* e) {
   for (double* p : {e->L, e->X, e->A, e->T1, e->Y, e->lu, e->d, e->e, e->tau, e->w, e->pv, e->tw,
                     e->scal})
     cudaFree(p);
+  cudaFree(e->xch);
   cudaFree(e->status);
   cudaFree(e->gstatus);
   cudaFreeHost(e->hstatus);
@@ -1038,29 +1091,24 @@ int eigen_values(EigenSolver* es, const double* F, double* w_out, int nev) {
   }
   // tridiagonalise
   {
-    int nn = n;
-    int blocks = es->coop_blocks;
-    const int need = (n * 32 + 255) / 256;
-    if (blocks > need) blocks = need > 0 ? need : 1;
-    // shared-memory resident path when every block can hold its columns
-    int nb = blocks;
-    const size_t ncpb = (n + nb - 1) / nb;
-    const size_t smem = sizeof(double) * (ncpb * n + 2 * (size_t)n);
-    if (smem <= TRIDIAG_SMEM_MAX) {
-      double* vbuf = es->pv;
-      double* pbuf = es->pv + (n + 1);
-      void* args[] = {&nn, &es->A, &es->d, &es->e, &es->tau, &vbuf, &pbuf};
-      ++g_kernel_launches;
-      const int tk = prof_kbegin(s);
-      ck(cudaLaunchCooperativeKernel((void*)k_tridiag_smem, nb, 256, args, smem, s), "tridiag_smem");
-      prof_kend(KS_TRIDIAG, tk, s);
+    const int tk = prof_kbegin(s);
+    if (n <= TRIDIAG_FIXED_MAX) {
+      tridiag_fixed(n, es->A, es->d, es->e, es->tau, es->xch, s);
     } else {
-      void* args[] = {&nn, &es->A, &es->d, &es->e, &es->tau, &es->pv, &es->scal};
+      int nn = n, blocks = std::min(es->coop_blocks, (n * 32 + 255) / 256);
+      // shared-memory resident while every block can hold its columns
+      const size_t smem = sizeof(double) * tridiag_smem_doubles(n, blocks);
       ++g_kernel_launches;
-      const int tk = prof_kbegin(s);
-      ck(cudaLaunchCooperativeKernel((void*)k_tridiag, blocks, 256, args, 0, s), "tridiag");
-      prof_kend(KS_TRIDIAG, tk, s);
+      if (smem <= TRIDIAG_SMEM_MAX && n <= 256 * TRIDIAG_ROWS) {
+        void* args[] = {&nn, &es->A, &es->d, &es->e, &es->tau, &es->pv};
+        ck(cudaLaunchCooperativeKernel((void*)k_tridiag_smem, blocks, 256, args, smem, s),
+           "tridiag_smem");
+      } else {
+        void* args[] = {&nn, &es->A, &es->d, &es->e, &es->tau, &es->pv, &es->scal};
+        ck(cudaLaunchCooperativeKernel((void*)k_tridiag, blocks, 256, args, 0, s), "tridiag");
+      }
     }
+    prof_kend(KS_TRIDIAG, tk, s);
   }
   if (nev <= 0 || nev > n) nev = n;
   g_kernel_launches += 2;
@@ -1153,257 +1201,12 @@ bool eigen_gemm_failed(EigenSolver* es) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Batched eigensolver: one thread-block cluster per molecule for the tridiagonalisation (the
-// columns stay in the cluster's shared memory, the barrier is the cluster's hardware barrier
-// instead of a grid barrier), blockIdx.z over molecules for the other steps.  The eigenvalues
+// Batched eigensolver: blockIdx.z over molecules (the tridiagonalisation in tridiag.cu: one CTA or
+// thread-block cluster per molecule).  The eigenvalues
 // are written straight into emo; icount (from the Fermi filling) bounds the vectors.
 // ------------------------------------------------------------------------------------------
 #define BMOL const MolPtrs& q = mp[list[blockIdx.z]]
 #define BARGS const MolPtrs* __restrict__ mp, const int* __restrict__ list
-
-// Householder tridiagonalisation of one molecule per thread-block cluster, lower-triangle
-// storage.  Column j lives in CTA j % nb of the cluster, packed (rows j .. n-1 only), so the
-// cluster holds n^2/2 doubles instead of n^2 and each element costs four FMAs per step
-// instead of six:
-//   p = A v   a column's dot product covers its rows r >= c; the rows above the diagonal are
-//             the same elements seen from their own columns, so every CTA also scatters
-//             A(r, c) v_c into a partial vector (one thread per row, no atomics), and each CTA
-//             sums the nb partial vectors through distributed shared memory;
-//   A -= v w^T + w v^T on the stored lower part only, w = t p + K v formed once per row.
-// Two cluster barriers per column, as in the full-storage form; v and tau of a step are read
-// from the owner CTA's shared memory.  The reflectors also go to global A (column-major, below
-// the subdiagonal) for the back-transformation.
-__device__ __forceinline__ size_t sym_off(int s, int n, int b, int nb) {
-  return (size_t)s * n - (size_t)s * b - (size_t)nb * s * (s - 1) / 2;
-}
-constexpr int TRI_WARPS = 8;  // warps of a kb_tridiag CTA (256 threads)
-__host__ __device__ inline size_t sym_tridiag_doubles(int n, int nb) {
-  const size_t ncpb = (size_t)(n + nb - 1) / nb;  // CTA 0 owns the most columns
-  // packed columns, four vectors (+1) and one row accumulator per warp
-  return ncpb * n - (size_t)nb * ncpb * (ncpb - 1) / 2 + (4 + TRI_WARPS) * (size_t)n + 1;
-}
-__global__ void __launch_bounds__(256) kb_tridiag(BARGS) {
-  cg::cluster_group cl = cg::this_cluster();
-  BMOL;
-  const int n = q.m.nao;
-  const int nb = (int)cl.num_blocks(), b = (int)cl.block_rank();
-  double* Ag = q.A;
-  double* d = q.ed;
-  double* e = q.ee;
-  double* tau = q.etau;
-  extern __shared__ double sm[];
-  const int ncpb = b < n ? (n - b + nb - 1) / nb : 0;
-  // the vectors first: other CTAs address spart and svpub at the same offset in their view
-  double* sv = sm;             // [n] v of the current step
-  double* sw = sv + n;         // [n] w = t p + K v
-  double* spart = sw + n;      // [n] this CTA's part of p (read by the others)
-  double* svpub = spart + n;   // [n + 1] v and tau published by the owner
-  double* wrow = svpub + n + 1;  // [TRI_WARPS][n] per-warp row accumulators of p, kept zero
-  double* scol = wrow + (size_t)TRI_WARPS * n;  // packed columns (their total differs by CTA)
-  __shared__ double red[32];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwb = blockDim.x >> 5;
-  for (int s = 0; s < ncpb; ++s) {
-    const int j = b + s * nb;
-    double* col = scol + sym_off(s, n, b, nb) - j;
-    for (int r = j + tid; r < n; r += blockDim.x) col[r] = Ag[r + (size_t)j * n];
-  }
-  for (size_t u = tid; u < (size_t)TRI_WARPS * n; u += blockDim.x) wrow[u] = 0.0;
-  __syncthreads();
-  auto column = [&](int s) { return scol + sym_off(s, n, b, nb) - (b + s * nb); };  // col[r], r >= c
-  // owner of column i builds reflector i from its stored column and publishes v, tau
-  auto reflector = [&](int i) {
-    double* col = column(i / nb);
-    const double alpha = col[i + 1];
-    double ss = 0.0;
-    for (int r = i + 2 + tid; r < n; r += blockDim.x) ss += col[r] * col[r];
-    ss = block_sum256(ss, red);
-    double t = 0.0, beta = alpha;
-    if (ss > 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + ss), alpha);
-      t = (beta - alpha) / beta;
-    }
-    const double sc = ss > 0.0 ? 1.0 / (alpha - beta) : 0.0;
-    for (int r = i + 2 + tid; r < n; r += blockDim.x) {
-      const double v = col[r] * sc;
-      col[r] = v;
-      svpub[r] = v;
-      Ag[r + (size_t)i * n] = v;
-    }
-    if (tid == 0) {
-      svpub[i + 1] = 1.0;
-      svpub[n] = t;
-      tau[i] = t;
-      e[i] = beta;
-      d[i] = col[i];
-    }
-  };
-  if (n == 1 && b == 0 && tid == 0) d[0] = scol[0];
-  if (n > 1 && b == 0) reflector(0);
-  cl.sync();
-  for (int i = 0; i < n - 1; ++i) {
-    // v_i and tau_i from the owner of column i
-    const double* pv = cl.map_shared_rank(svpub, i % nb);
-    for (int r = i + 1 + tid; r < n; r += blockDim.x) sv[r] = pv[r];
-    const double t = pv[n];
-    const int s0 = i < b ? 0 : (i - b) / nb + 1;  // first owned column > i
-    if (t != 0.0) {
-      __syncthreads();
-      // p from the owned columns c > i, one warp per column and one pass over its stored rows
-      // r >= c: the column's dot product sum_r A(r, c) v_r goes to p_c, and A(r, c) v_c (r > c,
-      // the elements above the diagonal seen from their rows) into the warp's row accumulator
-      double* acc = wrow + (size_t)wid * n;
-      for (int s2 = s0 + wid; s2 < ncpb; s2 += nwb) {
-        const int c = b + s2 * nb;
-        const double* col = column(s2);
-        const double vc = sv[c];
-        double dot = 0.0;
-        int r = c + lane;
-        if (r == c) {  // the diagonal: dot only
-          dot = col[r] * sv[r];
-          r += 32;
-        }
-        for (; r < n; r += 32) {
-          const double a = col[r];
-          dot = fma(a, sv[r], dot);
-          acc[r] = fma(a, vc, acc[r]);
-        }
-        dot = wred(dot);
-        if (lane == 0) acc[c] += dot;
-        __syncwarp();
-      }
-      __syncthreads();
-      // this CTA's part of p: the sum of the warp accumulators, which are zeroed again
-      for (int r = i + 1 + tid; r < n; r += blockDim.x) {
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < TRI_WARPS; ++w) {
-          s += wrow[(size_t)w * n + r];
-          wrow[(size_t)w * n + r] = 0.0;
-        }
-        spart[r] = s;
-      }
-    }
-    cl.sync();
-    if (t != 0.0) {
-      // p = t * (sum of the nb partial vectors), K = -t/2 p.v (same order in every CTA)
-      double kk = 0.0;
-      for (int r = i + 1 + tid; r < n; r += blockDim.x) {
-        double p = 0.0;
-        for (int q2 = 0; q2 < nb; ++q2) p += cl.map_shared_rank(spart, q2)[r];
-        p *= t;
-        sw[r] = p;
-        kk = fma(p, sv[r], kk);
-      }
-      kk = block_sum256(kk, red);
-      const double K = -0.5 * t * kk;
-      for (int r = i + 1 + tid; r < n; r += blockDim.x) sw[r] = fma(K, sv[r], sw[r]);
-      __syncthreads();
-      // rank-2 update of the owned columns c > i, one warp per column
-      for (int s2 = s0 + wid; s2 < ncpb; s2 += nwb) {
-        const int c = b + s2 * nb;
-        double* col = column(s2);
-        const double vc = sv[c], wc = sw[c];
-        for (int r = c + lane; r < n; r += 32) col[r] = fma(-sv[r], wc, fma(-sw[r], vc, col[r]));
-      }
-    }
-    __syncthreads();
-    if ((i + 1) % nb == b) {
-      if (i + 1 < n - 1) reflector(i + 1);
-      else if (tid == 0) d[n - 1] = column((n - 1) / nb)[n - 1];
-    }
-    cl.sync();
-  }
-}
-// Small molecules (the whole n x n matrix in one CTA's shared memory): the same Householder
-// reduction with everything on chip.  Per column: warp 0 builds the reflector (no block
-// reduction), the warps form p = t A22 v column by column, every warp reduces K = -t/2 p.v
-// for itself, w = p + K v is formed once per row, and all threads apply the symmetric rank-2
-// update to the lower triangle only (two FMAs per stored element, half the elements of the
-// full block).  p_j then reads column j from the diagonal down and the rest of it, above the
-// diagonal, as row j of the lower triangle (the same elements by symmetry); the columns are
-// ld = n | 1 doubles apart, so those row reads hit distinct banks.  Five block barriers per
-// column.  The reflectors and the diagonal go to global memory at the end in the layout the
-// back-transformation reads (column-major A, v below the subdiagonal).
-constexpr int TRI_SMALL_MAX = 156;  // n (n | 1) + 2n doubles <= 200 KB
-__host__ __device__ constexpr size_t tri_small_doubles(int n) {
-  return (size_t)n * (size_t)(n | 1) + 2 * (size_t)n;
-}
-static_assert(sizeof(double) * tri_small_doubles(TRI_SMALL_MAX) <= TRIDIAG_SMEM_MAX,
-              "the largest small tridiagonalisation fits the shared-memory attribute");
-__global__ void __launch_bounds__(256) kb_tridiag_small(BARGS) {
-  BMOL;
-  const int n = q.m.nao, ld = n | 1;
-  extern __shared__ double sm[];
-  double* a = sm;                    // [n][ld] column-major; the lower triangle is kept current
-  double* sv = sm + (size_t)n * ld;  // [n] reflector (sv[i+1] = 1)
-  double* sp = sv + n;               // [n] p, then w
-  __shared__ double s_t;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-  const double* A0 = q.A;
-  for (int t = tid; t < n * n; t += blockDim.x) a[(size_t)(t / n) * ld + t % n] = A0[t];
-  __syncthreads();
-  for (int i = 0; i < n - 1; ++i) {
-    const int r0 = i + 1;  // trailing block rows/cols r0 .. n-1
-    if (wid == 0) {        // reflector of column i
-      double* col = a + (size_t)i * ld;
-      const double alpha = col[r0];
-      double s = 0.0;
-      for (int r = r0 + 1 + lane; r < n; r += 32) s += col[r] * col[r];
-      s = wred(s);
-      double t = 0.0, beta = alpha;
-      if (s > 0.0) {
-        beta = -copysign(sqrt(alpha * alpha + s), alpha);
-        t = (beta - alpha) / beta;
-      }
-      const double sc = s > 0.0 ? 1.0 / (alpha - beta) : 0.0;
-      for (int r = r0 + 1 + lane; r < n; r += 32) {
-        const double v = col[r] * sc;
-        col[r] = v;
-        sv[r] = v;
-      }
-      if (lane == 0) {
-        sv[r0] = 1.0;
-        s_t = t;
-        q.etau[i] = t;
-        q.ee[i] = beta;
-        q.ed[i] = col[i];
-      }
-    }
-    __syncthreads();
-    const double t = s_t;
-    if (t != 0.0) {
-      // p_j = t * A22(:, j) . v  (warp per column): rows j .. n-1 from column j, rows
-      // r0 .. j-1 from row j
-      for (int j = r0 + wid; j < n; j += nw) {
-        const double* col = a + (size_t)j * ld;
-        double acc = 0.0;
-        for (int r = j + lane; r < n; r += 32) acc += col[r] * sv[r];
-        for (int r = r0 + lane; r < j; r += 32) acc += a[(size_t)r * ld + j] * sv[r];
-        acc = wred(acc) * t;
-        if (lane == 0) sp[j] = acc;
-      }
-      __syncthreads();
-      // K = -1/2 t (p . v), each warp for itself
-      double kk = 0.0;
-      for (int r = r0 + lane; r < n; r += 32) kk += sp[r] * sv[r];
-      const double K = -0.5 * t * wred(kk);
-      __syncthreads();  // every warp has read p
-      // w = p + K v once per row, then two FMAs per element: A -= v w^T + w v^T (lower part)
-      for (int r = r0 + tid; r < n; r += blockDim.x) sp[r] = fma(K, sv[r], sp[r]);
-      __syncthreads();
-      for (int c = r0 + wid; c < n; c += nw) {  // warp per column, v_c and w_c in registers
-        double* col = a + (size_t)c * ld;
-        const double vc = sv[c], wc = sp[c];
-        for (int r = c + lane; r < n; r += 32) col[r] = fma(-sv[r], wc, fma(-sp[r], vc, col[r]));
-      }
-    }
-    __syncthreads();
-  }
-  if (tid == 0) q.ed[n - 1] = a[(size_t)(n - 1) * ld + (n - 1)];
-  // reflectors (strictly below the subdiagonal of each column) for the back-transformation
-  double* Ag = q.A;
-  for (int t2 = tid; t2 < n * n; t2 += blockDim.x) Ag[t2] = a[(size_t)(t2 / n) * ld + t2 % n];
-}
 
 // Eigenvalues for the batch, one thread per eigenvalue (tri_eigenvalue: FP32 bisection, FP64
 // check, FP64 Illinois / bisection).  d, e^2 and their FP32 copies are staged in shared memory
@@ -1468,71 +1271,21 @@ __global__ void kb_scale_cols(BARGS, int mode) {
   scale_cols_dev(n, *q.icount, q.C, f, q.scratch);
 }
 
-// CTAs of the batched tridiagonalisation that should fit on one SM (1 or 2): with 2 the
-// clusters are made wide enough that each CTA holds at most ~110 KB, so a second molecule's CTA
-// computes while the first waits at a cluster barrier
-static int g_tridiag_ctas_per_sm = 2;
-// smallest cluster (1, 2, 4, 8 blocks) whose shared memory holds the lower triangle, within the
-// per-CTA budget of the chosen residency when possible
-static int tridiag_cluster(int n, size_t* smem) {
-  const size_t caps[2] = {g_tridiag_ctas_per_sm >= 2 ? (size_t)110 * 1024 : TRIDIAG_SMEM_MAX,
-                          TRIDIAG_SMEM_MAX};
-  for (size_t cap : caps)
-    for (int nb = 1; nb <= 8; nb *= 2) {
-      const size_t need = sizeof(double) * sym_tridiag_doubles(n, nb);
-      if (need <= cap) {
-        *smem = need;
-        return nb;
-      }
-    }
-  return 0;
-}
-void set_tridiag_ctas_per_sm(int k) { g_tridiag_ctas_per_sm = k >= 2 ? 2 : 1; }
-int get_tridiag_ctas_per_sm() { return g_tridiag_ctas_per_sm; }
-// buckets of at most TRI_SMALL_MAX orbitals: the one-CTA full-storage kernel (1, default) or the
-// packed lower-triangle kernel as a cluster of one CTA (0: two thirds of the FMAs, half the
-// shared memory, but row accumulators summed per column)
-static int g_tridiag_small = 1;
-void set_tridiag_small(int k) { g_tridiag_small = k ? 1 : 0; }
-int get_tridiag_small() { return g_tridiag_small; }
-int batch_tridiag_max_n() {
-  int n = 1;
-  size_t sm = 0;
-  while (tridiag_cluster(n + 1, &sm)) ++n;  // the second cap is the residency-independent one
-  return n;
-}
-
 static void batch_attributes() {
   static bool done = false;
   if (done) return;
-  ck(cudaFuncSetAttribute(kb_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)TRIDIAG_SMEM_MAX),
-     "smem attr batch tridiag");
-  ck(cudaFuncSetAttribute(kb_tridiag_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)TRIDIAG_SMEM_MAX),
-     "smem attr batch tridiag small");
   ck(cudaFuncSetAttribute(kb_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)BT_SMEM_MAX + (int)(BT_WARPS_B * sizeof(double) * 64)),
      "smem attr batch backtransform");
   done = true;
 }
 
-static void tridiag_cluster_b(const BatchLaunch& b);
-
 void eigen_values_b(const BatchLaunch& b) {
   if (!b.count) return;
   batch_attributes();
   gemm_b(b, GS_FX);
   gemm_b(b, GS_XTT);
-  if (b.nao_max <= TRI_SMALL_MAX && g_tridiag_small) {
-    const size_t sm_small = sizeof(double) * tri_small_doubles(b.nao_max);
-    ++g_kernel_launches;
-    const int tk = prof_kbegin(b.s);
-    kb_tridiag_small<<<dim3(1, 1, b.count), 256, sm_small, b.s>>>(b.mp, b.list);
-    prof_kend(KS_TRIDIAG, tk, b.s);
-  } else {
-    tridiag_cluster_b(b);
-  }
+  tridiag_fixed_b(b);
   ++g_kernel_launches;
   const int tm = prof_kbegin(b.s);
   if (b.nao_max > BIS_MAXN) throw std::runtime_error("batched eigenvalues: molecule too large");
@@ -1546,28 +1299,6 @@ void eigen_values_rest_b(const BatchLaunch& b) {
   ++g_kernel_launches;
   kb_eigvals<<<dim3((b.nao_max + EIG_BLOCK - 1) / EIG_BLOCK, 1, b.count), EIG_BLOCK, 0, b.s>>>(
       b.mp, b.list, 1);
-}
-
-static void tridiag_cluster_b(const BatchLaunch& b) {
-  size_t smem = 0;
-  const int nb = tridiag_cluster(b.nao_max, &smem);
-  if (!nb) throw std::runtime_error("batched tridiagonalisation: molecule too large");
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nb, 1, b.count);
-  cfg.blockDim = dim3(256, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = b.s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = nb;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  ++g_kernel_launches;
-  const int tk = prof_kbegin(b.s);
-  ck(cudaLaunchKernelEx(&cfg, kb_tridiag, b.mp, b.list), "batch tridiag");
-  prof_kend(KS_TRIDIAG, tk, b.s);
 }
 
 void eigen_vectors_b(const BatchLaunch& b) {

@@ -252,6 +252,13 @@ void eigen_destroy(EigenSolver*);
 // largest order the solver's buffers hold; eigen_resize switches to any order up to it
 int eigen_capacity(const EigenSolver*);
 void eigen_resize(EigenSolver*, int n);
+// fixed-point tridiagonalisation (tridiag.cu) of the symmetric column-major A (n x n, n up to
+// TRIDIAG_FIXED_MAX): d, e, tau and the reflectors below the subdiagonal of A, as dsytrd('L'); xch
+// holds tridiag_exchange_words(n) words
+constexpr int TRIDIAG_FIXED_MAX = 512;
+void tridiag_fixed(int n, double* A, double* d, double* e, double* tau, long long* xch,
+                   cudaStream_t s);
+size_t tridiag_exchange_words(int n);
 // factorise S once per geometry; returns 0 on success, >0 if S is not positive definite
 int eigen_set_overlap(EigenSolver*, const double* S);
 // eigenvalues (ascending) of F C = S C e; keeps the tridiagonal form for eigen_vectors.
@@ -513,6 +520,7 @@ void ogemm_b(const BatchLaunch& b, int site);
 extern bool g_split_gemm;
 // eigensolver steps for a bucket
 void cholesky_inverse_b(const BatchLaunch& b);          // S -> X (status into flag)
+void tridiag_fixed_b(const BatchLaunch& b);             // A -> ed, ee, etau (tridiag.cu)
 void eigen_values_b(const BatchLaunch& b);              // F -> emo (tridiagonal form kept)
 void eigen_values_rest_b(const BatchLaunch& b);         // emo[nev..n) after convergence
 void eigen_vectors_b(const BatchLaunch& b);             // icount lowest vectors into C
