@@ -646,9 +646,17 @@ __global__ void __launch_bounds__(32) k_eigvals(int n, int j0, int j1, int fill,
 
 // ------------------------------------------------------------------------------------------
 // inverse iteration: one thread per eigenvector (column j < k), Gaussian elimination with
-// partial pivoting of the tridiagonal T - w_j I, three solves from a pseudo-random start.
-// scratch layout [array][row][j] keeps the per-row accesses of a warp contiguous.
-// Y is written column-major [j][n].
+// partial pivoting of the tridiagonal T - w_j I, two solves from a pseudo-random start.
+//
+// Bound by the chain of FP64 instructions of one warp (64-71 cycles each, whatever the active
+// lanes): about 25 per row, six of them the division.  So the two pivot cases share one division
+// and one update by selecting operands, comparisons read the bit patterns, the reciprocals of the
+// pivots are formed once, the second superdiagonal is read back from e (it is e[r + 1] where rows
+// were interchanged, else 0), and the rows move through registers in blocks of 8, the next block's
+// loads issued before the current block's chain.  Scratch rows are contiguous over the warp's
+// vectors ([row][vector]); the finished columns go to Y (column-major [j][n]) through a
+// shared-memory transpose.  C200H402 (1202 rows, 601 vectors) 4.45 -> 1.89 ms, 192 rows and 96
+// vectors 540 -> 290 us, with the same bits.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ double hash_uniform(unsigned a, unsigned b) {
   unsigned h = a * 0x9E3779B1u ^ (b + 0x7F4A7C15u) * 0x85EBCA77u;
@@ -657,79 +665,182 @@ __device__ __forceinline__ double hash_uniform(unsigned a, unsigned b) {
   h ^= h >> 12;
   h *= 0x297A2D39u;
   h ^= h >> 15;
-  return (double)h / 4294967296.0 * 2.0 - 1.0;
+  return (double)(int)(h ^ 0x80000000u) * 0x1p-31;  // 2 h / 2^32 - 1, exactly
 }
 
+constexpr int INV_B = 8;       // rows in registers
+constexpr int INV_WARP = 32;   // threads of a block
 __device__ __forceinline__ void invit_dev(int n, int k0, int k, const double* __restrict__ d,
                         const double* __restrict__ e, const double* __restrict__ w,
                         const double* __restrict__ scal, double* lu, double* Y) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;  // vector k0 + j of the spectrum
-  if (j >= k) return;
+  __shared__ double tile[32][33];
+  if ((int)(blockIdx.x * blockDim.x) >= k) return;
+  const int lane = threadIdx.x;
+  const int jb = blockIdx.x * blockDim.x;
+  const int j = min(jb + lane, k - 1);  // vector k0 + j; idle lanes repeat the last one
+  const bool mine = jb + lane < k;
   const size_t nk = (size_t)n * k;
-  double* U0 = lu;
-  double* U1 = lu + nk;
-  double* U2 = lu + 2 * nk;
-  double* Lm = lu + 3 * nk;
-  double* PV = lu + 4 * nk;  // pivot flag stored as double
-#define AT(arr, r) arr[(size_t)(r) * k + j]
+  double* __restrict__ U1 = lu + j;           // first superdiagonal
+  double* __restrict__ R0 = lu + nk + j;      // 1 / pivot
+  double* __restrict__ Lm = lu + 2 * nk + j;  // multiplier
+  double* __restrict__ Yt = lu + 3 * nk + j;  // the vector
+  unsigned* PV = reinterpret_cast<unsigned*>(lu + 4 * nk) + j;  // interchange bits of 32 rows
   const double lam = w[k0 + j];
   const double tnorm = scal[1] > 0 ? scal[1] : 1.0;
   const double tiny = 2.220446049250313e-16 * tnorm;
+  auto absbits = [](double x) {
+    return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+  };
+  const unsigned long long btiny = absbits(tiny);
   // factorise T - lam I
-  double u0 = d[0] - lam, u1 = n > 1 ? e[0] : 0.0, u2 = 0.0;
+  double u0 = d[0] - lam, u1 = n > 1 ? e[0] : 0.0;
+  unsigned bits = 0u;
+  double ec = u1;  // e[r]
   for (int r = 0; r < n - 1; ++r) {
-    const double c = e[r];                                  // sub-diagonal of row r+1
+    const double c = ec;                                    // sub-diagonal of row r+1
     const double a1 = d[r + 1] - lam, b1 = r + 1 < n - 1 ? e[r + 1] : 0.0;
-    if (fabs(u0) >= fabs(c)) {
-      if (fabs(u0) < tiny) u0 = copysign(tiny, u0 == 0.0 ? 1.0 : u0);
-      const double l = c / u0;
-      AT(U0, r) = u0; AT(U1, r) = u1; AT(U2, r) = u2; AT(Lm, r) = l; AT(PV, r) = 0.0;
-      u0 = a1 - l * u1;
-      u1 = b1 - l * u2;
-      u2 = 0.0;
-    } else {
-      const double l = u0 / c;
-      AT(U0, r) = c; AT(U1, r) = a1; AT(U2, r) = b1; AT(Lm, r) = l; AT(PV, r) = 1.0;
-      const double n0 = u1 - l * a1, n1 = u2 - l * b1;
-      u0 = n0;
-      u1 = n1;
-      u2 = 0.0;
+    const bool keep = absbits(u0) >= absbits(c);
+    if (keep && absbits(u0) < btiny) u0 = copysign(tiny, u0 == 0.0 ? 1.0 : u0);
+    const double piv = keep ? u0 : c;
+    const double l = (keep ? c : u0) / piv;
+    if (mine) {
+      U1[(size_t)r * k] = keep ? u1 : a1;
+      R0[(size_t)r * k] = frcp(piv);
+      Lm[(size_t)r * k] = l;
     }
+    if (!keep) bits |= 1u << (r & 31);
+    if ((r & 31) == 31) {
+      if (mine) PV[(size_t)(r >> 5) * k] = bits;
+      bits = 0u;
+    }
+    // kept: u0' = a1 - l u1, u1' = b1; interchanged: u0' = u1 - l a1, u1' = -l b1
+    u0 = fma(-l, keep ? u1 : a1, keep ? a1 : u1);
+    u1 = keep ? b1 : -l * b1;
+    ec = b1;
   }
-  if (fabs(u0) < tiny) u0 = copysign(tiny, u0 == 0.0 ? 1.0 : u0);
-  AT(U0, n - 1) = u0; AT(U1, n - 1) = 0.0; AT(U2, n - 1) = 0.0;
-  double* y = Y + (size_t)(k0 + j) * n;
-  for (int r = 0; r < n; ++r) y[r] = hash_uniform(k0 + j + 1, r + 1);
+  if (mine) PV[(size_t)((n - 1) >> 5) * k] = bits;
+  if (absbits(u0) < btiny) u0 = copysign(tiny, u0 == 0.0 ? 1.0 : u0);
+  const double rlast = frcp(u0);
+  double scale = 1.0;
   for (int iter = 0; iter < 2; ++iter) {
-    // forward: apply row operations to the right-hand side
-    for (int r = 0; r < n - 1; ++r) {
-      const double l = AT(Lm, r);
-      if (AT(PV, r) == 0.0) {
-        y[r + 1] -= l * y[r];
-      } else {
-        const double t = y[r];
-        y[r] = y[r + 1];
-        y[r + 1] = t - l * y[r];
+    // forward: apply row operations to the right-hand side (start vector, or the scaled result of
+    // the first solve)
+    double cur = iter ? Yt[0] * scale : hash_uniform(k0 + j + 1, 1);
+    double yn[INV_B], ln[INV_B];
+#pragma unroll
+    for (int t = 0; t < INV_B; ++t) {
+      const int r = min(t, n - 2);
+      if (n > 1) {
+        ln[t] = Lm[(size_t)r * k];
+        if (iter) yn[t] = Yt[(size_t)(r + 1) * k];
       }
     }
+    for (int r0 = 0; r0 < n - 1; r0 += INV_B) {
+      double yv[INV_B], lv[INV_B];
+#pragma unroll
+      for (int t = 0; t < INV_B; ++t) {
+        yv[t] = iter ? yn[t] * scale : hash_uniform(k0 + j + 1, r0 + t + 2);
+        lv[t] = ln[t];
+      }
+      const unsigned pv = PV[(size_t)(r0 >> 5) * k] >> (r0 & 31);
+#pragma unroll
+      for (int t = 0; t < INV_B; ++t) {  // next block
+        const int r = min(r0 + INV_B + t, n - 2);
+        ln[t] = Lm[(size_t)r * k];
+        if (iter) yn[t] = Yt[(size_t)(r + 1) * k];
+      }
+#pragma unroll
+      for (int t = 0; t < INV_B; ++t)
+        if (r0 + t < n - 1) {
+          const bool sw = (pv >> t) & 1u;
+          const double p = sw ? yv[t] : cur, q = sw ? cur : yv[t];
+          if (mine) Yt[(size_t)(r0 + t) * k] = p;
+          cur = fma(-lv[t], p, q);
+        }
+    }
+    if (mine) Yt[(size_t)(n - 1) * k] = cur;
     // backward: U x = y
-    double x1 = 0.0, x2 = 0.0;
-    for (int r = n - 1; r >= 0; --r) {
-      const double v = (y[r] - AT(U1, r) * x1 - AT(U2, r) * x2) * frcp(AT(U0, r));
-      y[r] = v;
-      x2 = x1;
-      x1 = v;
+    double x1 = cur * rlast, x2 = 0.0;
+    if (mine) Yt[(size_t)(n - 1) * k] = x1;
+    double rn[INV_B], un[INV_B];
+#pragma unroll
+    for (int t = 0; t < INV_B; ++t) {
+      const size_t r = (size_t)max(n - 2 - t, 0) * k;
+      yn[t] = Yt[r];
+      un[t] = U1[r];
+      rn[t] = R0[r];
+    }
+    for (int r0 = n - 2; r0 >= 0; r0 -= INV_B) {  // rows r0, r0 - 1, ..
+      double yv[INV_B], uv[INV_B], rv[INV_B], ev[INV_B];
+      unsigned pv = 0u;
+#pragma unroll
+      for (int t = 0; t < INV_B; ++t) {
+        const int r = max(r0 - t, 0);
+        yv[t] = yn[t];
+        uv[t] = un[t];
+        rv[t] = rn[t];
+        ev[t] = r + 1 < n - 1 ? e[r + 1] : 0.0;
+      }
+      {
+        const int rl = max(r0 - INV_B + 1, 0);
+        const unsigned wl = PV[(size_t)(rl >> 5) * k], wh = PV[(size_t)(r0 >> 5) * k];
+        pv = __funnelshift_r(wl, (r0 >> 5) == (rl >> 5) ? 0u : wh, rl & 31) << (INV_B - 1 - (r0 - rl));
+      }  // bit INV_B - 1 - t: row r0 - t
+#pragma unroll
+      for (int t = 0; t < INV_B; ++t) {  // next block
+        const size_t r = (size_t)max(r0 - INV_B - t, 0) * k;
+        yn[t] = Yt[r];
+        un[t] = U1[r];
+        rn[t] = R0[r];
+      }
+      const bool any = __any_sync(0xffffffffu, (pv & ((1u << INV_B) - 1)) != 0u);
+#pragma unroll
+      for (int t = 0; t < INV_B; ++t)
+        if (r0 - t >= 0) {
+          double v = fma(-uv[t], x1, yv[t]);
+          if (any) v = fma(-(((pv >> (INV_B - 1 - t)) & 1u) ? ev[t] : 0.0), x2, v);
+          v *= rv[t];
+          if (mine) Yt[(size_t)(r0 - t) * k] = v;
+          x2 = x1;
+          x1 = v;
+        }
     }
     double nrm = 0.0;
-    for (int r = 0; r < n; ++r) nrm += y[r] * y[r];
-    nrm = 1.0 / sqrt(nrm);
-    for (int r = 0; r < n; ++r) y[r] *= nrm;
+    {
+#pragma unroll
+      for (int t = 0; t < INV_B; ++t) yn[t] = Yt[(size_t)min(t, n - 1) * k];
+      for (int r0 = 0; r0 < n; r0 += INV_B) {
+        double yv[INV_B];
+#pragma unroll
+        for (int t = 0; t < INV_B; ++t) {
+          yv[t] = yn[t];
+          yn[t] = Yt[(size_t)min(r0 + INV_B + t, n - 1) * k];
+        }
+#pragma unroll
+        for (int t = 0; t < INV_B; ++t)
+          if (r0 + t < n) nrm += yv[t] * yv[t];
+      }
+    }
+    scale = 1.0 / sqrt(nrm);
   }
-#undef AT
+  // Y[k0 + j][r], 32 rows at a time
+  const int cols = min(32, k - jb);
+  for (int r0 = 0; r0 < n; r0 += 32) {
+    __syncwarp();
+#pragma unroll 8
+    for (int t = 0; t < 32; ++t)
+      if (r0 + t < n) tile[t][lane] = Yt[(size_t)(r0 + t) * k] * scale;
+    __syncwarp();
+    if (r0 + lane < n)
+#pragma unroll 8
+      for (int t = 0; t < cols; ++t)
+        Y[(size_t)(k0 + jb + t) * n + r0 + lane] = tile[lane][t];
+  }
 }
-__global__ void k_invit(int n, int k0, int k, const double* __restrict__ d,
-                        const double* __restrict__ e, const double* __restrict__ w,
-                        const double* __restrict__ scal, double* lu, double* Y) {
+__global__ void __launch_bounds__(INV_WARP) k_invit(int n, int k0, int k,
+                        const double* __restrict__ d, const double* __restrict__ e,
+                        const double* __restrict__ w, const double* __restrict__ scal, double* lu,
+                        double* Y) {
   invit_dev(n, k0, k, d, e, w, scal, lu, Y);
 }
 
@@ -1141,7 +1252,7 @@ void eigen_vectors_range(EigenSolver* es, int k0, int k1, double* C) {
   if (k <= 0) return;
   ++g_kernel_launches;
   const int ti = prof_kbegin(s);
-  k_invit<<<(k + 15) / 16, 16, 0, s>>>(n, k0, k, es->d, es->e, es->w, es->scal, es->lu, es->Y);
+  k_invit<<<(k + INV_WARP - 1) / INV_WARP, INV_WARP, 0, s>>>(n, k0, k, es->d, es->e, es->w, es->scal, es->lu, es->Y);
   prof_kend(KS_INVIT, ti, s);
   ++g_kernel_launches;
   k_clusters<<<k, 256, 0, s>>>(n, k0, k1, es->d, es->e, es->w, es->scal, 1e-5, es->Y);
@@ -1239,7 +1350,7 @@ __global__ void __launch_bounds__(128) kb_eigvals(BARGS, int rest) {
   else if (!rest && j < n) q.emo[j] = TRI_SENTINEL;
 }
 
-__global__ void kb_invit(BARGS) {
+__global__ void __launch_bounds__(INV_WARP) kb_invit(BARGS) {
   BMOL;
   invit_dev(q.m.nao, 0, *q.icount, q.ed, q.ee, q.emo, q.escal, q.lu, q.Y);
 }
@@ -1306,9 +1417,8 @@ void eigen_vectors_b(const BatchLaunch& b) {
   batch_attributes();
   g_kernel_launches += 3;
   const int ti = prof_kbegin(b.s);
-  // one thread per vector; full warps (the one-molecule path keeps 16-thread blocks so that a
-  // single molecule's vectors spread over more SMs)
-  kb_invit<<<dim3((b.nao_max + 31) / 32, 1, b.count), 32, 0, b.s>>>(b.mp, b.list);
+  kb_invit<<<dim3((b.nao_max + INV_WARP - 1) / INV_WARP, 1, b.count), INV_WARP, 0, b.s>>>(b.mp,
+                                                                                          b.list);
   prof_kend(KS_INVIT, ti, b.s);
   kb_clusters<<<dim3(b.nao_max, 1, b.count), 256, 0, b.s>>>(b.mp, b.list);
   const int tb_ = prof_kbegin(b.s);
