@@ -502,10 +502,86 @@ __device__ TriBounds tri_bounds(int n, const double* __restrict__ d,
   return out;
 }
 
-// eigenvalue j of T; warp-collective (every lane of the warp calls it, inactive lanes too)
+// The FP64 stage with 16 lanes per eigenvalue: every round counts at 16 ascending points and keeps
+// the neighbouring pair that encloses the eigenvalue.  Round one takes both ends of the widened
+// bracket and rungs of a ladder (factor 4) around the FP32 result; a bracket that misses falls back
+// to the Gershgorin interval.  While the bracket of width W holds only this eigenvalue the points
+// are a ladder (factor 8, W/4 down to half a tolerance) around the secant point, so the bracket
+// shrinks to about the secant's error at every round; else, and within 8 tolerances (where the
+// rungs round to the same few numbers), they are equidistant.  Four or five
+// counts one after the other instead of nine (192 orbitals: see k_eigvals), same stopping rule.
+__device__ double tri_ladder(int n, const double* __restrict__ d, const double* __restrict__ e2,
+                             float flo, float fhi, int j, bool active, const TriBounds& b) {
+  const int sub = threadIdx.x & 15, lead = (threadIdx.x & 31) - sub;
+  const double wid = b.tnorm * 0x1p-16;
+  double lo = fmax(b.lo, (double)flo - wid), hi = fmin(b.hi, (double)fhi + wid);
+  double flm = 0.0, fhm = 0.0;
+  int fle = 0, fhe = 0, clo = 0, chi = n;
+  for (int it = 0; it < 80; ++it) {
+    const double W = hi - lo;
+    const double tol = 2.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + 4.0 * b.pivmin;
+    const double mid = 0.5 * (lo + hi);
+    const bool done = !active || W <= tol || !(mid > lo && mid < hi);
+    if (it > 0 && __all_sync(0xffffffffu, done)) break;
+    const bool iso = it > 0 && clo == j && chi == j + 1 && W > 8.0 * tol;
+    double x;
+    const int m = sub < 8 ? sub : 15 - sub;  // rung: 0 the outermost
+    if (it == 0 || iso) {
+      double c = 0.5 * ((double)flo + (double)fhi);
+      if (iso) {
+        const int E = max(fle, fhe);
+        const double a = scalbn(flm, fle - E), q = scalbn(fhm, fhe - E);
+        c = lo + a / (a - q) * W;
+      }
+      const double step = it == 0 ? scalbn(W, -1 - 2 * m) : fmax(scalbn(W, -2 - 3 * m), 0.5 * tol);
+      x = fmin(fmax(sub < 8 ? c - step : c + step, lo), hi);
+      if (it == 0) x = sub == 0 ? lo : sub == 15 ? hi : x;
+    } else {
+      x = lo + W * ((sub + 1) * (1.0 / 17.0));
+    }
+    double fm;
+    int fe;
+    const int c = sweep64(n, d, e2, x, fm, fe);
+    const unsigned above = (__ballot_sync(0xffffffffu, c > j) >> lead) & 0xFFFFu;
+    const int f = above ? __ffs(above) - 1 : 16;  // first point above the eigenvalue
+    const int il = lead + max(f - 1, 0), ih = lead + min(f, 15);
+    const double xl = __shfl_sync(0xffffffffu, x, il), xh = __shfl_sync(0xffffffffu, x, ih);
+    const double ml = __shfl_sync(0xffffffffu, fm, il), mh = __shfl_sync(0xffffffffu, fm, ih);
+    const int el = __shfl_sync(0xffffffffu, fe, il), eh = __shfl_sync(0xffffffffu, fe, ih);
+    const int cl = __shfl_sync(0xffffffffu, c, il), ch = __shfl_sync(0xffffffffu, c, ih);
+    if (it == 0 && (f == 0 || f == 16)) {  // the FP32 stage missed: full interval
+      lo = b.lo;
+      hi = b.hi;
+      continue;
+    }
+    if (done && it > 0) continue;
+    if (f > 0) {
+      lo = xl;
+      clo = cl;
+      flm = ml;
+      fle = el;
+    }
+    if (f < 16) {
+      hi = xh;
+      chi = ch;
+      fhm = mh;
+      fhe = eh;
+    }
+  }
+  return 0.5 * (lo + hi);
+}
+
+// eigenvalue j of T; warp-collective (every lane of the warp calls it, inactive lanes too).  A group
+// of 2^D neighbouring lanes shares one eigenvalue: in the FP32 stage its lanes evaluate the 2^D - 1
+// midpoints of the next D bisection levels at once (the same midpoints as level by level, so the
+// bracket is the same bit for bit; 2^D - 1 counts instead of D, in the time of one), and the FP64
+// check takes both ends at once.  Every lane of the group returns the eigenvalue.
+template <int D>
 __device__ double tri_eigenvalue(int n, const double* __restrict__ d, const double* __restrict__ e2,
                                  const float* __restrict__ fd, const float* __restrict__ fe2,
                                  int j, bool active, const TriBounds& b) {
+  constexpr int G = 1 << D;
+  const int sub = threadIdx.x & (G - 1), lead = (threadIdx.x & 31) - sub;
   // 1. FP32 bisection
   float flo = __double2float_rd(b.lo), fhi = __double2float_ru(b.hi);
   const float ftol = (float)(b.tnorm * 0x1p-21);
@@ -513,9 +589,36 @@ __device__ double tri_eigenvalue(int n, const double* __restrict__ d, const doub
     const float x = 0.5f * (flo + fhi);
     const bool done = !active || fhi - flo <= ftol || x <= flo || x >= fhi;
     if (__all_sync(0xffffffffu, done)) break;
-    if (done) continue;
-    if (sweep32(n, fd, fe2, x) > j) fhi = x;
-    else flo = x;
+    if constexpr (D == 0) {
+      if (done) continue;
+      if (sweep32(n, fd, fe2, x) > j) fhi = x;
+      else flo = x;
+    } else {
+      // lane sub evaluates node sub of the heap (1 the root, 2 q below and 2 q + 1 above node q)
+      float lo = flo, hi = fhi;
+      const int node = sub ? sub : 1;
+      for (int l = 30 - __clz(node); l >= 0; --l) {
+        const float m = 0.5f * (lo + hi);
+        if ((node >> l) & 1) lo = m;
+        else hi = m;
+      }
+      const int above = sweep32(n, fd, fe2, 0.5f * (lo + hi)) > j;
+      int q = 1;
+#pragma unroll
+      for (int l = 0; l < D; ++l) {
+        const float m = 0.5f * (flo + fhi);
+        const bool stop = !active || fhi - flo <= ftol || m <= flo || m >= fhi;
+        const int c = __shfl_sync(0xffffffffu, above, lead + (q & (G - 1)));
+        if (!stop) {
+          if (c) fhi = m;
+          else flo = m;
+          q = 2 * q + (c ? 0 : 1);
+        }
+      }
+    }
+  }
+  if constexpr (D == 4) {
+    if (n <= TRIDIAG_FIXED_MAX) return tri_ladder(n, d, e2, flo, fhi, j, active, b);
   }
   // 2. widened bracket, checked in FP64
   const double wid = b.tnorm * 0x1p-16;
@@ -523,9 +626,23 @@ __device__ double tri_eigenvalue(int n, const double* __restrict__ d, const doub
   double flm = 0.0, fhm = 0.0;
   int fle = 0, fhe = 0, clo = 0, chi = n;
   bool kl = false, kh = false;
+  if constexpr (D == 0) {
+    if (active) {
+      clo = sweep64(n, d, e2, lo, flm, fle);
+      chi = sweep64(n, d, e2, hi, fhm, fhe);
+    }
+  } else {  // even lanes the lower end, odd lanes the upper end
+    double fm;
+    int fe;
+    const int c = sweep64(n, d, e2, (sub & 1) ? hi : lo, fm, fe);
+    clo = __shfl_sync(0xffffffffu, c, lead);
+    chi = __shfl_sync(0xffffffffu, c, lead + 1);
+    flm = __shfl_sync(0xffffffffu, fm, lead);
+    fhm = __shfl_sync(0xffffffffu, fm, lead + 1);
+    fle = __shfl_sync(0xffffffffu, fe, lead);
+    fhe = __shfl_sync(0xffffffffu, fe, lead + 1);
+  }
   if (active) {
-    clo = sweep64(n, d, e2, lo, flm, fle);
-    chi = sweep64(n, d, e2, hi, fhm, fhe);
     kl = kh = true;
     if (clo > j || chi <= j) {  // the FP32 stage missed: full interval
       lo = b.lo;
@@ -624,22 +741,29 @@ __global__ void k_tri_prep(int n, const double* __restrict__ d, const double* __
     }
   }
 }
-// one-molecule path: eigenvalues j0 <= j < j1; with fill, w[j1 .. n) = TRI_SENTINEL
+// one-molecule path: eigenvalues j0 <= j < j1; with fill, w[j1 .. n) = TRI_SENTINEL.  One warp per
+// block (the warps of a single molecule spread over as many SMs as possible), 16 lanes per
+// eigenvalue: 2 warps per SM at 600 eigenvalues, so the extra FP32 counts cost no time
+constexpr int EIG_D = 4;
 __global__ void __launch_bounds__(32) k_eigvals(int n, int j0, int j1, int fill,
                                                  const double* __restrict__ d,
                                                  const double* __restrict__ ws,
                                                  const double* __restrict__ scal, double* w) {
-  const int j = j0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if ((int)(blockIdx.x * blockDim.x) + j0 >= n) return;  // whole warp beyond n
+  const int j = j0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> EIG_D);
   const float* fd = reinterpret_cast<const float*>(ws + n);
   const float* fe2 = fd + n;
+  if (j0 + (int)((blockIdx.x * blockDim.x) >> EIG_D) >= j1) {  // a warp of unwanted eigenvalues
+    if (fill && (threadIdx.x & ((1 << EIG_D) - 1)) == 0 && j < n) w[j] = TRI_SENTINEL;
+    return;
+  }
   TriBounds b;
   b.tnorm = scal[1];
   b.lo = scal[2];
   b.hi = scal[3];
   b.pivmin = scal[4];
   const bool active = j < j1;
-  const double v = tri_eigenvalue(n, d, ws, fd, fe2, j, active, b);
+  const double v = tri_eigenvalue<EIG_D>(n, d, ws, fd, fe2, j, active, b);
+  if ((threadIdx.x & ((1 << EIG_D) - 1)) != 0) return;
   if (active) w[j] = v;
   else if (fill && j < n) w[j] = TRI_SENTINEL;
 }
@@ -1225,8 +1349,7 @@ int eigen_values(EigenSolver* es, const double* F, double* w_out, int nev) {
   g_kernel_launches += 2;
   const int tm = prof_kbegin(s);
   k_tri_prep<<<(n + 255) / 256, 256, 0, s>>>(n, es->d, es->e, es->tw, es->scal);
-  // one warp per block: the warps of a single molecule spread over as many SMs as possible
-  k_eigvals<<<(n + 31) / 32, 32, 0, s>>>(n, 0, nev, 1, es->d, es->tw, es->scal, es->w);
+  k_eigvals<<<((n << EIG_D) + 31) / 32, 32, 0, s>>>(n, 0, nev, 1, es->d, es->tw, es->scal, es->w);
   prof_kend(KS_MULTISECT, tm, s);
   ck(cudaMemcpyAsync(w_out, es->w, sizeof(double) * n, cudaMemcpyDeviceToDevice, s), "w");
   return 0;
@@ -1239,7 +1362,7 @@ void eigen_values_rest(EigenSolver* es, int nev, double* w_out) {
   g_kernel_launches += 2;
   const int tm = prof_kbegin(s);
   k_tri_prep<<<(n + 255) / 256, 256, 0, s>>>(n, es->d, es->e, es->tw, es->scal);
-  k_eigvals<<<(n - nev + 31) / 32, 32, 0, s>>>(n, nev, n, 0, es->d, es->tw, es->scal, es->w);
+  k_eigvals<<<(((n - nev) << EIG_D) + 31) / 32, 32, 0, s>>>(n, nev, n, 0, es->d, es->tw, es->scal, es->w);
   prof_kend(KS_MULTISECT, tm, s);
   ck(cudaMemcpyAsync(w_out + nev, es->w + nev, sizeof(double) * (n - nev), cudaMemcpyDeviceToDevice, s),
      "w");
@@ -1324,14 +1447,22 @@ bool eigen_gemm_failed(EigenSolver* es) {
 // (every thread reads the same element at the same step).  rest = 0: eigenvalues j < nev and
 // the sentinel above them; rest = 1 (after the SCF): the eigenvalues nev <= j < n.
 constexpr int BIS_MAXN = 1024;
-// one warp per block: the Sturm counts are FP64-bound (a division per element), so spreading a
-// molecule's eigenvalues over more SMs shortens the kernel; each block stages d and e^2 again
+// one warp per block, so that a molecule's eigenvalues spread over the SMs; each block stages d
+// and e^2 again.  2^D lanes per eigenvalue (tri_eigenvalue)
 constexpr int EIG_BLOCK = 32;
-__global__ void __launch_bounds__(128) kb_eigvals(BARGS, int rest) {
+template <int D>
+__global__ void __launch_bounds__(EIG_BLOCK) kb_eigvals(BARGS, int rest) {
   BMOL;
   const int n = q.m.nao;
   const int j0 = rest ? q.nev : 0, j1 = rest ? n : q.nev;
-  if ((int)blockIdx.x * (int)blockDim.x + j0 >= n) return;
+  const int jw = j0 + (int)((blockIdx.x * EIG_BLOCK) >> D);  // the warp's first eigenvalue
+  const int j = j0 + (int)((blockIdx.x * EIG_BLOCK + threadIdx.x) >> D);
+  const bool head = (threadIdx.x & ((1 << D) - 1)) == 0;
+  if (jw >= n) return;
+  if (jw >= j1) {
+    if (!rest && head && j < n) q.emo[j] = TRI_SENTINEL;
+    return;
+  }
   __shared__ double sd[BIS_MAXN], se2[BIS_MAXN];
   __shared__ float fd[BIS_MAXN], fe2[BIS_MAXN];
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -1343,11 +1474,22 @@ __global__ void __launch_bounds__(128) kb_eigvals(BARGS, int rest) {
   }
   const TriBounds b = tri_bounds(n, q.ed, q.ee);  // ends with a block barrier
   if (blockIdx.x == 0 && threadIdx.x == 0 && !rest) q.escal[1] = b.tnorm;
-  const int j = j0 + blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = j < j1;
-  const double v = tri_eigenvalue(n, sd, se2, fd, fe2, j, active, b);
+  const double v = tri_eigenvalue<D>(n, sd, se2, fd, fe2, j, active, b);
+  if (!head) return;
   if (active) q.emo[j] = v;
   else if (!rest && j < n) q.emo[j] = TRI_SENTINEL;
+}
+// lanes per eigenvalue: 16, 4 or 1, as many as keep a launch at about eight warps per SM (the FP32
+// counts of a group are 15 for 4 levels, 3 for 2: time is saved only while issue slots are free)
+static void eigvals_launch(const BatchLaunch& b, int rest) {
+  const long long warps = (long long)b.nao_max * b.count, limit = 8LL * 32 * device_sm_count();
+  const int D = warps * 16 <= limit ? 4 : warps * 4 <= limit ? 2 : 0;
+  const dim3 grid((unsigned)(((b.nao_max << D) + EIG_BLOCK - 1) / EIG_BLOCK), 1, b.count);
+  ++g_kernel_launches;
+  if (D == 4) kb_eigvals<4><<<grid, EIG_BLOCK, 0, b.s>>>(b.mp, b.list, rest);
+  else if (D == 2) kb_eigvals<2><<<grid, EIG_BLOCK, 0, b.s>>>(b.mp, b.list, rest);
+  else kb_eigvals<0><<<grid, EIG_BLOCK, 0, b.s>>>(b.mp, b.list, rest);
 }
 
 __global__ void __launch_bounds__(INV_WARP) kb_invit(BARGS) {
@@ -1397,19 +1539,15 @@ void eigen_values_b(const BatchLaunch& b) {
   gemm_b(b, GS_FX);
   gemm_b(b, GS_XTT);
   tridiag_fixed_b(b);
-  ++g_kernel_launches;
   const int tm = prof_kbegin(b.s);
   if (b.nao_max > BIS_MAXN) throw std::runtime_error("batched eigenvalues: molecule too large");
-  kb_eigvals<<<dim3((b.nao_max + EIG_BLOCK - 1) / EIG_BLOCK, 1, b.count), EIG_BLOCK, 0, b.s>>>(
-      b.mp, b.list, 0);
+  eigvals_launch(b, 0);
   prof_kend(KS_MULTISECT, tm, b.s);
 }
 
 void eigen_values_rest_b(const BatchLaunch& b) {
   if (!b.count) return;
-  ++g_kernel_launches;
-  kb_eigvals<<<dim3((b.nao_max + EIG_BLOCK - 1) / EIG_BLOCK, 1, b.count), EIG_BLOCK, 0, b.s>>>(
-      b.mp, b.list, 1);
+  eigvals_launch(b, 1);
 }
 
 void eigen_vectors_b(const BatchLaunch& b) {
