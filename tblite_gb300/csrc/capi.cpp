@@ -924,6 +924,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   b.omega = w.b_omega.p;
   b.work = w.b_work.p;
   b.status = w.b_status.p;
+  b.ordered = n > TRIDIAG_FIXED_MAX;
 
   const double econv = 1.0e-6 * c->accuracy, pconv = 2.0e-5 * c->accuracy;
   const double target_kt = c->etemp;

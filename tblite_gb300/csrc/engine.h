@@ -234,6 +234,7 @@ struct BroydenState {
   double *q, *qlast, *dq, *dqlast, *df, *u, *a, *omega;  // device
   double* work;   // device scratch [memory*memory + 2*memory + 64]
   int* status;    // device status word (0 ok, !=0 singular)
+  bool ordered = false;  // keep the order of summation of a large molecule (tridiag_fixed)
 };
 void launch_broyden_next(BroydenState& b, cudaStream_t s);
 // with_mp: the mixer vector holds the atomic multipoles too (GFN2); GFN1 mixes shell charges
@@ -254,7 +255,10 @@ int eigen_capacity(const EigenSolver*);
 void eigen_resize(EigenSolver*, int n);
 // fixed-point tridiagonalisation (tridiag.cu) of the symmetric column-major A (n x n, n up to
 // TRIDIAG_FIXED_MAX): d, e, tau and the reflectors below the subdiagonal of A, as dsytrd('L'); xch
-// holds tridiag_exchange_words(n) words
+// holds tridiag_exchange_words(n) words.  Larger molecules keep the FP64 reduction, and with it the
+// order of every sum of their SCF: a long chain's dipole (0.06 a.u. over 200 carbons) turns a change
+// of 1e-16 anywhere in the iteration into 1e-9 of itself, so results comparable to the last digits
+// need the same roundings there
 constexpr int TRIDIAG_FIXED_MAX = 512;
 void tridiag_fixed(int n, double* A, double* d, double* e, double* tau, long long* xch,
                    cudaStream_t s);

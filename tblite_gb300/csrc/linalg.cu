@@ -27,14 +27,19 @@ namespace tb {
 // computed, the others (and the lower half of a diagonal tile) are written twice (C(i,j) and
 // C(j,i)), so C is exactly symmetric.
 // ------------------------------------------------------------------------------------------
+// Four warps per tile, one per scheduler: an FP64 instruction takes its scheduler 64-76 cycles, so
+// two warps (the earlier form) left half of the SM's FP64 rate unused.  The next k tile is loaded
+// into registers while the current one is multiplied (two shared-memory buffers, one barrier per
+// k tile); every output keeps its sum over k in order.
 template <int BM, int BN, int BK, int TM, int TN>
 __device__ __forceinline__ void gemm_dev(int M, int N, int K, double alpha, const double* __restrict__ A, int lda, bool ta,
            const double* __restrict__ B, int ldb, bool tb, double beta, double* __restrict__ C,
            int ldc, int kmode) {
   constexpr int NT = (BM / TM) * (BN / TN);
-  __shared__ double As[BK][BM + 1];
-  __shared__ double Bs[BK][BN + 1];
-  static_assert(!(BM != BN), "square tiles");
+  constexpr int LA = BM * BK / NT, LB = BK * BN / NT;  // elements a thread loads per k tile
+  __shared__ double As[2][BK][BM + 1];
+  __shared__ double Bs[2][BK][BN + 1];
+  static_assert(BM == BN && NT == 128, "square tiles, four warps");
   const int i0 = blockIdx.y * BM, j0 = blockIdx.x * BN;
   const bool sym = (kmode & KM_SYM) != 0;
   if (sym && i0 < j0) return;  // above the diagonal: written by the mirror tile
@@ -50,34 +55,58 @@ __device__ __forceinline__ void gemm_dev(int M, int N, int K, double alpha, cons
   for (int a = 0; a < TM; ++a)
 #pragma unroll
     for (int b = 0; b < TN; ++b) acc[a][b] = 0.0;
-  for (int k0 = kbeg; k0 < kend; k0 += BK) {
-    for (int t = tid; t < BM * BK; t += NT) {
+  double ra[LA], rb[LB];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < LA; ++q) {
+      const int t = tid + q * NT;
       const int ii = ta ? t / BK : t % BM, kk = ta ? t % BK : t / BM;
       const int gi = i0 + ii, gk = k0 + kk;
-      double v = 0.0;
-      if (gi < M && gk < kend) v = ta ? A[gk + (size_t)gi * lda] : A[gi + (size_t)gk * lda];
-      As[kk][ii] = v;
+      ra[q] = 0.0;
+      if (gi < M && gk < kend) ra[q] = ta ? A[gk + (size_t)gi * lda] : A[gi + (size_t)gk * lda];
     }
-    for (int t = tid; t < BK * BN; t += NT) {
+#pragma unroll
+    for (int q = 0; q < LB; ++q) {
+      const int t = tid + q * NT;
       const int kk = tb ? t / BN : t % BK, jj = tb ? t % BN : t / BK;
       const int gk = k0 + kk, gj = j0 + jj;
-      double v = 0.0;
-      if (gj < N && gk < kend) v = tb ? B[gj + (size_t)gk * ldb] : B[gk + (size_t)gj * ldb];
-      Bs[kk][jj] = v;
+      rb[q] = 0.0;
+      if (gj < N && gk < kend) rb[q] = tb ? B[gj + (size_t)gk * ldb] : B[gk + (size_t)gj * ldb];
     }
-    __syncthreads();
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int q = 0; q < LA; ++q) {
+      const int t = tid + q * NT;
+      As[buf][ta ? t % BK : t / BM][ta ? t / BK : t % BM] = ra[q];
+    }
+#pragma unroll
+    for (int q = 0; q < LB; ++q) {
+      const int t = tid + q * NT;
+      Bs[buf][tb ? t / BN : t % BK][tb ? t % BN : t / BK] = rb[q];
+    }
+  };
+  if (kbeg < kend) {
+    load(kbeg);
+    store(0);
+  }
+  __syncthreads();
+  for (int k0 = kbeg, buf = 0; k0 < kend; k0 += BK, buf ^= 1) {
+    const bool more = k0 + BK < kend;
+    if (more) load(k0 + BK);
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       double a[TM], b[TN];
 #pragma unroll
-      for (int x = 0; x < TM; ++x) a[x] = As[kk][tr * TM + x];
+      for (int x = 0; x < TM; ++x) a[x] = As[buf][kk][tr * TM + x];
 #pragma unroll
-      for (int y = 0; y < TN; ++y) b[y] = Bs[kk][tc * TN + y];
+      for (int y = 0; y < TN; ++y) b[y] = Bs[buf][kk][tc * TN + y];
 #pragma unroll
       for (int x = 0; x < TM; ++x)
 #pragma unroll
         for (int y = 0; y < TN; ++y) acc[x][y] = fma(a[x], b[y], acc[x][y]);
     }
+    if (more) store(buf ^ 1);
     __syncthreads();
   }
 #pragma unroll
@@ -131,11 +160,11 @@ cudaError_t gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const do
   if ((long long)((M + 31) / 32) * ((N + 31) / 32) < 2LL * device_sm_count()) {
     dim3 grid((N + 15) / 16, (M + 15) / 16);
     ++g_kernel_launches;
-    e = cudaLaunchKernel((const void*)k_gemm<16, 16, 16, 2, 2>, grid, dim3(64), args, 0, s);
+    e = cudaLaunchKernel((const void*)k_gemm<16, 16, 16, 2, 1>, grid, dim3(128), args, 0, s);
   } else {
     dim3 grid((N + 31) / 32, (M + 31) / 32);
     ++g_kernel_launches;
-    e = cudaLaunchKernel((const void*)k_gemm<32, 32, 16, 4, 4>, grid, dim3(64), args, 0, s);
+    e = cudaLaunchKernel((const void*)k_gemm<32, 32, 16, 4, 2>, grid, dim3(128), args, 0, s);
   }
   prof_kend(KS_GEMM, tk, s);
   return e;
@@ -361,10 +390,10 @@ void gemm_b(const BatchLaunch& b, int site) {
   ++g_kernel_launches;
   if (b.nao_max <= 128) {
     const unsigned t = (b.nao_max + 15) / 16;
-    kb_gemm<16, 16, 16, 2, 2><<<dim3(t, t, b.count), 64, 0, b.s>>>(b.mp, b.list, site);
+    kb_gemm<16, 16, 16, 2, 1><<<dim3(t, t, b.count), 128, 0, b.s>>>(b.mp, b.list, site);
   } else {
     const unsigned t = (b.nao_max + 31) / 32;
-    kb_gemm<32, 32, 16, 4, 4><<<dim3(t, t, b.count), 64, 0, b.s>>>(b.mp, b.list, site);
+    kb_gemm<32, 32, 16, 4, 2><<<dim3(t, t, b.count), 128, 0, b.s>>>(b.mp, b.list, site);
   }
   prof_kend(KS_GEMM, tk, b.s);
 }

@@ -17,6 +17,8 @@
 // instead of being stored: one warp per atom walks all partners.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "engine.h"
 
 namespace tb {
@@ -702,9 +704,12 @@ void launch_fock(int n, const int* ao_at, const double* H, const double* S, cons
 // Mulliken: column sums over row chunks.  partial[chunk][11][n]:
 //   0: sum_r P S, 1-3: sum_r P D_k, 4-9: sum_r P Q_q, 10: sum_r P H
 // ------------------------------------------------------------------------------------
-constexpr int MULL_ROWS = 64;
+// rows per chunk: 11 FP64 multiply-adds per row and column, so short chunks spread a molecule
+// over more SMs (68 orbitals: 64 rows 80 us, see the table of kernels for 16)
+// (above 512 orbitals the one-molecule path keeps its order of summation, see tridiag_fixed)
+__host__ __device__ constexpr int mull_rows(int n) { return n <= 512 ? 16 : 64; }
 
-int mulliken_chunks(int n) { return (n + MULL_ROWS - 1) / MULL_ROWS; }
+int mulliken_chunks(int n) { return (n + mull_rows(n) - 1) / mull_rows(n); }
 
 __device__ __forceinline__ void mull_partial_dev(int n, const double* __restrict__ P,
                                                       const double* __restrict__ S,
@@ -719,7 +724,7 @@ __device__ __forceinline__ void mull_partial_dev(int n, const double* __restrict
   double acc[11];
 #pragma unroll
   for (int k = 0; k < 11; ++k) acc[k] = 0.0;
-  const int r0 = chunk * MULL_ROWS, r1 = min(n, r0 + MULL_ROWS);
+  const int r0 = chunk * mull_rows(n), r1 = min(n, r0 + mull_rows(n));
   for (int r = r0; r < r1; ++r) {
     const size_t rc = (size_t)r * n + c;
     const double pv = P[rc];
@@ -742,34 +747,35 @@ __global__ void __launch_bounds__(128) k_mull_partial(int n, const double* __res
   mull_partial_dev(n, P, S, H, D, Q, partial);
 }
 
-// one thread per atom: reduce chunks for its orbitals, fill shells/atoms
+// 16 threads per atom, one per sum (population, 3 dipole, 6 quadrupole, band energy): reduce the
+// chunks of its orbitals, fill shells/atoms
+constexpr int MULL_LANES = 16;
 __device__ __forceinline__ void mull_reduce_dev(DevMol m, const double* __restrict__ partial, int nchunk,
                               double* qsh, double* qat, double* dpat, double* qpat,
                               double* eband) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m.nat) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = t / MULL_LANES, k = t % MULL_LANES;
+  if (i >= m.nat || k >= 11) return;
   const int n = m.nao;
-  double d[3] = {0, 0, 0}, q[6] = {0, 0, 0, 0, 0, 0}, e = 0.0, qa = 0.0;
+  const double* __restrict__ pk = partial + (size_t)k * n;
+  double sum = 0.0, qa = 0.0;
   for (int s = m.at_sh[i]; s < m.at_sh[i + 1]; ++s) {
-    double ps = 0.0;
     const int o = m.sh_ao[s], no = 2 * m.sh_l[s] + 1;
+    if (k == 0) sum = 0.0;
     for (int mu = o; mu < o + no; ++mu) {
-      for (int ch = 0; ch < nchunk; ++ch) {
-        const double* pp = partial + (size_t)ch * 11 * n;
-        ps += pp[mu];
-        for (int k = 0; k < 3; ++k) d[k] += pp[(1 + k) * (size_t)n + mu];
-        for (int k = 0; k < 6; ++k) q[k] += pp[(4 + k) * (size_t)n + mu];
-        e += pp[10 * (size_t)n + mu];
-      }
+#pragma unroll 4
+      for (int ch = 0; ch < nchunk; ++ch) sum += pk[(size_t)ch * 11 * n + mu];
     }
-    const double v = m.sh_refocc[s] - ps;
-    qsh[s] = v;
-    qa += v;
+    if (k == 0) {
+      const double v = m.sh_refocc[s] - sum;
+      qsh[s] = v;
+      qa += v;
+    }
   }
-  qat[i] = qa;
-  for (int k = 0; k < 3; ++k) dpat[3 * i + k] = -d[k];
-  for (int k = 0; k < 6; ++k) qpat[6 * i + k] = -q[k];
-  eband[i] = e;
+  if (k == 0) qat[i] = qa;
+  else if (k < 4) dpat[3 * i + k - 1] = -sum;
+  else if (k < 10) qpat[6 * i + k - 4] = -sum;
+  else eband[i] = sum;
 }
 __global__ void k_mull_reduce(DevMol m, const double* __restrict__ partial, int nchunk,
                               double* qsh, double* qat, double* dpat, double* qpat,
@@ -786,9 +792,14 @@ void launch_mulliken(const DevMol& m, const double* P, const double* S, const do
   k_mull_partial<<<dim3((n + 127) / 128, nchunk), 128, 0, s>>>(n, P, S, H, D, Q, partial);
   prof_kend(KS_MULLIKEN, tk, s);
   ++g_kernel_launches;
-  k_mull_reduce<<<(m.nat + 127) / 128, 128, 0, s>>>(m, partial, nchunk, qsh, qat, dpat, qpat,
-                                                    eband);
+  k_mull_reduce<<<(m.nat * MULL_LANES + 127) / 128, 128, 0, s>>>(m, partial, nchunk, qsh, qat, dpat,
+                                                                 qpat, eband);
 }
+
+// threads of a one-block kernel over n elements: no more warps than elements need, since every
+// warp of a block sum takes its scheduler the same five FP64 additions (the sums are the same bit
+// for bit as with 1024 threads, the missing warps would add zeros)
+static int one_block(int n) { return n >= 1024 ? 1024 : n <= 32 ? 32 : (n + 31) / 32 * 32; }
 
 // ------------------------------------------------------------------------------------
 // Fermi filling (one block).  Both spin channels share the eigenvalues.
@@ -852,7 +863,7 @@ __device__ double fermi_channel(int n, const double* emo, double nel, double kt,
   double s = 0.0;
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
     const double o = occ[k];
-    s += log(pow(o, o) * pow(1.0 - o, 1.0 - o));
+    if (o != 0.0 && o != 1.0) s += log(pow(o, o) * pow(1.0 - o, 1.0 - o));  // else log(1) = 0
   }
   s = block_sum(s, red);
   if (threadIdx.x == 0) *ts += s * kt;
@@ -869,7 +880,13 @@ __device__ __forceinline__ void fermi_dev(int n, const double* emo, double nalp,
   if (threadIdx.x == 0) *ts = 0.0;
   __syncthreads();
   const double efa = fermi_channel(n, emo, nalp, kt, fa, red, ts);
-  const double efb = fermi_channel(n, emo, nbet, kt, fb, red, ts);
+  double efb = efa;
+  if (nalp == nbet) {  // closed shell: the same filling twice
+    for (int k = threadIdx.x; k < n; k += blockDim.x) fb[k] = fa[k];
+    if (threadIdx.x == 0) *ts += *ts;
+  } else {
+    efb = fermi_channel(n, emo, nbet, kt, fb, red, ts);
+  }
   if (threadIdx.x == 0)
     ncols[1] = (nev < n && !(emo[nev - 1] >= fmax(efa, efb) + 51.0 * kt)) ? 1 : 0;
   int last = -1;
@@ -895,7 +912,7 @@ void launch_fermi(int n, const double* emo, double nalp, double nbet, double kt,
                   double* ts, int* ncols, cudaStream_t s, int nev) {
   // fa, fb scratch follow focc in memory: focc[n], fa[n], fb[n]
   ++g_kernel_launches;
-  k_fermi<<<1, 1024, 0, s>>>(n, emo, nalp, nbet, kt, focc + n, focc + 2 * n, focc, ts, ncols,
+  k_fermi<<<1, one_block(n), 0, s>>>(n, emo, nalp, nbet, kt, focc + n, focc + 2 * n, focc, ts, ncols,
                              nev > 0 ? nev : n);
 }
 
@@ -967,13 +984,14 @@ __global__ void k_diff(int nd, const double* vout, const double* q, double* dq, 
 void launch_diff(int nd, const double* vout, const double* q, double* dq, double* err,
                  cudaStream_t s) {
   ++g_kernel_launches;
-  k_diff<<<1, 1024, 0, s>>>(nd, vout, q, dq, err);
+  k_diff<<<1, one_block(nd), 0, s>>>(nd, vout, q, dq, err);
 }
 
 // ------------------------------------------------------------------------------------
 // Broyden step (one block).  Same recurrences as the reference; the overlap matrix a(i,j)
 // is kept between calls and only the row of the newest history vector is recomputed
-// (the other rows are unchanged dot products).
+// (the other rows are unchanged dot products).  ordered: dot products and back substitution keep
+// the order of summation of a block sum and of a row by row solution.
 // ------------------------------------------------------------------------------------
 __device__ double block_dot(int nd, const double* x, const double* y, double* red) {
   double s = 0.0;
@@ -983,7 +1001,7 @@ __device__ double block_dot(int nd, const double* x, const double* y, double* re
 
 __device__ __forceinline__ void broyden_dev(int nd, int memory, int iter, double alpha, double* q, double* qlast,
                           const double* dq, double* dqlast, double* df, double* u, double* a,
-                          double* omega, double* work, int* status) {
+                          double* omega, double* work, int* status, bool ordered) {
   __shared__ double red[32];
   if (iter == 1) {
     for (int t = threadIdx.x; t < nd; t += blockDim.x) {
@@ -1011,80 +1029,95 @@ __device__ __forceinline__ void broyden_dev(int nd, int memory, int iter, double
   inv = 1.0 / inv;
   for (int t = threadIdx.x; t < nd; t += blockDim.x) dfn[t] *= inv;
   __syncthreads();
-  // history indices, c vector, a row
-  double* beta = work;                      // [nhist][nhist]
-  double* cvec = work + memory * memory;    // [nhist]
-  for (int ih = 0; ih < nhist; ++ih) {
-    const int i = (first + ih - 1) % memory;
-    const double dfi_dq = block_dot(nd, df + (size_t)i * nd, dq, red);
-    const double aij = block_dot(nd, df + (size_t)i * nd, dfn, red);
-    if (threadIdx.x == 0) {
-      cvec[ih] = omega[i] * dfi_dq;
-      a[(size_t)i * memory + it1] = aij;
-      a[(size_t)it1 * memory + i] = aij;
+  // history indices, c vector, a row: one warp per dot product (a block sum would take every warp
+  // five FP64 additions per product)
+  constexpr int NS = 48;  // histories up to this order are solved in shared memory
+  __shared__ double sbeta[NS * NS], sfac[NS], sc[NS];
+  double* beta = nhist <= NS ? sbeta : work;                  // [nhist][nhist]
+  double* cvec = nhist <= NS ? sc : work + memory * memory;   // [nhist]
+  double* fac = nhist <= NS ? sfac : cvec + memory;           // [nhist]
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (ordered) {
+    for (int ih = 0; ih < nhist; ++ih) {
+      const int i = (first + ih - 1) % memory;
+      const double dfi_dq = block_dot(nd, df + (size_t)i * nd, dq, red);
+      const double aij = block_dot(nd, df + (size_t)i * nd, dfn, red);
+      if (threadIdx.x == 0) {
+        cvec[ih] = omega[i] * dfi_dq;
+        a[(size_t)i * memory + it1] = aij;
+        a[(size_t)it1 * memory + i] = aij;
+      }
+    }
+  }
+  for (int t = wid; !ordered && t < 2 * nhist; t += nw) {
+    const int ih = t >> 1, i = (first + ih - 1) % memory;
+    const double *x = df + (size_t)i * nd, *y = (t & 1) ? dfn : dq;
+    double s0 = 0.0, s1 = 0.0;
+    int k = lane;
+    for (; k + 32 < nd; k += 64) {
+      s0 = fma(x[k], y[k], s0);
+      s1 = fma(x[k + 32], y[k + 32], s1);
+    }
+    if (k < nd) s0 = fma(x[k], y[k], s0);
+    s0 = warp_sum(s0 + s1);
+    if (lane == 0) {
+      if (t & 1) {
+        a[(size_t)i * memory + it1] = s0;
+        a[(size_t)it1 * memory + i] = s0;
+      } else {
+        cvec[ih] = omega[i] * s0;
+      }
     }
   }
   __syncthreads();
+  // solve beta^T x = c by Gaussian elimination with partial pivoting (getrf + getrs 't'); warp 0
+  // finds and swaps the pivot row and forms the multipliers, all threads apply them
   for (int t = threadIdx.x; t < nhist * nhist; t += blockDim.x) {
-    const int ih = t / nhist, jh = t % nhist;
+    const int jh = t / nhist, ih = t % nhist;  // transposed
     const int i = (first + ih - 1) % memory, j = (first + jh - 1) % memory;
     beta[t] = omega[i] * omega[j] * a[(size_t)i * memory + j] + (ih == jh ? omega0 * omega0 : 0.0);
   }
-  __syncthreads();
-  // solve beta^T x = c by Gaussian elimination with partial pivoting (getrf + getrs 't')
-  __shared__ int piv;
   __shared__ int fail;
   if (threadIdx.x == 0) fail = 0;
   __syncthreads();
-  // transpose in place to solve beta^T
-  for (int t = threadIdx.x; t < nhist * nhist; t += blockDim.x) {
-    const int i = t / nhist, j = t % nhist;
-    if (i < j) {
-      const double x = beta[i * nhist + j];
-      beta[i * nhist + j] = beta[j * nhist + i];
-      beta[j * nhist + i] = x;
-    }
-  }
-  __syncthreads();
   for (int k = 0; k < nhist; ++k) {
-    if (threadIdx.x == 0) {
-      int p = k;
-      double best = fabs(beta[k * nhist + k]);
-      for (int i = k + 1; i < nhist; ++i) {
-        const double v = fabs(beta[i * nhist + k]);
-        if (v > best) {
-          best = v;
-          p = i;
+    if (wid == 0) {
+      unsigned long long best = 0ull;  // |value| as bits, then the first row that has it
+      for (int i = k + lane; i < nhist; i += 32)
+        best = max(best, (unsigned long long)__double_as_longlong(fabs(beta[i * nhist + k])));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+      int p = nhist;
+      for (int i = k + lane; i < nhist; i += 32)
+        if ((unsigned long long)__double_as_longlong(fabs(beta[i * nhist + k])) == best) p = min(p, i);
+      p = __reduce_min_sync(0xffffffffu, p);
+      if (best == 0ull) {
+        if (lane == 0) fail = k + 1;
+      } else {
+        if (p != k) {
+          for (int j = lane; j < nhist; j += 32) {
+            const double x = beta[k * nhist + j];
+            beta[k * nhist + j] = beta[p * nhist + j];
+            beta[p * nhist + j] = x;
+          }
+          if (lane == 0) {
+            const double x = cvec[k];
+            cvec[k] = cvec[p];
+            cvec[p] = x;
+          }
+          __syncwarp();
         }
+        const double pivv = beta[k * nhist + k];
+        for (int i = k + 1 + lane; i < nhist; i += 32) fac[i] = beta[i * nhist + k] / pivv;
       }
-      piv = p;
-      if (best == 0.0) fail = k + 1;
     }
     __syncthreads();
     if (fail) break;
-    const int p = piv;
-    if (p != k) {
-      for (int j = threadIdx.x; j < nhist; j += blockDim.x) {
-        const double x = beta[k * nhist + j];
-        beta[k * nhist + j] = beta[p * nhist + j];
-        beta[p * nhist + j] = x;
-      }
-      if (threadIdx.x == 0) {
-        const double x = cvec[k];
-        cvec[k] = cvec[p];
-        cvec[p] = x;
-      }
-    }
-    __syncthreads();
-    const double pivv = beta[k * nhist + k];
-    for (int t = threadIdx.x; t < (nhist - k - 1) * (nhist - k); t += blockDim.x) {
-      const int i = k + 1 + t / (nhist - k), j = k + t % (nhist - k);
-      const double f = beta[i * nhist + k] / pivv;
-      if (j > k) beta[i * nhist + j] -= f * beta[k * nhist + j];
-    }
-    __syncthreads();
-    for (int i = k + 1 + threadIdx.x; i < nhist; i += blockDim.x) {
-      cvec[i] -= beta[i * nhist + k] / pivv * cvec[k];
+    const int rem = nhist - k - 1;
+    for (int t = threadIdx.x; t < rem * (rem + 1); t += blockDim.x) {
+      const int i = k + 1 + t / (rem + 1), j = k + 1 + t % (rem + 1);
+      if (j < nhist) beta[i * nhist + j] = fma(-fac[i], beta[k * nhist + j], beta[i * nhist + j]);
+      else cvec[i] = fma(-fac[i], cvec[k], cvec[i]);
     }
     __syncthreads();
   }
@@ -1092,13 +1125,28 @@ __device__ __forceinline__ void broyden_dev(int nd, int memory, int iter, double
     if (threadIdx.x == 0) *status = fail;
     return;
   }
-  if (threadIdx.x == 0) {
-    for (int i = nhist - 1; i >= 0; --i) {
-      double s = cvec[i];
-      for (int j = i + 1; j < nhist; ++j) s -= beta[i * nhist + j] * cvec[j];
-      cvec[i] = s / beta[i * nhist + i];
+  // back substitution by columns: the diagonal's reciprocals first, then one solved element at a
+  // time leaves all the rows above it (ordered: row by row, one thread)
+  for (int i = threadIdx.x; i < nhist; i += blockDim.x) fac[i] = 1.0 / beta[i * nhist + i];
+  __syncthreads();
+  if (wid == 0) {
+    if (ordered && lane == 0)
+      for (int i = nhist - 1; i >= 0; --i) {
+        double x = cvec[i];
+        for (int j = i + 1; j < nhist; ++j) x -= beta[i * nhist + j] * cvec[j];
+        cvec[i] = x / beta[i * nhist + i];
+      }
+    __syncwarp();
+    for (int i = nhist - 1; !ordered && i >= 0; --i) {
+      const double x = cvec[i] * fac[i];
+      for (int l = lane; l < i; l += 32) cvec[l] = fma(-beta[l * nhist + i], x, cvec[l]);
+      __syncwarp();
+      if (lane == 0) cvec[i] = x;
     }
-    *status = 0;
+    for (int ih = lane; ih < nhist; ih += 32) fac[ih] = omega[(first + ih - 1) % memory];
+    __syncwarp();
+    for (int ih = lane; ih < nhist; ih += 32) fac[ih] *= cvec[ih];
+    if (lane == 0) *status = 0;
   }
   __syncthreads();
   double* un = u + (size_t)it1 * nd;
@@ -1106,22 +1154,19 @@ __device__ __forceinline__ void broyden_dev(int nd, int memory, int iter, double
     un[t] = alpha * dfn[t] + inv * (q[t] - qlast[t]);
     dqlast[t] = dq[t];
     qlast[t] = q[t];
-    q[t] = q[t] + alpha * dq[t];
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < nd; t += blockDim.x) {
-    double v = q[t];
-    for (int ih = 0; ih < nhist; ++ih) {
-      const int i = (first + ih - 1) % memory;
-      v -= omega[i] * cvec[ih] * u[(size_t)i * nd + t];
-    }
+    double v = q[t] + alpha * dq[t];
+    // (each thread reads its own element of the new history vector)
+#pragma unroll 4
+    for (int ih = 0; ih < nhist; ++ih)
+      v = fma(-fac[ih], u[(size_t)((first + ih - 1) % memory) * nd + t], v);
     q[t] = v;
   }
 }
 __global__ void k_broyden(int nd, int memory, int iter, double alpha, double* q, double* qlast,
                           const double* dq, double* dqlast, double* df, double* u, double* a,
-                          double* omega, double* work, int* status) {
-  broyden_dev(nd, memory, iter, alpha, q, qlast, dq, dqlast, df, u, a, omega, work, status);
+                          double* omega, double* work, int* status, bool ordered) {
+  broyden_dev(nd, memory, iter, alpha, q, qlast, dq, dqlast, df, u, a, omega, work, status,
+              ordered);
 }
 
 __device__ __forceinline__ void eelec_init_dev(int nat, const double* ts, const double* eband, double* eelec) {
@@ -1154,8 +1199,8 @@ void launch_fe(int n, const double* f, const double* e, double* out, cudaStream_
 void launch_broyden_next(BroydenState& b, cudaStream_t s) {
   b.iter += 1;
   ++g_kernel_launches;
-  k_broyden<<<1, 1024, 0, s>>>(b.ndim, b.memory, b.iter, b.damp, b.q, b.qlast, b.dq, b.dqlast,
-                               b.df, b.u, b.a, b.omega, b.work, b.status);
+  k_broyden<<<1, std::max(256, one_block(b.ndim)), 0, s>>>(b.ndim, b.memory, b.iter, b.damp, b.q, b.qlast, b.dq, b.dqlast,
+                               b.df, b.u, b.a, b.omega, b.work, b.status, b.ordered);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1401,10 +1446,12 @@ __global__ void kb_mull_reduce(BARGS) {
 void launch_mulliken_b(const BatchLaunch& b) {
   if (!b.count) return;
   ++g_kernel_launches;
-  kb_mull_partial<<<bgrid((b.nao_max + 127) / 128, b, mulliken_chunks(b.nao_max)), 128, 0,
+  // (the molecules of up to 512 orbitals in a wider bucket have the shorter chunks)
+  const int chunks = std::max(mulliken_chunks(b.nao_max), mulliken_chunks(std::min(b.nao_max, 512)));
+  kb_mull_partial<<<bgrid((b.nao_max + 127) / 128, b, chunks), 128, 0,
                     b.s>>>(b.mp, b.list);
   ++g_kernel_launches;
-  kb_mull_reduce<<<bgrid((b.nat_max + 127) / 128, b), 128, 0, b.s>>>(b.mp, b.list);
+  kb_mull_reduce<<<bgrid((b.nat_max * MULL_LANES + 127) / 128, b), 128, 0, b.s>>>(b.mp, b.list);
 }
 
 __global__ void kb_fermi(BARGS) {
@@ -1418,7 +1465,7 @@ __global__ void kb_fermi(BARGS) {
 void launch_fermi_b(const BatchLaunch& b) {
   if (!b.count) return;
   ++g_kernel_launches;
-  kb_fermi<<<bgrid(1, b), 1024, 0, b.s>>>(b.mp, b.list);
+  kb_fermi<<<bgrid(1, b), one_block(b.nao_max), 0, b.s>>>(b.mp, b.list);
 }
 
 __global__ void kb_pack(BARGS, int output) {
@@ -1453,18 +1500,18 @@ __global__ void kb_diff(BARGS) {
 void launch_diff_b(const BatchLaunch& b) {
   if (!b.count) return;
   ++g_kernel_launches;
-  kb_diff<<<bgrid(1, b), 1024, 0, b.s>>>(b.mp, b.list);
+  kb_diff<<<bgrid(1, b), one_block(b.nd_max), 0, b.s>>>(b.mp, b.list);
 }
 
 __global__ void kb_broyden(BARGS, int iter) {
   BMOL;
   broyden_dev(q.nd, q.memory, iter, q.damp, q.bq, q.bqlast, q.bdq, q.bdqlast, q.bdf, q.bu, q.ba,
-              q.bomega, q.bwork, q.bstatus);
+              q.bomega, q.bwork, q.bstatus, false);
 }
 void launch_broyden_b(const BatchLaunch& b, int iter) {
   if (!b.count) return;
   ++g_kernel_launches;
-  kb_broyden<<<bgrid(1, b), 1024, 0, b.s>>>(b.mp, b.list, iter);
+  kb_broyden<<<bgrid(1, b), std::max(256, one_block(b.nd_max)), 0, b.s>>>(b.mp, b.list, iter);
 }
 
 __global__ void kb_eelec_init(BARGS) {
