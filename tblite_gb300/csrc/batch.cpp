@@ -291,15 +291,15 @@ void layout(Plan& pl, Region* R) {
   }
   if (pl.wbo_ch > 0) pl.wbo = piece<double>(R, RR, (size_t)pl.wbo_ch * na * na);
   if (pl.sp2) {
-    pl.img = piece<uint16_t>(R, RS, pimage_bytes((int)n, (int)n) / sizeof(uint16_t));
+    pl.img = piece<uint16_t>(R, RS, pimage_bytes((int)n, (int)n, true) / sizeof(uint16_t));
     pl.iexp = piece<int>(R, RS, pimage_lines((int)n));
-    pl.img2 = piece<uint16_t>(R, RS, pimage_bytes((int)n, (int)n) / sizeof(uint16_t));
+    pl.img2 = piece<uint16_t>(R, RS, pimage_bytes((int)n, (int)n, true) / sizeof(uint16_t));
     pl.iexp2 = piece<int>(R, RS, pimage_lines((int)n));
     pl.sp2s = piece<double>(R, RS, 8);
     pl.sp2i = piece<int>(R, RZ, 8);  // zeroed: the pipeline status starts clear
     pl.sp2p = piece<unsigned long long>(R, RS, 3 * (size_t)sp2_slot_count((int)n));
-    pl.ximg0 = piece<uint16_t>(R, RS, pimage_bytes((int)n, (int)n) / sizeof(uint16_t));
-    pl.ximg1 = piece<uint16_t>(R, RS, pimage_bytes((int)n, (int)n) / sizeof(uint16_t));
+    pl.ximg0 = piece<uint16_t>(R, RS, pimage_bytes((int)n, (int)n, true) / sizeof(uint16_t));
+    pl.ximg1 = piece<uint16_t>(R, RS, pimage_bytes((int)n, (int)n, true) / sizeof(uint16_t));
     pl.xexp0 = piece<int>(R, RS, pimage_lines((int)n));
     pl.xexp1 = piece<int>(R, RS, pimage_lines((int)n));
   }

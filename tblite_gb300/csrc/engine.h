@@ -282,14 +282,15 @@ void eigen_vectors(EigenSolver*, int k, double* C);
 void eigen_vectors_range(EigenSolver*, int k0, int k1, double* C);
 
 // pipelined split GEMM (ozaki_pipe.cu): a matrix is split once into a slice image (per line a
-// power-of-two exponent and eight BF16 slices in the tensor cores' shared-memory layout), then
-// C = op(A) op(B) runs from two images
+// power-of-two exponent and seven or eight BF16 slices in the tensor cores' shared-memory layout),
+// then C = op(A) op(B) runs from two images
 struct PImage {
   int lines = 0, K = 0;
-  uint16_t* data = nullptr;  // pimage_bytes(lines, K) bytes
+  bool balanced = false;     // splitting: balanced digits, or 7-bit digits of the magnitude
+  uint16_t* data = nullptr;  // pimage_bytes(lines, K, balanced) bytes
   int* e = nullptr;          // pimage_lines(lines) ints
 };
-size_t pimage_bytes(int lines, int K);
+size_t pimage_bytes(int lines, int K, bool balanced);
 int pimage_lines(int lines);
 // line i, position k: M[i + k ld] (kcontig 0) or M[k + i ld] (kcontig 1)
 void psplit(const double* M, int ld, int kcontig, int lines, int K, PImage& img, cudaStream_t s);

@@ -1,25 +1,40 @@
 // Pipelined FP64-accurate split GEMM on the BF16 tensor cores for the one-molecule path.
 //
-// Same splitting as ozaki.cu: eight 7-bit slices per FP64 value, x = 2^e sum_p a_p 2^-7p, stored
-// pre-scaled in BF16, and the 36 exact slice products a_p b_q with p + q <= 7 (zero based).  The
-// operands are split once per matrix instead of once per tile pair, and the products are grouped
-// so that each tensor-core instruction is wide:
+// Two splittings (struct Balanced, struct Magnitude).  Balanced: x = 2^e sum_p d_p 2^(-7 - 8p),
+// p = 0..6, with digits d_p in [-128, 128]: seven slices in BF16, and the 28 slice products d_p d_q
+// with p + q <= 6 (zero based).  Magnitude, the splitting of ozaki.cu: eight 7-bit digits of |x| with
+// x's sign, 36 products with p + q <= 7.  Balanced radix-256 digits have the same magnitude bound
+// (products <= 2^14, so as many of them sum exactly in FP32) and hold one bit more each, and what
+// is rounded or dropped has no sign bias: 28 products instead of 36 and a smaller error (A A^T of
+// 3072: 8.5e-16 against 1.2e-15).  The batch and tblite_gb300_split_gemm use Balanced.  The
+// one-molecule projection (purify.cu) keeps Magnitude and with it its results: its bias loses
+// 2e-10 electrons of 4000 (500 waters), which the dipole of a cluster far from the origin shows at
+// 5e-10, so the splittings' results differ visibly there although both are within the solver's
+// tolerance.  The operands are split once per matrix instead of once per tile pair, and the
+// products are grouped so that each tensor-core instruction is wide (figures of Balanced;
+// Magnitude in brackets where they differ):
 //
 //   psplit   turns a matrix into a slice image: per line (row of op(A) or column of op(B)) a
-//            power-of-two exponent, and the eight BF16 slices laid out exactly as the tensor
+//            power-of-two exponent, and the BF16 slices laid out exactly as the tensor
 //            cores read them from shared memory, K-major lines of 64 bytes with the 64-byte
 //            swizzle: image[k chunk of 32][slice][line block of 64][64 x 64 bytes];
 //   pgemm    (kernel k_opipe) one 128 x 64 output tile per CTA, 10 warps.  Warp 0 streams the
-//            slices of each k chunk (96 KB: A 64 KB, B 32 KB) with cp.async.bulk into a
+//            slices of each k chunk (84 KB: A 56 KB, B 28 KB) with cp.async.bulk into a
 //            two-stage shared-memory ring (mbarrier complete_tx).  Warp 1 issues the MMAs: the B
-//            slices of a stage lie one after another, so a_p times [b_q0 .. b_q0+3] is a single
+//            slices of a stage lie one after another, so d_p times [d_q0 .. d_q0+3] is a single
 //            M 128 x N 256 x K 16 tcgen05.mma whose four 64-column blocks land in the TMEM
 //            accumulators of the levels p + q0 .. p + q0 + 3 (one accumulator of 64 columns per
-//            level 0..7, 512 columns); 13 MMAs per k step instead of 36.  Warps 2..9 drain the
-//            levels 0..5 every 5 chunks (160 values of k): they hold exact integers (at most 6
-//            products of < 2^14 each per k: < 2^24) that go into one int64 per element.  The
-//            levels 6..7 (< 2^-42 of the leading level) stay in FP32 over the whole of k (their
-//            rounding is < 2^-56 of the result) and are read with the output at the end.
+//            level 0..6); 10 [13] MMAs per k step.  Warps 2..9 drain the levels 0..4 [0..5] every
+//            6 [5] chunks (192 [160] values of k): they hold exact integers (at most 5 [6]
+//            products of <= 2^14 each per k: < 2^24) that go into one int64 per element.  The
+//            levels 5..6 [6..7] (weight 2^-40 [2^-42] of the
+//            leading level and a random sum of balanced digits) stay in FP32 over the whole of k
+//            (their rounding is below 2^-53 of the largest possible element) and are read with
+//            the output at the end.
+//
+// Bound by the tensor pipe (896 [1152] cycles per k step of 16) and, at the end of every window, by the
+// conversion of the drained sums (8 cycles per warp and conversion): the drain's loads are issued
+// one level ahead, level 0 (below 2^22) is converted by an FP32 addition instead.
 //
 // Every wait is bounded; a wait that runs out sets a CTA-wide abort flag, the other roles leave
 // their loops, copies and MMAs still in flight are waited for (bounded), TMEM is freed and the
@@ -40,17 +55,36 @@ namespace tb {
 
 namespace {
 
-constexpr int PP_M = 128, PP_N = 64, PP_KC = 32, PP_FLUSH = 5, PP_THREADS = 320;
-constexpr int PP_LEVELS = 8;    // TMEM accumulators, one per level p + q = 0..7
-constexpr int PP_EXACT = 6;     // levels 0..5 are drained as exact integers
-constexpr int PP_KMAX = 12288;  // |int64 level sums| < 1.02 * 2^49 K < 2^63
+constexpr int PP_M = 128, PP_N = 64, PP_KC = 32, PP_THREADS = 320;
+struct Balanced {
+  static constexpr int SLICES = 7;  // BF16 slices of an operand
+  static constexpr int LEVELS = 7;  // TMEM accumulators, one per level p + q
+  static constexpr int EXACT = 5;   // levels 0 .. EXACT - 1 are drained as exact integers
+  static constexpr int FLUSH = 6;   // k chunks per window
+  static constexpr int BITS = 8;    // of a digit
+  // the MMAs of a k step from slice 1 on, four bits each, the first one lowest: A slice p, first B
+  // slice q, number of B slices
+  static constexpr int GROUPS = 8;
+  static constexpr uint64_t GP = 0x65432211, GQ = 0x00004040, GN = 0x12341424;
+};
+struct Magnitude {
+  static constexpr int SLICES = 8, LEVELS = 8, EXACT = 6, FLUSH = 5, BITS = 7, GROUPS = 10;
+  static constexpr uint64_t GP = 0x7654332211, GQ = 0x0000404040, GN = 0x1234142434;
+};
+// |int64 level sums| < 1.01 * 2^46 K (Balanced), 1.02 * 2^49 K (Magnitude): below 2^63
+constexpr int PP_KMAX = 12288;
 constexpr int PP_STAGES = 2;    // the producer's bookkeeping below assumes two
-constexpr int PP_A_BYTES = 8 * 8192;  // 8 slices x 128 lines x 64 B
-constexpr int PP_B_BYTES = 8 * 4096;  // 8 slices x 64 lines x 64 B
-constexpr int PP_STAGE_BYTES = PP_A_BYTES + PP_B_BYTES;
-constexpr int PP_SMEM = PP_STAGES * PP_STAGE_BYTES + 1024;
+template <class Sch>
+constexpr int PP_A_BYTES = Sch::SLICES * 8192;  // slices x 128 lines x 64 B
+template <class Sch>
+constexpr int PP_B_BYTES = Sch::SLICES * 4096;  // slices x 64 lines x 64 B
+template <class Sch>
+constexpr int PP_STAGE_BYTES = PP_A_BYTES<Sch> + PP_B_BYTES<Sch>;
+template <class Sch>
+constexpr int PP_SMEM = PP_STAGES * PP_STAGE_BYTES<Sch> + 1024;
 constexpr int PP_TMEM_COLS = 512;
-static_assert(PP_LEVELS * PP_N == PP_TMEM_COLS, "one 64-column accumulator per level");
+static_assert(Magnitude::LEVELS * PP_N <= PP_TMEM_COLS && Balanced::LEVELS * PP_N <= PP_TMEM_COLS,
+              "one 64-column accumulator per level");
 constexpr int PP_GROUP = 8;  // row blocks per tile group
 constexpr int PP_WAIT = 1 << 22;
 // polls of a pipeline wait (stage full / empty, accumulators ready / free) before it gives up
@@ -96,16 +130,41 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
   return false;
 }
 
-// 16 consecutive TMEM columns of this thread's lane (one row of the tile) into v
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+// 32 consecutive TMEM columns of this thread's lane (one row of the tile) into v; tmem_wait before
+// v is used
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&v)[32]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-      "%14,%15}, [%16];"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
         "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15])
+        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
+        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
+        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(addr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// waits for this thread's TMEM loads; the loaded registers pass through, so that no use of them
+// moves above it
+__device__ __forceinline__ void tmem_wait(uint32_t (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]),
+                 "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]),
+                 "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]),
+                 "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
+                 "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27])
+               :
+               : "memory");
+  asm volatile("" : "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])::"memory");
+}
+
+// x 2^(55 - e), rounded: |x| < 2^e gives at most 2^55; zero and subnormals give zero
+__device__ __forceinline__ long long fixed55(uint64_t bits, int e) {
+  const int ex = (int)((bits >> 52) & 0x7FF);
+  if (ex == 0) return 0ll;
+  const uint64_t m = (bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+  const int sh = ex - e - 1020;
+  const uint64_t w = sh >= 0 ? m << sh : (sh > -64 ? ((m >> (-sh - 1)) + 1) >> 1 : 0ull);
+  return (bits >> 63) ? -(long long)w : (long long)w;
 }
 
 // |x| 2^(56 - e) as an integer (< 2^56 for |x| < 2^e): zero and subnormals give zero
@@ -129,6 +188,52 @@ __device__ __forceinline__ uint32_t bf16x2_sub(uint32_t a, uint32_t b) {
   return r.u;
 }
 
+// the balanced digits of two fixed-point values |W| <= 2^55 + 2^46 as packed BF16 pairs, w[p] =
+// (digit p of W0, digit p of W1).  Adding 128 to every digit turns the digits into the bytes of one
+// integer; a byte b gives the BF16 number 128 + (b & 127) by its mantissa field, and subtracting
+// 128 (b >= 128) or 256 (b < 128) leaves the digit b - 128, both elements in one BF16x2 subtraction
+// (exact: at most 8 significant bits).  The top digit + 128 may be 256: its lane then holds -128
+// and the sign is cleared.
+__device__ __forceinline__ void digits_pair(long long W0, long long W1,
+                                            uint32_t (&w)[Balanced::SLICES]) {
+  constexpr long long BIAS = 0x0080808080808080ll;
+  const unsigned long long V0 = (unsigned long long)(W0 + BIAS), V1 = (unsigned long long)(W1 + BIAS);
+  const uint32_t l0 = (uint32_t)V0, h0 = (uint32_t)(V0 >> 32), l1 = (uint32_t)V1,
+                 h1 = (uint32_t)(V1 >> 32);
+  // 16-bit lanes whose low byte is digit p of each element (the top digit: all 16 bits)
+  const uint32_t R[Balanced::SLICES] = {__byte_perm(h0, h1, 0x7632), __byte_perm(h0, h1, 0x5511),
+                                 __byte_perm(h0, h1, 0x4400), __byte_perm(l0, l1, 0x7733),
+                                 __byte_perm(l0, l1, 0x6622), __byte_perm(l0, l1, 0x5511),
+                                 __byte_perm(l0, l1, 0x4400)};
+#pragma unroll
+  for (int p = 0; p < Balanced::SLICES; ++p)
+    w[p] = bf16x2_sub((R[p] & 0x007F007Fu) | 0x43004300u, (R[p] & 0x00800080u) ^ 0x43804380u);
+  w[0] ^= (R[0] & 0x01000100u) << 7;
+}
+// the slices of two values x0, x1 (bits) of a line of exponent e: w[p] = (slice p of x0, of x1)
+template <class Sch>
+__device__ __forceinline__ void split_pair(uint64_t x0, uint64_t x1, int e,
+                                           uint32_t (&w)[Sch::SLICES]) {
+  if constexpr (Sch::SLICES == Balanced::SLICES) {
+    digits_pair(fixed55(x0, e), fixed55(x1, e), w);
+  } else {
+    // digit p of |x| 2^(56 - e) is the 7-bit field at 49 - 7p, read from the 28-bit half that
+    // holds it; 128 + digit by the mantissa field, minus 128, and the sign (a zero digit of a
+    // negative element becomes -0, which adds nothing to a product)
+    const uint32_t signs = (uint32_t)(x0 >> 63) << 15 | (uint32_t)(x1 >> 63) << 31;
+    const uint64_t Y0 = fixed_bits(x0, e), Y1 = fixed_bits(x1, e);
+    const uint32_t h0 = (uint32_t)(Y0 >> 28), l0 = (uint32_t)Y0 & 0xFFFFFFFu;
+    const uint32_t h1 = (uint32_t)(Y1 >> 28), l1 = (uint32_t)Y1 & 0xFFFFFFFu;
+    const uint32_t R[4] = {__byte_perm(h0 >> 14, h1 >> 14, 0x5410), __byte_perm(h0, h1, 0x5410),
+                           __byte_perm(l0 >> 14, l1 >> 14, 0x5410), __byte_perm(l0, l1, 0x5410)};
+#pragma unroll
+    for (int p = 0; p < Sch::SLICES; ++p) {
+      const uint32_t mag = ((R[p >> 1] >> ((p & 1) ? 0 : 7)) & 0x007F007Fu) | 0x43004300u;
+      w[p] = bf16x2_sub(mag, 0x43004300u) | signs;
+    }
+  }
+}
+
 // |x| as bits: for non-negative doubles the unsigned order of the bit patterns is the numeric
 // order, so line maxima are integer maxima (no FP64 instruction, which this GPU issues at 1/64
 // of the FP32 rate); e = ilogb(max) + 1 is the biased exponent field minus 1022 for a normal
@@ -142,26 +247,33 @@ __device__ __forceinline__ int exp_of_max(unsigned long long mb) {
 }
 
 // ---- exponents: e = ilogb(max |x|) + 1 of every line ------------------------------------------
-// lines contiguous in memory (element (i, k) at M[i + k ld]): 32 lines per block, the 8 warps
-// take every 8th k (coalesced 256-byte rows), then a shared-memory reduction
+// lines contiguous in memory (element (i, k) at M[i + k ld]): L lines per block, the T / L groups
+// of threads take every (T / L)-th k (128-byte rows for L = 16), then a shared-memory reduction
+template <int L, int T>
 __device__ __forceinline__ void pexp_rows_dev(const double* __restrict__ M, int ld, int lines,
                                               int K, int Lp, int* e, int blk) {
-  __shared__ unsigned long long part[8][33];
-  const int li = threadIdx.x & 31, kg = threadIdx.x >> 5;
-  const int i = blk * 32 + li;
+  constexpr int G = T / L;
+  __shared__ unsigned long long part[G][L + 1];
+  const int li = threadIdx.x % L, kg = threadIdx.x / L;
+  const int i = blk * L + li;
   unsigned long long mx = 0ull;
-  if (i < lines)
-    for (int k = kg; k < K; k += 8) mx = max(mx, abs_bits(M[i + (size_t)k * ld]));
+  if (i < lines) {
+#pragma unroll 4
+    for (int k = kg; k < K; k += G) mx = max(mx, abs_bits(M[i + (size_t)k * ld]));
+  }
   part[kg][li] = mx;
   __syncthreads();
   if (kg == 0 && i < Lp) {
-    for (int g = 1; g < 8; ++g) mx = max(mx, part[g][li]);
+#pragma unroll 8
+    for (int g = 1; g < G; ++g) mx = max(mx, part[g][li]);
     e[i] = exp_of_max(mx);
   }
 }
-__global__ void __launch_bounds__(256) k_pexp_rows(const double* __restrict__ M, int ld,
+// one matrix: 16 lines and 1024 threads per block keep enough loads in flight (3072 x 3072 with
+// 32 lines and 256 threads took 57 us)
+__global__ void __launch_bounds__(1024) k_pexp_rows(const double* __restrict__ M, int ld,
                                                    int lines, int K, int Lp, int* e) {
-  pexp_rows_dev(M, ld, lines, K, Lp, e, blockIdx.x);
+  pexp_rows_dev<16, 1024>(M, ld, lines, K, Lp, e, blockIdx.x);
 }
 // k contiguous (element (i, k) at M[k + i ld]): one warp per line
 __global__ void k_pexp_cols(const double* __restrict__ M, int ld, int lines, int K, int Lp,
@@ -178,6 +290,7 @@ __global__ void k_pexp_cols(const double* __restrict__ M, int ld, int lines, int
 
 // ---- slice image: one block per (64 lines, 32 k); the FP64 tile goes through shared memory so
 // both memory orders read coalesced; each thread splits 8 consecutive k of one line
+template <class Sch>
 __device__ __forceinline__ void psplit_dev(const double* __restrict__ M, int ld, int kcontig,
                                            int lines, int K, int nlb, const int* __restrict__ e,
                                            uint16_t* img, int lb, int kc) {
@@ -203,41 +316,28 @@ __device__ __forceinline__ void psplit_dev(const double* __restrict__ M, int ld,
   const int li = t & 63, g = t >> 6;  // k group of 8: 0..3
   const int i = l0 + li;
   const int ei = e[i];
-  uint32_t w[8][4];
+  uint32_t w[Sch::SLICES][4];
 #pragma unroll
-  for (int c = 0; c < 8; c += 2) {  // two neighbouring k per step, as in kb_sp2_slice
-    uint32_t hh[2], ll[2], signs = 0u;
+  for (int c = 0; c < 8; c += 2) {  // two neighbouring k per step
+    uint32_t g2[Sch::SLICES];
+    split_pair<Sch>((uint64_t)__double_as_longlong(tile[li][8 * g + c]),
+                    (uint64_t)__double_as_longlong(tile[li][8 * g + c + 1]), ei, g2);
 #pragma unroll
-    for (int d = 0; d < 2; ++d) {
-      const uint64_t bits = (uint64_t)__double_as_longlong(tile[li][8 * g + c + d]);
-      signs |= (uint32_t)(bits >> 63) << (15 + 16 * d);
-      const uint64_t Y = fixed_bits(bits, ei);  // |x| 2^(56 - e) < 2^56; zero and subnormals: 0
-      hh[d] = (uint32_t)(Y >> 28);
-      ll[d] = (uint32_t)Y & 0xFFFFFFFu;
-    }
-    const uint32_t R[4] = {__byte_perm(hh[0] >> 14, hh[1] >> 14, 0x5410),
-                           __byte_perm(hh[0], hh[1], 0x5410),
-                           __byte_perm(ll[0] >> 14, ll[1] >> 14, 0x5410),
-                           __byte_perm(ll[0], ll[1], 0x5410)};
-#pragma unroll
-    for (int p = 0; p < 8; ++p) {
-      const uint32_t bias = ((uint32_t)(134 - 7 * p) << 7) * 0x10001u;
-      const uint32_t mag = ((R[p >> 1] >> ((p & 1) ? 0 : 7)) & 0x007F007Fu) | bias;
-      w[p][c >> 1] = bf16x2_sub(mag, bias) | signs;
-    }
+    for (int p = 0; p < Sch::SLICES; ++p) w[p][c >> 1] = g2[p];
   }
   // [k chunk][slice][line block][64 lines x 64 B, 16-byte chunks swizzled]
 #pragma unroll
-  for (int p = 0; p < 8; ++p) {
-    const size_t off = (((size_t)kc * 8 + p) * nlb + lb) * 2048 + li * 32 +
+  for (int p = 0; p < Sch::SLICES; ++p) {
+    const size_t off = (((size_t)kc * Sch::SLICES + p) * nlb + lb) * 2048 + li * 32 +
                        ((g ^ ((li >> 1) & 3)) << 3);
     *reinterpret_cast<uint4*>(img + off) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
   }
 }
+template <class Sch>
 __global__ void __launch_bounds__(256) k_psplit(const double* __restrict__ M, int ld, int kcontig,
                                                 int lines, int K, int nlb,
                                                 const int* __restrict__ e, uint16_t* img) {
-  psplit_dev(M, ld, kcontig, lines, K, nlb, e, img, blockIdx.x, blockIdx.y);
+  psplit_dev<Sch>(M, ld, kcontig, lines, K, nlb, e, img, blockIdx.x, blockIdx.y);
 }
 
 struct PipeArgs {
@@ -260,42 +360,53 @@ struct PipeArgs {
 };
 
 // line exponent of every projection iterate: the spectrum of D stays in [0, 1], so every element
-// has |x| <= 1 < 2^SP2_E and the slices hold x to an absolute 2^-55 (an FP64 iterate's own
-// rounding is 2^-53 relative to its O(1) diagonal); an element at or above 2^SP2_E stops the
-// molecule.  During the projection the iterate lives in Y as signed 64-bit integers W = x 2^55
-// (SP2_FRAC fractional bits): |W| < 2^56, and the magnitude's two 28-bit halves are the slices'
-// source directly.
-constexpr int SP2_E = 1;
-constexpr int SP2_FRAC = 56 - SP2_E;
+// has |x| <= 1 = 2^SP2_E (up to rounding) and the slices hold x to an absolute 2^-55 (an FP64
+// iterate's own rounding is 2^-53 relative to its O(1) diagonal); an element at or above
+// SP2_LIMIT stops the molecule.  During the projection the iterate lives in Y as signed 64-bit
+// integers W = x 2^55 (SP2_FRAC fractional bits), which are the digits' source directly.
+constexpr int SP2_E = 0;
+constexpr int SP2_FRAC = 55 - SP2_E;
+constexpr long long SP2_LIMIT = (1ll << 55) + (1ll << 46);           // the top digit reaches 128
 constexpr long long SP2_BAD = (long long)0x8000000000000000ull;  // an element out of range
 
 __device__ __forceinline__ int slice_off(int line, int k, int nlb) {
   // image[k chunk][slice][line block][64 lines x 32 k], 16-byte groups swizzled (slice 0)
   const int li = line & 63, g = (k >> 3) & 3;
-  return (((k >> 5) * 8) * nlb + (line >> 6)) * 2048 + li * 32 + ((g ^ ((li >> 1) & 3)) << 3) +
+  return (((k >> 5) * Balanced::SLICES) * nlb + (line >> 6)) * 2048 + li * 32 + ((g ^ ((li >> 1) & 3)) << 3) +
          (k & 7);
 }
 
 
-// C element (i, j) of a finished tile from the exact levels T, the FP32 levels v6 + v7 and the
-// scale 2^sc: C = (T + F 2^35) 2^(sc - 35), F = levels 6 + 7 summed in FP32 (F < 2^-42 of the
-// result, so its rounding is below 2^-66); the power of two goes into the exponent field by an
-// integer add where the result stays normal: three FP64 operations per element (two conversions
-// and an add) instead of six
-__device__ __forceinline__ double tile_value(long long T, uint32_t v6, uint32_t v7, int sc) {
-  const float ff = (__uint_as_float(v6) + __uint_as_float(v7)) * 0x1p35f;
-  const double sum = (double)T + (double)ff;
+// C element (i, j) of a finished tile from the exact levels T (units of the last one, E), the two
+// FP32 levels va and vb and the scale 2^sc: C = (T + F) 2^(sc - BITS E), F = va 2^-BITS + vb
+// 2^(-2 BITS); the power of two goes into the exponent field by an integer add where the result
+// stays normal: three FP64 operations per element (two conversions and an add)
+template <class Sch>
+__device__ __forceinline__ float low_levels(uint32_t va, uint32_t vb) {
+  constexpr float f = 1.0f / (1 << Sch::BITS);
+  return fmaf(__uint_as_float(vb), f, __uint_as_float(va)) * f;
+}
+template <class Sch>
+__device__ __forceinline__ double tile_value(long long T, uint32_t va, uint32_t vb, int sc) {
+  constexpr int U = Sch::BITS * (Sch::EXACT - 1);
+  const double sum = (double)T + (double)low_levels<Sch>(va, vb);
   const long long sb = __double_as_longlong(sum);
   const int se = (int)((sb >> 52) & 0x7FF);
   if (sum == 0.0) return 0.0;
-  if (se > 0 && se + (sc - 35) > 0 && se + (sc - 35) < 2047)
-    return __longlong_as_double(sb + ((long long)(sc - 35) << 52));
-  return ldexp(sum, sc - 35);  // subnormal or out-of-range result: the general path
+  if (se > 0 && se + (sc - U) > 0 && se + (sc - U) < 2047)
+    return __longlong_as_double(sb + ((long long)(sc - U) << 52));
+  return ldexp(sum, sc - U);  // subnormal or out-of-range result: the general path
+}
+// T + iv 2^sh for a level's integer sum
+__device__ __forceinline__ long long add_level(long long T, int iv, int mul) {
+  long long r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(iv), "r"(mul), "l"(T));
+  return r;
 }
 
 // one 128 x 64 output tile (number b in the grouped order) of the product a (FIXED: the
 // projection's fixed-point epilogue, a.fixed set)
-template <bool FIXED = false>
+template <class Sch, bool FIXED = false>
 __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
   // ---- tile of this CTA: groups of PP_GROUP row blocks, column blocks inside a group
   const int mt = (a.M + PP_M - 1) / PP_M, nt = (a.N + PP_N - 1) / PP_N;
@@ -337,7 +448,7 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base;
   const int nkc = a.nkc;
-  const int nwin = (nkc + PP_FLUSH - 1) / PP_FLUSH;
+  const int nwin = (nkc + Sch::FLUSH - 1) / Sch::FLUSH;
 
   if (warp == 0) {
     // ---- producer: one elected lane streams the slices of every k chunk
@@ -353,13 +464,13 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
         }
         const uint32_t bar = su32(&full[s]);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                     "r"(PP_STAGE_BYTES)
+                     "r"(PP_STAGE_BYTES<Sch>)
                      : "memory");
-        unsigned char* st = smem + (size_t)s * PP_STAGE_BYTES;
+        unsigned char* st = smem + (size_t)s * PP_STAGE_BYTES<Sch>;
         {  // per slice: A 8 KB (two line blocks), B 4 KB
 #pragma unroll 1
-          for (int p = 0; p < 8; ++p) {
-            const size_t blk = (size_t)c * 8 + p;
+          for (int p = 0; p < Sch::SLICES; ++p) {
+            const size_t blk = (size_t)c * Sch::SLICES + p;
             const uint16_t* srcA = a.A + (blk * a.nlbA + lbA) * 2048;
             const uint16_t* srcB = a.B + (blk * a.nlbB + lbB) * 2048;
             asm volatile(
@@ -369,7 +480,7 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
                 : "memory");
             asm volatile(
                 "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], "
-                "%2, [%3];" ::"r"(su32(st + PP_A_BYTES + p * 4096)),
+                "%2, [%3];" ::"r"(su32(st + PP_A_BYTES<Sch> + p * 4096)),
                 "l"(srcB), "r"(4096), "r"(bar)
                 : "memory");
           }
@@ -388,8 +499,8 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
       const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PP_M >> 4) << 24);
       for (int c = 0; c < nkc; ++c) {
         const int s = c % PP_STAGES;
-        const int win = c / PP_FLUSH;
-        const bool win_start = (c % PP_FLUSH) == 0;
+        const int win = c / Sch::FLUSH;
+        const bool win_start = (c % Sch::FLUSH) == 0;
         if (win_start && win > 0 &&
             !wait_bar(su32(&accfree), (uint32_t)((win - 1) & 1), abort)) {
           atomicExch(&abort_flag, 1);
@@ -400,39 +511,45 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t stA = su32(smem + (size_t)s * PP_STAGE_BYTES);
-        const uint32_t stB = stA + PP_A_BYTES;
-        // slice 0 goes in three MMAs (levels 0..3, 4..5, 6..7), the others in groups of four
-        // B slices; a window starts with the first two overwriting the exact levels, the
-        // levels 6..7 are overwritten only by the very first MMA of the tile.  The 13 groups
-        // (A slice p, first B slice q0, B slices nq) are a compile-time table, so the issue is
-        // a straight sequence: descriptors are the stage's base descriptors plus constants
-        // (the start-address field holds address / 16; every address stays inside the stage)
-        constexpr int GP[13] = {0, 0, 0, 1, 1, 2, 2, 3, 3, 4, 5, 6, 7};
-        constexpr int GQ[13] = {0, 4, 6, 0, 4, 0, 4, 0, 4, 0, 0, 0, 0};
-        constexpr int GN[13] = {4, 2, 2, 4, 3, 4, 2, 4, 1, 4, 3, 2, 1};
+        const uint32_t stA = su32(smem + (size_t)s * PP_STAGE_BYTES<Sch>);
+        const uint32_t stB = stA + PP_A_BYTES<Sch>;
+        // groups (A slice p, first B slice q0, B slices nq); slice 0 covers every level and comes
+        // first: at the start of a window it overwrites the exact levels while the FP32 levels go
+        // on (overwritten only by the very first MMA of the tile), so there it takes three MMAs.
+        // The groups are a compile-time table, so the issue is a straight sequence: descriptors
+        // are the stage's base descriptors plus constants (the start-address field holds
+        // address / 16; every address stays inside the stage)
         const uint64_t dA = sdesc_sw64(stA), dB = sdesc_sw64(stB);
+        auto mma = [&](int ks, int pg, int q0, int nq, uint32_t acc) {
+          const uint32_t idesc = idesc0 | ((uint32_t)((nq * PP_N) >> 3) << 17);
+          const uint64_t da = dA + (uint64_t)((pg * 8192 + ks * 32) >> 4);
+          const uint64_t db = dB + (uint64_t)((q0 * 4096 + ks * 32) >> 4);
+          asm volatile(
+              "{\n\t.reg .pred pd;\n\tsetp.ne.b32 pd, %4, 0;\n\t"
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, pd;\n\t}" ::"r"(
+                  tmem + (uint32_t)((pg + q0) * PP_N)),
+              "l"(da), "l"(db), "r"(idesc), "r"(acc));
+        };
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-          for (int g = 0; g < 13; ++g) {
-            const int pg = GP[g], q0 = GQ[g], nq = GN[g];
-            const bool first = ks == 0 && pg == 0 && (q0 < PP_EXACT ? win_start : c == 0);
-            const uint32_t acc = first ? 0u : 1u;
-            const uint32_t idesc = idesc0 | ((uint32_t)((nq * PP_N) >> 3) << 17);
-            const uint64_t da = dA + (uint64_t)((pg * 8192 + ks * 32) >> 4);
-            const uint64_t db = dB + (uint64_t)((q0 * 4096 + ks * 32) >> 4);
-            asm volatile(
-                "{\n\t.reg .pred pd;\n\tsetp.ne.b32 pd, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, pd;\n\t}" ::"r"(
-                    tmem + (uint32_t)((pg + q0) * PP_N)),
-                "l"(da), "l"(db), "r"(idesc), "r"(acc));
+        for (int ks = 0; ks < 2; ++ks) {
+          const bool start = ks == 0 && win_start;
+          mma(ks, 0, 0, 4, start ? 0u : 1u);
+          if (Sch::SLICES == 7 && !start) {
+            mma(ks, 0, 4, 3, 1u);
+          } else {
+            mma(ks, 0, 4, Sch::EXACT - 4, start ? 0u : 1u);
+            mma(ks, 0, Sch::EXACT, 2, ks == 0 && c == 0 ? 0u : 1u);
           }
+#pragma unroll
+          for (int g = 0; g < Sch::GROUPS; ++g)
+            mma(ks, (int)(Sch::GP >> (4 * g)) & 15, (int)(Sch::GQ >> (4 * g)) & 15,
+                (int)(Sch::GN >> (4 * g)) & 15, 1u);
+        }
         asm volatile(
             "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                 su32(&empty[s]))
             : "memory");
-        if ((c % PP_FLUSH) == PP_FLUSH - 1 || c == nkc - 1)
+        if ((c % Sch::FLUSH) == Sch::FLUSH - 1 || c == nkc - 1)
           asm volatile(
               "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                   su32(&accf))
@@ -453,7 +570,7 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
 #pragma unroll
     for (int c = 0; c < 32; ++c) T[c] = 0;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(32 * half);
-    bool ok = true;
+    bool ok = true, mirror = false;
     for (int w = 0; w < nwin; ++w) {
       // warp-uniform decision: the TMEM loads below are .sync.aligned
       const bool got = wait_bar(su32(&accf), (uint32_t)(w & 1), abort);
@@ -463,81 +580,104 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
+      // the next level's load is in flight while a level is converted
+      uint32_t va[32], vb[32];
+      tmem_ld32(lane_base, va);
+      tmem_wait(va);
 #pragma unroll
-      for (int lv = 0; lv < PP_EXACT; ++lv) {
+      for (int lv = 0; lv < Sch::EXACT; ++lv) {
+        uint32_t(&v)[32] = (lv & 1) ? vb : va;
+        uint32_t(&vn)[32] = (lv & 1) ? va : vb;
+        if (lv + 1 < Sch::EXACT) tmem_ld32(lane_base + (uint32_t)((lv + 1) * PP_N), vn);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t v[16];
-          tmem_ld16(lane_base + (uint32_t)(lv * PP_N + 16 * h), v);
-#pragma unroll
-          for (int t = 0; t < 16; ++t) {
-            const float f = __uint_as_float(v[t]);
-            const long long iv =
-                (long long)__float2int_rn(f * __uint_as_float((uint32_t)(127 + 7 * lv) << 23));
-            T[16 * h + t] += iv * (1LL << (7 * (PP_EXACT - 1 - lv)));
+        for (int t = 0; t < 32; ++t) {
+          const float f = __uint_as_float(v[t]);
+          if (lv == 0) {  // |f| <= 192 * 2^14 < 2^22: read off the sum with 1.5 * 2^23
+            const int iv = (int)(__float_as_uint(f + 12582912.f) - 0x4B400000u);
+            T[t] = (long long)((unsigned long long)T[t] +
+                               ((unsigned long long)(long long)iv << (Sch::BITS * (Sch::EXACT - 1))));
+          } else {
+            T[t] = add_level(T[t], __float2int_rn(f), 1 << (Sch::BITS * (Sch::EXACT - 1 - lv)));
           }
         }
+        if (lv + 1 < Sch::EXACT) tmem_wait(vn);
       }
-
       asm volatile("tcgen05.fence::before_thread_sync;");
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(&accfree)) : "memory");
     }
     if (__all_sync(0xffffffffu, (ok && !*abort) ? 1 : 0)) {
-      // C = 2^(eA + eB - 14) (T 2^-35 + F), F = levels 6 + 7
+      // C = 2^(eA + eB - 14) (T + F) 2^(-BITS (EXACT - 1)).  A symmetric product's mirror image
+      // goes through shared memory (the stages are free: every copy and MMA of the tile has
+      // completed), so that both triangles are written in full sectors
       const int i = i0 + row;
       const int ei = i < a.M ? a.eA[i] + a.eshiftA : 0;
+      long long* mir = reinterpret_cast<long long*>(smem);  // [PP_N][PP_M + 1]
+      uint32_t v5[32], v6[32];
+      tmem_ld32(lane_base + (uint32_t)(Sch::EXACT * PP_N), v5);
+      tmem_ld32(lane_base + (uint32_t)((Sch::EXACT + 1) * PP_N), v6);
+      tmem_wait(v5);
+      tmem_wait(v6);
+      if constexpr (FIXED) {
+        // the projection iterate in fixed point: the product is (T + F) 2^(sc - 32) with
+        // sc = 2 SP2_E - 14, i.e. W = (T + F) 2^9 in units of 2^-55 (F rounded to an
+        // integer there: an absolute 2^-56); |T| < 2^53 keeps T 2^9 exact, else the element is
+        // marked out of range
+        long long* W = reinterpret_cast<long long*>(a.C);
+        static_assert(2 * SP2_E - 14 - Sch::BITS * (Sch::EXACT - 1) + SP2_FRAC == 9,
+                      "fixed-point scale of the product");
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t v6[16], v7[16];
-        tmem_ld16(lane_base + (uint32_t)(6 * PP_N + 16 * h), v6);
-        tmem_ld16(lane_base + (uint32_t)(7 * PP_N + 16 * h), v7);
-        if constexpr (FIXED) {
-          if (i < a.M) {
-          // the projection iterate in fixed point: the product is (T + F 2^35) 2^(sc - 35) with
-          // sc = 2 SP2_E - 14, i.e. W = T 2^8 + F 2^43 in units of 2^-55 (F rounded to an
-          // integer there: an absolute 2^-56); |T| < 2^54 keeps T 2^8 exact, else the element is
-          // marked out of range
-          long long* W = reinterpret_cast<long long*>(a.C);
-          static_assert(2 * SP2_E - 14 - 35 + SP2_FRAC == 8, "fixed-point scale of the product");
+        for (int t8 = 0; t8 < 32; t8 += 8) {
+          long long old[8];
 #pragma unroll
-          for (int t8 = 0; t8 < 16; t8 += 8) {
-            long long old[8];
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              const int j = j0 + 32 * half + 16 * h + t8 + t;
-              old[t] = (a.sub2 && j < a.N && i >= j) ? W[i + (size_t)j * a.ldc] : 0ll;
-            }
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              const int j = j0 + 32 * half + 16 * h + t8 + t;
-              if (j < a.N && i >= j) {
-                const long long tv = T[16 * h + t8 + t];
-                const float ff = (__uint_as_float(v6[t8 + t]) + __uint_as_float(v7[t8 + t])) *
-                                 0x1p43f;
-                // unsigned arithmetic: wrap-around instead of undefined overflow, and the
-                // out-of-range cases are replaced below
-                unsigned long long w =
-                    ((unsigned long long)tv << 8) + (unsigned long long)(long long)__float2int_rn(ff);
-                if (a.sub2) w = 2ull * (unsigned long long)old[t] - w;
-                if (tv >= (1ll << 54) || tv <= -(1ll << 54) || fabsf(ff) >= 0x1p30f ||
-                    old[t] == SP2_BAD)
-                  w = (unsigned long long)SP2_BAD;
-                W[i + (size_t)j * a.ldc] = (long long)w;
-                if (i != j) W[j + (size_t)i * a.ldc] = (long long)w;
-              }
-            }
+          for (int t = 0; t < 8; ++t) {
+            const int j = j0 + 32 * half + t8 + t;
+            old[t] = (a.sub2 && j < a.N && i < a.M && i >= j) ? W[i + (size_t)j * a.ldc] : 0ll;
           }
-          }
-        } else if (i < a.M) {
 #pragma unroll
-          for (int t = 0; t < 16; ++t) {
-            const int j = j0 + 32 * half + 16 * h + t;
-            if (j < a.N && !(a.sym && i < j)) {
-              const double val = tile_value(T[16 * h + t], v6[t], v7[t], ei + a.eB[j] - 14);
-              a.C[i + (size_t)j * a.ldc] = val;
-              if (a.sym && i != j) a.C[j + (size_t)i * a.ldc] = val;
-            }
+          for (int t = 0; t < 8; ++t) {
+            const int jl = 32 * half + t8 + t, j = j0 + jl;
+            const long long tv = T[t8 + t];
+            const float ff = low_levels<Sch>(v5[t8 + t], v6[t8 + t]) * 0x1p9f;
+            // unsigned arithmetic: wrap-around instead of undefined overflow, and the
+            // out-of-range cases are replaced below
+            unsigned long long w =
+                ((unsigned long long)tv << 9) + (unsigned long long)(long long)__float2int_rn(ff);
+            if (a.sub2) w = 2ull * (unsigned long long)old[t] - w;
+            if (tv >= (1ll << 53) || tv <= -(1ll << 53) || fabsf(ff) >= 0x1p30f ||
+                old[t] == SP2_BAD)
+              w = (unsigned long long)SP2_BAD;
+            if (i < a.M && j < a.N && i >= j) W[i + (size_t)j * a.ldc] = (long long)w;
+            mir[jl * (PP_M + 1) + row] = (long long)w;
           }
+        }
+      } else {
+#pragma unroll
+        for (int t = 0; t < 32; ++t) {
+          const int jl = 32 * half + t, j = j0 + jl;
+          const bool in = i < a.M && j < a.N;
+          const double val = in ? tile_value<Sch>(T[t], v5[t], v6[t], ei + a.eB[j] - 14) : 0.0;
+          if (in && !(a.sym && i < j)) a.C[i + (size_t)j * a.ldc] = val;
+          if (a.sym) mir[jl * (PP_M + 1) + row] = __double_as_longlong(val);
+        }
+      }
+      if (FIXED || a.sym) {
+        // rows of the mirror image: 16 per warp, two columns of the tile per lane.  All eight
+        // epilogue warps take this branch or none does, unless a wait ran out in one of them:
+        // the abort flag is read again behind a barrier that every one of them passes
+        mirror = true;
+      }
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (__all_sync(0xffffffffu, (mirror && !*abort) ? 1 : 0)) {
+      const long long* mir = reinterpret_cast<const long long*>(smem);
+      long long* W = reinterpret_cast<long long*>(a.C);
+#pragma unroll 4
+      for (int k = 0; k < 16; ++k) {
+        const int r = (warp - 2) * 16 + k, i = i0 + r;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int jl = lane + 32 * h, j = j0 + jl;
+          if (i < a.M && j < a.N && i > j) W[j + (size_t)i * a.ldc] = mir[jl * (PP_M + 1) + r];
         }
       }
     }
@@ -549,7 +689,10 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(PP_TMEM_COLS));
 }
-__global__ void __launch_bounds__(PP_THREADS, 1) k_opipe(PipeArgs a) { opipe_tile(a, blockIdx.x); }
+template <class Sch>
+__global__ void __launch_bounds__(PP_THREADS, 1) k_opipe(PipeArgs a) {
+  opipe_tile<Sch>(a, blockIdx.x);
+}
 
 // ---- batched spectral projection on the pipe, two launches per step for every molecule of the
 // list still iterating (blockIdx.y / blockIdx.z walks the molecules): kb_opipe_sq squares the
@@ -663,7 +806,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) kb_opipe_sq(const MolPtrs* __re
       atomicAdd(&g_pipe_batch_flops, 2ull * (unsigned long long)min(PP_M, n - i0) *
                                          (unsigned long long)min(PP_N, n - j0) * (unsigned)n);
   }
-  opipe_tile<true>(a, blockIdx.x);
+  opipe_tile<Balanced, true>(a, blockIdx.x);
 }
 
 // ---- the slice image of the iterate and the decision: each warp owns one line i of D (column i
@@ -675,13 +818,6 @@ __global__ void __launch_bounds__(PP_THREADS, 1) kb_opipe_sq(const MolPtrs* __re
 // elements k, k + 1 of a 64-element segment (coalesced loads), so each slice plane gets one
 // 32-bit word per lane.  Padding lines and positions get zero slices.
 //
-// Slice p of a fixed-point value Y < 2^56 is the 7-bit field a = (Y >> (49 - 7p)) & 127 (read
-// from the 28-bit half that holds it); its BF16 value a 2^-7p is read off the BF16 number whose
-// exponent field is 134 - 7p and mantissa field a: that number is 2^(7 - 7p) + a 2^-7p exactly,
-// and subtracting 2^(7 - 7p) leaves a 2^-7p (exact: at most 7 significant bits).  Two
-// elements go through one BF16x2 subtraction, and the signs go in with one OR (a zero slice of
-// a negative element becomes -0, which adds nothing to a product).
-
 // the square of Y < 2^56 as a (2^56, 2^28, 1) limb triple: Y = h 2^28 + l, Y^2 = h^2 2^56 +
 // 2 h l 2^28 + l^2 (every partial product below 2^56, so per-lane sums of up to 256 stay exact)
 struct Sq3 {
@@ -735,9 +871,8 @@ __global__ void __launch_bounds__(256) kb_sp2_slice(const MolPtrs* __restrict__ 
           if (k + e >= n) continue;
           const double x = ((k + e == i ? emax : 0.0) - am[k + e]) * f;
           const uint64_t bits = (uint64_t)__double_as_longlong(x);
-          const long long m = (long long)fixed_bits(bits, SP2_E);
           const long long w =
-              ((bits >> 52) & 0x7FF) >= (uint64_t)(1023 + SP2_E) ? SP2_BAD : ((bits >> 63) ? -m : m);
+              ((bits >> 52) & 0x7FF) > (uint64_t)(1023 + SP2_E) ? SP2_BAD : fixed55(bits, SP2_E);
           y[k + e] = w;
           (e ? w1 : w0) = w;
         }
@@ -751,29 +886,20 @@ __global__ void __launch_bounds__(256) kb_sp2_slice(const MolPtrs* __restrict__ 
     // molecule) and their 28-bit halves
     const unsigned long long a0 = w0 < 0 ? 0ull - (unsigned long long)w0 : (unsigned long long)w0;
     const unsigned long long a1 = w1 < 0 ? 0ull - (unsigned long long)w1 : (unsigned long long)w1;
-    const bool bad0 = a0 >= (1ull << 56), bad1 = a1 >= (1ull << 56);
+    const bool bad0 = a0 >= (unsigned long long)SP2_LIMIT,
+               bad1 = a1 >= (unsigned long long)SP2_LIMIT;
     over = over || bad0 || bad1;
     const unsigned long long m0 = bad0 ? 0ull : a0, m1 = bad1 ? 0ull : a1;
     const uint32_t h0 = (uint32_t)(m0 >> 28), l0 = (uint32_t)m0 & 0xFFFFFFFu;
     const uint32_t h1 = (uint32_t)(m1 >> 28), l1 = (uint32_t)m1 & 0xFFFFFFFu;
     sq.add(h0, l0);
     sq.add(h1, l1);
-    const uint32_t signs = (w0 < 0 ? 0x8000u : 0u) | (w1 < 0 ? 0x80000000u : 0u);
     const size_t off = (size_t)slice_off(i, k, nlb);
-    // both elements at once: 16-bit lanes hold the two elements' bits 0..15 of a half (slices
-    // 3 and 2 of h, 7 and 6 of l) or its bits 14..29 (slices 1 and 0, 5 and 4); a shift and a
-    // mask put a slice's 7-bit field of both elements in the lanes' mantissa fields, the
-    // exponent field 134 - 7p makes each lane 2^(7-7p) + a 2^-7p exactly, and one BF16x2
-    // subtraction of 2^(7-7p) leaves the packed pair of slices (exact: a has 7 bits)
-    const uint32_t R[4] = {__byte_perm(h0 >> 14, h1 >> 14, 0x5410), __byte_perm(h0, h1, 0x5410),
-                           __byte_perm(l0 >> 14, l1 >> 14, 0x5410), __byte_perm(l0, l1, 0x5410)};
+    uint32_t w[Balanced::SLICES];
+    digits_pair(bad0 ? 0 : w0, bad1 ? 0 : w1, w);
 #pragma unroll
-    for (int pp = 0; pp < 8; ++pp) {
-      const uint32_t bias = ((uint32_t)(134 - 7 * pp) << 7) * 0x10001u;
-      const uint32_t mag = ((R[pp >> 1] >> ((pp & 1) ? 0 : 7)) & 0x007F007Fu) | bias;
-      const uint32_t w = bf16x2_sub(mag, bias);
-      *reinterpret_cast<uint32_t*>(q.img + off + pp * plane) = w | signs;
-    }
+    for (int pp = 0; pp < Balanced::SLICES; ++pp)
+      *reinterpret_cast<uint32_t*>(q.img + off + pp * plane) = w[pp];
   }
   if (init && lane == 0) q.iexp[i] = SP2_E;
   // block partial sums (exact integers): warp trees, then the warps in order
@@ -856,7 +982,7 @@ __global__ void __launch_bounds__(256) kb_pexp_site(const MolPtrs* __restrict__ 
   int* e = xdst >= 0 ? q.xexp[xdst] : which ? q.iexp2 : q.iexp;
   if (!L.kcontig) {
     if ((int)blockIdx.x * 32 >= lp) return;
-    pexp_rows_dev(L.M, L.ld, L.lines, L.K, lp, e, blockIdx.x);
+    pexp_rows_dev<32, 256>(L.M, L.ld, L.lines, L.K, lp, e, blockIdx.x);
     return;
   }
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -876,7 +1002,7 @@ __global__ void __launch_bounds__(256) kb_psplit_site(const MolPtrs* __restrict_
   const SiteLines L = site_lines(site_of(q, site), which);
   const int lp = lines_padded(L.lines), nkc = (L.K + PP_KC - 1) / PP_KC;
   if ((int)blockIdx.x >= lp / 64 || (int)blockIdx.y >= nkc) return;
-  psplit_dev(L.M, L.ld, L.kcontig, L.lines, L.K, lp / 64,
+  psplit_dev<Balanced>(L.M, L.ld, L.kcontig, L.lines, L.K, lp / 64,
              xdst >= 0 ? q.xexp[xdst] : which ? q.iexp2 : q.iexp,
              xdst >= 0 ? q.ximg[xdst] : which ? q.img2 : q.img, blockIdx.x, blockIdx.y);
 }
@@ -913,7 +1039,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) kb_opipe_site(const MolPtrs* __
       atomicAdd(&g_pipe_batch_flops, 2ull * (unsigned long long)min(PP_M, s.M - i0) *
                                          (unsigned long long)min(PP_N, s.N - j0) * (unsigned)s.K);
   }
-  opipe_tile(a, blockIdx.x);
+  opipe_tile<Balanced>(a, blockIdx.x);
 }
 
 }  // namespace
@@ -922,7 +1048,8 @@ void pipe_site_b(const BatchLaunch& b, int site) {
   if (!b.count) return;
   static bool attr = false;
   if (!attr) {
-    ck(cudaFuncSetAttribute(kb_opipe_site, cudaFuncAttributeMaxDynamicSharedMemorySize, PP_SMEM),
+    ck(cudaFuncSetAttribute(kb_opipe_site, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            PP_SMEM<Balanced>),
        "smem attr batched pipelined split gemm");
     attr = true;
   }
@@ -940,7 +1067,7 @@ void pipe_site_b(const BatchLaunch& b, int site) {
   prof_kend(KS_PIPE_PREP, tk, b.s);
   ++g_kernel_launches;
   tk = prof_kbegin(b.s);
-  kb_opipe_site<<<dim3(tiles, b.count), PP_THREADS, PP_SMEM, b.s>>>(b.mp, b.list, site);
+  kb_opipe_site<<<dim3(tiles, b.count), PP_THREADS, PP_SMEM<Balanced>, b.s>>>(b.mp, b.list, site);
   prof_kend(KS_PIPE, tk, b.s);
 }
 
@@ -987,7 +1114,8 @@ void sp2_square_b(const BatchLaunch& b) {
   if (!b.count) return;
   static bool attr = false;
   if (!attr) {
-    ck(cudaFuncSetAttribute(kb_opipe_sq, cudaFuncAttributeMaxDynamicSharedMemorySize, PP_SMEM),
+    ck(cudaFuncSetAttribute(kb_opipe_sq, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            PP_SMEM<Balanced>),
        "smem attr batched pipelined split gemm");
     attr = true;
   }
@@ -995,14 +1123,14 @@ void sp2_square_b(const BatchLaunch& b) {
   const int tiles = ((n + PP_M - 1) / PP_M) * ((n + PP_N - 1) / PP_N);
   const int tk = prof_kbegin(b.s);
   ++g_kernel_launches;
-  kb_opipe_sq<<<dim3(tiles, b.count), PP_THREADS, PP_SMEM, b.s>>>(b.mp, b.list);
+  kb_opipe_sq<<<dim3(tiles, b.count), PP_THREADS, PP_SMEM<Balanced>, b.s>>>(b.mp, b.list);
   prof_kend(KS_PIPE, tk, b.s);
 }
 
-size_t pimage_bytes(int lines, int K) {
+size_t pimage_bytes(int lines, int K, bool balanced) {
   const size_t lp = (size_t)((lines + PP_M - 1) / PP_M) * PP_M;
   const size_t kp = (size_t)((K + PP_KC - 1) / PP_KC) * PP_KC;
-  return lp * kp * 8 * sizeof(uint16_t);
+  return lp * kp * (balanced ? Balanced::SLICES : Magnitude::SLICES) * sizeof(uint16_t);
 }
 int pimage_lines(int lines) { return ((lines + PP_M - 1) / PP_M) * PP_M; }
 int sp2_slot_count(int n) { return sp2_slots(n); }
@@ -1017,9 +1145,13 @@ void psplit(const double* M, int ld, int kcontig, int lines, int K, PImage& img,
   const int nkc = (K + PP_KC - 1) / PP_KC;
   g_kernel_launches += 2;
   if (kcontig) k_pexp_cols<<<(lp * 32 + 255) / 256, 256, 0, s>>>(M, ld, lines, K, lp, img.e);
-  else k_pexp_rows<<<lp / 32, 256, 0, s>>>(M, ld, lines, K, lp, img.e);
-  k_psplit<<<dim3(lp / 64, nkc), 256, 0, s>>>(M, ld, kcontig, lines, K, lp / 64, img.e,
-                                              img.data);
+  else k_pexp_rows<<<lp / 16, 1024, 0, s>>>(M, ld, lines, K, lp, img.e);
+  if (img.balanced)
+    k_psplit<Balanced><<<dim3(lp / 64, nkc), 256, 0, s>>>(M, ld, kcontig, lines, K, lp / 64, img.e,
+                                                          img.data);
+  else
+    k_psplit<Magnitude><<<dim3(lp / 64, nkc), 256, 0, s>>>(M, ld, kcontig, lines, K, lp / 64,
+                                                           img.e, img.data);
 }
 
 // C = 2^eshiftA op(A) op(B) from two slice images (A.K == B.K); sym: the product is symmetric
@@ -1028,9 +1160,14 @@ void pgemm(const PImage& A, const PImage& B, double* C, int ldc, bool sym, int* 
   if (A.lines <= 0 || B.lines <= 0) return;
   if (A.K != B.K) throw std::runtime_error("split GEMM: inner dimensions differ");
   if (A.K > PP_KMAX) throw std::runtime_error("split GEMM: inner dimension above 12288");
+  if (A.balanced != B.balanced) throw std::runtime_error("split GEMM: operands split differently");
   static bool attr = false;
   if (!attr) {
-    ck(cudaFuncSetAttribute(k_opipe, cudaFuncAttributeMaxDynamicSharedMemorySize, PP_SMEM),
+    ck(cudaFuncSetAttribute(k_opipe<Balanced>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            PP_SMEM<Balanced>),
+       "smem attr pipelined split gemm");
+    ck(cudaFuncSetAttribute(k_opipe<Magnitude>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            PP_SMEM<Magnitude>),
        "smem attr pipelined split gemm");
     attr = true;
   }
@@ -1054,7 +1191,8 @@ void pgemm(const PImage& A, const PImage& B, double* C, int ldc, bool sym, int* 
                        : 2ull * a.M * a.N * A.K;
   const int tk = prof_kbegin(s);
   ++g_kernel_launches;
-  k_opipe<<<mt * nt, PP_THREADS, PP_SMEM, s>>>(a);
+  if (A.balanced) k_opipe<Balanced><<<mt * nt, PP_THREADS, PP_SMEM<Balanced>, s>>>(a);
+  else k_opipe<Magnitude><<<mt * nt, PP_THREADS, PP_SMEM<Magnitude>, s>>>(a);
   prof_kend(KS_GEMM, tk, s);
 }
 
@@ -1075,12 +1213,13 @@ extern "C" int tblite_gb300_split_gemm(int m, int n, int k, const double* a, con
   if (m <= 0 || n <= 0 || k <= 0 || !a || !b || !c || (sym && m != n)) return -1;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   PImage ia, ib;
+  ia.balanced = ib.balanced = true;
   int* st = nullptr;
   int hst = 0;
   int rc = 0;
-  if (cudaMalloc(&ia.data, pimage_bytes(m, k)) != cudaSuccess ||
+  if (cudaMalloc(&ia.data, pimage_bytes(m, k, true)) != cudaSuccess ||
       cudaMalloc(&ia.e, sizeof(int) * pimage_lines(m)) != cudaSuccess ||
-      cudaMalloc(&ib.data, pimage_bytes(n, k)) != cudaSuccess ||
+      cudaMalloc(&ib.data, pimage_bytes(n, k, true)) != cudaSuccess ||
       cudaMalloc(&ib.e, sizeof(int) * pimage_lines(n)) != cudaSuccess ||
       cudaMalloc(&st, sizeof(int)) != cudaSuccess) {
     rc = -2;

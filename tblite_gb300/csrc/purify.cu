@@ -372,7 +372,7 @@ Purifier* purify_create(int n, cudaStream_t s) {
   ck(cudaMemsetAsync(p->status, 0, sizeof(int), s), "purify status");
   ck(cudaMallocHost(&p->hsc, sizeof(double) * 16), "purify hsc");
   for (PImage& im : p->img) {
-    ck(cudaMalloc(&im.data, pimage_bytes(n, n)), "purify image");
+    ck(cudaMalloc(&im.data, pimage_bytes(n, n, false)), "purify image");
     ck(cudaMalloc(&im.e, sizeof(int) * pimage_lines(n)), "purify image e");
   }
   return p;
@@ -399,7 +399,9 @@ static void read_scalars(Purifier* p, int count) {
   stream_wait(p->s);
 }
 // C = A B (n x n, column-major; sym: C is symmetric, the tiles on and below the diagonal are
-// computed and mirrored).  The pipelined GEMM first splits A into image slot sa (its rows) and
+// computed and mirrored).  The pipelined GEMM first splits A into image slot sa (every left operand
+// here is symmetric, so its rows are read as its columns, which are contiguous: the exponents of
+// 3072 lines take 20 us that way, 57 us by rows) and
 // B into slot sb (its columns), unless keep_a / keep_b say the slot already holds that image.
 static void product(Purifier* p, const double* A, int sa, bool keep_a, const double* B, int sb,
                     bool keep_b, double* C, bool sym) {
@@ -409,7 +411,7 @@ static void product(Purifier* p, const double* A, int sa, bool keep_a, const dou
           p->s);
     return;
   }
-  if (!keep_a) psplit(A, n, 0, n, n, p->img[sa], p->s);
+  if (!keep_a) psplit(A, n, 1, n, n, p->img[sa], p->s);
   if (!keep_b && !(sb == sa && B == A)) psplit(B, n, 1, n, n, p->img[sb], p->s);
   pgemm(p->img[sa], p->img[sb], C, n, sym, p->status, p->s);
 }
@@ -457,7 +459,7 @@ int purify_set_overlap(Purifier* p, const double* S) {
   ++g_kernel_launches;
   k_scale_dev<<<eb, 256, 0, p->s>>>(nn, Z, p->sc + 2);
   if (Z != p->Z) ck(cudaMemcpyAsync(p->Z, Z, sizeof(double) * nn, cudaMemcpyDeviceToDevice, p->s), "Z");
-  if (g_pipe_gemm) psplit(p->Z, n, 0, n, n, p->img[2], p->s);  // Z stays split (symmetric)
+  if (g_pipe_gemm) psplit(p->Z, n, 1, n, n, p->img[2], p->s);  // Z stays split (symmetric)
   return it;
 }
 
