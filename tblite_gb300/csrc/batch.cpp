@@ -182,7 +182,7 @@ struct Plan {
   // offsets (region, offset) of every array
   Piece xyz, at_z, at_sh, sh_atom, sh_l, sh_nprim, sh_alpha, sh_coeff, sh_ao, ao_sh, ao_at, sh_se0,
       sh_kcn, sh_shpoly, sh_zeta, sh_hub, sh_gam3, sh_refocc, at_en, at_rad, at_rcov, at_mprad,
-      at_vcn, at_dkern, at_qkern, at_repa, at_repz, sh_valence, at_gam3;
+      at_vcn, at_dkern, at_qkern, at_repa, at_repz, sh_valence, sh_perm, at_gam3;
   Piece d3_sp, d3_nref, d3_refcn, d3_c6ref, d3_r4r2, d3_rcov, d3_cn, d3_w, d3_dw, d3_dEdcn;
   Piece d4_sp, d4_nref, d4_ngw, d4_refcn, d4_refq, d4_zeff, d4_gam, d4_r4r2, d4_rcov, d4_en,
       d4_c6ref;
@@ -202,7 +202,7 @@ struct Plan {
 
 struct Bucket {
   int first, last;  // range in the sorted plan
-  int nat_max = 0, nsh_max = 0, nao_max = 0, nd_max = 0;
+  int nat_max = 0, nsh_max = 0, nao_max = 0, nd_max = 0, np_max = 0;
   bool sp2 = false;
   int sp2_steps = SP2_MAX_STEPS;  // step budget of the next projection
 };
@@ -238,6 +238,7 @@ void layout(Plan& pl, Region* R) {
                    &pl.at_qkern, &pl.at_repa, &pl.at_repz, &pl.at_gam3})
     *p = piece<double>(R, RU, na);
   pl.sh_valence = piece<int>(R, RU, ns);
+  pl.sh_perm = piece<int>(R, RU, ns);
   if (pl.has_d3) {
     pl.d3_nref = piece<int>(R, RU, na);
     pl.d3_refcn = piece<double>(R, RU, na * D4_MREF);
@@ -391,6 +392,8 @@ MolPtrs make_ptrs(const Plan& pl, const Bases& db) {
   m.at_repa = db.at<double>(pl.at_repa);
   m.at_repz = db.at<double>(pl.at_repz);
   m.sh_valence = db.at<int>(pl.sh_valence);
+  m.sh_perm = db.at<int>(pl.sh_perm);
+  m.ns = pl.c->n_s;
   m.at_gam3 = db.at<double>(pl.at_gam3);
   q.has_d4 = pl.has_d4 ? 1 : 0;
   q.has_d3 = pl.has_d3 ? 1 : 0;
@@ -571,6 +574,7 @@ std::vector<Bucket> make_buckets(const std::vector<Plan>& plans) {
            plans[j].sp2 == b.sp2) {
       b.nat_max = std::max(b.nat_max, plans[j].nat);
       b.nsh_max = std::max(b.nsh_max, plans[j].nsh);
+      b.np_max = std::max(b.np_max, plans[j].nsh - plans[j].c->n_s);
       b.nao_max = std::max(b.nao_max, plans[j].nao);
       b.nd_max = std::max(b.nd_max, plans[j].nd);
       ++j;
@@ -648,6 +652,7 @@ std::vector<int> run_chunk(std::vector<Plan>& plans, Arena& ar, _tblite_context*
     stage(hb, pl.at_repa, c->at_repa);
     stage(hb, pl.at_repz, c->at_repz);
     stage(hb, pl.sh_valence, c->sh_valence);
+    stage(hb, pl.sh_perm, c->sh_perm);
     stage(hb, pl.at_gam3, c->at_gam3);
     if (pl.has_d3) {
       stage(hb, pl.d3_nref, c->d3_nref);
@@ -707,6 +712,7 @@ std::vector<int> run_chunk(std::vector<Plan>& plans, Arena& ar, _tblite_context*
       L.list = d_list + pos;
       L.nat_max = b.nat_max;
       L.nsh_max = b.nsh_max;
+      L.np_max = b.np_max;
       L.nao_max = b.nao_max;
       L.nd_max = b.nd_max;
       L.sp2 = b.sp2 ? 1 : 0;

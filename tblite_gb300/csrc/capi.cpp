@@ -307,6 +307,13 @@ static void build_calculator(_tblite_calculator* c, const _tblite_structure* mol
     c->at_repz.push_back(e->zeff);
     c->at_gam3.push_back(method == 1 ? e->gam3 : 0.0);
   }
+  // shells by kind for the pair kernels: s, then p, each by number of primitives
+  c->sh_perm.resize(c->nsh);
+  for (int s = 0; s < c->nsh; ++s) c->sh_perm[s] = s;
+  std::stable_sort(c->sh_perm.begin(), c->sh_perm.end(), [&](int x, int y) {
+    return c->sh_l[x] != c->sh_l[y] ? c->sh_l[x] < c->sh_l[y] : c->sh_nprim[x] < c->sh_nprim[y];
+  });
+  c->n_s = (int)std::count(c->sh_l.begin(), c->sh_l.end(), 0);
   c->model.pair_mode = pairs_gfn1 ? 1 : 0;
   if (mol->nat > 1) {
     if (method == 2) build_d4_data(c, mol);
@@ -428,6 +435,7 @@ static void ensure_workspace(_tblite_calculator* c) {
     w.at_repa.upload(c->at_repa, s);
     w.at_repz.upload(c->at_repz, s);
     w.sh_valence.upload(c->sh_valence, s);
+    w.sh_perm.upload(c->sh_perm, s);
     w.at_gam3.upload(c->at_gam3, s);
     if (c->has_d3) {
       w.d3_nref.upload(c->d3_nref, s);
@@ -663,6 +671,8 @@ static DevMol dev_mol(const _tblite_calculator* c) {
   m.at_repa = w.at_repa.p;
   m.at_repz = w.at_repz.p;
   m.sh_valence = w.sh_valence.p;
+  m.sh_perm = w.sh_perm.p;
+  m.ns = c->n_s;
   m.at_gam3 = w.at_gam3.p;
   return m;
 }

@@ -76,6 +76,8 @@ struct DevMol {
   const double* at_qkern;  // AES quadrupole kernel
   const double* at_repa;   // repulsion alpha
   const double* at_repz;   // repulsion zeff
+  const int* sh_perm;      // [nsh] s shells, then p shells, each by number of primitives
+  int ns;                  // number of s shells
   const int* sh_valence;   // GFN1: 1 for the first shell of its angular momentum on the atom
   const double* at_gam3;   // GFN1: atom-resolved third-order hardness derivative
 };
@@ -424,6 +426,7 @@ struct BatchLaunch {
   const int* list;
   int count;
   int nat_max, nsh_max, nao_max, nd_max;
+  int np_max;     // p shells
   int sp2;        // the bucket's density comes from the spectral projection (sp2.cu)
   int sp2_steps;  // its step budget in this SCF iteration
   cudaStream_t s;

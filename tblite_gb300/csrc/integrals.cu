@@ -48,7 +48,7 @@ __device__ __forceinline__ double O1(const Moments& M, int k, int p, int b, doub
 __device__ __forceinline__ int cexp(int l, int c, int k) { return (l == 1 && c == k) ? 1 : 0; }
 
 // ---------------------------------------------------------------------------------------
-// H0 build: one thread per (shell pair ish >= jsh, ket orbital mi)
+// H0 build over the shell pairs ish >= jsh (ish the ket)
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void tri_index(long long t, int& i, int& j) {
   // t = i*(i+1)/2 + j, 0 <= j <= i
@@ -102,30 +102,33 @@ __device__ __forceinline__ double hscale_of(const DevMol& m, const Gfn2Scalars& 
   return zij * p.kshell[m.sh_l[jsh]][m.sh_l[ish]] * (1.0 + p.enscale * den);
 }
 
-__device__ __forceinline__ void build_h0_dev(DevMol m, Gfn2Scalars p, const double* __restrict__ se, double* S,
-                           double* H, double* D, double* Q, long long npair) {
-  const long long gid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long t = gid / 3;
-  const int mi = (int)(gid % 3);
-  if (t >= npair) return;
-  int ish, jsh;
-  tri_index(t, ish, jsh);
-  const int li = m.sh_l[ish], lj = m.sh_l[jsh];
-  if (mi > 2 * li) return;
+// Shell pairs are walked by kind: DevMol.sh_perm lists the s shells, then the p shells, each by
+// number of primitives, and the pairs come as s-s, then s-p, then p-p, each kind from a multiple of
+// 32 on.  An FP64 instruction costs a warp the same whatever its active lanes do, so a warp of
+// mixed kinds pays for every kind in turn (for water 16 units of component pairs where its lanes
+// need 2.25 on average) and for the longest primitive loops among its lanes.
+__device__ __forceinline__ long long pad32(long long t) { return (t + 31) & ~31ll; }
+
+// ket shell ish >= bra shell jsh of angular momenta LI, LJ; NI ket components from the cartesian
+// component CI on.  The products are written as rounded multiplications and one FMA, so that a factor
+// known to be 1 changes no rounding.
+template <int LI, int LJ, int NI, int CI>
+__device__ __forceinline__ void build_h0_pair(const DevMol& m, const Gfn2Scalars& p,
+                           const double* __restrict__ se, double* S,
+                           double* H, double* D, double* Q, int ish, int jsh) {
+  constexpr int NJ = 2 * LJ + 1;
   const int iat = m.sh_atom[ish], jat = m.sh_atom[jsh];
   double vec[3];
-  double r2 = 0.0;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    vec[k] = m.xyz[3 * iat + k] - m.xyz[3 * jat + k];
-    r2 += vec[k] * vec[k];
-  }
+  for (int k = 0; k < 3; ++k) vec[k] = m.xyz[3 * iat + k] - m.xyz[3 * jat + k];
+  // written out so that every kind rounds alike: the integrals are the same bit for bit whatever
+  // the kind is compiled to
+  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(vec[0], vec[0]), __dmul_rn(vec[1], vec[1])),
+                              __dmul_rn(vec[2], vec[2]));
   const bool onsite = iat == jat;
   if (!onsite && (r2 > p.h0_cutoff * p.h0_cutoff || r2 < 2.220446049250313e-16)) return;
-  const int ci = li == 1 ? cart_of_sph_p(mi) : 0;
-  const int ncj = 2 * lj + 1;
-  // accumulators per bra cartesian component: S, M1[3], M2[6] about A
-  double aS[3] = {0, 0, 0}, aM1[3][3] = {{0}}, aM2[3][6] = {{0}};
+  // accumulators per ket and bra component: S, M1[3], M2[6] about A
+  double aS[NI][NJ] = {{0}}, aM1[NI][NJ][3] = {{{0}}}, aM2[NI][NJ][6] = {{{0}}};
   const int npi = m.sh_nprim[ish], npj = m.sh_nprim[jsh];
   const double pi3 = 5.568327996831708;  // pi^(3/2)
   for (int ip = 0; ip < npi; ++ip) {
@@ -142,24 +145,32 @@ __device__ __forceinline__ void build_h0_dev(DevMol m, Gfn2Scalars p, const doub
       for (int k = 0; k < 3; ++k) pa[k] = -vec[k] * aj * oeta;
       Moments M;
       gauss_moments(pa, eta, M);
-      for (int cj = 0; cj < ncj; ++cj) {
-        double V[3][3];  // [dir][e] = O(a+e, b)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const int a = cexp(li, ci, k), b = cexp(lj, cj, k);
+      for (int ii = 0; ii < NI; ++ii) {
+        const int ci = CI + ii;
 #pragma unroll
-          for (int e = 0; e < 3; ++e) V[k][e] = O1(M, k, a + e, b, vec[k]);
+        for (int cj = 0; cj < NJ; ++cj) {
+          double V[3][3];  // [dir][e] = O(a+e, b)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const int a = cexp(LI, ci, k), b = cexp(LJ, cj, k);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) V[k][e] = O1(M, k, a + e, b, vec[k]);
+          }
+          auto add = [&](double& acc, int ex, int ey, int ez) {
+            acc = fma(__dmul_rn(__dmul_rn(cc, V[0][ex]), V[1][ey]), V[2][ez], acc);
+          };
+          add(aS[ii][cj], 0, 0, 0);
+          add(aM1[ii][cj][0], 1, 0, 0);
+          add(aM1[ii][cj][1], 0, 1, 0);
+          add(aM1[ii][cj][2], 0, 0, 1);
+          add(aM2[ii][cj][0], 2, 0, 0);  // xx
+          add(aM2[ii][cj][1], 1, 1, 0);  // xy
+          add(aM2[ii][cj][2], 0, 2, 0);  // yy
+          add(aM2[ii][cj][3], 1, 0, 1);  // xz
+          add(aM2[ii][cj][4], 0, 1, 1);  // yz
+          add(aM2[ii][cj][5], 0, 0, 2);  // zz
         }
-        aS[cj] += cc * V[0][0] * V[1][0] * V[2][0];
-        aM1[cj][0] += cc * V[0][1] * V[1][0] * V[2][0];
-        aM1[cj][1] += cc * V[0][0] * V[1][1] * V[2][0];
-        aM1[cj][2] += cc * V[0][0] * V[1][0] * V[2][1];
-        aM2[cj][0] += cc * V[0][2] * V[1][0] * V[2][0];  // xx
-        aM2[cj][1] += cc * V[0][1] * V[1][1] * V[2][0];  // xy
-        aM2[cj][2] += cc * V[0][0] * V[1][2] * V[2][0];  // yy
-        aM2[cj][3] += cc * V[0][1] * V[1][0] * V[2][1];  // xz
-        aM2[cj][4] += cc * V[0][0] * V[1][1] * V[2][1];  // yz
-        aM2[cj][5] += cc * V[0][0] * V[1][0] * V[2][2];  // zz
       }
     }
   }
@@ -173,23 +184,27 @@ __device__ __forceinline__ void build_h0_dev(DevMol m, Gfn2Scalars p, const doub
   }
   const int n = m.nao;
   const size_t nn = (size_t)n * n;
-  const int io = m.sh_ao[ish] + mi, jo0 = m.sh_ao[jsh];
+  const int jo0 = m.sh_ao[jsh];
   const bool write_t = ish != jsh;
-  for (int cj = 0; cj < ncj; ++cj) {
-    const int mj = lj == 1 ? sph_of_cart_p(cj) : 0;
+#pragma unroll
+  for (int ii = 0; ii < NI; ++ii)
+#pragma unroll
+  for (int cj = 0; cj < NJ; ++cj) {
+    const int io = m.sh_ao[ish] + (LI == 1 ? sph_of_cart_p(CI + ii) : 0);
+    const int mj = LJ == 1 ? sph_of_cart_p(cj) : 0;
     const int jo = jo0 + mj;
-    const double s = aS[cj];
+    const double s = aS[ii][cj];
     double dA[3], dB[3], qA[6], qB[6];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      dA[k] = aM1[cj][k];
-      dB[k] = aM1[cj][k] + vec[k] * s;  // (r-B) = (r-A) + vec
+      dA[k] = aM1[ii][cj][k];
+      dB[k] = aM1[ii][cj][k] + vec[k] * s;  // (r-B) = (r-A) + vec
     }
     const int qa[6] = {0, 0, 1, 0, 1, 2}, qb[6] = {0, 1, 1, 2, 2, 2};
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      qA[q] = aM2[cj][q];
-      qB[q] = aM2[cj][q] + vec[qa[q]] * aM1[cj][qb[q]] + vec[qb[q]] * aM1[cj][qa[q]]
+      qA[q] = aM2[ii][cj][q];
+      qB[q] = aM2[ii][cj][q] + vec[qa[q]] * aM1[ii][cj][qb[q]] + vec[qb[q]] * aM1[ii][cj][qa[q]]
               + vec[qa[q]] * vec[qb[q]] * s;
     }
     // traceless
@@ -219,9 +234,48 @@ __device__ __forceinline__ void build_h0_dev(DevMol m, Gfn2Scalars p, const doub
     }
   }
 }
+// tasks of the H0 build: one thread per s-s and s-p pair, three per p-p pair (the three ket
+// components one kind after the other, so that the component is known at compile time)
+__host__ __device__ inline long long h0_tasks(long long nsh, long long np) {
+  return nsh * (nsh + 1) / 2 + np * (np + 1) + 5 * 32;
+}
+__device__ __forceinline__ void build_h0_dev(const DevMol& m, const Gfn2Scalars& p,
+                           const double* __restrict__ se, double* S, double* H, double* D,
+                           double* Q) {
+  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int ns = m.ns, np = m.nsh - m.ns;
+  const long long nss = (long long)ns * (ns + 1) / 2, nsp = (long long)ns * np;
+  if (t < pad32(nss)) {
+    if (t >= nss) return;
+    int i, j;
+    tri_index(t, i, j);
+    const int a = m.sh_perm[i], b = m.sh_perm[j];
+    build_h0_pair<0, 0, 1, 0>(m, p, se, S, H, D, Q, max(a, b), min(a, b));
+    return;
+  }
+  t -= pad32(nss);
+  if (t < pad32(nsp)) {
+    if (t >= nsp) return;
+    const int a = m.sh_perm[ns + (int)(t / ns)], b = m.sh_perm[(int)(t % ns)];  // p, s
+    if (a > b) build_h0_pair<1, 0, 3, 0>(m, p, se, S, H, D, Q, a, b);
+    else build_h0_pair<0, 1, 1, 0>(m, p, se, S, H, D, Q, b, a);
+    return;
+  }
+  t -= pad32(nsp);
+  const long long npp = (long long)np * (np + 1) / 2;
+  const int c = (int)(t / max(pad32(npp), 1ll));
+  t -= c * pad32(npp);
+  if (c > 2 || t >= npp) return;
+  int i, j;
+  tri_index(t, i, j);
+  const int x = m.sh_perm[ns + i], y = m.sh_perm[ns + j], a = max(x, y), b = min(x, y);
+  if (c == 0) build_h0_pair<1, 1, 1, 0>(m, p, se, S, H, D, Q, a, b);
+  else if (c == 1) build_h0_pair<1, 1, 1, 1>(m, p, se, S, H, D, Q, a, b);
+  else build_h0_pair<1, 1, 1, 2>(m, p, se, S, H, D, Q, a, b);
+}
 __global__ void k_build_h0(DevMol m, Gfn2Scalars p, const double* __restrict__ se, double* S,
-                           double* H, double* D, double* Q, long long npair) {
-  build_h0_dev(m, p, se, S, H, D, Q, npair);
+                           double* H, double* D, double* Q) {
+  build_h0_dev(m, p, se, S, H, D, Q);
 }
 
 void launch_build_h0(const DevMol& m, const Gfn2Scalars& p, const double* se, double* S,
@@ -231,11 +285,10 @@ void launch_build_h0(const DevMol& m, const Gfn2Scalars& p, const double* se, do
   cudaMemsetAsync(H, 0, nn * sizeof(double), s);
   cudaMemsetAsync(D, 0, 3 * nn * sizeof(double), s);
   cudaMemsetAsync(Q, 0, 6 * nn * sizeof(double), s);
-  const long long npair = (long long)m.nsh * (m.nsh + 1) / 2;
-  const long long nthr = npair * 3;
+  const long long nthr = h0_tasks(m.nsh, m.nsh - m.ns);
   const int bs = 128;
   ++g_kernel_launches;
-  k_build_h0<<<(unsigned)((nthr + bs - 1) / bs), bs, 0, s>>>(m, p, se, S, H, D, Q, npair);
+  k_build_h0<<<(unsigned)((nthr + bs - 1) / bs), bs, 0, s>>>(m, p, se, S, H, D, Q);
 }
 
 // One primitive pair of the H0 gradient for shells of angular momenta LI (bra, A) and LJ
@@ -312,28 +365,23 @@ __device__ __forceinline__ void h0g_prim(const Moments& M, const double (&vec)[3
 }
 
 // ---------------------------------------------------------------------------------------
-// H0 gradient: one thread per cross-atom shell pair (ish > jsh).  The reference formula
+// H0 gradient: one thread per cross-atom shell pair, by kind (of an s-p pair the p shell is ish).
+// The reference formula
 // (h0.f90:528-560) is contracted on the fly:
 //   dG = sum_ji [ sval dS + 2 P hij S dsv - P d<j|O|i>/dR_A ] ,
 //   sval = -P (v_j + v_i) + 2 P hij - 2 W,
 // where O is the multipole potential operator of atoms A and B written as a polynomial in
 // (r - A).  The operator on A moves with A, which adds  P (vA_c S + sum_b (1+d_cb) wA_cb D_b).
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void h0_gradient_dev(DevMol m, Gfn2Scalars p, const double* __restrict__ se,
+template <int LI, int LJ>
+__device__ __forceinline__ void h0_gradient_pair(const DevMol& m, const Gfn2Scalars& p,
+                              const double* __restrict__ se,
                               const double* __restrict__ P, const double* __restrict__ W,
                               const double* __restrict__ vao, const double* __restrict__ vdp,
-                              const double* __restrict__ vqp, double* grad, double* sigma,
-                              double* dEdcn, long long npair) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  // every thread reaches the warp-wide virial sum at the end: pairs that contribute nothing
-  // (outside the list, on one atom, beyond the cutoff) skip the work, not the sum
-  double vec[3] = {0.0, 0.0, 0.0}, dG[3] = {0.0, 0.0, 0.0};
-  do {
-  if (t >= npair) break;
-  int ish, jsh;
-  tri_index(t, ish, jsh);
+                              const double* __restrict__ vqp, double* grad,
+                              double* dEdcn, int ish, int jsh, double (&vec)[3], double (&dG)[3]) {
   const int iat = m.sh_atom[ish], jat = m.sh_atom[jsh];
-  if (iat == jat) break;
+  if (iat == jat) return;
   double r2 = 0.0;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -342,15 +390,15 @@ __device__ __forceinline__ void h0_gradient_dev(DevMol m, Gfn2Scalars p, const d
   }
   if (r2 > p.h0_cutoff * p.h0_cutoff || r2 < 2.220446049250313e-16) {
     vec[0] = vec[1] = vec[2] = 0.0;
-    break;
+    return;
   }
-  const int li = m.sh_l[ish], lj = m.sh_l[jsh];
-  const int nci = 2 * li + 1, ncj = 2 * lj + 1;
+  constexpr int nci = 2 * LI + 1, ncj = 2 * LJ + 1;
   const double rr = sqrt(sqrt(r2) / (m.at_rad[iat] + m.at_rad[jat]));
   const double polyi = 1.0 + m.sh_shpoly[ish] * rr, polyj = 1.0 + m.sh_shpoly[jsh] * rr;
   const double poly = polyi * polyj;
   const double dpoly = (polyi * m.sh_shpoly[jsh] + polyj * m.sh_shpoly[ish]) * 0.5 * rr / r2;
-  const double hs = hscale_of(m, p, ish, jsh, iat, jat) * poly;
+  const double hs = (ish > jsh ? hscale_of(m, p, ish, jsh, iat, jat)
+                               : hscale_of(m, p, jsh, ish, jat, iat)) * poly;
   const double hij = 0.5 * (se[ish] + se[jsh]) * hs;
   // potential operator coefficients in (r-A) monomials
   double vA[3], vB[3], wA[6], wB[6];
@@ -388,10 +436,12 @@ __device__ __forceinline__ void h0_gradient_dev(DevMol m, Gfn2Scalars p, const d
   const int n = m.nao;
   const int io0 = m.sh_ao[ish], jo0 = m.sh_ao[jsh];
   double ws[3][3], wp[3][3];
+#pragma unroll
   for (int cj = 0; cj < ncj; ++cj) {
-    const int ja = jo0 + (lj == 1 ? sph_of_cart_p(cj) : 0);
+    const int ja = jo0 + (LJ == 1 ? sph_of_cart_p(cj) : 0);
+#pragma unroll
     for (int ci = 0; ci < nci; ++ci) {
-      const int ia = io0 + (li == 1 ? sph_of_cart_p(ci) : 0);
+      const int ia = io0 + (LI == 1 ? sph_of_cart_p(ci) : 0);
       const double pij = P[(size_t)ja * n + ia];
       const double wij = W[(size_t)ja * n + ia];
       wp[cj][ci] = pij;
@@ -415,20 +465,7 @@ __device__ __forceinline__ void h0_gradient_dev(DevMol m, Gfn2Scalars p, const d
       for (int k = 0; k < 3; ++k) pa[k] = -vec[k] * aj * oeta;
       Moments M;
       gauss_moments(pa, eta, M);
-      switch (2 * li + lj) {  // shell kinds as template arguments: the 1-d factors of all
-        case 0:               // angular components are shared by the compiler
-          h0g_prim<0, 0>(M, vec, ai, cc, wp, ws, c0, c1, c2, dG, PS, PD);
-          break;
-        case 1:
-          h0g_prim<0, 1>(M, vec, ai, cc, wp, ws, c0, c1, c2, dG, PS, PD);
-          break;
-        case 2:
-          h0g_prim<1, 0>(M, vec, ai, cc, wp, ws, c0, c1, c2, dG, PS, PD);
-          break;
-        default:
-          h0g_prim<1, 1>(M, vec, ai, cc, wp, ws, c0, c1, c2, dG, PS, PD);
-          break;
-      }
+      h0g_prim<LI, LJ>(M, vec, ai, cc, wp, ws, c0, c1, c2, dG, PS, PD);
     }
   }
   // operator on A moves with A;  symmetric quadrupole weight matrix of atom A
@@ -449,7 +486,39 @@ __device__ __forceinline__ void h0_gradient_dev(DevMol m, Gfn2Scalars p, const d
     atomicAdd(grad + 3 * iat + c, dG[c]);
     atomicAdd(grad + 3 * jat + c, -dG[c]);
   }
-  } while (false);
+}
+__device__ __forceinline__ void h0_gradient_dev(const DevMol& m, const Gfn2Scalars& p,
+                              const double* __restrict__ se,
+                              const double* __restrict__ P, const double* __restrict__ W,
+                              const double* __restrict__ vao, const double* __restrict__ vdp,
+                              const double* __restrict__ vqp, double* grad, double* sigma,
+                              double* dEdcn) {
+  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int ns = m.ns, np = m.nsh - m.ns;
+  const long long nss = (long long)ns * (ns + 1) / 2, nsp = (long long)ns * np;
+  // every thread reaches the warp-wide virial sum at the end: pairs that contribute nothing
+  // (outside the list, on one atom, beyond the cutoff) skip the work, not the sum
+  double vec[3] = {0.0, 0.0, 0.0}, dG[3] = {0.0, 0.0, 0.0};
+  int i, j;
+  if (t < pad32(nss)) {
+    if (t < nss) {
+      tri_index(t, i, j);
+      h0_gradient_pair<0, 0>(m, p, se, P, W, vao, vdp, vqp, grad, dEdcn, m.sh_perm[i],
+                             m.sh_perm[j], vec, dG);
+    }
+  } else if (t < pad32(nss) + pad32(nsp)) {
+    t -= pad32(nss);
+    if (t < nsp)
+      h0_gradient_pair<1, 0>(m, p, se, P, W, vao, vdp, vqp, grad, dEdcn,
+                             m.sh_perm[ns + (int)(t / ns)], m.sh_perm[(int)(t % ns)], vec, dG);
+  } else {
+    t -= pad32(nss) + pad32(nsp);
+    if (t < (long long)np * (np + 1) / 2) {
+      tri_index(t, i, j);
+      h0_gradient_pair<1, 1>(m, p, se, P, W, vao, vdp, vqp, grad, dEdcn, m.sh_perm[ns + i],
+                             m.sh_perm[ns + j], vec, dG);
+    }
+  }
   // virial: the six distinct elements of the symmetric 3 x 3 summed over the warp, then one
   // atomic per element and warp (every pair of a molecule adds to the same nine numbers)
   const int va[6] = {0, 0, 1, 0, 1, 2}, vb[6] = {0, 1, 1, 2, 2, 2};
@@ -468,8 +537,8 @@ __global__ void k_h0_gradient(DevMol m, Gfn2Scalars p, const double* __restrict_
                               const double* __restrict__ P, const double* __restrict__ W,
                               const double* __restrict__ vao, const double* __restrict__ vdp,
                               const double* __restrict__ vqp, double* grad, double* sigma,
-                              double* dEdcn, long long npair) {
-  h0_gradient_dev(m, p, se, P, W, vao, vdp, vqp, grad, sigma, dEdcn, npair);
+                              double* dEdcn) {
+  h0_gradient_dev(m, p, se, P, W, vao, vdp, vqp, grad, sigma, dEdcn);
 }
 
 // on-site CN derivative of the diagonal levels: dEdcn_A += sum_{mu in A} dse/dcn P_mumu
@@ -491,11 +560,11 @@ __global__ void k_h0_onsite_dcn(DevMol m, const double* __restrict__ P, double* 
 void launch_h0_gradient(const DevMol& m, const Gfn2Scalars& p, const double* se, const double* P,
                         const double* W, const double* vao, const double* vdp, const double* vqp,
                         double* grad, double* sigma, double* dEdcn, cudaStream_t s) {
-  const long long npair = (long long)m.nsh * (m.nsh + 1) / 2;
+  const long long npair = (long long)m.nsh * (m.nsh + 1) / 2 + 64;
   const int bs = 128;
   ++g_kernel_launches;
   k_h0_gradient<<<(unsigned)((npair + bs - 1) / bs), bs, 0, s>>>(m, p, se, P, W, vao, vdp, vqp,
-                                                                   grad, sigma, dEdcn, npair);
+                                                                   grad, sigma, dEdcn);
   ++g_kernel_launches;
   k_h0_onsite_dcn<<<(m.nat + 127) / 128, 128, 0, s>>>(m, P, dEdcn);
 }
@@ -513,16 +582,15 @@ void launch_h0_gradient(const DevMol& m, const Gfn2Scalars& p, const double* se,
 // d ln hscale / d zeta_i = wexp (1/(2 zeta_i) - 1/(zeta_i + zeta_j)) off-site.  The same form
 // holds for on-site pairs (no H0 scaling there) and for i == j (bra and ket derivatives equal).
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void zeta_grad_dev(const DevMol& m, const Gfn2Scalars& p,
+template <int LI, int LJ>
+__device__ __forceinline__ void zeta_grad_pair(const DevMol& m, const Gfn2Scalars& p,
                                               const double* __restrict__ se,
                                               const double* __restrict__ P,
                                               const double* __restrict__ W,
                                               const double* __restrict__ vao,
                                               const double* __restrict__ vdp,
                                               const double* __restrict__ vqp, double* dz,
-                                              long long t) {
-  if (t >= (long long)m.nsh * m.nsh) return;
-  const int ish = (int)(t / m.nsh), jsh = (int)(t % m.nsh);
+                                              int ish, int jsh) {
   const int iat = m.sh_atom[ish], jat = m.sh_atom[jsh];
   double vec[3];
   double r2 = 0.0;
@@ -533,8 +601,7 @@ __device__ __forceinline__ void zeta_grad_dev(const DevMol& m, const Gfn2Scalars
   }
   const bool onsite = iat == jat;
   if (!onsite && (r2 > p.h0_cutoff * p.h0_cutoff || r2 < 2.220446049250313e-16)) return;
-  const int li = m.sh_l[ish], lj = m.sh_l[jsh];
-  const int nci = 2 * li + 1, ncj = 2 * lj + 1;
+  constexpr int nci = 2 * LI + 1, ncj = 2 * LJ + 1;
   double hij, dhij = 0.0;
   if (onsite) {
     hij = 0.5 * (se[ish] + se[jsh]);
@@ -576,16 +643,18 @@ __device__ __forceinline__ void zeta_grad_dev(const DevMol& m, const Gfn2Scalars
   const int n = m.nao;
   const int io0 = m.sh_ao[ish], jo0 = m.sh_ao[jsh];
   double ws[3][3], wp[3][3];
+#pragma unroll
   for (int cj = 0; cj < ncj; ++cj) {
-    const int ja = jo0 + (lj == 1 ? sph_of_cart_p(cj) : 0);
+    const int ja = jo0 + (LJ == 1 ? sph_of_cart_p(cj) : 0);
+#pragma unroll
     for (int ci = 0; ci < nci; ++ci) {
-      const int ia = io0 + (li == 1 ? sph_of_cart_p(ci) : 0);
+      const int ia = io0 + (LI == 1 ? sph_of_cart_p(ci) : 0);
       const double pij = P[(size_t)ja * n + ia];
       wp[cj][ci] = pij;
       ws[cj][ci] = -pij * (vao[ja] + vao[ia]) + 2.0 * pij * hij - 2.0 * W[(size_t)ja * n + ia];
     }
   }
-  const double gl = 0.75 + 0.5 * li;
+  constexpr double gl = 0.75 + 0.5 * LI;
   double accd = 0.0, accs = 0.0;
   const int npi = m.sh_nprim[ish], npj = m.sh_nprim[jsh];
   const double pi3 = 5.568327996831708;
@@ -603,12 +672,14 @@ __device__ __forceinline__ void zeta_grad_dev(const DevMol& m, const Gfn2Scalars
       for (int k = 0; k < 3; ++k) pa[k] = -vec[k] * aj * oeta;
       Moments M;
       gauss_moments(pa, eta, M);
+#pragma unroll
       for (int cj = 0; cj < ncj; ++cj) {
+#pragma unroll
         for (int ci = 0; ci < nci; ++ci) {
           double V[3][5];  // (x-A)^(a+e) (x-B)^b, e = 0..4
 #pragma unroll
           for (int k = 0; k < 3; ++k) {
-            const int a = cexp(li, ci, k), b = cexp(lj, cj, k);
+            const int a = cexp(LI, ci, k), b = cexp(LJ, cj, k);
 #pragma unroll
             for (int e = 0; e < 5; ++e) V[k][e] = O1(M, k, a + e, b, vec[k]);
           }
@@ -633,6 +704,38 @@ __device__ __forceinline__ void zeta_grad_dev(const DevMol& m, const Gfn2Scalars
   const double val = 2.0 / m.sh_zeta[ish] * accd + 2.0 * dhij * accs;
   atomicAdd(dz + ish, val);
 }
+// ordered pairs by kind: s-s, s-p, p-s, p-p
+__device__ __forceinline__ void zeta_grad_dev(const DevMol& m, const Gfn2Scalars& p,
+                                              const double* __restrict__ se,
+                                              const double* __restrict__ P,
+                                              const double* __restrict__ W,
+                                              const double* __restrict__ vao,
+                                              const double* __restrict__ vdp,
+                                              const double* __restrict__ vqp, double* dz,
+                                              long long t) {
+  const int ns = m.ns, np = m.nsh - m.ns;
+  const long long nss = (long long)ns * ns, nsp = (long long)ns * np;
+  const int* __restrict__ sp = m.sh_perm;
+  const int* __restrict__ pp = m.sh_perm + ns;
+  if (t < pad32(nss)) {
+    if (t < nss)
+      zeta_grad_pair<0, 0>(m, p, se, P, W, vao, vdp, vqp, dz, sp[t / ns], sp[t % ns]);
+    return;
+  }
+  t -= pad32(nss);
+  if (t < pad32(nsp)) {
+    if (t < nsp) zeta_grad_pair<0, 1>(m, p, se, P, W, vao, vdp, vqp, dz, sp[t / np], pp[t % np]);
+    return;
+  }
+  t -= pad32(nsp);
+  if (t < pad32(nsp)) {
+    if (t < nsp) zeta_grad_pair<1, 0>(m, p, se, P, W, vao, vdp, vqp, dz, pp[t / ns], sp[t % ns]);
+    return;
+  }
+  t -= pad32(nsp);
+  if (t < (long long)np * np)
+    zeta_grad_pair<1, 1>(m, p, se, P, W, vao, vdp, vqp, dz, pp[t / np], pp[t % np]);
+}
 __global__ void k_zeta_grad(DevMol m, Gfn2Scalars p, const double* __restrict__ se,
                             const double* __restrict__ P, const double* __restrict__ W,
                             const double* __restrict__ vao, const double* __restrict__ vdp,
@@ -645,7 +748,7 @@ void launch_zeta_grad(const DevMol& m, const Gfn2Scalars& p, const double* se, c
                       const double* W, const double* vao, const double* vdp, const double* vqp,
                       double* dz, cudaStream_t s) {
   cudaMemsetAsync(dz, 0, sizeof(double) * m.nsh, s);
-  const long long np = (long long)m.nsh * m.nsh;
+  const long long np = (long long)m.nsh * m.nsh + 96;
   ++g_kernel_launches;
   k_zeta_grad<<<(unsigned)((np + 127) / 128), 128, 0, s>>>(m, p, se, P, W, vao, vdp, vqp, dz);
 }
@@ -654,13 +757,12 @@ void launch_zeta_grad(const DevMol& m, const Gfn2Scalars& p, const double* se, c
 __global__ void kb_build_h0(const MolPtrs* __restrict__ mp, const int* __restrict__ list,
                             Gfn2Scalars p) {
   const MolPtrs& q = mp[list[blockIdx.z]];
-  const long long npair = (long long)q.m.nsh * (q.m.nsh + 1) / 2;
   p.h0_cutoff = q.h0_cutoff;
-  build_h0_dev(q.m, p, q.se, q.S, q.H, q.D, q.Q, npair);
+  build_h0_dev(q.m, p, q.se, q.S, q.H, q.D, q.Q);
 }
 void launch_build_h0_b(const BatchLaunch& b, const Gfn2Scalars& p) {
   if (!b.count) return;
-  const long long nthr = (long long)b.nsh_max * (b.nsh_max + 1) / 2 * 3;
+  const long long nthr = h0_tasks(b.nsh_max, b.np_max);
   ++g_kernel_launches;
   kb_build_h0<<<dim3((unsigned)((nthr + 127) / 128), 1, b.count), 128, 0, b.s>>>(b.mp, b.list, p);
 }
@@ -669,9 +771,8 @@ void launch_build_h0_b(const BatchLaunch& b, const Gfn2Scalars& p) {
 __global__ void kb_h0_gradient(const MolPtrs* __restrict__ mp, const int* __restrict__ list,
                                Gfn2Scalars p) {
   const MolPtrs& q = mp[list[blockIdx.z]];
-  const long long npair = (long long)q.m.nsh * (q.m.nsh + 1) / 2;
   p.h0_cutoff = q.h0_cutoff;
-  h0_gradient_dev(q.m, p, q.se, q.P, q.F, q.vao, q.vdp, q.vqp, q.grad, q.sigma, q.dEdcn, npair);
+  h0_gradient_dev(q.m, p, q.se, q.P, q.F, q.vao, q.vdp, q.vqp, q.grad, q.sigma, q.dEdcn);
 }
 __global__ void kb_h0_onsite_dcn(const MolPtrs* __restrict__ mp, const int* __restrict__ list) {
   const MolPtrs& q = mp[list[blockIdx.z]];
@@ -688,14 +789,14 @@ __global__ void kb_zeta_grad(const MolPtrs* __restrict__ mp, const int* __restri
 }
 void launch_zeta_grad_b(const BatchLaunch& b, const Gfn2Scalars& p) {
   if (!b.count) return;
-  const long long np = (long long)b.nsh_max * b.nsh_max;
+  const long long np = (long long)b.nsh_max * b.nsh_max + 96;
   ++g_kernel_launches;
   kb_zeta_grad<<<dim3((unsigned)((np + 127) / 128), 1, b.count), 128, 0, b.s>>>(b.mp, b.list, p);
 }
 
 void launch_h0_gradient_b(const BatchLaunch& b, const Gfn2Scalars& p) {
   if (!b.count) return;
-  const long long npair = (long long)b.nsh_max * (b.nsh_max + 1) / 2;
+  const long long npair = (long long)b.nsh_max * (b.nsh_max + 1) / 2 + 64;
   ++g_kernel_launches;
   kb_h0_gradient<<<dim3((unsigned)((npair + 127) / 128), 1, b.count), 128, 0, b.s>>>(b.mp, b.list,
                                                                                      p);
