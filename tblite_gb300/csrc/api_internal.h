@@ -120,7 +120,22 @@ struct Workspace {
       d4_atm;
   EigenSolver* eig = nullptr;
   Purifier* pur = nullptr;
+  // mapped host memory for what an SCF iteration reports (grow-only)
+  double* host = nullptr;
+  size_t host_n = 0;
+  double* host_words(size_t count) {
+    if (count > host_n) {
+      if (host) cudaFreeHost(host);
+      host = nullptr;
+      host_n = 0;
+      cuda_check(cudaHostAlloc((void**)&host, sizeof(double) * count, cudaHostAllocMapped),
+                 "cudaHostAlloc");
+      host_n = count;
+    }
+    return host;
+  }
   ~Workspace() {
+    if (host) cudaFreeHost(host);
     if (eig) eigen_destroy(eig);
     if (pur) purify_destroy(pur);
     if (stream) cudaStreamDestroy(stream);

@@ -965,7 +965,29 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   std::vector<int> h_cnt(2);
   // eigenvalues per iteration: the occupied levels and a margin (the rest once converged)
   int nev = scf_eigenvalue_count(n, std::max(nalp, nbet));
+  int nvec = 0;  // eigenvectors computed
   double kt = target_kt;
+  // one wait per iteration: what the host reads comes through mapped host memory in one kernel
+  int h_status = 0;
+  cuda_check(cudaMemsetAsync(w.b_status.p, 0, sizeof(int), s), "status");
+  auto collect = [&]() {
+    double* h = w.host_words(nat + 5);
+    launch_collect(nat, w.eelec.p, w.scal.p, w.icount.p, w.b_status.p, h, s);
+    stream_wait(s);
+    std::copy(h, h + nat, h_eelec.begin());
+    h_scal.assign(h + nat, h + nat + 2);
+    h_cnt[0] = (int)h[nat + 2];
+    h_cnt[1] = (int)h[nat + 3];
+    h_status = (int)h[nat + 4];
+  };
+  // the Fermi level needs more levels than were computed: all of them from now on
+  auto more_levels = [&]() { return h_cnt[1] != 0; };
+  auto fill_more_levels = [&]() {
+    eigen_values_rest(w.eig, nev, w.emo.p);
+    nev = n;
+    launch_fermi(n, w.emo.p, nalp, nbet, kt, w.focc.p, w.scal.p, w.icount.p, s, nev);
+    collect();
+  };
   while (!converged && iscf < c->max_iter) {
     const double elast = eelec_sum;
     if (elevated_kt > target_kt) {  // singlepoint.f90:286-296
@@ -977,10 +999,6 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
     if (iscf > 0) {
       g_prof.begin(PH_MIXER, s);
       launch_broyden_next(b, s);
-      int st = 0;
-      cuda_check(cudaMemcpyAsync(&st, w.b_status.p, sizeof(int), cudaMemcpyDeviceToHost, s), "st");
-      stream_wait(s);
-      if (st != 0) throw std::runtime_error("Broyden mixing failed to obtain next iteration");
       launch_unpack(m, w.b_q.p, w.qsh.p, w.qat.p, w.dpat.p, w.qpat.p, s, with_mp);
       g_prof.end(s);
     }
@@ -1013,22 +1031,22 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
         throw std::runtime_error("(sygvd) failed to solve eigenvalue problem. info=" +
                                  std::to_string(info));
       launch_fermi(n, w.emo.p, nalp, nbet, kt, w.focc.p, w.scal.p, w.icount.p, s, nev);
-      w.icount.download(h_cnt, 2, s);
-      stream_wait(s);
-      if (h_cnt[1] != 0) {  // the Fermi level needs more levels: all of them from now on
-        eigen_values_rest(w.eig, nev, w.emo.p);
-        nev = n;
-        launch_fermi(n, w.emo.p, nalp, nbet, kt, w.focc.p, w.scal.p, w.icount.p, s, nev);
-        w.icount.download(h_cnt, 2, s);
-        stream_wait(s);
+      if (n > TRIDIAG_FIXED_MAX) {  // vectors of the occupied levels only
+        collect();
+        if (more_levels()) fill_more_levels();
+        nvec = h_cnt[0];
+      } else {
+        // every computed level: the empty ones among them carry zero occupations, so the host
+        // need not know the count before it launches the rest of the iteration
+        nvec = nev;
       }
-      eigen_vectors(w.eig, h_cnt[0], w.C.p);
+      eigen_vectors(w.eig, nvec, w.C.p);
       g_prof.end(s);
       g_prof.begin(PH_DENSITY, s);
-      density_matrix(n, h_cnt[0], w.C.p, w.focc.p, w.P.p, w.scratch.p, s,
-                     eigen_gemm_status(w.eig));
+      density_matrix(n, nvec, w.C.p, w.focc.p, w.P.p, w.scratch.p, s, eigen_gemm_status(w.eig));
       g_prof.end(s);
     }
+    auto analyse = [&]() {
     g_prof.begin(PH_MULLIKEN, s);
     launch_mulliken(m, w.P.p, w.S.p, w.H.p, w.D.p, w.Q.p, w.mull.p, mulliken_chunks(n), w.qsh_o.p,
                     w.qat_o.p, w.dpat_o.p, w.qpat_o.p, w.eband.p, s);
@@ -1042,9 +1060,19 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
     if (c->has_field)
       launch_field_energy(nat, w.xyz.p, c->efield, w.qat_o.p, w.dpat_o.p, w.eelec.p, s);
     g_prof.end(s);
-    w.eelec.download(h_eelec, nat, s);
-    w.scal.download(h_scal, 2, s);
-    stream_wait(s);
+    collect();
+    };
+    analyse();
+    // the Broyden step that began this iteration (its status came with the rest)
+    if (iscf > 1 && h_status != 0)
+      throw std::runtime_error("Broyden mixing failed to obtain next iteration");
+    if (!purify && n <= TRIDIAG_FIXED_MAX && more_levels()) {  // the density again, all levels
+      fill_more_levels();
+      nvec = n;
+      eigen_vectors(w.eig, nvec, w.C.p);
+      density_matrix(n, nvec, w.C.p, w.focc.p, w.P.p, w.scratch.p, s, eigen_gemm_status(w.eig));
+      analyse();
+    }
     eelec_sum = 0.0;
     for (int i = 0; i < nat; ++i) eelec_sum += h_eelec[i];
     const bool econv_ok = fabs(eelec_sum - elast) < econv;
@@ -1115,7 +1143,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   if (!purify) {  // the projection has no orbitals
     g_prof.begin(PH_EIGEN, s);
     eigen_values_rest(w.eig, nev, w.emo.p);
-    eigen_vectors_range(w.eig, h_cnt[0], (int)n, w.C.p);
+    eigen_vectors_range(w.eig, nvec, (int)n, w.C.p);
     g_prof.end(s);
   }
   // Wiberg/Mayer bond orders (post_processing/wbo.f90:60-115): closed shell from P; restricted

@@ -329,6 +329,10 @@ enum { KM_NONE = 0, KM_LT_COLEND = 1, KM_LT_ROWEND = 2, KM_GE_ROWBEG = 3, KM_SYM
 cudaError_t gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const double* A, int lda,
             const double* B, int ldb, double beta, double* C, int ldc, int kmode, cudaStream_t s);
 
+// what the host reads of an SCF iteration, into mapped host memory out[nat + 5]: atomic energies,
+// scal[0..1], icount[0..1], Broyden status
+void launch_collect(int nat, const double* eelec, const double* scal, const int* icount,
+                    const int* status, double* out, cudaStream_t s);
 // eelec[i] = ts/nat + eband[i]
 void launch_eelec_init(int nat, const double* ts, const double* eband, double* eelec,
                        cudaStream_t s);

@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <chrono>
 
 #include "engine.h"
 
@@ -30,6 +31,15 @@ void stream_wait(cudaStream_t s) {
   thread_local cudaEvent_t ev = nullptr;
   if (!ev) cudaEventCreateWithFlags(&ev, cudaEventBlockingSync | cudaEventDisableTiming);
   cudaEventRecord(ev, s);
+  // a short wait is polled (waking a sleeping thread takes tens of microseconds, which every SCF
+  // iteration of a small molecule would pay), a longer one sleeps
+  if (cudaPeekAtLastError() == cudaSuccess) {  // (an error waiting to be read is left as it is)
+    const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(400);
+    do {
+      if (cudaEventQuery(ev) != cudaErrorNotReady) return;
+      cudaGetLastError();  // "not ready" counts as the last error
+    } while (std::chrono::steady_clock::now() < until);
+  }
   cudaEventSynchronize(ev);
 }
 
@@ -1175,6 +1185,20 @@ __device__ __forceinline__ void eelec_init_dev(int nat, const double* ts, const 
 }
 __global__ void k_eelec_init(int nat, const double* ts, const double* eband, double* eelec) {
   eelec_init_dev(nat, ts, eband, eelec);
+}
+
+__global__ void k_collect(int nat, const double* eelec, const double* scal, const int* icount,
+                          const int* status, double* out) {
+  for (int t = threadIdx.x; t < nat + 5; t += blockDim.x)
+    out[t] = t < nat       ? eelec[t]
+             : t < nat + 2 ? scal[t - nat]
+             : t < nat + 4 ? (double)icount[t - nat - 2]
+                           : (double)*status;
+}
+void launch_collect(int nat, const double* eelec, const double* scal, const int* icount,
+                    const int* status, double* out, cudaStream_t s) {
+  ++g_kernel_launches;
+  k_collect<<<1, one_block(nat + 5), 0, s>>>(nat, eelec, scal, icount, status, out);
 }
 
 void launch_eelec_init(int nat, const double* ts, const double* eband, double* eelec,
