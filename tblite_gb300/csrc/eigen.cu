@@ -1307,6 +1307,12 @@ int eigen_set_overlap(EigenSolver* e, const double* S) {
   const int n = e->n;
   // a new geometry: the tensor-core status word starts clear
   ck(cudaMemsetAsync(e->gstatus, 0, sizeof(int), e->stream), "gstatus");
+  if (cholinv_fixed(n, S, e->X, e->status, e->stream)) {
+    ck(cudaMemcpyAsync(e->hstatus, e->status, sizeof(int), cudaMemcpyDeviceToHost, e->stream),
+       "Cholesky status");
+    stream_wait(e->stream);
+    if (*e->hstatus == 0) return 0;  // else outside the fixed-point range: in FP64
+  }
   ck(cudaMemcpyAsync(e->L, S, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, e->stream),
      "copy S");
   return cholesky_inverse(n, e->L, e->X, e->status, e->hstatus, e->stream);

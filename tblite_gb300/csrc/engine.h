@@ -266,6 +266,9 @@ void tridiag_fixed(int n, double* A, double* d, double* e, double* tau, long lon
                    cudaStream_t s);
 size_t tridiag_exchange_words(int n);
 // factorise S once per geometry; returns 0 on success, >0 if S is not positive definite
+// X = L^-T of S = L L^T in fixed point (cholinv.cu), n up to TRIDIAG_FIXED_MAX; false: not launched.
+// *status (device) 0: done, 1: outside the fixed-point range, X not written
+bool cholinv_fixed(int n, const double* S, double* X, int* status, cudaStream_t s);
 int eigen_set_overlap(EigenSolver*, const double* S);
 // eigenvalues (ascending) of F C = S C e; keeps the tridiagonal form for eigen_vectors.
 // Only the nev lowest are computed (nev <= 0: all); e[nev..n) = 1e300, which the Fermi
@@ -531,6 +534,7 @@ void pipe_x_images_b(const BatchLaunch& b);
 void ogemm_b(const BatchLaunch& b, int site);
 extern bool g_split_gemm;
 // eigensolver steps for a bucket
+bool cholinv_fixed_b(const BatchLaunch& b);  // the same for the batch (status into estatus)
 void cholesky_inverse_b(const BatchLaunch& b);          // S -> X (status into flag)
 void tridiag_fixed_b(const BatchLaunch& b);             // A -> ed, ee, etau (tridiag.cu)
 void eigen_values_b(const BatchLaunch& b);              // F -> emo (tridiagonal form kept)

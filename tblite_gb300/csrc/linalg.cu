@@ -407,8 +407,9 @@ void gemm_b(const BatchLaunch& b, int site) {
 // update runs on the FP64 pipe instead of waiting on L2.  A pivot that is not positive marks
 // the molecule failed (flag -2); it is read after a barrier, so the whole block leaves together.
 constexpr int CHOL_NB = 16;
-__global__ void __launch_bounds__(256) kb_cholesky(BARGS) {
+__global__ void __launch_bounds__(256) kb_cholesky(BARGS, int rest) {
   BMOL;
+  if (rest && *q.estatus == 0) return;  // done in fixed point
   const int n = q.m.nao;
   double* A = q.T1;
   extern __shared__ double pan[];  // [CHOL_NB][m] panel, column-major (m = n - j0 rows)
@@ -510,8 +511,9 @@ __device__ __forceinline__ void tri_col_load(const double* __restrict__ L, int n
     v[t] = (k > i && k <= j) ? L[k + (size_t)i * n] : 0.0;
   }
 }
-__global__ void kb_tri_inv_t(BARGS) {
+__global__ void kb_tri_inv_t(BARGS, int rest) {
   BMOL;
+  if (rest && *q.estatus == 0) return;
   if (*q.flag < 0) return;
   const int n = q.m.nao;
   if (n > 32 * TRI_INV_R) {
@@ -571,6 +573,8 @@ __global__ void kb_tri_inv_t(BARGS) {
 
 void cholesky_inverse_b(const BatchLaunch& b) {
   if (!b.count) return;
+  // fixed point first (cholinv.cu); what leaves its range, or does not fit, follows in FP64
+  const int rest = cholinv_fixed_b(b) ? 1 : 0;
   g_kernel_launches += 2;
   const size_t smem = (size_t)CHOL_NB * b.nao_max * sizeof(double);
   static size_t attr = 0;  // the kernel's static shared memory comes on top of smem
@@ -582,8 +586,9 @@ void cholesky_inverse_b(const BatchLaunch& b) {
                                "' in batched Cholesky shared memory");
     attr = smem;
   }
-  kb_cholesky<<<dim3(1, 1, b.count), 256, smem, b.s>>>(b.mp, b.list);
-  kb_tri_inv_t<<<dim3((b.nao_max * 32 + 255) / 256, 1, b.count), 256, 0, b.s>>>(b.mp, b.list);
+  kb_cholesky<<<dim3(1, 1, b.count), 256, smem, b.s>>>(b.mp, b.list, rest);
+  kb_tri_inv_t<<<dim3((b.nao_max * 32 + 255) / 256, 1, b.count), 256, 0, b.s>>>(b.mp, b.list,
+                                                                               rest);
 }
 
 #undef BMOL
