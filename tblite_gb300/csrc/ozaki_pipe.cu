@@ -49,6 +49,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 #include "engine.h"
 
@@ -63,14 +64,9 @@ struct Balanced {
   static constexpr int EXACT = 5;   // levels 0 .. EXACT - 1 are drained as exact integers
   static constexpr int FLUSH = 6;   // k chunks per window
   static constexpr int BITS = 8;    // of a digit
-  // the MMAs of a k step from slice 1 on, four bits each, the first one lowest: A slice p, first B
-  // slice q, number of B slices
-  static constexpr int GROUPS = 8;
-  static constexpr uint64_t GP = 0x65432211, GQ = 0x00004040, GN = 0x12341424;
 };
 struct Magnitude {
-  static constexpr int SLICES = 8, LEVELS = 8, EXACT = 6, FLUSH = 5, BITS = 7, GROUPS = 10;
-  static constexpr uint64_t GP = 0x7654332211, GQ = 0x0000404040, GN = 0x1234142434;
+  static constexpr int SLICES = 8, LEVELS = 8, EXACT = 6, FLUSH = 5, BITS = 7;
 };
 // |int64 level sums| < 1.01 * 2^46 K (Balanced), 1.02 * 2^49 K (Magnitude): below 2^63
 constexpr int PP_KMAX = 12288;
@@ -84,6 +80,7 @@ constexpr int PP_STAGE_BYTES = PP_A_BYTES<Sch> + PP_B_BYTES<Sch>;
 template <class Sch>
 constexpr int PP_SMEM = PP_STAGES * PP_STAGE_BYTES<Sch> + 1024;
 constexpr int PP_TMEM_COLS = 512;
+constexpr int PP_LOW = 4;  // levels 0 .. 3 are handed to the drain first
 static_assert(Magnitude::LEVELS * PP_N <= PP_TMEM_COLS && Balanced::LEVELS * PP_N <= PP_TMEM_COLS,
               "one 64-column accumulator per level");
 constexpr int PP_GROUP = 8;  // row blocks per tile group
@@ -422,7 +419,7 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem =
       smem_raw + ((1024 - (su32(smem_raw) & 1023)) & 1023);  // 1 KB aligned stages
-  __shared__ __align__(8) uint64_t full[PP_STAGES], empty[PP_STAGES], accf, accfree, fin;
+  __shared__ __align__(8) uint64_t full[PP_STAGES], empty[PP_STAGES], accf[2], accfree[2], fin;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -433,8 +430,10 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&full[s])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&empty[s])));
     }
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&accf)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;" ::"r"(su32(&accfree)));
+    for (int h = 0; h < 2; ++h) {  // 0: levels below PP_LOW, 1: the others
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&accf[h])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 256;" ::"r"(su32(&accfree[h])));
+    }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&fin)));
     asm volatile("fence.mbarrier_init.release.cluster;");
     abort_flag = 0;
@@ -502,22 +501,21 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
         const int s = c % PP_STAGES;
         const int win = c / Sch::FLUSH;
         const bool win_start = (c % Sch::FLUSH) == 0;
-        if (win_start && win > 0 &&
-            !wait_bar(su32(&accfree), (uint32_t)((win - 1) & 1), abort)) {
-          atomicExch(&abort_flag, 1);
-          break;
-        }
-        if (!wait_bar(su32(&full[s]), (uint32_t)((c / PP_STAGES) & 1), abort)) {
+        const bool win_end = (c % Sch::FLUSH) == Sch::FLUSH - 1 || c == nkc - 1;
+        if (!wait_bar(su32(&full[s]), (uint32_t)((c / PP_STAGES) & 1), abort) ||
+            (win_start && win > 0 &&
+             !wait_bar(su32(&accfree[0]), (uint32_t)((win - 1) & 1), abort))) {
           atomicExch(&abort_flag, 1);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t stA = su32(smem + (size_t)s * PP_STAGE_BYTES<Sch>);
         const uint32_t stB = stA + PP_A_BYTES<Sch>;
-        // groups (A slice p, first B slice q0, B slices nq); slice 0 covers every level and comes
-        // first: at the start of a window it overwrites the exact levels while the FP32 levels go
-        // on (overwritten only by the very first MMA of the tile), so there it takes three MMAs.
-        // The groups are a compile-time table, so the issue is a straight sequence: descriptors
+        // groups (A slice p, first B slice q0, B slices nq), first those of the levels below
+        // PP_LOW, then the others: the drain of either half runs under the MMAs of the other.  At
+        // the start of a window slice 0, which covers every level, overwrites the exact levels;
+        // the FP32 levels go on (overwritten only by the very first MMA of the tile).  The groups
+        // are known at compile time, so the issue is a straight sequence: descriptors
         // are the stage's base descriptors plus constants (the start-address field holds
         // address / 16; every address stays inside the stage)
         const uint64_t dA = sdesc_sw64(stA), dB = sdesc_sw64(stB);
@@ -533,28 +531,40 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
         };
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
-          const bool start = ks == 0 && win_start;
-          mma(ks, 0, 0, 4, start ? 0u : 1u);
-          if (Sch::SLICES == 7 && !start) {
-            mma(ks, 0, 4, 3, 1u);
-          } else {
-            mma(ks, 0, 4, Sch::EXACT - 4, start ? 0u : 1u);
-            mma(ks, 0, Sch::EXACT, 2, ks == 0 && c == 0 ? 0u : 1u);
-          }
 #pragma unroll
-          for (int g = 0; g < Sch::GROUPS; ++g)
-            mma(ks, (int)(Sch::GP >> (4 * g)) & 15, (int)(Sch::GQ >> (4 * g)) & 15,
-                (int)(Sch::GN >> (4 * g)) & 15, 1u);
+          for (int p = 0; p < PP_LOW; ++p)
+            mma(ks, p, 0, PP_LOW - p, p == 0 && ks == 0 && win_start ? 0u : 1u);
         }
-        asm volatile(
-            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                su32(&empty[s]))
-            : "memory");
-        if ((c % Sch::FLUSH) == Sch::FLUSH - 1 || c == nkc - 1)
+        auto commit = [&](uint64_t* bar) {
           asm volatile(
               "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                  su32(&accf))
+                  su32(bar))
               : "memory");
+        };
+        if (win_end) commit(&accf[0]);
+        if (win_start && win > 0) {
+          if (!wait_bar(su32(&accfree[1]), (uint32_t)((win - 1) & 1), abort)) {
+            atomicExch(&abort_flag, 1);
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;");
+        }
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+          if (ks == 0 && win_start) {
+            mma(ks, 0, PP_LOW, Sch::EXACT - PP_LOW, 0u);
+            mma(ks, 0, Sch::EXACT, Sch::LEVELS - Sch::EXACT, c == 0 ? 0u : 1u);
+          } else {
+            mma(ks, 0, PP_LOW, Sch::LEVELS - PP_LOW, 1u);
+          }
+#pragma unroll
+          for (int p = 1; p < Sch::SLICES; ++p) {
+            const int q = p < PP_LOW ? PP_LOW - p : 0;
+            mma(ks, p, q, Sch::LEVELS - p - q, 1u);
+          }
+        }
+        commit(&empty[s]);
+        if (win_end) commit(&accf[1]);
       }
       // every MMA issued so far has completed before TMEM is read for the last time or freed
       asm volatile(
@@ -572,24 +582,19 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
     for (int c = 0; c < 32; ++c) T[c] = 0;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(32 * half);
     bool ok = true, mirror = false;
-    for (int w = 0; w < nwin; ++w) {
-      // warp-uniform decision: the TMEM loads below are .sync.aligned
-      const bool got = wait_bar(su32(&accf), (uint32_t)(w & 1), abort);
-      if (!__all_sync(0xffffffffu, got ? 1 : 0)) {
-        atomicExch(&abort_flag, 1);
-        ok = false;
-        break;
-      }
+    // the exact levels LO .. HI - 1 of a window into T; the next level's load is in flight while a
+    // level is converted
+    auto drain = [&](auto lo, auto hi) {
+      constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
       asm volatile("tcgen05.fence::after_thread_sync;");
-      // the next level's load is in flight while a level is converted
       uint32_t va[32], vb[32];
-      tmem_ld32(lane_base, va);
+      tmem_ld32(lane_base + (uint32_t)(LO * PP_N), va);
       tmem_wait(va);
 #pragma unroll
-      for (int lv = 0; lv < Sch::EXACT; ++lv) {
-        uint32_t(&v)[32] = (lv & 1) ? vb : va;
-        uint32_t(&vn)[32] = (lv & 1) ? va : vb;
-        if (lv + 1 < Sch::EXACT) tmem_ld32(lane_base + (uint32_t)((lv + 1) * PP_N), vn);
+      for (int lv = LO; lv < HI; ++lv) {
+        uint32_t(&v)[32] = ((lv - LO) & 1) ? vb : va;
+        uint32_t(&vn)[32] = ((lv - LO) & 1) ? va : vb;
+        if (lv + 1 < HI) tmem_ld32(lane_base + (uint32_t)((lv + 1) * PP_N), vn);
 #pragma unroll
         for (int t = 0; t < 32; ++t) {
           const float f = __uint_as_float(v[t]);
@@ -601,10 +606,24 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
             T[t] = add_level(T[t], __float2int_rn(f), 1 << (Sch::BITS * (Sch::EXACT - 1 - lv)));
           }
         }
-        if (lv + 1 < Sch::EXACT) tmem_wait(vn);
+        if (lv + 1 < HI) tmem_wait(vn);
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(&accfree)) : "memory");
+    };
+    for (int w = 0; w < nwin && ok; ++w) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        // warp-uniform decision: the TMEM loads are .sync.aligned
+        const bool got = wait_bar(su32(&accf[h]), (uint32_t)(w & 1), abort);
+        if (!__all_sync(0xffffffffu, got ? 1 : 0)) {
+          atomicExch(&abort_flag, 1);
+          ok = false;
+          break;
+        }
+        if (h == 0) drain(std::integral_constant<int, 0>(), std::integral_constant<int, PP_LOW>());
+        else drain(std::integral_constant<int, PP_LOW>(), std::integral_constant<int, Sch::EXACT>());
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(&accfree[h])) : "memory");
+      }
     }
     if (__all_sync(0xffffffffu, (ok && !*abort) ? 1 : 0)) {
       // C = 2^(eA + eB - 14) (T + F) 2^(-BITS (EXACT - 1)).  A symmetric product's mirror image
