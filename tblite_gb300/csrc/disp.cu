@@ -15,14 +15,9 @@
 #include <stdexcept>
 
 #include "engine.h"
+#include "warp_sums.cuh"
 
 namespace tb {
-
-__device__ __forceinline__ double wsum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
 // D4 coordination number, dcount/dr
 __device__ __forceinline__ void d4_count(const DevD4& d, int i, int j, double r, double& c,
@@ -52,7 +47,7 @@ __device__ __forceinline__ void d4_cn_dev(DevMol m, DevD4 d, double* cn) {
     d4_count(d, i, j, sqrt(r2), c, dc);
     acc += c;
   }
-  acc = wsum(acc);
+  acc = warp_sum(acc);
   if (lane == 0) cn[i] = acc;
 }
 __global__ void k_d4_cn(DevMol m, DevD4 d, double* cn) {
@@ -229,7 +224,7 @@ __device__ __forceinline__ void d4_pair_dev(DevMol m, DevD4 d, const double* __r
     }
   }
   if (MODE < 2) {
-    for (int r = 0; r < D4_MREF; ++r) u[r] = wsum(u[r]);
+    warp_sums(u);
     if (lane == 0) {
       double acc = 0.0;
       if (MODE == 0) {
@@ -241,9 +236,7 @@ __device__ __forceinline__ void d4_pair_dev(DevMol m, DevD4 d, const double* __r
       }
     }
   } else {
-    for (int k = 0; k < 3; ++k) g[k] = wsum(g[k]);
-    for (int k = 0; k < 9; ++k) sg[k] = wsum(sg[k]);
-    dcn = wsum(dcn);
+    warp_sums_grad(g, sg, dcn);
     if (lane == 0) {
       for (int k = 0; k < 3; ++k) grad[3 * i + k] += g[k];
       for (int k = 0; k < 9; ++k) sig_at[9 * i + k] += sg[k];
@@ -283,15 +276,24 @@ __global__ void k_d4_c6(int nat, DevD4 d, const double* __restrict__ gwv,
 
 // Axilrod-Teller-Muto term (disp/d4.f90 three-body part, d4 get_atm_dispersion).  Every factor
 // of a triple (i, j, l) that is a product over its three pairs is tabulated per pair first
-// (k_d4_atm_pairs): r^2, 1/r, the damping ratio (r0/r)^(alpha/3), sqrt|C6| and
+// (k_d4_atm_pairs): r^2, 1/r^2, the damping ratio (r0/r)^(alpha/3), sqrt|C6| / r^3 and
 // dC6_ij/dCN_i / (2 C6_ij) in both index orders, so that no pow or sqrt and a single division
 // remain per triple.  Each triple i < j < l is then evaluated once (k_d4_atm): its energy goes
 // 1/3 to each atom, its CN derivatives to the three atoms, and its derivatives with respect to
 // the three squared distances into a pair matrix Gamma (upper triangle); the forces and the
 // virial follow from Gamma in one pass over the pairs (k_d4_atm_grad):
 //   dE/dR_i = sum_j 2 Gamma_ij (R_i - R_j),  sigma = sum_{i<j} 2 Gamma_ij v_ij v_ij^T.
-// tab layout [8][nat][nat]: r^2 (+inf beyond the cutoff), 1/r, ratio, sqrt|C6|, dq, dq^T,
+// tab layout [8][nat][nat]: r^2 (+inf beyond the cutoff), 1/r^2, ratio, sqrt|C6| / r^3, dq, dq^T,
 // Gamma rows written by their owner atom, Gamma of the (j, l) pairs accumulated atomically.
+//
+// What bounds the triples is the FP64 pipe: an instruction costs a warp 64 to 76 cycles whatever
+// its active lanes do.  So lanes are not left idle (the partners of i inside the cutoff are listed
+// first, and of those the ones inside the cutoff of j are queued until 32 are together), and a
+// triple is 45 FP64 instructions (77 before): with a, b, c the squared distances,
+// p_a = a - b + c and so on, P = p_a p_b p_c,
+//   E = K (1 + p),  K = c9 fdmp / (r_ij r_jl r_il)^3,  p = 0.375 P / (a b c),
+//   dE/dx = K 0.375 / (a b c) dP/dx + M / x,
+//   M = E alpha/6 (1 - fdmp) - K (2.5 p + 1.5),  dP/da = 2 a p_b - p_c p_a, ...
 constexpr int ATM_TABLES = 8;
 __device__ __forceinline__ void d4_atm_pairs_dev(DevMol m, DevD4 d, const double* __restrict__ c6,
                                                  const double* __restrict__ dc6, double* tab,
@@ -317,7 +319,9 @@ __device__ __forceinline__ void d4_atm_pairs_dev(DevMol m, DevD4 d, const double
     const double r0 = d.a1 * sqrt(3.0 * d.r4r2[i] * d.r4r2[j]) + d.a2;
     w = pow(r0 * ir, d.atm_alpha / 3.0);
     const double c = c6[t];
-    sc = sqrt(fabs(c));
+    sc = sqrt(fabs(c)) * ir;
+    ir *= ir;
+    sc *= ir;
     dq = c != 0.0 ? dc6[t] / (2.0 * c) : 0.0;
     dqt = c != 0.0 ? dc6[(size_t)j * nat + i] / (2.0 * c) : 0.0;
   }
@@ -334,19 +338,27 @@ __global__ void k_d4_atm_pairs(DevMol m, DevD4 d, const double* __restrict__ c6,
   d4_atm_pairs_dev(m, d, c6, dc6, tab, eat);
 }
 
-// one warp per atom i, triples i < j < l: j warp-uniform, the lanes walk l > j.  The warp keeps
-// three rows in shared memory (3 nat doubles): Gamma_i. (roles (i, j) and (i, l)), the energy
-// thirds and the CN derivatives of the partners; Gamma of the (j, l) pairs goes to global memory
-// with coalesced atomics.  eat and dEdcn are accumulated (eat is zeroed by the pairs kernel).
+constexpr int ATM_WARPS = 2;  // warps of a block at most
+// twice a positive finite number below 2^1022, without the FP64 pipe
+__device__ __forceinline__ double twice(double x) {
+  return __hiloint2double(__double2hiint(x) + (1 << 20), __double2loint(x));
+}
+// one warp per atom i, triples i < j < l: j warp-uniform, the lanes take the l queued for it.  The
+// warp keeps three rows in shared memory (3 nat doubles): Gamma_i. (roles (i, j) and (i, l)), the
+// energies and the CN derivatives of the partners; Gamma of the (j, l) pairs goes to global memory
+// with coalesced atomics.  The list of partners stands in i's row of Gamma until that is written.
+// eat and dEdcn are accumulated (eat is zeroed by the pairs kernel).
 __device__ __forceinline__ void d4_atm_dev(DevMol m, DevD4 d, double* tab, double* eat,
                                            double* dEdcn, double* srow) {
+  __shared__ int queue[ATM_WARPS][64];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nat = m.nat;
   if (warp >= nat) return;
   const int i = warp;
+  int* qu = queue[threadIdx.x >> 5];
   const size_t nn = (size_t)nat * nat;
   const double* R2 = tab;
-  const double* IR = tab + nn;
+  const double* I2 = tab + nn;
   const double* W = tab + 2 * nn;
   const double* SC = tab + 3 * nn;
   const double* DQ = tab + 4 * nn;
@@ -356,81 +368,93 @@ __device__ __forceinline__ void d4_atm_dev(DevMol m, DevD4 d, double* tab, doubl
   double* sG = srow;
   double* sE = srow + nat;
   double* sD = srow + 2 * nat;
+  const double cut2 = d.disp3_cutoff * d.disp3_cutoff;
+  const double a6 = d.atm_alpha / 6.0;
+  const size_t ri = (size_t)i * nat;
+  int* list = reinterpret_cast<int*>(GO + ri);
+  const unsigned below = (1u << lane) - 1;
+  int count = 0;
+  for (int l0 = i + 1; l0 < nat; l0 += 32) {
+    const int l = l0 + lane;
+    const bool in = l < nat && R2[ri + l] <= cut2;
+    const unsigned mask = __ballot_sync(0xffffffffu, in);
+    if (in) list[count + __popc(mask & below)] = l;
+    count += __popc(mask);
+  }
   for (int l = lane; l < nat; l += 32) {
     sG[l] = 0.0;
     sE[l] = 0.0;
     sD[l] = 0.0;
   }
   __syncwarp();
-  const double cut2 = d.disp3_cutoff * d.disp3_cutoff;
-  const double a6 = d.atm_alpha / 6.0;
-  const size_t ri = (size_t)i * nat;
-  double ei = 0.0, di = 0.0;
-  for (int j = i + 1; j < nat; ++j) {
-    const double a = R2[ri + j];
-    if (!(a <= cut2)) continue;  // beyond the cutoff (warp uniform)
+  for (int jj = 0; jj + 1 < count; ++jj) {
+    const int j = list[jj];
     const size_t rj = (size_t)j * nat;
-    const double irij = IR[ri + j], wij = W[ri + j], scij = SC[ri + j];
-    const double dqij = DQ[ri + j], dqji = DQT[ri + j];
-    const double ia = irij * irij;
-    double gA = 0.0, eJ = 0.0, dJ = 0.0;
-    for (int l = j + 1 + lane; l < nat; l += 32) {
-      const double c = R2[ri + l], b = R2[rj + l];
-      if (!(c <= cut2) || !(b <= cut2)) continue;
-      const double iril = IR[ri + l], irjl = IR[rj + l];
-      const double c9 = -d.s9 * scij * SC[ri + l] * SC[rj + l];
-      const double t = wij * W[ri + l] * W[rj + l];
-      const double ir1 = irij * iril * irjl;
-      const double ir2 = ir1 * ir1, ir3 = ir2 * ir1, ir5 = ir3 * ir2;
-      const double fdmp = 1.0 / (1.0 + 6.0 * t);
+    const double a = R2[ri + j], ia = I2[ri + j];
+    const double w6 = 6.0 * W[ri + j], c9 = -d.s9 * SC[ri + j], k0 = 0.375 * ia, a2 = 2.0 * a;
+    double v[3] = {0.0, 0.0, 0.0};  // sums over l: Gamma_ij, E, CN derivative of j
+    auto triple = [&](int l) {
+      const double c = R2[ri + l], b = R2[rj + l], ic = I2[ri + l], ib = I2[rj + l];
+      const double fdmp = 1.0 / fma(w6 * W[ri + l], W[rj + l], 1.0);
+      const double K = c9 * SC[ri + l] * SC[rj + l] * fdmp;
+      const double k2 = k0 * ic * ib;
       // angular factor in the squared distances a = r2ij, b = r2jl, c = r2il
-      const double ib = irjl * irjl, ic = iril * iril;
-      const double pa = a - b + c, pb = -a + b + c, pc = a + b - c;
-      const double P = pc * pa * pb;
-      const double ang = 0.375 * P * ir5 + ir3;
-      const double E = ang * fdmp * c9;
-      const double dPa = pa * pb + pc * pb - pc * pa;
-      const double dPc = -pa * pb + pc * pb + pc * pa;
-      const double dPb = pa * pb - pc * pb + pc * pa;
-      const double g0 = ang * (-6.0 * fdmp * fdmp) * (-a6) * t;
-      const double h = 0.375 * ir5, q = 2.5 * P * h, s = 1.5 * ir3;
-      const double dEa = c9 * ((dPa * h - (q + s) * ia) * fdmp + g0 * ia);
-      const double dEb = c9 * ((dPb * h - (q + s) * ib) * fdmp + g0 * ib);
-      const double dEc = c9 * ((dPc * h - (q + s) * ic) * fdmp + g0 * ic);
-      const double e3 = E * (1.0 / 3.0);
-      ei += e3;
-      eJ += e3;
-      sE[l] += e3;
-      gA += dEa;
-      sG[l] += dEc;
-      atomicAdd(GB + rj + l, dEb);
-      // dE/dCN through C6_pq = sqrt: E dC6_pq/dCN_p / (2 C6_pq)
-      di += E * (dqij + DQ[ri + l]);
-      dJ += E * (dqji + DQ[rj + l]);
-      sD[l] += E * (DQT[ri + l] + DQT[rj + l]);
+      const double s = c - b, pa = a + s, pc = a - s, pb = (b + c) - a;
+      const double x = pc * pa, y = pc * pb, z = pa * pb;
+      const double p = k2 * (x * pb);
+      const double E = fma(K, p, K), kk = K * k2;
+      const double M = fma(E, fma(-a6, fdmp, a6), -(K * fma(2.5, p, 1.5)));
+      v[0] = fma(M, ia, fma(kk, fma(a2, pb, -x), v[0]));
+      sG[l] = fma(M, ic, fma(kk, fma(twice(c), pc, -z), sG[l]));
+      atomicAdd(GB + rj + l, fma(M, ib, kk * fma(twice(b), pa, -y)));
+      // dE/dCN through C6_pq = sqrt: E dC6_pq/dCN_p / (2 C6_pq); the pairs with i at the end
+      v[1] += E;
+      sE[l] += E;
+      v[2] = fma(E, DQ[rj + l], v[2]);
+      sD[l] = fma(E, DQT[rj + l], sD[l]);
+    };
+    int held = 0;
+    for (int k = jj + 1; k < count; k += 32) {
+      const int l = k + lane < count ? list[k + lane] : 0;
+      const bool in = k + lane < count && R2[rj + l] <= cut2;
+      const unsigned mask = __ballot_sync(0xffffffffu, in);
+      if (in) qu[held + __popc(mask & below)] = l;
+      held += __popc(mask);
+      __syncwarp();
+      if (held >= 32) {
+        triple(qu[lane]);
+        held -= 32;
+        const int rest = qu[32 + lane];
+        __syncwarp();
+        qu[lane] = rest;
+        __syncwarp();
+      }
     }
-    gA = wsum(gA);
-    eJ = wsum(eJ);
-    dJ = wsum(dJ);
-    if (lane == 0) {
-      sG[j] += gA;
-      sE[j] += eJ;
-      sD[j] += dJ;
-    }
+    if (lane < held) triple(qu[lane]);
+    __syncwarp();
+    warp_sums(v);
+    if (lane == 0) sG[j] += v[0];
+    if (lane == 1) sE[j] += v[1];
+    if (lane == 2) sD[j] += v[2];
     __syncwarp();
   }
-  ei = wsum(ei);
-  di = wsum(di);
+  // the three atoms of a triple share its energy; every triple of i stands in sE twice
+  double ei = 0.0, di = 0.0;
   for (int l = lane; l < nat; l += 32) {
-    if (l > i) GO[ri + l] = sG[l];
-    if (l != i) {
-      if (sE[l] != 0.0) atomicAdd(eat + l, sE[l]);
-      if (sD[l] != 0.0) atomicAdd(dEdcn + l, sD[l]);
-    }
+    if (l <= i) continue;
+    const double e = sE[l];
+    GO[ri + l] = sG[l];
+    if (e == 0.0 && sD[l] == 0.0) continue;
+    ei += e;
+    di = fma(e, DQ[ri + l], di);
+    atomicAdd(eat + l, e * (1.0 / 3.0));
+    atomicAdd(dEdcn + l, fma(e, DQT[ri + l], sD[l]));
   }
+  double t[2] = {ei, di};
+  warp_sums(t);
   if (lane == 0) {
-    atomicAdd(eat + i, ei);
-    atomicAdd(dEdcn + i, di);
+    atomicAdd(eat + i, t[0] * (1.0 / 6.0));
+    atomicAdd(dEdcn + i, t[1]);
   }
 }
 __global__ void k_d4_atm(DevMol m, DevD4 d, double* tab, double* eat, double* dEdcn) {
@@ -460,8 +484,7 @@ __device__ __forceinline__ void d4_atm_grad_dev(DevMol m, const double* __restri
     for (int p = 0; p < 3; ++p)
       for (int q = 0; q < 3; ++q) sg[3 * p + q] += G * v[p] * v[q];
   }
-  for (int k = 0; k < 3; ++k) g[k] = wsum(g[k]);
-  for (int k = 0; k < 9; ++k) sg[k] = wsum(sg[k]);
+  warp_sums_grad(g, sg);
   if (lane == 0) {
     for (int k = 0; k < 3; ++k) grad[3 * i + k] += g[k];
     for (int k = 0; k < 9; ++k) sig_at[9 * i + k] += sg[k];
@@ -475,7 +498,7 @@ __global__ void k_d4_atm_grad(DevMol m, const double* __restrict__ tab, double* 
 // warps per block of k_d4_atm: its shared memory holds 3 nat doubles per warp
 static inline int atm_warps(int nat) {
   const size_t per = (size_t)3 * nat * sizeof(double);
-  if (per * 2 <= 200 * 1024) return 2;
+  if (per * ATM_WARPS <= 200 * 1024) return ATM_WARPS;
   if (per <= 200 * 1024) return 1;
   return 0;
 }
@@ -510,8 +533,7 @@ __device__ __forceinline__ void d4_cn_grad_dev(DevMol m, DevD4 d, const double* 
     for (int a = 0; a < 3; ++a)
       for (int b = 0; b < 3; ++b) sg[3 * a + b] += 0.5 * f * v[a] * v[b];
   }
-  for (int k = 0; k < 3; ++k) g[k] = wsum(g[k]);
-  for (int k = 0; k < 9; ++k) sg[k] = wsum(sg[k]);
+  warp_sums_grad(g, sg);
   if (lane == 0) {
     for (int k = 0; k < 3; ++k) grad[3 * i + k] += g[k];
     for (int k = 0; k < 9; ++k) sig_at[9 * i + k] += sg[k];
@@ -617,7 +639,7 @@ __device__ __forceinline__ void d3_setup_dev(const DevMol& m, const DevD3& d) {
     d3_count(sqrt(r2), d.rcov[i] + d.rcov[j], d.k1, c, dc);
     acc += c;
   }
-  acc = wsum(acc);
+  acc = warp_sum(acc);
   if (lane != 0) return;
   d.cn[i] = acc;
   double w[D4_MREF], dw[D4_MREF], norm = 0.0, dnorm = 0.0;
@@ -691,12 +713,8 @@ __device__ __forceinline__ void d3_pair_dev(const DevMol& m, const DevD3& d, int
       dcn += dedc6 * dc6i;
     }
   }
-  e = wsum(e);
-  if (grad) {
-    dcn = wsum(dcn);
-    for (int k = 0; k < 3; ++k) g[k] = wsum(g[k]);
-    for (int k = 0; k < 9; ++k) sg[k] = wsum(sg[k]);
-  }
+  if (grad) warp_sums_grad(g, sg, e, dcn);
+  else e = warp_sum(e);
   if (lane != 0) return;
   eat[i] += e;
   if (!grad) return;
@@ -728,8 +746,7 @@ __device__ __forceinline__ void d3_cn_grad_dev(const DevMol& m, const DevD3& d, 
     for (int a = 0; a < 3; ++a)
       for (int b = 0; b < 3; ++b) sg[3 * a + b] += 0.5 * f * v[a] * v[b];
   }
-  for (int k = 0; k < 3; ++k) g[k] = wsum(g[k]);
-  for (int k = 0; k < 9; ++k) sg[k] = wsum(sg[k]);
+  warp_sums_grad(g, sg);
   if (lane == 0) {
     for (int k = 0; k < 3; ++k) grad[3 * i + k] += g[k];
     for (int k = 0; k < 9; ++k) sig_at[9 * i + k] += sg[k];
