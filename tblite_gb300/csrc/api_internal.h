@@ -94,7 +94,7 @@ struct Workspace {
       sh_refocc, at_en, at_rad, at_rcov, at_mprad, at_vcn, at_dkern, at_qkern, at_repa, at_repz;
   DBuf<int> at_z, at_sh, sh_atom, sh_l, sh_nprim, sh_ao, ao_sh, ao_at;
   // geometry dependent
-  DBuf<double> cn, se, mrad, dmrdcn, S, H, D, Q, F, C, P, W, emo, focc, scratch;
+  DBuf<double> cn, se, mrad, dmrdcn, ctab, S, H, D, Q, F, C, P, W, emo, focc, scratch;
   // SCF state
   DBuf<double> qsh, qat, dpat, qpat, qsh_o, qat_o, dpat_o, qpat_o, vsh, vat, vdp, vqp, vao;
   DBuf<double> mull, eband, eelec, erep, vec_out, scal;

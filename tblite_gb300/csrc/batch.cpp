@@ -308,7 +308,7 @@ void layout(Plan& pl, Region* R) {
   pl.cn = piece<double>(R, RS, na);
   pl.se = piece<double>(R, RS, ns);
   pl.mrad = piece<double>(R, RS, na);
-  pl.ctab = piece<double>(R, RS, ns * ns + 3 * na * na);
+  pl.ctab = piece<double>(R, RS, coulomb_table_words(ns, na));
   pl.dmrdcn = piece<double>(R, RS, na);
   for (Piece* p : {&pl.F, &pl.P, &pl.C, &pl.scratch, &pl.X, &pl.A, &pl.T1, &pl.Y})
     *p = piece<double>(R, RS, nn);

@@ -830,6 +830,9 @@ void electron_counts(const _tblite_calculator* c, const _tblite_structure* mol, 
   *nbet_out = (nocc - diff) / 2;
 }
 
+// doubles of the largest pair table of the electrostatics (1 GiB: about 5000 atoms)
+constexpr size_t COULOMB_TABLE_MAX = (size_t)1 << 27;
+
 static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
                         _tblite_calculator* c, _tblite_result* res) {
   if (mol->nat != c->nat) throw std::runtime_error("structure does not match calculator");
@@ -868,6 +871,14 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   g_prof.begin(PH_SETUP, s);
   launch_cn(m, p, w.cn.p, s);
   launch_setup_levels(m, p, w.cn.p, w.se.p, w.mrad.p, w.dmrdcn.p, s);
+  // the table's pair terms are the ones evaluated in place but for their last bits, which a large
+  // molecule keeps (see tridiag_fixed); it stays small beside the matrices
+  const size_t ctab_words = coulomb_table_words(nsh, nat);
+  const bool ctab = (purify || n <= TRIDIAG_FIXED_MAX) && ctab_words <= COULOMB_TABLE_MAX;
+  if (ctab) {
+    w.ctab.alloc(ctab_words);
+    launch_coulomb_table(m, p, w.mrad.p, w.ctab.p, s);
+  }
   launch_build_h0(m, p, w.se.p, w.S.p, w.H.p, w.D.p, w.Q.p, s);
   cuda_check(cudaMemsetAsync(w.grad.p, 0, sizeof(double) * 3 * nat, s), "zero");
   cuda_check(cudaMemsetAsync(w.sig_at.p, 0, sizeof(double) * 9 * nat, s), "zero");
@@ -1005,7 +1016,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
     ++iscf;
     g_prof.begin(PH_POTENTIAL, s);
     launch_coulomb_potential(m, p, w.mrad.p, w.qsh.p, w.qat.p, w.dpat.p, w.qpat.p, w.vsh.p, w.vat.p,
-                             w.vdp.p, w.vqp.p, s);
+                             w.vdp.p, w.vqp.p, ctab ? w.ctab.p : nullptr, s);
     if (c->has_d4) d4_potential(m, d4, d4w, w.qat.p, w.vat.p, s);
     if (c->solv) solv_potential(dsolv, w.xyz.p, w.qat.p, w.vat.p, s);
     if (c->has_field) launch_field_potential(nat, w.xyz.p, c->efield, w.vat.p, w.vdp.p, s);
@@ -1054,7 +1065,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
     launch_diff((int)nd, w.vec_out.p, w.b_q.p, w.b_dq.p, w.scal.p + 1, s);  // mixer%diff
     launch_eelec_init(nat, w.scal.p, w.eband.p, w.eelec.p, s);
     launch_coulomb_energy(m, p, w.mrad.p, w.qsh_o.p, w.qat_o.p, w.dpat_o.p, w.qpat_o.p, w.eelec.p,
-                          s);
+                          ctab ? w.ctab.p : nullptr, s);
     if (c->has_d4) d4_energy(m, d4, d4w, w.qat_o.p, w.eelec.p, s);
     if (c->solv) solv_energy(dsolv, w.xyz.p, w.qat_o.p, w.eelec.p, s);
     if (c->has_field)

@@ -200,14 +200,19 @@ void launch_field_potential(int nat, const double* xyz, const double* efield, do
                             double* vdp, cudaStream_t s);
 void launch_field_energy(int nat, const double* xyz, const double* efield, const double* qat,
                          const double* dpat, double* eat, cudaStream_t s);
+// pair table of the electrostatics, coulomb_table_words(nsh, nat) doubles, once per geometry; the
+// potential and the energy read it, or evaluate the pairs themselves (tab == nullptr)
+inline size_t coulomb_table_words(size_t nsh, size_t nat) { return nsh * nsh + 3 * nat * nat; }
+void launch_coulomb_table(const DevMol& m, const Gfn2Scalars& p, const double* mrad, double* tab,
+                          cudaStream_t s);
 void launch_coulomb_potential(const DevMol& m, const Gfn2Scalars& p, const double* mrad,
                               const double* qsh, const double* qat, const double* dpat,
                               const double* qpat, double* vsh, double* vat, double* vdp,
-                              double* vqp, cudaStream_t s);
+                              double* vqp, const double* tab, cudaStream_t s);
 // per-atom electrostatic energy (es2 + es3 + AES incl. kernels), added into eat
 void launch_coulomb_energy(const DevMol& m, const Gfn2Scalars& p, const double* mrad,
                            const double* qsh, const double* qat, const double* dpat,
-                           const double* qpat, double* eat, cudaStream_t s);
+                           const double* qpat, double* eat, const double* tab, cudaStream_t s);
 void launch_coulomb_gradient(const DevMol& m, const Gfn2Scalars& p, const double* mrad,
                              const double* dmrdcn, const double* qsh, const double* qat,
                              const double* dpat, const double* qpat, double* grad, double* sigma,

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "engine.h"
+#include "warp_sums.cuh"
 
 namespace tb {
 
@@ -31,7 +32,8 @@ __device__ __forceinline__ void gauss_moments(const double pa[3], double eta, Mo
     const double a = pa[k], a2 = a * a, a3 = a2 * a;
     M.m[k][0] = 1.0;
     M.m[k][1] = a;
-    M.m[k][2] = a2 + s2;
+    // (not fused, as where a2 is needed again: the same rounding for every kind of pair)
+    M.m[k][2] = __dadd_rn(a2, s2);
     M.m[k][3] = a3 + 3.0 * a * s2;
     M.m[k][4] = a2 * a2 + 6.0 * a2 * s2 + 3.0 * s2 * s2;
     M.m[k][5] = a3 * a2 + 10.0 * a3 * s2 + 15.0 * a * s2 * s2;
@@ -522,14 +524,17 @@ __device__ __forceinline__ void h0_gradient_dev(const DevMol& m, const Gfn2Scala
   // virial: the six distinct elements of the symmetric 3 x 3 summed over the warp, then one
   // atomic per element and warp (every pair of a molecule adds to the same nine numbers)
   const int va[6] = {0, 0, 1, 0, 1, 2}, vb[6] = {0, 1, 1, 2, 2, 2};
+  double v[6];
 #pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    double v = 0.5 * (vec[va[e]] * dG[vb[e]] + dG[va[e]] * vec[vb[e]]);
+  for (int e = 0; e < 6; ++e)
+    v[e] = 0.5 * (vec[va[e]] * dG[vb[e]] + dG[va[e]] * vec[vb[e]]);
+  warp_sums(v);
+  if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0 && v != 0.0) {
-      atomicAdd(sigma + 3 * va[e] + vb[e], v);
-      if (va[e] != vb[e]) atomicAdd(sigma + 3 * vb[e] + va[e], v);
+    for (int e = 0; e < 6; ++e) {
+      if (v[e] == 0.0) continue;
+      atomicAdd(sigma + 3 * va[e] + vb[e], v[e]);
+      if (va[e] != vb[e]) atomicAdd(sigma + 3 * vb[e] + va[e], v[e]);
     }
   }
 }

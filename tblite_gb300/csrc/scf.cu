@@ -21,6 +21,7 @@
 #include <chrono>
 
 #include "engine.h"
+#include "warp_sums.cuh"
 
 namespace tb {
 
@@ -41,12 +42,6 @@ void stream_wait(cudaStream_t s) {
     } while (std::chrono::steady_clock::now() < until);
   }
   cudaEventSynchronize(ev);
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
 }
 
 // x^e for the small integer exponents of the damping functions, pow() otherwise
@@ -144,10 +139,7 @@ __device__ __forceinline__ void cn_grad_dev(DevMol m, Gfn2Scalars p, const doubl
     for (int a = 0; a < 3; ++a)
       for (int b = 0; b < 3; ++b) sg[3 * a + b] += 0.5 * f * v[a] * v[b];
   }
-  for (int k = 0; k < 3; ++k) {
-    g[k] = warp_sum(g[k]);
-  }
-  for (int k = 0; k < 9; ++k) sg[k] = warp_sum(sg[k]);
+  warp_sums_grad(g, sg);
   if (lane == 0) {
     for (int k = 0; k < 3; ++k) grad[3 * i + k] += g[k];
     for (int k = 0; k < 9; ++k) sig_at[9 * i + k] += sg[k];
@@ -282,13 +274,34 @@ __device__ __forceinline__ void coulomb_table_dev(DevMol m, Gfn2Scalars p,
   }
 }
 
-// tab: the pair table of coulomb_table_dev, or nullptr to evaluate the pair terms here
-template <int MODE>
-__device__ __forceinline__ void coulomb_dev(DevMol m, Gfn2Scalars p, const double* __restrict__ mrad,
-                          const double* __restrict__ qsh, const double* __restrict__ qat,
-                          const double* __restrict__ dpat, const double* __restrict__ qpat,
-                          double* vsh, double* vat, double* vdp, double* vqp, double* eat,
-                          const double* __restrict__ tab = nullptr) {
+// gamma of the shells s and t of two atoms at distance r1, from the table where there is one
+__device__ __forceinline__ double gam_pair(const DevMol& m, const Gfn2Scalars& p, const double* tab,
+                                           double r1, int s, int t) {
+  return tab ? tab[(size_t)s * m.nsh + t]
+             : gam_kernel(r1, eta_avg(m.sh_hub[s], m.sh_hub[t], p.harmonic), p.gexp);
+}
+__device__ __forceinline__ void aes_scalars(const DevMol& m, const Gfn2Scalars& p,
+                                            const double* tab, const double* mrad, double r1,
+                                            int i, int j, double& g3f3, double& g5f5,
+                                            double& g3f5) {
+  if (tab) {
+    const size_t plane = (size_t)m.nat * m.nat, ij = (size_t)i * m.nat + j;
+    const double* aes = tab + (size_t)m.nsh * m.nsh;
+    g3f3 = aes[ij];
+    g5f5 = aes[plane + ij];
+    g3f5 = aes[2 * plane + ij];
+  } else {
+    aes_pair(r1, mrad[i], mrad[j], p, g3f3, g5f5, g3f5);
+  }
+}
+
+// tab: the pair table of coulomb_table_dev, or nullptr to evaluate the pair terms here.  The sixteen
+// sums over the warp cost as much as the pairs of a molecule of 50 atoms when each is taken alone.
+__device__ __forceinline__ void coulomb_potential_dev(DevMol m, Gfn2Scalars p,
+                          const double* __restrict__ mrad, const double* __restrict__ qsh,
+                          const double* __restrict__ qat, const double* __restrict__ dpat,
+                          const double* __restrict__ qpat, double* vsh, double* vat, double* vdp,
+                          double* vqp, const double* __restrict__ tab) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= m.nat) return;
   const int i = warp;
@@ -302,8 +315,8 @@ __device__ __forceinline__ void coulomb_dev(DevMol m, Gfn2Scalars p, const doubl
   const double qa_i = qat[i], ri = mrad[i];
   double ush[MAXSH] = {0, 0, 0};     // sum_j gamma q_j for shells of i
   double uat = 0.0;                  // vat_i
-  double ud[3] = {0, 0, 0};          // vdp_i: sd + dd parts
-  double udd[3] = {0, 0, 0};         // dd part only (energy needs 1/2 of it)
+  double ud[3] = {0, 0, 0};          // vdp_i: charges of the partners
+  double udd[3] = {0, 0, 0};         // vdp_i: their dipoles
   double uq[6] = {0, 0, 0, 0, 0, 0};  // vqp_i
   const int nsh = m.nsh, nat = m.nat;
   const double* aes = tab + (size_t)nsh * nsh;
@@ -353,76 +366,146 @@ __device__ __forceinline__ void coulomb_dev(DevMol m, Gfn2Scalars p, const doubl
     }
     for (int k = 0; k < 6; ++k) uq[k] += sq[k] * qa_j;
   }
-  for (int a = 0; a < MAXSH; ++a) ush[a] = warp_sum(ush[a]);
-  uat = warp_sum(uat);
-  for (int k = 0; k < 3; ++k) {
-    ud[k] = warp_sum(ud[k]);
-    udd[k] = warp_sum(udd[k]);
+  double u[MAXSH + 13] = {ush[0], ush[1], ush[2], uat,   ud[0], ud[1], ud[2], udd[0],
+                          udd[1], udd[2], uq[0],  uq[1], uq[2], uq[3], uq[4], uq[5]};
+  static_assert(MAXSH == 3, "three shells per atom");
+  constexpr int UAT = MAXSH, UD = UAT + 1, UDD = UD + 3, UQ = UDD + 3;
+  if (tab) {
+    warp_sums(u);
+  } else {  // one by one, as the loop above was compiled with: its roundings stay the same
+    for (int k = 0; k < MAXSH + 13; ++k) u[k] = warp_sum(u[k]);
   }
-  for (int k = 0; k < 6; ++k) uq[k] = warp_sum(uq[k]);
   if (lane != 0) return;
-  // on-site gamma block
-  double gsh[MAXSH];
-  for (int a = 0; a < nsi; ++a) {
-    double acc = ush[a];
+#pragma unroll
+  for (int a = 0; a < MAXSH; ++a) {
+    if (a >= nsi) break;
+    double acc = u[a];  // and the on-site gamma block
     for (int b = 0; b < nsi; ++b)
       acc += eta_avg(m.sh_hub[is0 + a], m.sh_hub[is0 + b], p.harmonic) * qsh[is0 + b];
-    gsh[a] = acc;
+    const double q = qsh[is0 + a];
+    vsh[is0 + a] = acc + (p.third_atom ? 0.0 : q * q * m.sh_gam3[is0 + a]);
   }
   const double mpscale[6] = {1, 2, 1, 2, 2, 1};
-  if (MODE == 0) {
-    for (int a = 0; a < nsi; ++a) {
-      const double q = qsh[is0 + a];
-      vsh[is0 + a] = gsh[a] + (p.third_atom ? 0.0 : q * q * m.sh_gam3[is0 + a]);
+  vat[i] = u[UAT] + (p.third_atom ? qa_i * qa_i * m.at_gam3[i] : 0.0);
+  for (int k = 0; k < 3; ++k)
+    vdp[3 * i + k] =
+        p.aes ? u[UD + k] + u[UDD + k] + 2.0 * m.at_dkern[i] * di[k] : 0.0;
+  for (int k = 0; k < 6; ++k)
+    vqp[6 * i + k] =
+        p.aes ? u[UQ + k] + 2.0 * m.at_qkern[i] * qi[k] * mpscale[k] : 0.0;
+}
+
+// energy of atom i (added to eat): the potentials of i contracted with its charges and moments
+// pair by pair, half the FP64 work of forming them, and one sum over the warp
+__device__ __forceinline__ void coulomb_energy_dev(DevMol m, Gfn2Scalars p,
+                          const double* __restrict__ mrad, const double* __restrict__ qsh,
+                          const double* __restrict__ qat, const double* __restrict__ dpat,
+                          const double* __restrict__ qpat, double* eat,
+                          const double* __restrict__ tab) {
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (warp >= m.nat) return;
+  const int i = warp;
+  const int is0 = m.at_sh[i], nsi = m.at_sh[i + 1] - is0;
+  const double mpscale[6] = {1, 2, 1, 2, 2, 1};
+  double xi[3], di[3], qi[6], qs[MAXSH] = {0.0, 0.0, 0.0};
+  for (int k = 0; k < 3; ++k) {
+    xi[k] = m.xyz[3 * i + k];
+    di[k] = dpat[3 * i + k];
+  }
+  for (int k = 0; k < 6; ++k) qi[k] = mpscale[k] * qpat[6 * i + k];
+#pragma unroll
+  for (int a = 0; a < MAXSH; ++a)
+    if (a < nsi) qs[a] = 0.5 * qsh[is0 + a];
+  double e = 0.0;
+  const int nat = m.nat;
+  for (int j = lane; j < nat; j += 32) {
+    if (j == i) continue;
+    double v[3];
+    for (int k = 0; k < 3; ++k) v[k] = xi[k] - m.xyz[3 * j + k];  // R_i - R_j
+    const double r1 = tab ? 0.0 : sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+    const int js0 = m.at_sh[j], nsj = m.at_sh[j + 1] - js0;
+#pragma unroll
+    for (int a = 0; a < MAXSH; ++a) {
+      if (a >= nsi) break;
+      double acc = 0.0;
+      for (int b = 0; b < nsj; ++b)
+        acc += gam_pair(m, p, tab, r1, is0 + a, js0 + b) * qsh[js0 + b];
+      e += qs[a] * acc;
     }
-    vat[i] = uat + (p.third_atom ? qa_i * qa_i * m.at_gam3[i] : 0.0);
-    for (int k = 0; k < 3; ++k)
-      vdp[3 * i + k] = p.aes ? ud[k] + udd[k] + 2.0 * m.at_dkern[i] * di[k] : 0.0;
-    for (int k = 0; k < 6; ++k)
-      vqp[6 * i + k] = p.aes ? uq[k] + 2.0 * m.at_qkern[i] * qi[k] * mpscale[k] : 0.0;
-  } else {
-    double e = 0.0;
-    for (int a = 0; a < nsi; ++a) {
-      const double q = qsh[is0 + a];
-      e += 0.5 * gsh[a] * q + (p.third_atom ? 0.0 : q * q * q * m.sh_gam3[is0 + a] / 3.0);
-    }
-    if (p.third_atom) e += qa_i * qa_i * qa_i * m.at_gam3[i] / 3.0;
-    if (!p.aes) {
-      eat[i] += e;
-      return;
-    }
-    for (int k = 0; k < 3; ++k) e += di[k] * (ud[k] + 0.5 * udd[k]);
-    for (int k = 0; k < 6; ++k) e += qi[k] * uq[k];
+    if (!p.aes) continue;
+    double g3f3, g5f5, g3f5;
+    aes_scalars(m, p, tab, mrad, r1, i, j, g3f3, g5f5, g3f5);
+    const double* dj = dpat + 3 * j;
+    const double vi = v[0] * di[0] + v[1] * di[1] + v[2] * di[2];
+    const double vj = v[0] * dj[0] + v[1] * dj[1] + v[2] * dj[2];
+    const double dd = di[0] * dj[0] + di[1] * dj[1] + di[2] * dj[2];
+    const double qv = (qi[0] * v[0] + qi[1] * v[1] + qi[3] * v[2]) * v[0] +
+                      (qi[2] * v[1] + qi[4] * v[2]) * v[1] + qi[5] * v[2] * v[2];
+    // charge-dipole, charge-quadrupole, half of the dipole-dipole term
+    e += qat[j] * (g5f5 * qv - g3f3 * vi);
+    e += 0.5 * dd * g3f5 - 1.5 * vi * vj * g5f5;
+  }
+  e = warp_sum(e);
+  if (lane != 0) return;
+  for (int a = 0; a < nsi; ++a) {
+    const double q = qsh[is0 + a];
+    double acc = 0.0;  // on-site gamma block
+    for (int b = 0; b < nsi; ++b)
+      acc += eta_avg(m.sh_hub[is0 + a], m.sh_hub[is0 + b], p.harmonic) * qsh[is0 + b];
+    e += 0.5 * acc * q + (p.third_atom ? 0.0 : q * q * q * m.sh_gam3[is0 + a] / 3.0);
+  }
+  if (p.third_atom) {
+    const double q = qat[i];
+    e += q * q * q * m.at_gam3[i] / 3.0;
+  }
+  if (p.aes) {
     double d2 = 0.0, q2 = 0.0;
     for (int k = 0; k < 3; ++k) d2 += di[k] * di[k];
-    for (int k = 0; k < 6; ++k) q2 += qi[k] * qi[k] * mpscale[k];
+    for (int k = 0; k < 6; ++k) q2 += qi[k] * qpat[6 * i + k];
     e += m.at_dkern[i] * d2 + m.at_qkern[i] * q2;
-    eat[i] += e;
   }
+  eat[i] += e;
 }
-template <int MODE>
+template <int MODE, bool TAB>
 __global__ void k_coulomb(DevMol m, Gfn2Scalars p, const double* __restrict__ mrad,
                           const double* __restrict__ qsh, const double* __restrict__ qat,
                           const double* __restrict__ dpat, const double* __restrict__ qpat,
-                          double* vsh, double* vat, double* vdp, double* vqp, double* eat) {
-  coulomb_dev<MODE>(m, p, mrad, qsh, qat, dpat, qpat, vsh, vat, vdp, vqp, eat);
+                          double* vsh, double* vat, double* vdp, double* vqp, double* eat,
+                          const double* __restrict__ tab) {
+  if (MODE == 0)
+    coulomb_potential_dev(m, p, mrad, qsh, qat, dpat, qpat, vsh, vat, vdp, vqp,
+                          TAB ? tab : nullptr);
+  else
+    coulomb_energy_dev(m, p, mrad, qsh, qat, dpat, qpat, eat, TAB ? tab : nullptr);
+}
+__global__ void k_coulomb_table(DevMol m, Gfn2Scalars p, const double* __restrict__ mrad,
+                                double* tab) {
+  coulomb_table_dev(m, p, mrad, tab);
+}
+
+void launch_coulomb_table(const DevMol& m, const Gfn2Scalars& p, const double* mrad, double* tab,
+                          cudaStream_t s) {
+  ++g_kernel_launches;
+  k_coulomb_table<<<(m.nat * 32 + 63) / 64, 64, 0, s>>>(m, p, mrad, tab);
 }
 
 void launch_coulomb_potential(const DevMol& m, const Gfn2Scalars& p, const double* mrad,
                               const double* qsh, const double* qat, const double* dpat,
                               const double* qpat, double* vsh, double* vat, double* vdp,
-                              double* vqp, cudaStream_t s) {
+                              double* vqp, const double* tab, cudaStream_t s) {
   ++g_kernel_launches;
-  k_coulomb<0><<<(m.nat * 32 + 63) / 64, 64, 0, s>>>(m, p, mrad, qsh, qat, dpat, qpat, vsh, vat,
-                                                         vdp, vqp, nullptr);
+  auto kernel = tab ? k_coulomb<0, true> : k_coulomb<0, false>;
+  kernel<<<(m.nat * 32 + 63) / 64, 64, 0, s>>>(m, p, mrad, qsh, qat, dpat, qpat, vsh, vat, vdp, vqp,
+                                               nullptr, tab);
 }
 
 void launch_coulomb_energy(const DevMol& m, const Gfn2Scalars& p, const double* mrad,
                            const double* qsh, const double* qat, const double* dpat,
-                           const double* qpat, double* eat, cudaStream_t s) {
+                           const double* qpat, double* eat, const double* tab, cudaStream_t s) {
   ++g_kernel_launches;
-  k_coulomb<1><<<(m.nat * 32 + 63) / 64, 64, 0, s>>>(m, p, mrad, qsh, qat, dpat, qpat, nullptr,
-                                                         nullptr, nullptr, nullptr, eat);
+  auto kernel = tab ? k_coulomb<1, true> : k_coulomb<1, false>;
+  kernel<<<(m.nat * 32 + 63) / 64, 64, 0, s>>>(m, p, mrad, qsh, qat, dpat, qpat, nullptr, nullptr,
+                                               nullptr, nullptr, eat, tab);
 }
 
 // ------------------------------------------------------------------------------------
@@ -517,9 +600,7 @@ __device__ __forceinline__ void coulomb_grad_dev(DevMol m, Gfn2Scalars p, const 
       for (int b = 0; b < 3; ++b)
         sg[3 * a + b] += 0.5 * gp[a] * w[b] - 0.25 * (v[a] * ga[b] + ga[a] * v[b]);
   }
-  for (int k = 0; k < 3; ++k) g[k] = warp_sum(g[k]);
-  for (int k = 0; k < 9; ++k) sg[k] = warp_sum(sg[k]);
-  dEdr = warp_sum(dEdr);
+  warp_sums_grad(g, sg, dEdr);
   if (lane == 0) {
     for (int k = 0; k < 3; ++k) grad[3 * i + k] += g[k];
     for (int k = 0; k < 9; ++k) sig_at[9 * i + k] += sg[k];
@@ -572,9 +653,7 @@ __device__ __forceinline__ void repulsion_dev(DevMol m, Gfn2Scalars p, double* e
     for (int a2 = 0; a2 < 3; ++a2)
       for (int c = 0; c < 3; ++c) sg[3 * a2 + c] += 0.5 * f * v[a2] * v[c];
   }
-  e = warp_sum(e);
-  for (int k = 0; k < 3; ++k) g[k] = warp_sum(g[k]);
-  for (int k = 0; k < 9; ++k) sg[k] = warp_sum(sg[k]);
+  warp_sums_grad(g, sg, e);
   if (lane == 0) {
     erep[i] = e;
     if (grad) {
@@ -1396,11 +1475,10 @@ template <int MODE>
 __global__ void kb_coulomb(BARGS, Gfn2Scalars p) {
   BMOL;
   if (MODE == 0)
-    coulomb_dev<0>(q.m, p, q.mrad, q.qsh, q.qat, q.dpat, q.qpat, q.vsh, q.vat, q.vdp, q.vqp,
-                   nullptr, q.ctab);
+    coulomb_potential_dev(q.m, p, q.mrad, q.qsh, q.qat, q.dpat, q.qpat, q.vsh, q.vat, q.vdp,
+                          q.vqp, q.ctab);
   else
-    coulomb_dev<1>(q.m, p, q.mrad, q.qsh_o, q.qat_o, q.dpat_o, q.qpat_o, nullptr, nullptr,
-                   nullptr, nullptr, q.eelec, q.ctab);
+    coulomb_energy_dev(q.m, p, q.mrad, q.qsh_o, q.qat_o, q.dpat_o, q.qpat_o, q.eelec, q.ctab);
 }
 void launch_coulomb_potential_b(const BatchLaunch& b, const Gfn2Scalars& p) {
   if (!b.count) return;
