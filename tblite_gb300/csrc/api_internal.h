@@ -107,6 +107,7 @@ struct Workspace {
   DBuf<double> wbo, ones, pgrad, zgrad;
   // GFN1 per-shell/atom data and D3 dispersion (data and work)
   DBuf<int> sh_valence, sh_perm, d3_nref;
+  DBuf<float> sh_amin;
   DBuf<double> at_gam3, d3_refcn, d3_c6ref, d3_r4r2, d3_rcov, d3_cn, d3_w, d3_dw, d3_dEdcn;
   DBuf<int> d3_sp;
   // implicit solvation: per-atom model arrays [9][nat], grid [230][4], work [4][nat]
@@ -180,6 +181,7 @@ struct _tblite_calculator {
   ModelConstants model;
   std::vector<int> sh_perm;      // s shells, then p shells, each by number of primitives
   int n_s = 0;                   // number of s shells
+  std::vector<float> sh_amin;    // smallest exponent of a shell
   std::vector<int> sh_valence;   // GFN1: first shell of its angular momentum on the atom
   std::vector<double> at_gam3;   // GFN1: atom-resolved third-order hardness derivative
   // D3 data per atom (GFN1, molecules with pairs)

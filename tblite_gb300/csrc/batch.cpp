@@ -182,7 +182,7 @@ struct Plan {
   // offsets (region, offset) of every array
   Piece xyz, at_z, at_sh, sh_atom, sh_l, sh_nprim, sh_alpha, sh_coeff, sh_ao, ao_sh, ao_at, sh_se0,
       sh_kcn, sh_shpoly, sh_zeta, sh_hub, sh_gam3, sh_refocc, at_en, at_rad, at_rcov, at_mprad,
-      at_vcn, at_dkern, at_qkern, at_repa, at_repz, sh_valence, sh_perm, at_gam3;
+      at_vcn, at_dkern, at_qkern, at_repa, at_repz, sh_valence, sh_perm, sh_amin, at_gam3;
   Piece d3_sp, d3_nref, d3_refcn, d3_c6ref, d3_r4r2, d3_rcov, d3_cn, d3_w, d3_dw, d3_dEdcn;
   Piece d4_sp, d4_nref, d4_ngw, d4_refcn, d4_refq, d4_zeff, d4_gam, d4_r4r2, d4_rcov, d4_en,
       d4_c6ref;
@@ -239,6 +239,7 @@ void layout(Plan& pl, Region* R) {
     *p = piece<double>(R, RU, na);
   pl.sh_valence = piece<int>(R, RU, ns);
   pl.sh_perm = piece<int>(R, RU, ns);
+  pl.sh_amin = piece<float>(R, RU, ns);
   if (pl.has_d3) {
     pl.d3_nref = piece<int>(R, RU, na);
     pl.d3_refcn = piece<double>(R, RU, na * D4_MREF);
@@ -394,6 +395,7 @@ MolPtrs make_ptrs(const Plan& pl, const Bases& db) {
   m.sh_valence = db.at<int>(pl.sh_valence);
   m.sh_perm = db.at<int>(pl.sh_perm);
   m.ns = pl.c->n_s;
+  m.sh_amin = db.at<float>(pl.sh_amin);
   m.at_gam3 = db.at<double>(pl.at_gam3);
   q.has_d4 = pl.has_d4 ? 1 : 0;
   q.has_d3 = pl.has_d3 ? 1 : 0;
@@ -653,6 +655,7 @@ std::vector<int> run_chunk(std::vector<Plan>& plans, Arena& ar, _tblite_context*
     stage(hb, pl.at_repz, c->at_repz);
     stage(hb, pl.sh_valence, c->sh_valence);
     stage(hb, pl.sh_perm, c->sh_perm);
+    stage(hb, pl.sh_amin, c->sh_amin);
     stage(hb, pl.at_gam3, c->at_gam3);
     if (pl.has_d3) {
       stage(hb, pl.d3_nref, c->d3_nref);

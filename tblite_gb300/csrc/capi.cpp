@@ -167,6 +167,15 @@ static void orthogonalize_s(int ni, const double* ai, const double* ci, int& nj,
 // Within a form every element record entry and every global constant of the record is used;
 // anything else (another form, d shells, the halogen-bond correction, element-pair factors
 // other than the form's own) is refused with an error.
+// smallest primitive exponent of every shell (screening of shell pairs); follows sh_alpha
+static void smallest_exponents(_tblite_calculator* c) {
+  c->sh_amin.resize(c->nsh);
+  for (int s = 0; s < c->nsh; ++s) {
+    const double* a = c->sh_alpha.data() + (size_t)s * MAXG;
+    c->sh_amin[s] = (float)*std::min_element(a, a + c->sh_nprim[s]);
+  }
+}
+
 static void build_calculator(_tblite_calculator* c, const _tblite_structure* mol,
                              const ParamRecord& rec) {
   int method = 0;
@@ -314,6 +323,7 @@ static void build_calculator(_tblite_calculator* c, const _tblite_structure* mol
     return c->sh_l[x] != c->sh_l[y] ? c->sh_l[x] < c->sh_l[y] : c->sh_nprim[x] < c->sh_nprim[y];
   });
   c->n_s = (int)std::count(c->sh_l.begin(), c->sh_l.end(), 0);
+  smallest_exponents(c);
   c->model.pair_mode = pairs_gfn1 ? 1 : 0;
   if (mol->nat > 1) {
     if (method == 2) build_d4_data(c, mol);
@@ -407,6 +417,7 @@ static void ensure_workspace(_tblite_calculator* c) {
   if (c->params_dirty && w.nat == c->nat && w.nao == c->nao && w.nsh == c->nsh) {
     w.sh_alpha.upload(c->sh_alpha, s);
     w.sh_coeff.upload(c->sh_coeff, s);
+    w.sh_amin.upload(c->sh_amin, s);
     w.sh_zeta.upload(c->sh_zeta, s);
     w.sh_se0.upload(c->sh_se0, s);
     w.sh_kcn.upload(c->sh_kcn, s);
@@ -436,6 +447,7 @@ static void ensure_workspace(_tblite_calculator* c) {
     w.at_repz.upload(c->at_repz, s);
     w.sh_valence.upload(c->sh_valence, s);
     w.sh_perm.upload(c->sh_perm, s);
+    w.sh_amin.upload(c->sh_amin, s);
     w.at_gam3.upload(c->at_gam3, s);
     if (c->has_d3) {
       w.d3_nref.upload(c->d3_nref, s);
@@ -673,6 +685,7 @@ static DevMol dev_mol(const _tblite_calculator* c) {
   m.sh_valence = w.sh_valence.p;
   m.sh_perm = w.sh_perm.p;
   m.ns = c->n_s;
+  m.sh_amin = w.sh_amin.p;
   m.at_gam3 = w.at_gam3.p;
   return m;
 }
@@ -1700,6 +1713,7 @@ void tblite_gb300_set_calculator_slater_exponents(tblite_context ctx, tblite_cal
     calc->sh_zeta[i] = zeta[i];
   }
   calc->min_alpha = min_alpha;
+  smallest_exponents(calc);
   calc->params_dirty = true;
 }
 

@@ -78,6 +78,7 @@ struct DevMol {
   const double* at_repz;   // repulsion zeff
   const int* sh_perm;      // [nsh] s shells, then p shells, each by number of primitives
   int ns;                  // number of s shells
+  const float* sh_amin;    // [nsh] smallest exponent of a shell
   const int* sh_valence;   // GFN1: 1 for the first shell of its angular momentum on the atom
   const double* at_gam3;   // GFN1: atom-resolved third-order hardness derivative
 };

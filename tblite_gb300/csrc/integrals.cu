@@ -54,8 +54,7 @@ __device__ __forceinline__ int cexp(int l, int c, int k) { return (l == 1 && c =
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void tri_index(long long t, int& i, int& j) {
   // t = i*(i+1)/2 + j, 0 <= j <= i
-  double d = sqrt(8.0 * (double)t + 1.0);
-  i = (int)((d - 1.0) * 0.5);
+  i = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);  // corrected below
   while ((long long)i * (i + 1) / 2 > t) --i;
   while ((long long)(i + 1) * (i + 2) / 2 <= t) ++i;
   j = (int)(t - (long long)i * (i + 1) / 2);
@@ -105,19 +104,97 @@ __device__ __forceinline__ double hscale_of(const DevMol& m, const Gfn2Scalars& 
 }
 
 // Shell pairs are walked by kind: DevMol.sh_perm lists the s shells, then the p shells, each by
-// number of primitives, and the pairs come as s-s, then s-p, then p-p, each kind from a multiple of
-// 32 on.  An FP64 instruction costs a warp the same whatever its active lanes do, so a warp of
+// number of primitives, and the pairs come as s-s, then s-p, then p-p, each kind from a full warp
+// on.  An FP64 instruction costs a warp the same whatever its active lanes do, so a warp of
 // mixed kinds pays for every kind in turn (for water 16 units of component pairs where its lanes
-// need 2.25 on average) and for the longest primitive loops among its lanes.
-__device__ __forceinline__ long long pad32(long long t) { return (t + 31) & ~31ll; }
+// need 2.25 on average) and for the longest primitive loops among its lanes.  Two forms:
+//
+// G == 1, one lane per pair.  A warp tests `rounds` times 32 pairs and queues the ones with any
+// primitive pair to evaluate until 32 are together: of the p-p pairs of 64 waters four in five lie
+// beyond the reach of their exponents, and lanes left idle by them cost as much as busy ones.
+// G == 8, eight lanes per pair, each with every eighth primitive pair, for molecules and batches
+// that leave the chip empty otherwise: the primitive loop of a pair is the length of the kernel
+// there.
+constexpr int WALK_G = 8;
+constexpr int WALK_THREADS = 128;
+// the form and the rounds for a number of tasks: 8 lanes while that is at most eight warps per
+// scheduler, several rounds once the warps left are still as many
+struct Walk {
+  int lanes, rounds;
+};
+inline Walk walk_of(long long tasks) {
+  const long long full = (long long)device_sm_count() * 4 * 8 * 32;  // lanes
+  if (tasks * WALK_G <= full) return {WALK_G, 1};
+  return {1, tasks >= 4 * full ? 8 : tasks >= full ? 4 : 1};
+}
+// tasks of a kind padded to whole warps
+__host__ __device__ inline long long walk_pad(long long t, int G, int rounds) {
+  const int w = 32 / G * rounds;
+  return (t + w - 1) / w * w;
+}
+inline unsigned walk_blocks(long long padded, const Walk& w) {
+  const long long per = (long long)WALK_THREADS / w.lanes * w.rounds;
+  return (unsigned)((padded + per - 1) / per);
+}
+// a warp's tasks base + [0, 32 / G rounds) of `count`: work(t) for those with test(t), all lanes of a
+// task's group together
+template <int G, class Test, class Work>
+__device__ __forceinline__ void walk(long long base, long long count, int rounds, Test test,
+                                     Work work) {
+  const int lane = threadIdx.x & 31;
+  if constexpr (G > 1) {
+    const long long t = base + lane / G;
+    if (t < count && test(t)) work(t);
+  } else {
+    if (rounds == 1) {
+      const long long t = base + lane;
+      if (t < count && test(t)) work(t);
+      return;
+    }
+    __shared__ int queue[WALK_THREADS / 32][64];
+    int* q = queue[threadIdx.x >> 5];
+    int held = 0;
+    for (int r = 0; r < rounds; ++r) {
+      const long long t = base + 32 * r + lane;
+      const bool in = t < count && test(t);
+      const unsigned mask = __ballot_sync(0xffffffffu, in);
+      if (in) q[held + __popc(mask & ((1u << lane) - 1))] = 32 * r + lane;
+      held += __popc(mask);
+      __syncwarp();
+      const bool last = r == rounds - 1;
+      while (held >= 32 || (last && held > 0)) {
+        if (lane < held) work(base + q[lane]);
+        __syncwarp();
+        held = max(held - 32, 0);
+        const int rest = q[32 + lane];
+        __syncwarp();
+        q[lane] = rest;
+        __syncwarp();
+      }
+    }
+  }
+}
+// false if every primitive pair of the two shells is screened, or the atoms are beyond the cutoff:
+// by the smallest exponents in FP32, with a margin
+__device__ __forceinline__ bool shells_near(const DevMol& m, const Gfn2Scalars& p, int a, int b) {
+  const int ia = m.sh_atom[a], ib = m.sh_atom[b];
+  if (ia == ib) return true;
+  double v[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v[k] = m.xyz[3 * ia + k] - m.xyz[3 * ib + k];
+  const double r2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+  if (r2 > p.h0_cutoff * p.h0_cutoff * 1.0001) return false;
+  const float x = m.sh_amin[a], y = m.sh_amin[b];
+  return !(x * y / (x + y) * (float)r2 > (float)INTCUT * 1.001f);
+}
 
 // ket shell ish >= bra shell jsh of angular momenta LI, LJ; NI ket components from the cartesian
 // component CI on.  The products are written as rounded multiplications and one FMA, so that a factor
-// known to be 1 changes no rounding.
-template <int LI, int LJ, int NI, int CI>
+// known to be 1 changes no rounding.  sub: this lane's place in the pair's group of G.
+template <int G, int LI, int LJ, int NI, int CI>
 __device__ __forceinline__ void build_h0_pair(const DevMol& m, const Gfn2Scalars& p,
                            const double* __restrict__ se, double* S,
-                           double* H, double* D, double* Q, int ish, int jsh) {
+                           double* H, double* D, double* Q, int ish, int jsh, int sub) {
   constexpr int NJ = 2 * LJ + 1;
   const int iat = m.sh_atom[ish], jat = m.sh_atom[jsh];
   double vec[3];
@@ -130,13 +207,15 @@ __device__ __forceinline__ void build_h0_pair(const DevMol& m, const Gfn2Scalars
   const bool onsite = iat == jat;
   if (!onsite && (r2 > p.h0_cutoff * p.h0_cutoff || r2 < 2.220446049250313e-16)) return;
   // accumulators per ket and bra component: S, M1[3], M2[6] about A
-  double aS[NI][NJ] = {{0}}, aM1[NI][NJ][3] = {{{0}}}, aM2[NI][NJ][6] = {{{0}}};
+  double acc[NI * NJ * 10];
+#pragma unroll
+  for (int k = 0; k < NI * NJ * 10; ++k) acc[k] = 0.0;
   const int npi = m.sh_nprim[ish], npj = m.sh_nprim[jsh];
   const double pi3 = 5.568327996831708;  // pi^(3/2)
-  for (int ip = 0; ip < npi; ++ip) {
-    const double ai = m.sh_alpha[ish * MAXG + ip];
-    const double ci_ = m.sh_coeff[ish * MAXG + ip];
-    for (int jp = 0; jp < npj; ++jp) {
+  for (int t = sub; t < npi * npj; t += G) {
+      const int ip = t / npj, jp = t - ip * npj;
+      const double ai = m.sh_alpha[ish * MAXG + ip];
+      const double ci_ = m.sh_coeff[ish * MAXG + ip];
       const double aj = m.sh_alpha[jsh * MAXG + jp];
       const double eta = ai + aj, oeta = 1.0 / eta;
       const double est = ai * aj * r2 * oeta;
@@ -159,22 +238,27 @@ __device__ __forceinline__ void build_h0_pair(const DevMol& m, const Gfn2Scalars
 #pragma unroll
             for (int e = 0; e < 3; ++e) V[k][e] = O1(M, k, a + e, b, vec[k]);
           }
-          auto add = [&](double& acc, int ex, int ey, int ez) {
-            acc = fma(__dmul_rn(__dmul_rn(cc, V[0][ex]), V[1][ey]), V[2][ez], acc);
+          double* A = acc + (ii * NJ + cj) * 10;
+          auto add = [&](int k, int ex, int ey, int ez) {
+            A[k] = fma(__dmul_rn(__dmul_rn(cc, V[0][ex]), V[1][ey]), V[2][ez], A[k]);
           };
-          add(aS[ii][cj], 0, 0, 0);
-          add(aM1[ii][cj][0], 1, 0, 0);
-          add(aM1[ii][cj][1], 0, 1, 0);
-          add(aM1[ii][cj][2], 0, 0, 1);
-          add(aM2[ii][cj][0], 2, 0, 0);  // xx
-          add(aM2[ii][cj][1], 1, 1, 0);  // xy
-          add(aM2[ii][cj][2], 0, 2, 0);  // yy
-          add(aM2[ii][cj][3], 1, 0, 1);  // xz
-          add(aM2[ii][cj][4], 0, 1, 1);  // yz
-          add(aM2[ii][cj][5], 0, 0, 2);  // zz
+          add(0, 0, 0, 0);
+          add(1, 1, 0, 0);
+          add(2, 0, 1, 0);
+          add(3, 0, 0, 1);
+          add(4, 2, 0, 0);  // xx
+          add(5, 1, 1, 0);  // xy
+          add(6, 0, 2, 0);  // yy
+          add(7, 1, 0, 1);  // xz
+          add(8, 0, 1, 1);  // yz
+          add(9, 0, 0, 2);  // zz
         }
       }
     }
+  if constexpr (G > 1) {
+    const unsigned mask = ((1u << G) - 1) << ((threadIdx.x & 31) & ~(G - 1));
+    group_sums<G>(acc, mask);
+    if (sub != 0) return;
   }
   double hij;
   if (!onsite) {
@@ -195,18 +279,19 @@ __device__ __forceinline__ void build_h0_pair(const DevMol& m, const Gfn2Scalars
     const int io = m.sh_ao[ish] + (LI == 1 ? sph_of_cart_p(CI + ii) : 0);
     const int mj = LJ == 1 ? sph_of_cart_p(cj) : 0;
     const int jo = jo0 + mj;
-    const double s = aS[ii][cj];
+    const double* A = acc + (ii * NJ + cj) * 10;
+    const double s = A[0];
     double dA[3], dB[3], qA[6], qB[6];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      dA[k] = aM1[ii][cj][k];
-      dB[k] = aM1[ii][cj][k] + vec[k] * s;  // (r-B) = (r-A) + vec
+      dA[k] = A[1 + k];
+      dB[k] = A[1 + k] + vec[k] * s;  // (r-B) = (r-A) + vec
     }
     const int qa[6] = {0, 0, 1, 0, 1, 2}, qb[6] = {0, 1, 1, 2, 2, 2};
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      qA[q] = aM2[ii][cj][q];
-      qB[q] = aM2[ii][cj][q] + vec[qa[q]] * aM1[ii][cj][qb[q]] + vec[qb[q]] * aM1[ii][cj][qa[q]]
+      qA[q] = A[4 + q];
+      qB[q] = A[4 + q] + vec[qa[q]] * A[1 + qb[q]] + vec[qb[q]] * A[1 + qa[q]]
               + vec[qa[q]] * vec[qb[q]] * s;
     }
     // traceless
@@ -236,48 +321,82 @@ __device__ __forceinline__ void build_h0_pair(const DevMol& m, const Gfn2Scalars
     }
   }
 }
-// tasks of the H0 build: one thread per s-s and s-p pair, three per p-p pair (the three ket
-// components one kind after the other, so that the component is known at compile time)
-__host__ __device__ inline long long h0_tasks(long long nsh, long long np) {
-  return nsh * (nsh + 1) / 2 + np * (np + 1) + 5 * 32;
+// tasks of the H0 build: one per s-s and s-p pair, three per p-p pair (the three ket components one
+// kind after the other, so that the component is known at compile time)
+inline long long h0_padded(long long nsh, long long np, const Walk& w) {
+  // (a batch's molecules have at most nsh shells and np p shells: any split of them stays below)
+  return walk_pad(nsh * (nsh + 1) / 2, w.lanes, w.rounds) + 3LL * 32 * w.rounds +
+         3 * walk_pad(np * (np + 1) / 2, w.lanes, w.rounds);
 }
+template <int G>
 __device__ __forceinline__ void build_h0_dev(const DevMol& m, const Gfn2Scalars& p,
                            const double* __restrict__ se, double* S, double* H, double* D,
-                           double* Q) {
-  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+                           double* Q, int rounds) {
+  const int sub = threadIdx.x & (G - 1);
+  const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  long long t = w * (32 / G * rounds);  // first task of the warp
   const int ns = m.ns, np = m.nsh - m.ns;
   const long long nss = (long long)ns * (ns + 1) / 2, nsp = (long long)ns * np;
-  if (t < pad32(nss)) {
-    if (t >= nss) return;
-    int i, j;
-    tri_index(t, i, j);
-    const int a = m.sh_perm[i], b = m.sh_perm[j];
-    build_h0_pair<0, 0, 1, 0>(m, p, se, S, H, D, Q, max(a, b), min(a, b));
-    return;
-  }
-  t -= pad32(nss);
-  if (t < pad32(nsp)) {
-    if (t >= nsp) return;
-    const int a = m.sh_perm[ns + (int)(t / ns)], b = m.sh_perm[(int)(t % ns)];  // p, s
-    if (a > b) build_h0_pair<1, 0, 3, 0>(m, p, se, S, H, D, Q, a, b);
-    else build_h0_pair<0, 1, 1, 0>(m, p, se, S, H, D, Q, b, a);
-    return;
-  }
-  t -= pad32(nsp);
   const long long npp = (long long)np * (np + 1) / 2;
-  const int c = (int)(t / max(pad32(npp), 1ll));
-  t -= c * pad32(npp);
-  if (c > 2 || t >= npp) return;
-  int i, j;
-  tri_index(t, i, j);
-  const int x = m.sh_perm[ns + i], y = m.sh_perm[ns + j], a = max(x, y), b = min(x, y);
-  if (c == 0) build_h0_pair<1, 1, 1, 0>(m, p, se, S, H, D, Q, a, b);
-  else if (c == 1) build_h0_pair<1, 1, 1, 1>(m, p, se, S, H, D, Q, a, b);
-  else build_h0_pair<1, 1, 1, 2>(m, p, se, S, H, D, Q, a, b);
+  const long long pss = walk_pad(nss, G, rounds), psp = walk_pad(nsp, G, rounds);
+  const long long ppp = walk_pad(npp, G, rounds);
+  const int* __restrict__ sp = m.sh_perm;
+  const int* __restrict__ pp = m.sh_perm + ns;
+  auto tri = [&](const int* list, long long u, int& a, int& b) {
+    int i, j;
+    tri_index(u, i, j);
+    a = max(list[i], list[j]);
+    b = min(list[i], list[j]);
+  };
+  if (t < pss) {
+    walk<G>(t, nss, rounds,
+            [&](long long u) {
+              int a, b;
+              tri(sp, u, a, b);
+              return shells_near(m, p, a, b);
+            },
+            [&](long long u) {
+              int a, b;
+              tri(sp, u, a, b);
+              build_h0_pair<G, 0, 0, 1, 0>(m, p, se, S, H, D, Q, a, b, sub);
+            });
+    return;
+  }
+  t -= pss;
+  if (t < psp) {
+    walk<G>(t, nsp, rounds,
+            [&](long long u) { return shells_near(m, p, pp[u / ns], sp[u % ns]); },
+            [&](long long u) {
+              const int a = pp[u / ns], b = sp[u % ns];
+              if (a > b) build_h0_pair<G, 1, 0, 3, 0>(m, p, se, S, H, D, Q, a, b, sub);
+              else build_h0_pair<G, 0, 1, 1, 0>(m, p, se, S, H, D, Q, b, a, sub);
+            });
+    return;
+  }
+  t -= psp;
+  if (ppp == 0) return;
+  const int c = (int)(t / ppp);
+  t -= c * ppp;
+  if (c > 2) return;
+  walk<G>(t, npp, rounds,
+          [&](long long u) {
+            int a, b;
+            tri(pp, u, a, b);
+            return shells_near(m, p, a, b);
+          },
+          [&](long long u) {
+            int a, b;
+            tri(pp, u, a, b);
+            if (c == 0) build_h0_pair<G, 1, 1, 1, 0>(m, p, se, S, H, D, Q, a, b, sub);
+            else if (c == 1) build_h0_pair<G, 1, 1, 1, 1>(m, p, se, S, H, D, Q, a, b, sub);
+            else build_h0_pair<G, 1, 1, 1, 2>(m, p, se, S, H, D, Q, a, b, sub);
+          });
 }
-__global__ void k_build_h0(DevMol m, Gfn2Scalars p, const double* __restrict__ se, double* S,
-                           double* H, double* D, double* Q) {
-  build_h0_dev(m, p, se, S, H, D, Q);
+template <int G>
+__global__ void __launch_bounds__(WALK_THREADS)
+    k_build_h0(DevMol m, Gfn2Scalars p, const double* __restrict__ se, double* S, double* H,
+               double* D, double* Q, int rounds) {
+  build_h0_dev<G>(m, p, se, S, H, D, Q, rounds);
 }
 
 void launch_build_h0(const DevMol& m, const Gfn2Scalars& p, const double* se, double* S,
@@ -287,10 +406,13 @@ void launch_build_h0(const DevMol& m, const Gfn2Scalars& p, const double* se, do
   cudaMemsetAsync(H, 0, nn * sizeof(double), s);
   cudaMemsetAsync(D, 0, 3 * nn * sizeof(double), s);
   cudaMemsetAsync(Q, 0, 6 * nn * sizeof(double), s);
-  const long long nthr = h0_tasks(m.nsh, m.nsh - m.ns);
-  const int bs = 128;
+  const Walk w = walk_of(h0_padded(m.nsh, m.nsh - m.ns, {1, 1}));
+  const unsigned blocks = walk_blocks(h0_padded(m.nsh, m.nsh - m.ns, w), w);
   ++g_kernel_launches;
-  k_build_h0<<<(unsigned)((nthr + bs - 1) / bs), bs, 0, s>>>(m, p, se, S, H, D, Q);
+  if (w.lanes == 1)
+    k_build_h0<1><<<blocks, WALK_THREADS, 0, s>>>(m, p, se, S, H, D, Q, w.rounds);
+  else
+    k_build_h0<WALK_G><<<blocks, WALK_THREADS, 0, s>>>(m, p, se, S, H, D, Q, w.rounds);
 }
 
 // One primitive pair of the H0 gradient for shells of angular momenta LI (bra, A) and LJ
@@ -367,7 +489,7 @@ __device__ __forceinline__ void h0g_prim(const Moments& M, const double (&vec)[3
 }
 
 // ---------------------------------------------------------------------------------------
-// H0 gradient: one thread per cross-atom shell pair, by kind (of an s-p pair the p shell is ish).
+// H0 gradient over the cross-atom shell pairs, by kind (of an s-p pair the p shell is ish).
 // The reference formula
 // (h0.f90:528-560) is contracted on the fly:
 //   dG = sum_ji [ sval dS + 2 P hij S dsv - P d<j|O|i>/dR_A ] ,
@@ -375,25 +497,22 @@ __device__ __forceinline__ void h0g_prim(const Moments& M, const double (&vec)[3
 // where O is the multipole potential operator of atoms A and B written as a polynomial in
 // (r - A).  The operator on A moves with A, which adds  P (vA_c S + sum_b (1+d_cb) wA_cb D_b).
 // ---------------------------------------------------------------------------------------
-template <int LI, int LJ>
+template <int G, int LI, int LJ>
 __device__ __forceinline__ void h0_gradient_pair(const DevMol& m, const Gfn2Scalars& p,
                               const double* __restrict__ se,
                               const double* __restrict__ P, const double* __restrict__ W,
                               const double* __restrict__ vao, const double* __restrict__ vdp,
                               const double* __restrict__ vqp, double* grad,
-                              double* dEdcn, int ish, int jsh, double (&vec)[3], double (&dG)[3]) {
+                              double* dEdcn, int ish, int jsh, int sub, double (&vir)[6]) {
   const int iat = m.sh_atom[ish], jat = m.sh_atom[jsh];
   if (iat == jat) return;
-  double r2 = 0.0;
+  double vec[3], dG[3] = {0.0, 0.0, 0.0}, r2 = 0.0;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     vec[k] = m.xyz[3 * iat + k] - m.xyz[3 * jat + k];
     r2 += vec[k] * vec[k];
   }
-  if (r2 > p.h0_cutoff * p.h0_cutoff || r2 < 2.220446049250313e-16) {
-    vec[0] = vec[1] = vec[2] = 0.0;
-    return;
-  }
+  if (r2 > p.h0_cutoff * p.h0_cutoff || r2 < 2.220446049250313e-16) return;
   constexpr int nci = 2 * LI + 1, ncj = 2 * LJ + 1;
   const double rr = sqrt(sqrt(r2) / (m.at_rad[iat] + m.at_rad[jat]));
   const double polyi = 1.0 + m.sh_shpoly[ish] * rr, polyj = 1.0 + m.sh_shpoly[jsh] * rr;
@@ -453,22 +572,32 @@ __device__ __forceinline__ void h0_gradient_pair(const DevMol& m, const Gfn2Scal
   double PS = 0.0, PD[3] = {0, 0, 0};
   const int npi = m.sh_nprim[ish], npj = m.sh_nprim[jsh];
   const double pi3 = 5.568327996831708;
-  for (int ip = 0; ip < npi; ++ip) {
+  for (int t = sub; t < npi * npj; t += G) {
+    const int ip = t / npj, jp = t - ip * npj;
     const double ai = m.sh_alpha[ish * MAXG + ip];
     const double ci_ = m.sh_coeff[ish * MAXG + ip];
-    for (int jp = 0; jp < npj; ++jp) {
-      const double aj = m.sh_alpha[jsh * MAXG + jp];
-      const double eta = ai + aj, oeta = 1.0 / eta;
-      const double est = ai * aj * r2 * oeta;
-      if (est > INTCUT) continue;
-      const double cc = ci_ * m.sh_coeff[jsh * MAXG + jp] * exp(-est) * pi3 * oeta * sqrt(oeta);
-      double pa[3];
+    const double aj = m.sh_alpha[jsh * MAXG + jp];
+    const double eta = ai + aj, oeta = 1.0 / eta;
+    const double est = ai * aj * r2 * oeta;
+    if (est > INTCUT) continue;
+    const double cc = ci_ * m.sh_coeff[jsh * MAXG + jp] * exp(-est) * pi3 * oeta * sqrt(oeta);
+    double pa[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) pa[k] = -vec[k] * aj * oeta;
-      Moments M;
-      gauss_moments(pa, eta, M);
-      h0g_prim<LI, LJ>(M, vec, ai, cc, wp, ws, c0, c1, c2, dG, PS, PD);
+    for (int k = 0; k < 3; ++k) pa[k] = -vec[k] * aj * oeta;
+    Moments M;
+    gauss_moments(pa, eta, M);
+    h0g_prim<LI, LJ>(M, vec, ai, cc, wp, ws, c0, c1, c2, dG, PS, PD);
+  }
+  if constexpr (G > 1) {
+    double v[7] = {dG[0], dG[1], dG[2], PS, PD[0], PD[1], PD[2]};
+    group_sums<G>(v, ((1u << G) - 1) << ((threadIdx.x & 31) & ~(G - 1)));
+    if (sub != 0) return;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      dG[k] = v[k];
+      PD[k] = v[4 + k];
     }
+    PS = v[3];
   }
   // operator on A moves with A;  symmetric quadrupole weight matrix of atom A
   const double wAm[3][3] = {{wA[0], wA[1], wA[3]}, {wA[1], wA[2], wA[4]}, {wA[3], wA[4], wA[5]}};
@@ -488,47 +617,74 @@ __device__ __forceinline__ void h0_gradient_pair(const DevMol& m, const Gfn2Scal
     atomicAdd(grad + 3 * iat + c, dG[c]);
     atomicAdd(grad + 3 * jat + c, -dG[c]);
   }
+  // virial: the six distinct elements of the symmetric 3 x 3
+#pragma unroll
+  for (int q = 0; q < 6; ++q)
+    vir[q] += 0.5 * (vec[qa[q]] * dG[qb[q]] + dG[qa[q]] * vec[qb[q]]);
 }
+inline long long h0_gradient_padded(long long nsh, const Walk& w) {
+  return walk_pad(nsh * (nsh + 1) / 2, w.lanes, w.rounds) + 3LL * 32 * w.rounds;
+}
+template <int G>
 __device__ __forceinline__ void h0_gradient_dev(const DevMol& m, const Gfn2Scalars& p,
                               const double* __restrict__ se,
                               const double* __restrict__ P, const double* __restrict__ W,
                               const double* __restrict__ vao, const double* __restrict__ vdp,
                               const double* __restrict__ vqp, double* grad, double* sigma,
-                              double* dEdcn) {
-  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+                              double* dEdcn, int rounds) {
+  const int sub = threadIdx.x & (G - 1);
+  const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  long long t = w * (32 / G * rounds);  // first task of the warp
   const int ns = m.ns, np = m.nsh - m.ns;
   const long long nss = (long long)ns * (ns + 1) / 2, nsp = (long long)ns * np;
-  // every thread reaches the warp-wide virial sum at the end: pairs that contribute nothing
-  // (outside the list, on one atom, beyond the cutoff) skip the work, not the sum
-  double vec[3] = {0.0, 0.0, 0.0}, dG[3] = {0.0, 0.0, 0.0};
-  int i, j;
-  if (t < pad32(nss)) {
-    if (t < nss) {
-      tri_index(t, i, j);
-      h0_gradient_pair<0, 0>(m, p, se, P, W, vao, vdp, vqp, grad, dEdcn, m.sh_perm[i],
-                             m.sh_perm[j], vec, dG);
-    }
-  } else if (t < pad32(nss) + pad32(nsp)) {
-    t -= pad32(nss);
-    if (t < nsp)
-      h0_gradient_pair<1, 0>(m, p, se, P, W, vao, vdp, vqp, grad, dEdcn,
-                             m.sh_perm[ns + (int)(t / ns)], m.sh_perm[(int)(t % ns)], vec, dG);
+  const long long npp = (long long)np * (np + 1) / 2;
+  const long long pss = walk_pad(nss, G, rounds), psp = walk_pad(nsp, G, rounds);
+  const int* __restrict__ sp = m.sh_perm;
+  const int* __restrict__ pp = m.sh_perm + ns;
+  double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  auto near = [&](int a, int b) {
+    return m.sh_atom[a] != m.sh_atom[b] && shells_near(m, p, a, b);
+  };
+  if (t < pss) {
+    walk<G>(t, nss, rounds,
+            [&](long long u) {
+              int i, j;
+              tri_index(u, i, j);
+              return near(sp[i], sp[j]);
+            },
+            [&](long long u) {
+              int i, j;
+              tri_index(u, i, j);
+              h0_gradient_pair<G, 0, 0>(m, p, se, P, W, vao, vdp, vqp, grad, dEdcn, sp[i], sp[j],
+                                        sub, v);
+            });
+  } else if (t < pss + psp) {
+    walk<G>(t - pss, nsp, rounds, [&](long long u) { return near(pp[u / ns], sp[u % ns]); },
+            [&](long long u) {
+              h0_gradient_pair<G, 1, 0>(m, p, se, P, W, vao, vdp, vqp, grad, dEdcn, pp[u / ns],
+                                        sp[u % ns], sub, v);
+            });
   } else {
-    t -= pad32(nss) + pad32(nsp);
-    if (t < (long long)np * (np + 1) / 2) {
-      tri_index(t, i, j);
-      h0_gradient_pair<1, 1>(m, p, se, P, W, vao, vdp, vqp, grad, dEdcn, m.sh_perm[ns + i],
-                             m.sh_perm[ns + j], vec, dG);
-    }
+    walk<G>(t - pss - psp, npp, rounds,
+            [&](long long u) {
+              int i, j;
+              tri_index(u, i, j);
+              return near(pp[i], pp[j]);
+            },
+            [&](long long u) {
+              int i, j;
+              tri_index(u, i, j);
+              h0_gradient_pair<G, 1, 1>(m, p, se, P, W, vao, vdp, vqp, grad, dEdcn, pp[i], pp[j],
+                                        sub, v);
+            });
   }
-  // virial: the six distinct elements of the symmetric 3 x 3 summed over the warp, then one
-  // atomic per element and warp (every pair of a molecule adds to the same nine numbers)
-  const int va[6] = {0, 0, 1, 0, 1, 2}, vb[6] = {0, 1, 1, 2, 2, 2};
-  double v[6];
+  // one atomic per element and warp (every pair of a molecule adds to the same nine numbers)
+  bool any = false;
 #pragma unroll
-  for (int e = 0; e < 6; ++e)
-    v[e] = 0.5 * (vec[va[e]] * dG[vb[e]] + dG[va[e]] * vec[vb[e]]);
+  for (int e = 0; e < 6; ++e) any = any || v[e] != 0.0;
+  if (!__any_sync(0xffffffffu, any)) return;
   warp_sums(v);
+  const int va[6] = {0, 0, 1, 0, 1, 2}, vb[6] = {0, 1, 1, 2, 2, 2};
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll
     for (int e = 0; e < 6; ++e) {
@@ -538,12 +694,14 @@ __device__ __forceinline__ void h0_gradient_dev(const DevMol& m, const Gfn2Scala
     }
   }
 }
-__global__ void k_h0_gradient(DevMol m, Gfn2Scalars p, const double* __restrict__ se,
-                              const double* __restrict__ P, const double* __restrict__ W,
-                              const double* __restrict__ vao, const double* __restrict__ vdp,
-                              const double* __restrict__ vqp, double* grad, double* sigma,
-                              double* dEdcn) {
-  h0_gradient_dev(m, p, se, P, W, vao, vdp, vqp, grad, sigma, dEdcn);
+template <int G>
+__global__ void __launch_bounds__(WALK_THREADS)
+    k_h0_gradient(DevMol m, Gfn2Scalars p, const double* __restrict__ se,
+                  const double* __restrict__ P, const double* __restrict__ W,
+                  const double* __restrict__ vao, const double* __restrict__ vdp,
+                  const double* __restrict__ vqp, double* grad, double* sigma, double* dEdcn,
+                  int rounds) {
+  h0_gradient_dev<G>(m, p, se, P, W, vao, vdp, vqp, grad, sigma, dEdcn, rounds);
 }
 
 // on-site CN derivative of the diagonal levels: dEdcn_A += sum_{mu in A} dse/dcn P_mumu
@@ -565,17 +723,21 @@ __global__ void k_h0_onsite_dcn(DevMol m, const double* __restrict__ P, double* 
 void launch_h0_gradient(const DevMol& m, const Gfn2Scalars& p, const double* se, const double* P,
                         const double* W, const double* vao, const double* vdp, const double* vqp,
                         double* grad, double* sigma, double* dEdcn, cudaStream_t s) {
-  const long long npair = (long long)m.nsh * (m.nsh + 1) / 2 + 64;
-  const int bs = 128;
+  const Walk w = walk_of(h0_gradient_padded(m.nsh, {1, 1}));
+  const unsigned blocks = walk_blocks(h0_gradient_padded(m.nsh, w), w);
   ++g_kernel_launches;
-  k_h0_gradient<<<(unsigned)((npair + bs - 1) / bs), bs, 0, s>>>(m, p, se, P, W, vao, vdp, vqp,
-                                                                   grad, sigma, dEdcn);
+  if (w.lanes == 1)
+    k_h0_gradient<1><<<blocks, WALK_THREADS, 0, s>>>(m, p, se, P, W, vao, vdp, vqp, grad, sigma,
+                                                     dEdcn, w.rounds);
+  else
+    k_h0_gradient<WALK_G><<<blocks, WALK_THREADS, 0, s>>>(m, p, se, P, W, vao, vdp, vqp, grad,
+                                                          sigma, dEdcn, w.rounds);
   ++g_kernel_launches;
   k_h0_onsite_dcn<<<(m.nat + 127) / 128, 128, 0, s>>>(m, P, dEdcn);
 }
 
 // ---------------------------------------------------------------------------------------
-// dE/dzeta of the Slater exponents (GFN2-xTB), one thread per ordered shell pair (i, j): the
+// dE/dzeta of the Slater exponents (GFN2-xTB), one lane per ordered shell pair (i, j): the
 // derivative acts on the i function only; pair (j, i) carries the one of zeta_j.  A primitive
 // of exponent alpha = alpha0 zeta^2 with its normalisation (2 alpha/pi)^(3/4) (4 alpha)^(l/2)
 // gives  d phi / d zeta = (2 / zeta) sum_k c_k [(3/4 + l/2) - alpha_k |r - A|^2] g_k ,  so the
@@ -710,6 +872,14 @@ __device__ __forceinline__ void zeta_grad_pair(const DevMol& m, const Gfn2Scalar
   atomicAdd(dz + ish, val);
 }
 // ordered pairs by kind: s-s, s-p, p-s, p-p
+inline long long zeta_padded(long long nsh, const Walk& w) {
+  return walk_pad(nsh * nsh, 1, w.rounds) + 4LL * 32 * w.rounds;
+}
+inline Walk zeta_walk(long long tasks) {
+  Walk w = walk_of(tasks);
+  w.lanes = 1;
+  return w;
+}
 __device__ __forceinline__ void zeta_grad_dev(const DevMol& m, const Gfn2Scalars& p,
                                               const double* __restrict__ se,
                                               const double* __restrict__ P,
@@ -717,94 +887,123 @@ __device__ __forceinline__ void zeta_grad_dev(const DevMol& m, const Gfn2Scalars
                                               const double* __restrict__ vao,
                                               const double* __restrict__ vdp,
                                               const double* __restrict__ vqp, double* dz,
-                                              long long t) {
+                                              int rounds) {
+  const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  long long t = w * (32 * rounds);  // first task of the warp
   const int ns = m.ns, np = m.nsh - m.ns;
   const long long nss = (long long)ns * ns, nsp = (long long)ns * np;
+  const long long pss = walk_pad(nss, 1, rounds), psp = walk_pad(nsp, 1, rounds);
   const int* __restrict__ sp = m.sh_perm;
   const int* __restrict__ pp = m.sh_perm + ns;
-  if (t < pad32(nss)) {
-    if (t < nss)
-      zeta_grad_pair<0, 0>(m, p, se, P, W, vao, vdp, vqp, dz, sp[t / ns], sp[t % ns]);
+  auto near = [&](int a, int b) { return shells_near(m, p, a, b); };
+  if (t < pss) {
+    walk<1>(t, nss, rounds, [&](long long u) { return near(sp[u / ns], sp[u % ns]); },
+            [&](long long u) {
+              zeta_grad_pair<0, 0>(m, p, se, P, W, vao, vdp, vqp, dz, sp[u / ns], sp[u % ns]);
+            });
     return;
   }
-  t -= pad32(nss);
-  if (t < pad32(nsp)) {
-    if (t < nsp) zeta_grad_pair<0, 1>(m, p, se, P, W, vao, vdp, vqp, dz, sp[t / np], pp[t % np]);
+  t -= pss;
+  if (t < psp) {
+    walk<1>(t, nsp, rounds, [&](long long u) { return near(sp[u / np], pp[u % np]); },
+            [&](long long u) {
+              zeta_grad_pair<0, 1>(m, p, se, P, W, vao, vdp, vqp, dz, sp[u / np], pp[u % np]);
+            });
     return;
   }
-  t -= pad32(nsp);
-  if (t < pad32(nsp)) {
-    if (t < nsp) zeta_grad_pair<1, 0>(m, p, se, P, W, vao, vdp, vqp, dz, pp[t / ns], sp[t % ns]);
+  t -= psp;
+  if (t < psp) {
+    walk<1>(t, nsp, rounds, [&](long long u) { return near(pp[u / ns], sp[u % ns]); },
+            [&](long long u) {
+              zeta_grad_pair<1, 0>(m, p, se, P, W, vao, vdp, vqp, dz, pp[u / ns], sp[u % ns]);
+            });
     return;
   }
-  t -= pad32(nsp);
-  if (t < (long long)np * np)
-    zeta_grad_pair<1, 1>(m, p, se, P, W, vao, vdp, vqp, dz, pp[t / np], pp[t % np]);
+  t -= psp;
+  walk<1>(t, (long long)np * np, rounds,
+          [&](long long u) { return near(pp[u / np], pp[u % np]); },
+          [&](long long u) {
+            zeta_grad_pair<1, 1>(m, p, se, P, W, vao, vdp, vqp, dz, pp[u / np], pp[u % np]);
+          });
 }
-__global__ void k_zeta_grad(DevMol m, Gfn2Scalars p, const double* __restrict__ se,
-                            const double* __restrict__ P, const double* __restrict__ W,
-                            const double* __restrict__ vao, const double* __restrict__ vdp,
-                            const double* __restrict__ vqp, double* dz) {
-  zeta_grad_dev(m, p, se, P, W, vao, vdp, vqp, dz,
-                blockIdx.x * (long long)blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(WALK_THREADS)
+    k_zeta_grad(DevMol m, Gfn2Scalars p, const double* __restrict__ se,
+                const double* __restrict__ P, const double* __restrict__ W,
+                const double* __restrict__ vao, const double* __restrict__ vdp,
+                const double* __restrict__ vqp, double* dz, int rounds) {
+  zeta_grad_dev(m, p, se, P, W, vao, vdp, vqp, dz, rounds);
 }
 
 void launch_zeta_grad(const DevMol& m, const Gfn2Scalars& p, const double* se, const double* P,
                       const double* W, const double* vao, const double* vdp, const double* vqp,
                       double* dz, cudaStream_t s) {
   cudaMemsetAsync(dz, 0, sizeof(double) * m.nsh, s);
-  const long long np = (long long)m.nsh * m.nsh + 96;
+  const Walk w = zeta_walk(zeta_padded(m.nsh, {1, 1}));
   ++g_kernel_launches;
-  k_zeta_grad<<<(unsigned)((np + 127) / 128), 128, 0, s>>>(m, p, se, P, W, vao, vdp, vqp, dz);
+  k_zeta_grad<<<walk_blocks(zeta_padded(m.nsh, w), w), WALK_THREADS, 0, s>>>(
+      m, p, se, P, W, vao, vdp, vqp, dz, w.rounds);
 }
 
 // batched launches (blockIdx.z walks the listed molecules; S, H, D, Q start zeroed)
-__global__ void kb_build_h0(const MolPtrs* __restrict__ mp, const int* __restrict__ list,
-                            Gfn2Scalars p) {
+template <int G>
+__global__ void __launch_bounds__(WALK_THREADS)
+    kb_build_h0(const MolPtrs* __restrict__ mp, const int* __restrict__ list, Gfn2Scalars p,
+                int rounds) {
   const MolPtrs& q = mp[list[blockIdx.z]];
   p.h0_cutoff = q.h0_cutoff;
-  build_h0_dev(q.m, p, q.se, q.S, q.H, q.D, q.Q);
+  build_h0_dev<G>(q.m, p, q.se, q.S, q.H, q.D, q.Q, rounds);
 }
 void launch_build_h0_b(const BatchLaunch& b, const Gfn2Scalars& p) {
   if (!b.count) return;
-  const long long nthr = h0_tasks(b.nsh_max, b.np_max);
+  const Walk w = walk_of(b.count * h0_padded(b.nsh_max, b.np_max, {1, 1}));
+  const dim3 grid(walk_blocks(h0_padded(b.nsh_max, b.np_max, w), w), 1, b.count);
   ++g_kernel_launches;
-  kb_build_h0<<<dim3((unsigned)((nthr + 127) / 128), 1, b.count), 128, 0, b.s>>>(b.mp, b.list, p);
+  if (w.lanes == 1)
+    kb_build_h0<1><<<grid, WALK_THREADS, 0, b.s>>>(b.mp, b.list, p, w.rounds);
+  else
+    kb_build_h0<WALK_G><<<grid, WALK_THREADS, 0, b.s>>>(b.mp, b.list, p, w.rounds);
 }
 
 // the energy-weighted density W sits in F once the SCF is done
-__global__ void kb_h0_gradient(const MolPtrs* __restrict__ mp, const int* __restrict__ list,
-                               Gfn2Scalars p) {
+template <int G>
+__global__ void __launch_bounds__(WALK_THREADS)
+    kb_h0_gradient(const MolPtrs* __restrict__ mp, const int* __restrict__ list, Gfn2Scalars p,
+                   int rounds) {
   const MolPtrs& q = mp[list[blockIdx.z]];
   p.h0_cutoff = q.h0_cutoff;
-  h0_gradient_dev(q.m, p, q.se, q.P, q.F, q.vao, q.vdp, q.vqp, q.grad, q.sigma, q.dEdcn);
+  h0_gradient_dev<G>(q.m, p, q.se, q.P, q.F, q.vao, q.vdp, q.vqp, q.grad, q.sigma, q.dEdcn,
+                     rounds);
 }
 __global__ void kb_h0_onsite_dcn(const MolPtrs* __restrict__ mp, const int* __restrict__ list) {
   const MolPtrs& q = mp[list[blockIdx.z]];
   h0_onsite_dcn_dev(q.m, q.P, q.dEdcn);
 }
 // W is in F after the gradient phase; zgrad was zeroed by kb_param_grad
-__global__ void kb_zeta_grad(const MolPtrs* __restrict__ mp, const int* __restrict__ list,
-                             Gfn2Scalars p) {
+__global__ void __launch_bounds__(WALK_THREADS)
+    kb_zeta_grad(const MolPtrs* __restrict__ mp, const int* __restrict__ list, Gfn2Scalars p,
+                 int rounds) {
   const MolPtrs& q = mp[list[blockIdx.z]];
   if (!q.param_grad) return;
   p.h0_cutoff = q.h0_cutoff;
-  zeta_grad_dev(q.m, p, q.se, q.P, q.F, q.vao, q.vdp, q.vqp, q.zgrad,
-                blockIdx.x * (long long)blockDim.x + threadIdx.x);
+  zeta_grad_dev(q.m, p, q.se, q.P, q.F, q.vao, q.vdp, q.vqp, q.zgrad, rounds);
 }
 void launch_zeta_grad_b(const BatchLaunch& b, const Gfn2Scalars& p) {
   if (!b.count) return;
-  const long long np = (long long)b.nsh_max * b.nsh_max + 96;
+  const Walk w = zeta_walk(b.count * zeta_padded(b.nsh_max, {1, 1}));
   ++g_kernel_launches;
-  kb_zeta_grad<<<dim3((unsigned)((np + 127) / 128), 1, b.count), 128, 0, b.s>>>(b.mp, b.list, p);
+  kb_zeta_grad<<<dim3(walk_blocks(zeta_padded(b.nsh_max, w), w), 1, b.count), WALK_THREADS, 0,
+                 b.s>>>(b.mp, b.list, p, w.rounds);
 }
 
 void launch_h0_gradient_b(const BatchLaunch& b, const Gfn2Scalars& p) {
   if (!b.count) return;
-  const long long npair = (long long)b.nsh_max * (b.nsh_max + 1) / 2 + 64;
+  const Walk w = walk_of(b.count * h0_gradient_padded(b.nsh_max, {1, 1}));
+  const dim3 grid(walk_blocks(h0_gradient_padded(b.nsh_max, w), w), 1, b.count);
   ++g_kernel_launches;
-  kb_h0_gradient<<<dim3((unsigned)((npair + 127) / 128), 1, b.count), 128, 0, b.s>>>(b.mp, b.list,
-                                                                                     p);
+  if (w.lanes == 1)
+    kb_h0_gradient<1><<<grid, WALK_THREADS, 0, b.s>>>(b.mp, b.list, p, w.rounds);
+  else
+    kb_h0_gradient<WALK_G><<<grid, WALK_THREADS, 0, b.s>>>(b.mp, b.list, p, w.rounds);
   ++g_kernel_launches;
   kb_h0_onsite_dcn<<<dim3((b.nat_max + 127) / 128, 1, b.count), 128, 0, b.s>>>(b.mp, b.list);
 }
