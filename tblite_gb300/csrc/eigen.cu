@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "warp_sums.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -290,22 +291,22 @@ __global__ void __launch_bounds__(256) k_tridiag_smem(int n, double* A, double* 
       s = wred(s);
       if (lane == 0) red[wid] = s;
       __syncthreads();
-      if (wid == 0) {
+      if (wid < 2) {  // each of the two divisions on a scheduler of its own
         s = 0.0;
         for (int k = 0; k < nwb; ++k) s += red[k];
         const double alpha = sn[i + 2];
-        double tn = 0.0, beta = alpha;
-        if (s > 0.0) {
-          beta = -copysign(sqrt(alpha * alpha + s), alpha);
-          tn = (beta - alpha) / beta;
-        }
-        const double sc = s > 0.0 ? 1.0 / (alpha - beta) : 0.0;
-        if (lane == 0) {
-          s_t = tn;
-          s_sc = sc;
-          if (own) {
-            tau[i + 1] = tn;
-            e[i + 1] = beta;
+        const double beta = s > 0.0 ? -copysign(sqrt(alpha * alpha + s), alpha) : alpha;
+        if (wid == 0) {
+          const double sc = s > 0.0 ? 1.0 / (alpha - beta) : 0.0;
+          if (lane == 0) s_sc = sc;
+        } else {
+          const double tn = s > 0.0 ? (beta - alpha) / beta : 0.0;
+          if (lane == 0) {
+            s_t = tn;
+            if (own) {
+              tau[i + 1] = tn;
+              e[i + 1] = beta;
+            }
           }
         }
       }
@@ -1202,12 +1203,14 @@ __device__ __forceinline__ void backtransform_dev(int n, int k, int chunk, bool 
   for (int gtop = (n - 2) / 4; gtop >= 0; gtop -= cb) {
     const int gbot = max(0, gtop - cb + 1);
     __syncthreads();
-    for (int g = gtop; g >= gbot; --g)
-      for (int a = 0; a < 4; ++a) {
-        double* sv = smem + (size_t)((gtop - g) * 4 + a) * n;
-        for (int r = 4 * g + 1 + threadIdx.x; r < n; r += blockDim.x)
-          sv[r] = bt_v(n, A, 4 * g + a, r);
-      }
+    // a warp per reflector: its rows are in flight together (one after the other per thread they
+    // took as long as the arithmetic)
+    for (int q = wid; q < 4 * (gtop - gbot + 1); q += W) {
+      const int j = 4 * (gtop - (q >> 2)) + (q & 3);
+      double* sv = smem + (size_t)q * n;
+#pragma unroll 8
+      for (int r = (j & ~3) + 1 + lane; r < n; r += 32) sv[r] = bt_v(n, A, j, r);
+    }
     __syncthreads();
     if (y) {
       for (int g = gtop; g >= gbot; --g) {
@@ -1215,23 +1218,26 @@ __device__ __forceinline__ void backtransform_dev(int n, int k, int chunk, bool 
         const double* v1 = v0 + n;
         const double* v2 = v1 + n;
         const double* v3 = v2 + n;
-        double w0 = 0.0, w1 = 0.0, w2 = 0.0, w3 = 0.0;
+        double w[4] = {0.0, 0.0, 0.0, 0.0};
+        // z = T w (upper triangular, column-major): row b on lane b, from its diagonal on, four
+        // operations for all rows
+        const int b = lane & 3;
+        const double* T = Tm + 16 * g + 5 * b;
+        const double t0 = T[0], t1 = b < 3 ? T[4] : 0.0, t2 = b < 2 ? T[8] : 0.0,
+                     t3 = b < 1 ? T[12] : 0.0;
         for (int r = 4 * g + 1 + lane; r < n; r += 32) {
           const double yr = y[r];
-          w0 = fma(v0[r], yr, w0);
-          w1 = fma(v1[r], yr, w1);
-          w2 = fma(v2[r], yr, w2);
-          w3 = fma(v3[r], yr, w3);
+          w[0] = fma(v0[r], yr, w[0]);
+          w[1] = fma(v1[r], yr, w[1]);
+          w[2] = fma(v2[r], yr, w[2]);
+          w[3] = fma(v3[r], yr, w[3]);
         }
-        w0 = wred(w0);
-        w1 = wred(w1);
-        w2 = wred(w2);
-        w3 = wred(w3);
-        const double* T = Tm + 16 * g;  // z = T w (upper triangular, column-major)
-        const double z0 = T[0] * w0 + T[4] * w1 + T[8] * w2 + T[12] * w3;
-        const double z1 = T[5] * w1 + T[9] * w2 + T[13] * w3;
-        const double z2 = T[10] * w2 + T[14] * w3;
-        const double z3 = T[15] * w3;
+        const double s = warp_sums4(w);  // six additions instead of twenty
+        const double x0 = warp_sum4_of(s, b), x1 = warp_sum4_of(s, b + 1),
+                     x2 = warp_sum4_of(s, b + 2), x3 = warp_sum4_of(s, b + 3);
+        const double zb = fma(t3, x3, fma(t2, x2, fma(t0, x0, __dmul_rn(t1, x1))));
+        const double z0 = __shfl_sync(0xffffffffu, zb, 0), z1 = __shfl_sync(0xffffffffu, zb, 1);
+        const double z2 = __shfl_sync(0xffffffffu, zb, 2), z3 = __shfl_sync(0xffffffffu, zb, 3);
         for (int r = 4 * g + 1 + lane; r < n; r += 32)
           y[r] -= fma(v0[r], z0, fma(v1[r], z1, fma(v2[r], z2, v3[r] * z3)));
         __syncwarp();
