@@ -414,10 +414,11 @@ struct MolPtrs {
   // open shell) and the output [channels][nat][nat]
   int wbo_ch;
   double* wbo;
-  // density by spectral projection (closed shells of a projection bucket, sp2.cu): the slice
-  // image of the iterate (in Y) and its line exponents, a second image (the columns of op(B) of
-  // a pipelined GEMM site), state doubles [8] and ints [8], partial sums of the iterate
-  // [3 sp2_slot_count(nao)] (trace and the 128-bit sum of squares per block of 8 lines), and the
+  // density by spectral projection (closed shells of a projection bucket, sp2.cu): two slice
+  // images for the iterates (in Y; the steps alternate) and for the rows of op(A) and the columns
+  // of op(B) of a pipelined GEMM site, their line exponents (iexp: the iterates' too), state
+  // doubles [8] and ints [8], partial sums of the iterate [3 sp2_slot_count(nao)] (trace and the
+  // 128-bit sum of squares per block of 8 lines or per tile), and the
   // steps of the last projection for the host
   uint16_t* img;
   int* iexp;
@@ -557,13 +558,14 @@ void sp2_density_b(const BatchLaunch& b, int steps);
 void sp2_gap_b(const BatchLaunch& b);
 void sp2_weighted_b(const BatchLaunch& b);
 void sp2_pipe_check_b(const BatchLaunch& b);  // flag -5 for a molecule whose pipe wait ran out
-// ozaki_pipe.cu: the squaring of a projection step of the iterating molecules (D^2 on the
-// tensor cores from the slice image; the next iterate D^2 or 2D - D^2 over D in Y, as signed
-// 64-bit fixed point in units of 2^-55 during the projection)
+// ozaki_pipe.cu: a projection step of the iterating molecules (D^2 on the tensor cores from the
+// slice image; the next iterate D^2 or 2D - D^2 over D in Y, as signed 64-bit fixed point in units
+// of 2^-55 during the projection; its slice image with its exact partial sums, and the next
+// decision)
 void sp2_square_b(const BatchLaunch& b);
-// ozaki_pipe.cu: the slice image of the iterate in Y with its exact partial sums, and the next
-// decision (init: D0 from A and the Gershgorin bounds into Y first)
-void sp2_slice_b(const BatchLaunch& b, bool init);
+// ozaki_pipe.cu: the first iterate D0 from A and the Gershgorin bounds into Y, its slice image and
+// the first decision
+void sp2_init_b(const BatchLaunch& b);
 // ozaki_pipe.cu: the converged iterate (fixed point during the projection) back to FP64 in Y
 void sp2_unfix_b(const BatchLaunch& b);
 int sp2_slot_count(int n);  // partial-sum slots of a molecule of n orbitals (3 words each)

@@ -290,8 +290,8 @@ __global__ void k_pexp_cols(const double* __restrict__ M, int ld, int lines, int
 // both memory orders read coalesced; each thread splits 8 consecutive k of one line
 template <class Sch>
 __device__ __forceinline__ void psplit_dev(const double* __restrict__ M, int ld, int kcontig,
-                                           int lines, int K, int nlb, const int* __restrict__ e,
-                                           uint16_t* img, int lb, int kc) {
+                                           int lines, int K, int nlb, int ei, uint16_t* img,
+                                           int lb, int kc) {
   __shared__ double tile[64][33];
   const int t = threadIdx.x;
   const int l0 = lb * 64, k0 = kc * PP_KC;
@@ -312,8 +312,6 @@ __device__ __forceinline__ void psplit_dev(const double* __restrict__ M, int ld,
   }
   __syncthreads();
   const int li = t & 63, g = t >> 6;  // k group of 8: 0..3
-  const int i = l0 + li;
-  const int ei = e[i];
   uint32_t w[Sch::SLICES][4];
 #pragma unroll
   for (int c = 0; c < 8; c += 2) {  // two neighbouring k per step
@@ -335,7 +333,8 @@ template <class Sch>
 __global__ void __launch_bounds__(256) k_psplit(const double* __restrict__ M, int ld, int kcontig,
                                                 int lines, int K, int nlb,
                                                 const int* __restrict__ e, uint16_t* img) {
-  psplit_dev<Sch>(M, ld, kcontig, lines, K, nlb, e, img, blockIdx.x, blockIdx.y);
+  psplit_dev<Sch>(M, ld, kcontig, lines, K, nlb, e[blockIdx.x * 64 + (threadIdx.x & 63)], img,
+                  blockIdx.x, blockIdx.y);
 }
 
 struct PipeArgs {
@@ -354,7 +353,11 @@ struct PipeArgs {
   // of 2^-SP2_FRAC instead of doubles (|D_ij| <= 1); sub2: C <- 2 C - product (the old element
   // read first), which turns D^2 into 2D - D^2 in place
   int sub2;
-  int fixed;
+  // the slice image of the new iterate (lines_padded(N) lines, exponent SP2_E), the tile's partial
+  // sums of it (three words) and the mark of an element out of range
+  uint16_t* img;
+  unsigned long long* part;
+  int* bad;
 };
 
 // line exponent of every projection iterate: the spectrum of D stays in [0, 1], so every element
@@ -402,19 +405,73 @@ __device__ __forceinline__ long long add_level(long long T, int iv, int mul) {
   return r;
 }
 
-// one 128 x 64 output tile (number b in the grouped order) of the product a (FIXED: the
-// projection's fixed-point epilogue, a.fixed set)
-template <class Sch, bool FIXED = false>
-__device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
-  // ---- tile of this CTA: groups of PP_GROUP row blocks, column blocks inside a group
-  const int mt = (a.M + PP_M - 1) / PP_M, nt = (a.N + PP_N - 1) / PP_N;
+// the squares of Y < 2^56 as a (2^56, 2^28, 1) limb triple: Y = h 2^28 + l, Y^2 = h^2 2^56 +
+// 2 h l 2^28 + l^2 (every partial product below 2^56, so per-lane sums of up to 256 stay exact)
+struct Sq3 {
+  unsigned long long hh = 0ull, hl = 0ull, ll = 0ull;
+  __device__ __forceinline__ void add(uint32_t h, uint32_t l) {
+    hh += (unsigned long long)h * h;
+    hl += (unsigned long long)h * l;
+    ll += (unsigned long long)l * l;
+  }
+  // the 128-bit value hh 2^56 + hl 2^29 + ll
+  __device__ __forceinline__ void value(unsigned long long& lo, unsigned long long& hi) const {
+    lo = hh << 56;
+    hi = hh >> 8;
+    const unsigned long long m = hl << 29, mh = hl >> 35;
+    lo += m;
+    hi += mh + (lo < m ? 1ull : 0ull);
+    lo += ll;
+    hi += (lo < ll ? 1ull : 0ull);
+  }
+};
+__device__ __forceinline__ void add128(unsigned long long& lo, unsigned long long& hi,
+                                       unsigned long long l, unsigned long long h) {
+  lo += l;
+  hi += h + (lo < l ? 1ull : 0ull);
+}
+
+// the iterate's element W for its image: zero if it is out of range, and its square
+__device__ __forceinline__ long long sp2_element(long long w, Sq3& sq, bool& over) {
+  // magnitudes (an out-of-range element, including the marker, counts as zero and stops the
+  // molecule) and their 28-bit halves
+  const unsigned long long a = w < 0 ? 0ull - (unsigned long long)w : (unsigned long long)w;
+  const bool bad = a >= (unsigned long long)SP2_LIMIT;
+  over = over || bad;
+  const unsigned long long m = bad ? 0ull : a;
+  sq.add((uint32_t)(m >> 28), (uint32_t)m & 0xFFFFFFFu);
+  return bad ? 0 : w;
+}
+// exact sums over the warp
+__device__ __forceinline__ void sp2_warp_sums(long long& tr, unsigned long long& lo,
+                                              unsigned long long& hi) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    tr += __shfl_xor_sync(0xffffffffu, tr, o);
+    add128(lo, hi, __shfl_xor_sync(0xffffffffu, lo, o), __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+}
+
+// rows and columns of tile b: groups of PP_GROUP row blocks, column blocks inside a group
+__device__ __forceinline__ void tile_origin(int M, int N, int b, int& i0, int& j0) {
+  const int mt = (M + PP_M - 1) / PP_M, nt = (N + PP_N - 1) / PP_N;
   const int gid = b / (PP_GROUP * nt);
   const int first = gid * PP_GROUP;
   const int gsize = min(mt - first, PP_GROUP);
   const int inner = b - gid * PP_GROUP * nt;
-  const int tm = first + inner % gsize, tn = inner / gsize;
-  const int i0 = tm * PP_M, j0 = tn * PP_N;
-  if (a.sym && i0 + PP_M - 1 < j0) return;  // strictly above the diagonal: mirrored
+  i0 = (first + inner % gsize) * PP_M;
+  j0 = (inner / gsize) * PP_N;
+}
+// a symmetric product skips the tiles strictly above the diagonal (mirrored from below it)
+__device__ __forceinline__ bool tile_above(int i0, int j0) { return i0 + PP_M - 1 < j0; }
+
+// one 128 x 64 output tile (number b in the grouped order) of the product a (FIXED: the
+// projection's fixed-point epilogue, a.fixed set)
+template <class Sch, bool FIXED = false>
+__device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
+  int i0, j0;
+  tile_origin(a.M, a.N, b, i0, j0);
+  if (a.sym && tile_above(i0, j0)) return;
 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem =
@@ -422,6 +479,8 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
   __shared__ __align__(8) uint64_t full[PP_STAGES], empty[PP_STAGES], accf[2], accfree[2], fin;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
+  __shared__ long long s_tr[8];
+  __shared__ unsigned long long s_lo[8], s_hi[8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile int* abort = &abort_flag;
 
@@ -701,10 +760,87 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
         }
       }
     }
+    if constexpr (FIXED) {
+      // The slice image of the new iterate, from the tile in shared memory: the lines i of the tile
+      // (k = its columns) and, for the blocks of 64 strictly below the diagonal, the lines j (k =
+      // its rows); of the block on the diagonal the elements on and below it, and their mirror
+      // images.  A block above the diagonal belongs to another tile.  Four lanes per line and
+      // chunk of 32, eight elements each, so that a warp writes eight whole lines.  A separate
+      // kernel read the iterate back for this: 44 ms of an ensemble's 237 ms, and a launch per
+      // step.
+      long long tr = 0;
+      Sq3 sq;
+      bool over = false;
+      if (__all_sync(0xffffffffu, (mirror && !*abort) ? 1 : 0)) {
+        const long long* mir = reinterpret_cast<const long long*>(smem);
+        const int g = lane & 3, cb = j0 / 64;
+        auto piece = [&](int line, int kc, auto element) {
+          const int k0 = 32 * kc + 8 * g;
+          uint32_t w[Sch::SLICES][4];
+#pragma unroll
+          for (int c = 0; c < 8; c += 2) {
+            long long x[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              x[e] = sp2_element(element(k0 + c + e), sq, over);
+              if (k0 + c + e == line) tr = x[e];  // (one line per lane holds its diagonal here)
+            }
+            uint32_t t[Sch::SLICES];
+            digits_pair(x[0], x[1], t);
+#pragma unroll
+            for (int p = 0; p < Sch::SLICES; ++p) w[p][c >> 1] = t[p];
+          }
+          const int li = line & 63;
+#pragma unroll
+          for (int p = 0; p < Sch::SLICES; ++p)
+            *reinterpret_cast<uint4*>(
+                a.img + (((size_t)kc * Sch::SLICES + p) * a.nlbA + (line >> 6)) * 2048 + li * 32 +
+                ((g ^ ((li >> 1) & 3)) << 3)) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+        };
+#pragma unroll 1
+        for (int u = (warp - 2) * 8 + (lane >> 2); u < 2 * PP_M; u += 64) {  // lines of rows
+          const int r = u & (PP_M - 1), i = i0 + r, kc = j0 / 32 + u / PP_M, rb = i >> 6;
+          if (rb < cb || kc >= nkc) continue;
+          piece(i, kc, [&](int k) {
+            // on the diagonal block an element above the diagonal is the one below it
+            return rb == cb && k > i ? mir[(i - j0) * (PP_M + 1) + (k - i0)]
+                                     : mir[(k - j0) * (PP_M + 1) + r];
+          });
+        }
+#pragma unroll 1
+        for (int u = (warp - 2) * 8 + (lane >> 2); u < 4 * PP_N; u += 64) {  // lines of columns
+          const int jl = u & (PP_N - 1), j = j0 + jl, kc = i0 / 32 + u / PP_N;
+          if ((kc >> 1) <= cb || kc >= nkc) continue;
+          piece(j, kc, [&](int k) { return mir[jl * (PP_M + 1) + (k - i0)]; });
+        }
+      }
+      unsigned long long lo, hi;
+      sq.value(lo, hi);
+      sp2_warp_sums(tr, lo, hi);
+      if (__any_sync(0xffffffffu, over ? 1 : 0) && lane == 0) *a.bad = 1;
+      if (lane == 0) {
+        s_tr[warp - 2] = tr;
+        s_lo[warp - 2] = lo;
+        s_hi[warp - 2] = hi;
+      }
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (tid == 0 && abort_flag) atomicExch(a.status, 1);
+  if constexpr (FIXED) {
+    if (tid == 0) {  // exact integers
+      long long t = 0;
+      unsigned long long lo = 0ull, hi = 0ull;
+      for (int u = 0; u < 8; ++u) {
+        t += s_tr[u];
+        add128(lo, hi, s_lo[u], s_hi[u]);
+      }
+      a.part[0] = (unsigned long long)t;
+      a.part[1] = lo;
+      a.part[2] = hi;
+    }
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(PP_TMEM_COLS));
@@ -714,44 +850,59 @@ __global__ void __launch_bounds__(PP_THREADS, 1) k_opipe(PipeArgs a) {
   opipe_tile<Sch>(a, blockIdx.x);
 }
 
-// ---- batched spectral projection on the pipe, two launches per step for every molecule of the
+// ---- batched spectral projection on the pipe, one launch per step for every molecule of the
 // list still iterating (blockIdx.y / blockIdx.z walks the molecules): kb_opipe_sq squares the
 // iterate D_k from its slice image and writes D_(k+1) = D_k^2, or 2 D_k - D_k^2 (the old element
-// read first), over D_k in Y; kb_sp2_slice then writes the slice image of D_(k+1) (every line
-// exponent SP2_E) with the partial sums of its trace and of its squared elements, and its last
-// block takes the next decision.  Molecules that left the batch or whose projection has
-// converged (sp2i[0] != 0) launch nothing.
+// read first), over D_k in Y, and the slice image of D_(k+1) (every line exponent SP2_E) into the
+// other of the molecule's two images, with the tile's partial sums of its trace and of its squared
+// elements; its last block takes the next decision.  Molecules that left the batch or whose
+// projection has converged (sp2i[0] != 0) launch nothing.
 __device__ __forceinline__ int lines_padded(int n) { return ((n + PP_M - 1) / PP_M) * PP_M; }
 __device__ __forceinline__ int sq_tiles(int n) {
   return ((n + PP_M - 1) / PP_M) * ((n + PP_N - 1) / PP_N);
 }
-// partial-sum slots of a molecule: one per block of kb_sp2_slice (8 lines)
+// partial-sum slots of a molecule: one per block of kb_sp2_init (8 lines) and one per tile
 __host__ __device__ __forceinline__ int sp2_slots(int n) {
-  return ((n + PP_M - 1) / PP_M) * PP_M / 8;
+  const int mt = (n + PP_M - 1) / PP_M, nt = (n + PP_N - 1) / PP_N;
+  return mt * (nt > PP_M / 8 ? nt : PP_M / 8);
+}
+// the image that holds the iterate after `steps` steps
+__device__ __forceinline__ uint16_t* sp2_image(const MolPtrs& q, int steps) {
+  return (steps & 1) ? q.img2 : q.img;
 }
 
-// The decision at a new iterate D, taken by one thread after every partial sum of D is written:
-// tr D in a fixed order, tr D^2 = sum of the squares of D's elements (D is symmetric) exactly in
-// 128-bit integers, read past L1 since other CTAs wrote them; then the idempotency error
+// The decision at a new iterate D, taken by one warp after every partial sum of D is written (the
+// slots 0 .. nslots - 1, without those of the tiles above the diagonal if they are tiles): tr D
+// and tr D^2 = sum of the squares of D's elements (D is symmetric) exactly in 128-bit integers,
+// read past L1 since other CTAs wrote them; then the idempotency error
 // tr(D - D^2), the stop test (the error no longer falls over two steps, Kruchinin, Rubensson,
 // Niklasson 2016, or reaches the rounding floor) and the update D^2 or 2D - D^2 whose trace is
 // closer to the occupied count (Niklasson 2002).  State: sp2i[0] converged, [1] steps taken,
 // [2] update of the next step (1 square, 0 2D - D^2, -1 none), [3] pipeline status; sp2s[2..4]
 // the last three idempotency errors, [4] set by a block that met an element outside the
 // fixed-point range (the molecule leaves).
-__device__ void sp2_decide(const MolPtrs& q, int nslots) {
+__device__ void sp2_decide(const MolPtrs& q, int nslots, bool tiles) {
   // tr D 2^55 as a signed 128-bit sum of the blocks' int64 sums, tr D^2 2^110 unsigned
-  unsigned long long tlo = 0ull, slo = 0ull, shi = 0ull;
-  long long thi = 0;
-  for (int t = 0; t < nslots; ++t) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long tlo = 0ull, thi_ = 0ull, slo = 0ull, shi = 0ull;
+  for (int t = lane; t < nslots; t += 32) {
+    if (tiles) {
+      int i0, j0;
+      tile_origin(q.m.nao, q.m.nao, t, i0, j0);
+      if (tile_above(i0, j0)) continue;
+    }
     const unsigned long long* pt = q.sp2p + 3 * t;
     const long long tv = (long long)__ldcg(pt);
-    tlo += (unsigned long long)tv;
-    thi += (tv < 0 ? -1 : 0) + (tlo < (unsigned long long)tv ? 1 : 0);
-    const unsigned long long l = __ldcg(pt + 1);
-    slo += l;
-    shi += __ldcg(pt + 2) + (slo < l ? 1ull : 0ull);
+    add128(tlo, thi_, (unsigned long long)tv, tv < 0 ? ~0ull : 0ull);
+    add128(slo, shi, __ldcg(pt + 1), __ldcg(pt + 2));
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    add128(tlo, thi_, __shfl_xor_sync(0xffffffffu, tlo, o), __shfl_xor_sync(0xffffffffu, thi_, o));
+    add128(slo, shi, __shfl_xor_sync(0xffffffffu, slo, o), __shfl_xor_sync(0xffffffffu, shi, o));
+  }
+  if (lane != 0) return;
+  const long long thi = (long long)thi_;
   const double tx = ((double)thi * 0x1p64 + (double)tlo) * 0x1p-55;
   const double tx2 = ((double)shi * 0x1p64 + (double)slo) * 0x1p-110;
   const int n = q.m.nao;
@@ -782,7 +933,8 @@ __device__ void sp2_decide(const MolPtrs& q, int nslots) {
 // the last of `units` CTAs of a molecule to finish takes the decision (no separate launch):
 // after the CTA's barrier one thread fences (cumulatively, the stores its barrier ordered before
 // it) and counts the finished units; the CTA that completes the count decides and resets it
-__device__ __forceinline__ void sp2_last_decides(const MolPtrs& q, int units) {
+__device__ __forceinline__ void sp2_last_decides(const MolPtrs& q, int units, int nslots,
+                                                 bool tiles) {
   __shared__ int last;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -790,10 +942,10 @@ __device__ __forceinline__ void sp2_last_decides(const MolPtrs& q, int units) {
     last = atomicAdd(q.sp2i + 5, 1) == units - 1;
   }
   __syncthreads();
-  if (!last || threadIdx.x != 0) return;
+  if (!last || threadIdx.x >= 32) return;
   __threadfence();
-  sp2_decide(q, units);  // one partial sum per unit
-  q.sp2i[5] = 0;
+  sp2_decide(q, nslots, tiles);
+  if (threadIdx.x == 0) q.sp2i[5] = 0;
 }
 __device__ __forceinline__ bool sq_skip(const MolPtrs& q) {
   return *q.flag < 0 || q.sp2i[0] != 0;
@@ -804,8 +956,13 @@ __global__ void __launch_bounds__(PP_THREADS, 1) kb_opipe_sq(const MolPtrs* __re
   const int n = q.m.nao;
   const int tiles = sq_tiles(n);
   if (sq_skip(q) || (int)blockIdx.x >= tiles) return;
+  int i0, j0;
+  tile_origin(n, n, blockIdx.x, i0, j0);
+  if (tile_above(i0, j0)) return;
+  // read by every tile before the last one to finish changes them
+  const int steps = q.sp2i[1] - 1;  // of the iterate to be squared (the decision counted this one)
   PipeArgs a{};
-  a.A = a.B = q.img;  // a symmetric matrix: its rows are its columns
+  a.A = a.B = sp2_image(q, steps);  // a symmetric matrix: its rows are its columns
   a.eA = a.eB = q.iexp;
   a.eshiftA = 0;
   a.nlbA = a.nlbB = lines_padded(n) / 64;
@@ -816,62 +973,33 @@ __global__ void __launch_bounds__(PP_THREADS, 1) kb_opipe_sq(const MolPtrs* __re
   a.sym = 1;
   a.status = q.sp2i + 3;
   a.sub2 = q.sp2i[2] == 0 ? 1 : 0;
-  a.fixed = 1;
-  if (threadIdx.x == 0) {  // the tile's useful area (the upper tiles of the symmetric product exit)
-    const int mt = (n + PP_M - 1) / PP_M, nt = (n + PP_N - 1) / PP_N;
-    const int b = blockIdx.x, gid = b / (PP_GROUP * nt), first = gid * PP_GROUP;
-    const int gsize = min(mt - first, PP_GROUP), inner = b - gid * PP_GROUP * nt;
-    const int i0 = (first + inner % gsize) * PP_M, j0 = (inner / gsize) * PP_N;
-    if (!(i0 + PP_M - 1 < j0))
-      atomicAdd(&g_pipe_batch_flops, 2ull * (unsigned long long)min(PP_M, n - i0) *
-                                         (unsigned long long)min(PP_N, n - j0) * (unsigned)n);
-  }
+  a.img = sp2_image(q, steps + 1);
+  a.part = q.sp2p + 3 * blockIdx.x;
+  a.bad = q.sp2i + 4;
+  if (threadIdx.x == 0)  // the tile's useful area
+    atomicAdd(&g_pipe_batch_flops, 2ull * (unsigned long long)min(PP_M, n - i0) *
+                                       (unsigned long long)min(PP_N, n - j0) * (unsigned)n);
   opipe_tile<Balanced, true>(a, blockIdx.x);
+  int units = 0;  // tiles on and below the diagonal: row block t has 2 t + 2 of them at most
+  const int mt = (n + PP_M - 1) / PP_M, nt = (n + PP_N - 1) / PP_N;
+  for (int t = 0; t < mt; ++t) units += min(2 * t + 2, nt);
+  sp2_last_decides(q, units, tiles, true);
 }
 
-// ---- the slice image of the iterate and the decision: each warp owns one line i of D (column i
-// in memory, which equals row i), held in Y as fixed-point integers W = x 2^55; at the start
-// (init) the line is D0 = (emax I - A) / (emax - emin), computed in FP64 and written to Y in
-// fixed point, else it is read from Y.  Its slices (exponent SP2_E) go to img, and the line's
-// diagonal element and the exact squares of its elements to the block's partial sums (exact
-// integers); the last block of the molecule takes the decision.  A lane holds two neighbouring
-// elements k, k + 1 of a 64-element segment (coalesced loads), so each slice plane gets one
-// 32-bit word per lane.  Padding lines and positions get zero slices.
-//
-// the square of Y < 2^56 as a (2^56, 2^28, 1) limb triple: Y = h 2^28 + l, Y^2 = h^2 2^56 +
-// 2 h l 2^28 + l^2 (every partial product below 2^56, so per-lane sums of up to 256 stay exact)
-struct Sq3 {
-  unsigned long long hh = 0ull, hl = 0ull, ll = 0ull;
-  __device__ __forceinline__ void add(uint32_t h, uint32_t l) {
-    hh += (unsigned long long)h * h;
-    hl += (unsigned long long)h * l;
-    ll += (unsigned long long)l * l;
-  }
-  // the 128-bit value hh 2^56 + hl 2^29 + ll
-  __device__ __forceinline__ void value(unsigned long long& lo, unsigned long long& hi) const {
-    lo = hh << 56;
-    hi = hh >> 8;
-    const unsigned long long m = hl << 29, mh = hl >> 35;
-    lo += m;
-    hi += mh + (lo < m ? 1ull : 0ull);
-    lo += ll;
-    hi += (lo < ll ? 1ull : 0ull);
-  }
-};
-__device__ __forceinline__ void add128(unsigned long long& lo, unsigned long long& hi,
-                                       unsigned long long l, unsigned long long h) {
-  lo += l;
-  hi += h + (lo < l ? 1ull : 0ull);
-}
-
-__global__ void __launch_bounds__(256) kb_sp2_slice(const MolPtrs* __restrict__ mp,
-                                                    const int* __restrict__ list, int init) {
+// ---- the first iterate and its decision: each warp owns one line i of D (column i in memory, which
+// equals row i), D0 = (emax I - A) / (emax - emin), computed in FP64 and written to Y in fixed point
+// (W = x 2^55).  Its slices (exponent SP2_E) go to img, and the line's diagonal element and the
+// exact squares of its elements to the block's partial sums (exact integers); the last block of the
+// molecule takes the decision.  A lane holds two neighbouring elements k, k + 1 of a 64-element
+// segment (coalesced loads), so each slice plane gets one 32-bit word per lane.  Padding lines and
+// positions get zero slices.
+__global__ void __launch_bounds__(256) kb_sp2_init(const MolPtrs* __restrict__ mp,
+                                                   const int* __restrict__ list) {
   const MolPtrs& q = mp[list[blockIdx.z]];
   const int n = q.m.nao, lp = lines_padded(n);
-  // uniform over the block; sp2i[0] changes only in the last block, after every block started
-  if ((int)blockIdx.x * 8 >= lp || *q.flag < 0 || (!init && q.sp2i[0] != 0)) return;
+  if ((int)blockIdx.x * 8 >= lp || *q.flag < 0) return;  // uniform over the block
   const int i = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const double emax = init ? q.sp2s[1] : 0.0, f = init ? 1.0 / (emax - q.sp2s[0]) : 0.0;
+  const double emax = q.sp2s[1], f = 1.0 / (emax - q.sp2s[0]);
   const int nkc = (n + PP_KC - 1) / PP_KC, nlb = lp / 64;
   const size_t plane = (size_t)nlb * 2048;
   long long dw = 0;  // the line's diagonal element (an integer select per element)
@@ -885,53 +1013,33 @@ __global__ void __launch_bounds__(256) kb_sp2_slice(const MolPtrs* __restrict__ 
     if ((k >> 5) >= nkc) continue;  // the last segment may hold one chunk only
     long long w0 = 0, w1 = 0;
     if (real) {
-      if (init) {  // D0 in FP64, then to fixed point (once per projection)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          if (k + e >= n) continue;
-          const double x = ((k + e == i ? emax : 0.0) - am[k + e]) * f;
-          const uint64_t bits = (uint64_t)__double_as_longlong(x);
-          const long long w =
-              ((bits >> 52) & 0x7FF) > (uint64_t)(1023 + SP2_E) ? SP2_BAD : fixed55(bits, SP2_E);
-          y[k + e] = w;
-          (e ? w1 : w0) = w;
-        }
-      } else {
-        if (k < n) w0 = y[k];
-        if (k + 1 < n) w1 = y[k + 1];
+      for (int e = 0; e < 2; ++e) {
+        if (k + e >= n) continue;
+        const double x = ((k + e == i ? emax : 0.0) - am[k + e]) * f;
+        const uint64_t bits = (uint64_t)__double_as_longlong(x);
+        const long long w =
+            ((bits >> 52) & 0x7FF) > (uint64_t)(1023 + SP2_E) ? SP2_BAD : fixed55(bits, SP2_E);
+        y[k + e] = w;
+        (e ? w1 : w0) = w;
       }
     }
     dw = k == i ? w0 : (k + 1 == i ? w1 : dw);
-    // magnitudes (an out-of-range element, including the marker, counts as zero and stops the
-    // molecule) and their 28-bit halves
-    const unsigned long long a0 = w0 < 0 ? 0ull - (unsigned long long)w0 : (unsigned long long)w0;
-    const unsigned long long a1 = w1 < 0 ? 0ull - (unsigned long long)w1 : (unsigned long long)w1;
-    const bool bad0 = a0 >= (unsigned long long)SP2_LIMIT,
-               bad1 = a1 >= (unsigned long long)SP2_LIMIT;
-    over = over || bad0 || bad1;
-    const unsigned long long m0 = bad0 ? 0ull : a0, m1 = bad1 ? 0ull : a1;
-    const uint32_t h0 = (uint32_t)(m0 >> 28), l0 = (uint32_t)m0 & 0xFFFFFFFu;
-    const uint32_t h1 = (uint32_t)(m1 >> 28), l1 = (uint32_t)m1 & 0xFFFFFFFu;
-    sq.add(h0, l0);
-    sq.add(h1, l1);
     const size_t off = (size_t)slice_off(i, k, nlb);
     uint32_t w[Balanced::SLICES];
-    digits_pair(bad0 ? 0 : w0, bad1 ? 0 : w1, w);
+    const long long x0 = sp2_element(w0, sq, over), x1 = sp2_element(w1, sq, over);
+    digits_pair(x0, x1, w);
 #pragma unroll
     for (int pp = 0; pp < Balanced::SLICES; ++pp)
       *reinterpret_cast<uint32_t*>(q.img + off + pp * plane) = w[pp];
   }
-  if (init && lane == 0) q.iexp[i] = SP2_E;
+  if (lane == 0) q.iexp[i] = SP2_E;
   // block partial sums (exact integers): warp trees, then the warps in order
   __shared__ long long s_tr[8];
   __shared__ unsigned long long s_lo[8], s_hi[8];
   unsigned long long flo, fhi;
   sq.value(flo, fhi);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    dw += __shfl_xor_sync(0xffffffffu, dw, o);  // one lane holds the diagonal, the others 0
-    add128(flo, fhi, __shfl_xor_sync(0xffffffffu, flo, o), __shfl_xor_sync(0xffffffffu, fhi, o));
-  }
+  sp2_warp_sums(dw, flo, fhi);  // (one lane holds the diagonal, the others 0)
   over = __any_sync(0xffffffffu, over ? 1 : 0) != 0;
   if (over && lane == 0) q.sp2i[4] = 1;
   const int w = threadIdx.x >> 5;
@@ -953,7 +1061,7 @@ __global__ void __launch_bounds__(256) kb_sp2_slice(const MolPtrs* __restrict__ 
     pt[1] = lo;
     pt[2] = hi;
   }
-  sp2_last_decides(q, lp / 8);
+  sp2_last_decides(q, lp / 8, lp / 8, false);
 }
 
 // after a projection: the converged iterate from fixed point back to FP64 in place (the products
@@ -982,8 +1090,8 @@ __device__ __forceinline__ SiteLines site_lines(const Site& s, int which) {
 // exponents of the lines: 32 lines per block (lines strided in memory) or one warp per line
 // (k contiguous); grid.x covers lines_padded / 8 blocks for the widest molecule
 // which operand image of a site is already split: -1 none (split it), 0 / 1 one of X's two
-// cached images (rows / columns of X), 2 the projection's last iterate image in img (op(B) = D
-// of X D: D is symmetric, so its columns are the lines img holds, exact for the fixed-point D)
+// cached images (rows / columns of X), 2 the image of the projection's last iterate (op(B) = D
+// of X D: D is symmetric, so its columns are the lines the image holds, exact for the fixed-point D)
 __host__ __device__ __forceinline__ int site_ximage(int site, int which) {
   if (site == GS_FX) return which ? 1 : -1;   // B = X: its columns
   if (site == GS_XTT) return which ? -1 : 1;  // A = X^T: rows of X^T are columns of X
@@ -1022,9 +1130,10 @@ __global__ void __launch_bounds__(256) kb_psplit_site(const MolPtrs* __restrict_
   const SiteLines L = site_lines(site_of(q, site), which);
   const int lp = lines_padded(L.lines), nkc = (L.K + PP_KC - 1) / PP_KC;
   if ((int)blockIdx.x >= lp / 64 || (int)blockIdx.y >= nkc) return;
+  const int* e = xdst >= 0 ? q.xexp[xdst] : which ? q.iexp2 : q.iexp;
   psplit_dev<Balanced>(L.M, L.ld, L.kcontig, L.lines, L.K, lp / 64,
-             xdst >= 0 ? q.xexp[xdst] : which ? q.iexp2 : q.iexp,
-             xdst >= 0 ? q.ximg[xdst] : which ? q.img2 : q.img, blockIdx.x, blockIdx.y);
+                       e[blockIdx.x * 64 + (threadIdx.x & 63)],
+                       xdst >= 0 ? q.ximg[xdst] : which ? q.img2 : q.img, blockIdx.x, blockIdx.y);
 }
 __global__ void __launch_bounds__(PP_THREADS, 1) kb_opipe_site(const MolPtrs* __restrict__ mp,
                                                               const int* __restrict__ list,
@@ -1037,7 +1146,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) kb_opipe_site(const MolPtrs* __
   PipeArgs a{};
   const int xa = site_ximage(site, 0), xb = site_ximage(site, 1);
   a.A = xa >= 0 ? q.ximg[xa] : q.img;  // (xa is never 2)
-  a.B = xb == 2 ? q.img : xb >= 0 ? q.ximg[xb] : q.img2;
+  a.B = xb == 2 ? sp2_image(q, q.sp2i[1]) : xb >= 0 ? q.ximg[xb] : q.img2;
   a.eA = xa >= 0 ? q.xexp[xa] : q.iexp;
   a.eB = xb == 2 ? q.iexp : xb >= 0 ? q.xexp[xb] : q.iexp2;
   a.eshiftA = s.alpha == 2.0 ? 1 : s.alpha == 0.5 ? -1 : 0;
@@ -1107,14 +1216,13 @@ void pipe_x_images_b(const BatchLaunch& b) {
   prof_kend(KS_PIPE_PREP, tk, b.s);
 }
 
-// the slice image of the iterate and the next decision for every listed molecule still
-// iterating (init: D0 from A and the Gershgorin bounds into Y first)
-void sp2_slice_b(const BatchLaunch& b, bool init) {
+// the first iterate D0 (from A and the Gershgorin bounds), its slice image and the first decision
+void sp2_init_b(const BatchLaunch& b) {
   if (!b.count) return;
   const int lp = pimage_lines(b.nao_max);
   const int tk = prof_kbegin(b.s);
   ++g_kernel_launches;
-  kb_sp2_slice<<<dim3(lp / 8, 1, b.count), 256, 0, b.s>>>(b.mp, b.list, init ? 1 : 0);
+  kb_sp2_init<<<dim3(lp / 8, 1, b.count), 256, 0, b.s>>>(b.mp, b.list);
   prof_kend(KS_PIPE_PREP, tk, b.s);
 }
 
@@ -1127,9 +1235,9 @@ void sp2_unfix_b(const BatchLaunch& b) {
   kb_sp2_unfix<<<dim3(blocks, 1, b.count), 256, 0, b.s>>>(b.mp, b.list);
 }
 
-// the squaring of a projection step for every listed molecule still iterating: D^2 on the
-// tensor cores from the iterate's slice image, and the next iterate (D^2 or 2D - D^2 as decided)
-// over D in Y
+// a projection step for every listed molecule still iterating: D^2 on the tensor cores from the
+// iterate's slice image, the next iterate (D^2 or 2D - D^2 as decided) over D in Y, its slice
+// image and the next decision
 void sp2_square_b(const BatchLaunch& b) {
   if (!b.count) return;
   static bool attr = false;

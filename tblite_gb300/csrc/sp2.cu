@@ -16,10 +16,10 @@
 // Per molecule and SCF iteration the eigensolver's tridiagonalisation, eigenvalues, inverse
 // iteration and back-transformation (FP64 cores) become ~25 symmetric squarings on the BF16
 // tensor cores with FP64-accurate operand splitting (ozaki_pipe.cu: kb_opipe_sq squares the
-// iterate from its slice image and writes the next iterate over it in the epilogue; kb_sp2_slice
-// writes the new iterate's slice image with one exponent for every line, sums its trace and,
-// exactly in integers, tr D^2 = sum of its squared elements, and its last block per molecule
-// takes the next decision, so a step is two launches and the decision needs no product).  Every
+// iterate from its slice image and, in the epilogue, writes the next iterate over it and that
+// one's slice image with one exponent for every line, sums its trace and, exactly in integers,
+// tr D^2 = sum of its squared elements; the last block per molecule takes the next decision, so a
+// step is one launch and the decision needs no product).  Every
 // molecule of a size bucket iterates in lockstep; each decides its own step on the device and
 // stops on its own (its later launches return at once).  The host launches a step budget per
 // bucket (the most steps any of its molecules took in the previous SCF iteration plus a margin);
@@ -50,7 +50,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // Gershgorin bounds of A and a fresh projection state: one block per 8 columns (a warp per
 // column) writes its columns' lowest and highest bound into its partial-sum slot (the slots of
-// the later slice passes, free here); the last block of the molecule to finish (a fence and the
+// the projection, free here); the last block of the molecule to finish (a fence and the
 // block count sp2i[5], zero between passes) takes the minimum and maximum over the slots in a
 // fixed order and resets the state
 __global__ void __launch_bounds__(256) kb_sp2_start(BARGS) {
@@ -138,11 +138,9 @@ void sp2_density_b(const BatchLaunch& b, int steps) {
   pipe_site_b(b, GS_XTT);  // A = X^T T1
   ++g_kernel_launches;
   kb_sp2_start<<<dim3(pimage_lines(b.nao_max) / 8, 1, b.count), 256, 0, b.s>>>(b.mp, b.list);
-  sp2_slice_b(b, true);  // D0, its slice image and the first decision
-  for (int k = 0; k < steps; ++k) {
-    sp2_square_b(b);         // D^2 and the next iterate over D
-    sp2_slice_b(b, false);  // its slice image and the next decision
-  }
+  sp2_init_b(b);  // D0, its slice image and the first decision
+  // the next iterate over D, its slice image and the next decision
+  for (int k = 0; k < steps; ++k) sp2_square_b(b);
   ++g_kernel_launches;
   kb_sp2_finish<<<dim3(1, 1, b.count), 32, 0, b.s>>>(b.mp, b.list);
   sp2_unfix_b(b);          // D from fixed point to FP64
