@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 #include "engine.h"
 #include "tridiag_fixed.cuh"
@@ -133,29 +134,53 @@ __device__ __forceinline__ void pass_group(const Exchange<MODE>& x, long long* a
   }
   const bool piv = x.b + s * x.nb == r0;  // column s is the next pivot column
   int cnt = 0;
-  for (int r = r0 + lane; r < n; r += 32) {
-    const int2 vr = v[r], wr = w[r], xr = vn[r];
-    long long t[CG];
+  // RR rows per lane in flight: a row's chain from its loads to the product's sums is some 300
+  // cycles, which few warps cannot fill with one row each
+  auto rows = [&](auto rr, int base) {
+    constexpr int RR = decltype(rr)::value;
+    int2 vr[RR], wr[RR], xr[RR];
+    long long t[RR][CG];
+    bool in[RR];
 #pragma unroll
-    for (int q = 0; q < CG; ++q) t[q] = on[q] ? a[(size_t)(s + q) * n + r] : 0;
+    for (int k = 0; k < RR; ++k) {
+      const int r = min(base + 32 * k + lane, n - 1);
+      in[k] = base + 32 * k + lane < n;
+      vr[k] = v[r];
+      wr[k] = w[r];
+      xr[k] = in[k] ? vn[r] : make_int2(0, 0);
 #pragma unroll
-    for (int q = 0; q < CG; ++q) {
-      t[q] = rank2(t[q], vr.x, vr.y, wr.x, wr.y, vc[q].x, vc[q].y, wc[q].x, wc[q].y);
-      mac(hi31(t[q]), lo31(t[q]), xr.x, xr.y, hh[q], cr[q]);
+      for (int q = 0; q < CG; ++q) t[k][q] = on[q] ? a[(size_t)(s + q) * n + r] : 0;
     }
 #pragma unroll
-    for (int q = 0; q < CG; ++q)
-      if (on[q]) a[(size_t)(s + q) * n + r] = t[q];
-    if (piv)
-      for (int k = 0; k < x.copies(); ++k) x.put(cp + r, k, t[0]);
-    if ((++cnt & 15) == 0) {  // cr stays below 2^63 for 16 terms
+    for (int k = 0; k < RR; ++k)
+#pragma unroll
+      for (int q = 0; q < CG; ++q) {
+        t[k][q] = rank2(t[k][q], vr[k].x, vr[k].y, wr[k].x, wr[k].y, vc[q].x, vc[q].y, wc[q].x,
+                        wc[q].y);
+        mac(hi31(t[k][q]), lo31(t[k][q]), xr[k].x, xr[k].y, hh[q], cr[q]);
+      }
+#pragma unroll
+    for (int k = 0; k < RR; ++k) {
+      const int r = base + 32 * k + lane;
+#pragma unroll
+      for (int q = 0; q < CG; ++q)
+        if (on[q] && in[k]) a[(size_t)(s + q) * n + r] = t[k][q];
+      if (piv && in[k])
+        for (int c = 0; c < x.copies(); ++c) x.put(cp + r, c, t[k][0]);
+    }
+    if ((cnt += RR) > 14) {  // cr stays below 2^63 for 16 terms
+      cnt = 0;
 #pragma unroll
       for (int q = 0; q < CG; ++q) {
         sum[q] += fold<4>(hh[q], cr[q]);
         hh[q] = cr[q] = 0;
       }
     }
-  }
+  };
+  constexpr int RR = CG > 2 ? 1 : 2;
+  int base = r0;
+  for (; base + 32 * (RR - 1) < n; base += 32 * RR) rows(std::integral_constant<int, RR>(), base);
+  if (RR > 1 && base < n) rows(std::integral_constant<int, 1>(), base);
 #pragma unroll
   for (int q = 0; q < CG; ++q) sum[q] += fold<4>(hh[q], cr[q]);
   // warp sums of the CG values, halving the values per exchange while more than one is left:
@@ -322,6 +347,7 @@ __device__ __forceinline__ void tri_body(const TriArgs& g, int nb, int b) {
   if constexpr (MODE == GRID) x.barrier();
   else __syncthreads();
 
+  int jm = 0, slot = 0;
   for (int i = -1; i < n - 1; ++i) {
     const int par = (i + 1) & 1;
     const long long* uin = x.u + par * n;
@@ -331,8 +357,7 @@ __device__ __forceinline__ void tri_body(const TriArgs& g, int nb, int b) {
     // warps with rows >= i + 1
     const int wlo = RPT == 1 ? (i + 1) >> 5 : 0, whi = RPT == 1 ? (n + 31) >> 5 : nw;
     const bool active = wid >= wlo && wid < whi;
-    const bool own = (i + 1) % nb == b;  // column i + 1 in slot
-    const int slot = (i + 1) / nb;
+    const bool own = jm == b;  // column i + 1 = slot nb + jm
     // ---- kappa = v.u; everything of the update that does not wait for it
     if (active) {
       long long kap = 0, cr[RPT];
@@ -430,8 +455,12 @@ __device__ __forceinline__ void tri_body(const TriArgs& g, int nb, int b) {
     }
     // ---- update and product of the owned columns j >= i + 2
     const int r0 = i + 2;
-    const int s0 = r0 <= b ? 0 : (r0 - b + nb - 1) / nb;
+    const int s0 = slot + (b <= jm ? 1 : 0);  // the first owned column after i + 1
     const int left = ncpb - s0;
+    if (++jm == nb) {
+      jm = 0;
+      ++slot;
+    }
     if (left > 2 * nw) {
       for (int s = s0 + 4 * wid; s < ncpb; s += 4 * nw)
         pass_group<MODE, 4>(x, a, s, ncpb, r0, v, w, vn, un, cn);

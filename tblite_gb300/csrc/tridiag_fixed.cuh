@@ -187,7 +187,7 @@ __host__ __device__ __forceinline__ Scalars scalars(const Reflector& f, long lon
   const unsigned long long h = umulhi(f.s, sa);
   const float hf = (float)(unsigned)(h >> 32) * 0x1p-31f;
 #ifdef __CUDA_ARCH__
-  const float y = __frcp_rn(hf);
+  const float y = __fdividef(1.0f, hf);
 #else
   const float y = 1.0f / hf;
 #endif
