@@ -1067,7 +1067,8 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
       eigen_vectors(w.eig, nvec, w.C.p);
       g_prof.end(s);
       g_prof.begin(PH_DENSITY, s);
-      density_matrix(n, nvec, w.C.p, w.focc.p, w.P.p, w.scratch.p, s, eigen_gemm_status(w.eig));
+      density_matrix(n, nvec, w.C.p, w.focc.p, w.P.p, w.scratch.p, s, eigen_gemm_status(w.eig),
+                     eigen_gemm_pair(w.eig));
       g_prof.end(s);
     }
     auto analyse = [&]() {
@@ -1094,7 +1095,8 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
       fill_more_levels();
       nvec = n;
       eigen_vectors(w.eig, nvec, w.C.p);
-      density_matrix(n, nvec, w.C.p, w.focc.p, w.P.p, w.scratch.p, s, eigen_gemm_status(w.eig));
+      density_matrix(n, nvec, w.C.p, w.focc.p, w.P.p, w.scratch.p, s, eigen_gemm_status(w.eig),
+                     eigen_gemm_pair(w.eig));
       analyse();
     }
     eelec_sum = 0.0;
@@ -1150,7 +1152,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   } else {
     launch_fe(n, w.focc.p, w.emo.p, w.vec_out.p, s);
     density_matrix(n, h_cnt[0], w.C.p, w.vec_out.p, w.W.p, w.scratch.p, s,
-                   eigen_gemm_status(w.eig));
+                   eigen_gemm_status(w.eig), eigen_gemm_pair(w.eig));
   }
   launch_h0_gradient(m, p, w.se.p, w.P.p, w.W.p, w.vao.p, w.vdp.p, w.vqp.p, w.grad.p, w.sigma.p,
                      w.dEdcn.p, s);
@@ -1188,7 +1190,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   } else {
     for (int sp = 0; sp < 2; ++sp) {  // W is free after the gradient: it holds the spin density
       density_matrix(n, h_cnt[0], w.C.p, w.focc.p + (size_t)(1 + sp) * n, w.W.p, w.scratch.p, s,
-                     eigen_gemm_status(w.eig));
+                     eigen_gemm_status(w.eig), eigen_gemm_pair(w.eig));
       gemm64(false, false, n, n, n, 1.0, w.W.p, n, w.S.p, n, 0.0, w.scratch.p, n, KM_NONE, s);
       launch_wbo(m, w.scratch.p, w.wbo.p + (size_t)sp * nat * nat, 2.0, s);
     }
@@ -1525,9 +1527,36 @@ void molecular_moments(const _tblite_structure* mol, _tblite_result* res) {
   }
 }
 
+// A pipelined product of a small molecule whose wait ran out (the SCF may end in any error then): the
+// calculation is repeated from the same start with the other split product, which the batch's
+// molecules count on when they are handed over for that reason.
 void run_singlepoint(_tblite_context* ctx, const _tblite_structure* mol, _tblite_calculator* c,
                      _tblite_result* res) {
-  singlepoint(ctx, mol, c, res);
+  const bool had = res->has_wfn;
+  const std::vector<double> qsh = res->qsh, dpat = res->dpat, qpat = res->qpat, qat = res->qat;
+  const int nat = res->nat, nsh = res->nsh, nao = res->nao;
+  try {
+    singlepoint(ctx, mol, c, res);
+    return;
+  } catch (...) {
+    if (!c->ws || !c->ws->eig || c->density_solver == 1 || !eigen_pair_failed(c->ws->eig)) throw;
+  }
+  res->has_wfn = had;
+  res->qsh = qsh;
+  res->dpat = dpat;
+  res->qpat = qpat;
+  res->qat = qat;
+  res->nat = nat;
+  res->nsh = nsh;
+  res->nao = nao;
+  eigen_set_pair(c->ws->eig, false);
+  try {
+    singlepoint(ctx, mol, c, res);
+  } catch (...) {
+    if (c->ws && c->ws->eig) eigen_set_pair(c->ws->eig, true);
+    throw;
+  }
+  if (c->ws && c->ws->eig) eigen_set_pair(c->ws->eig, true);
 }
 
 static void copy_msg(const std::string& msg, char* buffer, const int* buffersize) {
@@ -2386,7 +2415,7 @@ void tblite_get_singlepoint(tblite_context ctx, tblite_structure mol, tblite_cal
   }
   calc->default_post_processing();  // bond orders and molecular moments unless asked otherwise
   try {
-    singlepoint(ctx, mol, calc, res);
+    run_singlepoint(ctx, mol, calc, res);
   } catch (const std::exception& e) {
     ctx->push(e.what());
   }

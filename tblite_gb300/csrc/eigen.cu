@@ -37,6 +37,16 @@ static void ck(cudaError_t e, const char* what) {
 
 // GEMMs of the one-molecule path go to the tensor cores from 128 orbitals on
 static inline bool split_gemm(int n) { return g_split_gemm && n >= 128; }
+extern bool g_pipe_gemm;
+// The split products of a small molecule on the pipelined kernel: k_ogemm splits the operands of
+// every tile pair anew, 65 us at 192 orbitals and two exponent launches of 3 us; operand split and
+// pipelined product take 10 + 22 us, with a smaller error (28 products of balanced digits).  Above
+// TRIDIAG_FIXED_MAX k_ogemm's results stay (see there); below 128 orbitals the FP64 tiles are
+// faster (8 us at 68).
+constexpr int PAIR_MAX = TRIDIAG_FIXED_MAX;
+static inline bool pair_gemm(int n, const void* pair) {
+  return pair && split_gemm(n) && g_pipe_gemm && n <= PAIR_MAX;
+}
 
 struct EigenSolver {
   int n = 0;
@@ -48,6 +58,8 @@ struct EigenSolver {
   double *tw = nullptr;   // eigenvalue scratch: e^2 [n] (double), d and e^2 [n] (float)
   double *Y = nullptr;    // eigenvectors of T, column-major [k][n]
   int* status = nullptr;  // device
+  void* pair = nullptr;   // workspace of the pipelined products up to PAIR_MAX orbitals
+  bool pair_on = true;
   int* gstatus = nullptr; // device: 1 once a tensor-core GEMM did not answer
   int* hstatus = nullptr; // pinned
   int coop_blocks = 0;
@@ -1276,6 +1288,7 @@ EigenSolver* eigen_create(int n, cudaStream_t s) {
   ck(cudaMalloc(&e->xch, sizeof(long long) * tridiag_exchange_words(n)), "xch");
   ck(cudaMalloc(&e->scal, sizeof(double) * 8), "scal");
   ck(cudaMalloc(&e->status, sizeof(int)), "status");
+  if (n >= 128) ck(cudaMalloc(&e->pair, pair_work_bytes(std::min(n, PAIR_MAX))), "pair");
   ck(cudaMalloc(&e->gstatus, sizeof(int)), "gstatus");
   ck(cudaMemsetAsync(e->gstatus, 0, sizeof(int), s), "gstatus");
   ck(cudaMallocHost(&e->hstatus, sizeof(int)), "hstatus");
@@ -1303,6 +1316,7 @@ void eigen_destroy(EigenSolver* e) {
   cudaFree(e->xch);
   cudaFree(e->status);
   cudaFree(e->gstatus);
+  cudaFree(e->pair);
   cudaFreeHost(e->hstatus);
   delete e;
 }
@@ -1329,9 +1343,17 @@ int eigen_values(EigenSolver* es, const double* F, double* w_out, int nev) {
   cudaStream_t s = es->stream;
   // A = X^T (F X): X upper triangular
   if (split_gemm(n)) {  // BF16 tensor cores, FP64-accurate splitting (exponents in tw)
-    int* ex = reinterpret_cast<int*>(es->tw);
-    ogemm(false, false, n, n, n, F, es->X, es->T1, n, KM_LT_COLEND, ex, es->gstatus, s);
-    ogemm(true, false, n, n, n, es->X, es->T1, es->A, n, KM_LT_ROWEND | KM_SYM, ex, es->gstatus, s);
+    if (pair_gemm(n, eigen_gemm_pair(es))) {
+      pgemm_pair(n, false, false, n, n, n, F, n, es->X, n, es->T1, n, false, es->pair, es->gstatus,
+                 s);
+      pgemm_pair(n, true, false, n, n, n, es->X, n, es->T1, n, es->A, n, true, es->pair,
+                 es->gstatus, s);
+    } else {
+      int* ex = reinterpret_cast<int*>(es->tw);
+      ogemm(false, false, n, n, n, F, es->X, es->T1, n, KM_LT_COLEND, ex, es->gstatus, s);
+      ogemm(true, false, n, n, n, es->X, es->T1, es->A, n, KM_LT_ROWEND | KM_SYM, ex, es->gstatus,
+            s);
+    }
   } else {
     gemm64(false, false, n, n, n, 1.0, F, n, es->X, n, 0.0, es->T1, n, KM_LT_COLEND, s);
     gemm64(true, false, n, n, n, 1.0, es->X, n, es->T1, n, 0.0, es->A, n, KM_LT_ROWEND | KM_SYM, s);
@@ -1401,7 +1423,10 @@ void eigen_vectors_range(EigenSolver* es, int k0, int k1, double* C) {
       n, k, chunk, bt_ysmem(n), es->A, es->lu, Yk);
   prof_kend(KS_BACKTRANSFORM, tb_, s);
   // C = X Y (X upper triangular)
-  if (split_gemm(n))
+  if (pair_gemm(n, eigen_gemm_pair(es)))
+    pgemm_pair(n, false, false, n, k, n, es->X, n, Yk, n, C + (size_t)k0 * n, n, false, es->pair,
+               es->gstatus, s);
+  else if (split_gemm(n))
     ogemm(false, false, n, k, n, es->X, Yk, C + (size_t)k0 * n, n, KM_GE_ROWBEG,
           reinterpret_cast<int*>(es->tw), es->gstatus, s);
   else
@@ -1422,7 +1447,7 @@ __global__ void k_scale_cols(int n, int k, const double* C, const double* f, dou
 }
 
 void density_matrix(int n, int k, const double* C, const double* f, double* P, double* work,
-                    cudaStream_t s, int* status) {
+                    cudaStream_t s, int* status, void* pair) {
   if (k <= 0) {
     cudaMemsetAsync(P, 0, sizeof(double) * (size_t)n * n, s);
     return;
@@ -1431,7 +1456,9 @@ void density_matrix(int n, int k, const double* C, const double* f, double* P, d
   ++g_kernel_launches;
   k_scale_cols<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(n, k, C, f, work);
   // the split GEMM keeps its 2n exponents behind the scaled columns (needs k < n)
-  if (status && split_gemm(n) && k < n)
+  if (status && pair_gemm(n, pair) && k < n)
+    pgemm_pair(n, false, true, n, n, k, work, n, C, n, P, n, true, pair, status, s);
+  else if (status && split_gemm(n) && k < n)
     ogemm(false, true, n, n, k, work, C, P, n, KM_NONE | KM_SYM,
           reinterpret_cast<int*>(work + tot), status, s);
   else
@@ -1439,6 +1466,15 @@ void density_matrix(int n, int k, const double* C, const double* f, double* P, d
 }
 
 int* eigen_gemm_status(EigenSolver* es) { return es->gstatus; }
+void* eigen_gemm_pair(EigenSolver* es) { return es->pair_on ? es->pair : nullptr; }
+void eigen_set_pair(EigenSolver* es, bool on) { es->pair_on = on; }
+bool eigen_pair_failed(EigenSolver* es) {
+  int h = 0;
+  return pair_gemm(es->n, eigen_gemm_pair(es)) &&
+         cudaMemcpyAsync(&h, es->gstatus, sizeof(int), cudaMemcpyDeviceToHost, es->stream) ==
+             cudaSuccess &&
+         cudaStreamSynchronize(es->stream) == cudaSuccess && h != 0;
+}
 bool eigen_gemm_failed(EigenSolver* es) {
   int h = 0;
   ck(cudaMemcpyAsync(&h, es->gstatus, sizeof(int), cudaMemcpyDeviceToHost, es->stream), "gstatus");

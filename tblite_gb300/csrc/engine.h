@@ -309,6 +309,12 @@ void psplit(const double* M, int ld, int kcontig, int lines, int K, PImage& img,
 // set to 1 if a wait of the tensor-core pipeline ran out
 void pgemm(const PImage& A, const PImage& B, double* C, int ldc, bool sym, int* status,
            cudaStream_t s, int eshiftA = 0);
+// one product of dimensions up to n, operands split and multiplied in two launches; work holds
+// pair_work_bytes(n)
+size_t pair_work_bytes(int n);
+void pgemm_pair(int n, bool ta, bool tb, int M, int N, int K, const double* A, int lda,
+                const double* B, int ldb, double* C, int ldc, bool sym, void* work, int* status,
+                cudaStream_t s);
 
 // density by spectral projection (purify.cu): closed-shell, gapped systems at large n
 struct Purifier;
@@ -353,13 +359,16 @@ void launch_fe(int n, const double* f, const double* e, double* out, cudaStream_
 // may run on the tensor cores (split GEMM), which then keeps 2n ints behind the n*k scaled
 // columns in work
 void density_matrix(int n, int k, const double* C, const double* f, double* P, double* work,
-                    cudaStream_t s, int* status = nullptr);
+                    cudaStream_t s, int* status = nullptr, void* pair = nullptr);
 // split GEMM of the one-molecule path (ozaki.cu): C = op(A) op(B), column-major, leading
 // dimension ld; ex: M + ld ints of device scratch; status set to 1 if it did not complete
 void ogemm(bool ta, bool tb, int M, int N, int K, const double* A, const double* B, double* C,
            int ld, int kmode, int* ex, int* status, cudaStream_t s);
 // the eigensolver's tensor-core GEMM status word, and its check (synchronises the stream)
 int* eigen_gemm_status(EigenSolver*);
+void* eigen_gemm_pair(EigenSolver*);  // workspace of the small products (pgemm_pair), or null
+void eigen_set_pair(EigenSolver*, bool on);
+bool eigen_pair_failed(EigenSolver*);  // small products are on and one did not complete
 bool eigen_gemm_failed(EigenSolver*);
 // wbo[A][B] += scale * sum (PS)_{nu mu} (PS)_{mu nu} over the orbitals of atoms A != B
 void launch_wbo(const DevMol& m, const double* PS, double* wbo, double scale, cudaStream_t s);

@@ -1282,6 +1282,75 @@ void psplit(const double* M, int ld, int kcontig, int lines, int K, PImage& img,
                                                            img.e, img.data);
 }
 
+// ---- both operands of one small product in one launch: block (line block, k chunk, operand).  A
+// block finds the exponents of its 64 lines over all of k for itself (a few reads more per chunk
+// instead of a launch in between), the first chunk's block writes them, and each splits its chunk.
+struct SmallOperand {
+  const double* M;
+  int ld, kcontig, lines;
+  int* e;
+  uint16_t* img;
+};
+__global__ void __launch_bounds__(256) k_psplit_pair(SmallOperand oa, SmallOperand ob, int K) {
+  const SmallOperand o = blockIdx.z ? ob : oa;
+  const int lp = lines_padded(o.lines), lb = blockIdx.x, kc = blockIdx.y;
+  if (lb >= lp / 64) return;
+  __shared__ unsigned long long top[4][64];
+  __shared__ int se[64];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (o.kcontig) {
+    for (int li = wid; li < 64; li += 8) {
+      const int i = lb * 64 + li;
+      unsigned long long mx = 0ull;
+      if (i < o.lines) {
+#pragma unroll 4
+        for (int k = lane; k < K; k += 32) mx = max(mx, abs_bits(o.M[k + (size_t)i * o.ld]));
+      }
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+      if (lane == 0) se[li] = exp_of_max(mx);
+    }
+  } else {
+    const int li = tid & 63, g = tid >> 6, i = lb * 64 + li;
+    unsigned long long mx = 0ull;
+    if (i < o.lines) {
+#pragma unroll 8
+      for (int k = g; k < K; k += 4) mx = max(mx, abs_bits(o.M[i + (size_t)k * o.ld]));
+    }
+    top[g][li] = mx;
+    __syncthreads();
+    if (g == 0) se[li] = exp_of_max(max(max(top[0][li], top[1][li]), max(top[2][li], top[3][li])));
+  }
+  __syncthreads();
+  if (kc == 0 && tid < 64) o.e[lb * 64 + tid] = se[tid];
+  psplit_dev<Balanced>(o.M, o.ld, o.kcontig, o.lines, K, lp / 64, se[tid & 63], o.img, lb, kc);
+}
+
+// work of pgemm_pair for orders up to n
+static size_t pair_image(int n) { return (pimage_bytes(n, n, true) + 255) & ~(size_t)255; }
+size_t pair_work_bytes(int n) { return 2 * (pair_image(n) + sizeof(int) * pimage_lines(n)); }
+
+// C = op(A) op(B), column-major, all dimensions at most n: split and product in two launches
+void pgemm_pair(int n, bool ta, bool tb, int M, int N, int K, const double* A, int lda,
+                const double* B, int ldb, double* C, int ldc, bool sym, void* work, int* status,
+                cudaStream_t s) {
+  unsigned char* p = static_cast<unsigned char*>(work);
+  PImage ia, ib;
+  ia.balanced = ib.balanced = true;
+  ia.lines = M;
+  ib.lines = N;
+  ia.K = ib.K = K;
+  ia.data = reinterpret_cast<uint16_t*>(p);
+  ib.data = reinterpret_cast<uint16_t*>(p + pair_image(n));
+  ia.e = reinterpret_cast<int*>(p + 2 * pair_image(n));
+  ib.e = ia.e + pimage_lines(n);
+  const int lb = std::max(pimage_lines(M), pimage_lines(N)) / 64;
+  ++g_kernel_launches;
+  k_psplit_pair<<<dim3(lb, (K + PP_KC - 1) / PP_KC, 2), 256, 0, s>>>(
+      {A, lda, ta ? 1 : 0, M, ia.e, ia.data}, {B, ldb, tb ? 0 : 1, N, ib.e, ib.data}, K);
+  pgemm(ia, ib, C, ldc, sym, status, s, 0);
+}
+
 // C = 2^eshiftA op(A) op(B) from two slice images (A.K == B.K); sym: the product is symmetric
 void pgemm(const PImage& A, const PImage& B, double* C, int ldc, bool sym, int* status,
            cudaStream_t s, int eshiftA) {

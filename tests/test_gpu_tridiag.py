@@ -1,8 +1,9 @@
 """Fixed-point tridiagonalisation at the orders where its launch or its layout changes.
 
 Molecules of waters, ammonias and hydrogens are put together to a given number of orbitals: one
-CTA, 8-CTA cluster (64 .. 256), cooperative grid (257 .. 512, above 512 several rows per thread),
-and in a batch the one-CTA, cluster and 16-CTA cluster forms (up to 162, up to about 430, above).
+CTA, 8-CTA cluster (64 .. 256), cooperative grid (257 .. 512; one molecule of more orbitals takes
+the FP64 kernel), the tensor-core products (from 128 on, above 512 by another kernel), and in a
+batch the one-CTA, cluster and 16-CTA cluster forms (up to 162, up to about 430, above).
 The orbital energies are compared with LAPACK's of the oracle's converged Fock matrix; an SCF
 converged to 1e-9 Eh fixes them to well below the 1e-7 Eh used here.
 """
@@ -11,7 +12,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-ORBITALS = [2, 6, 7, 32, 33, 63, 64, 65, 161, 162, 163, 256, 257]
+ORBITALS = [2, 6, 7, 32, 33, 63, 64, 65, 127, 128, 161, 162, 163, 256, 257]
 LARGE = [433, 512, 513]
 
 
