@@ -747,7 +747,7 @@ __device__ __forceinline__ void opipe_tile(const PipeArgs& a, int b) {
       }
     }
     asm volatile("bar.sync 1, 256;" ::: "memory");
-    if (__all_sync(0xffffffffu, (mirror && !*abort) ? 1 : 0)) {
+    if (!FIXED && __all_sync(0xffffffffu, (mirror && !*abort) ? 1 : 0)) {
       const long long* mir = reinterpret_cast<const long long*>(smem);
       long long* W = reinterpret_cast<long long*>(a.C);
 #pragma unroll 4
@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) k_opipe(PipeArgs a) {
 // ---- batched spectral projection on the pipe, one launch per step for every molecule of the
 // list still iterating (blockIdx.y / blockIdx.z walks the molecules): kb_opipe_sq squares the
 // iterate D_k from its slice image and writes D_(k+1) = D_k^2, or 2 D_k - D_k^2 (the old element
-// read first), over D_k in Y, and the slice image of D_(k+1) (every line exponent SP2_E) into the
+// read first), over D_k in Y (on and below the diagonal), and the slice image of D_(k+1) (every line exponent SP2_E) into the
 // other of the molecule's two images, with the tile's partial sums of its trace and of its squared
 // elements; its last block takes the next decision.  Molecules that left the batch or whose
 // projection has converged (sp2i[0] != 0) launch nothing.
@@ -1065,16 +1065,38 @@ __global__ void __launch_bounds__(256) kb_sp2_init(const MolPtrs* __restrict__ m
 }
 
 // after a projection: the converged iterate from fixed point back to FP64 in place (the products
-// P = 2 X D X^T read it as doubles); every listed molecule of the projection bucket
+// P = 2 X D X^T read it as doubles); every listed molecule of the projection bucket.  The steps keep
+// the triangle on and below the diagonal: 32 x 32 tiles of it go to both places, the mirror image
+// through shared memory
 __global__ void __launch_bounds__(256) kb_sp2_unfix(const MolPtrs* __restrict__ mp,
                                                     const int* __restrict__ list) {
   const MolPtrs& q = mp[list[blockIdx.z]];
   if (*q.flag < 0) return;
-  const size_t nn = (size_t)q.m.nao * q.m.nao;
-  long long* w = reinterpret_cast<long long*>(q.Y);
-  for (size_t e = (size_t)blockIdx.x * 256 + threadIdx.x; e < nn; e += (size_t)gridDim.x * 256)
-    q.Y[e] = w[e] == SP2_BAD ? __longlong_as_double(0x7FF8000000000000ll)
-                             : (double)w[e] * 0x1p-55;
+  __shared__ double tile[32][33];
+  const int n = q.m.nao, nt = (n + 31) / 32, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long* w = reinterpret_cast<const long long*>(q.Y);
+  for (int t = blockIdx.x; t < nt * (nt + 1) / 2; t += gridDim.x) {
+    int ti = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+    while (ti * (ti + 1) / 2 > t) --ti;
+    while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+    const int tj = t - ti * (ti + 1) / 2;
+    const int i = 32 * ti + lane;
+    __syncthreads();
+    for (int c = wid; c < 32; c += 8) {
+      const int j = 32 * tj + c;
+      if (i >= n || j > i) continue;
+      const size_t e = i + (size_t)j * n;
+      const double x = w[e] == SP2_BAD ? __longlong_as_double(0x7FF8000000000000ll)
+                                       : (double)w[e] * 0x1p-55;
+      q.Y[e] = x;
+      tile[c][lane] = x;
+    }
+    __syncthreads();
+    for (int r = wid; r < 32; r += 8) {
+      const int row = 32 * ti + r, j = 32 * tj + lane;  // element (row, j) to (j, row)
+      if (row < n && j < row) q.Y[j + (size_t)row * n] = tile[lane][r];
+    }
+  }
 }
 
 // ---- batched GEMM sites on the pipe (projection buckets): the rows of op(A) go into img,
@@ -1229,8 +1251,7 @@ void sp2_init_b(const BatchLaunch& b) {
 // the projection iterate back to FP64 for every listed molecule (after the last step)
 void sp2_unfix_b(const BatchLaunch& b) {
   if (!b.count) return;
-  const size_t nn = (size_t)b.nao_max * b.nao_max;
-  const int blocks = (int)std::min<size_t>((nn + 1023) / 1024, 4096);
+  const int nt = (b.nao_max + 31) / 32, blocks = nt * (nt + 1) / 2;
   ++g_kernel_launches;
   kb_sp2_unfix<<<dim3(blocks, 1, b.count), 256, 0, b.s>>>(b.mp, b.list);
 }
