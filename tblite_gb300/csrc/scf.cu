@@ -13,8 +13,8 @@
 //   Mulliken                 src/tblite/wavefunction/mulliken.f90:37-100
 //   Fermi filling            src/tblite/wavefunction/fermi.f90:31-106, scf/iterator.f90:347-353
 //   Broyden                  src/tblite/scf/mixer/broyden.f90:148-278
-// Interaction matrices (gamma, AES) are evaluated on the fly inside the potential kernels
-// instead of being stored: one warp per atom walks all partners.
+// Interaction matrices (gamma, AES) are tabulated per pair once per geometry, or evaluated inside the
+// potential kernels where there is no table: one warp per atom walks all partners.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -708,7 +708,7 @@ __device__ __forceinline__ void fock_dev(int n, const int* __restrict__ ao_at,
                                               const double* __restrict__ vqp, double* F) {
   const int I = blockIdx.y, J = blockIdx.x;
   if (I > J) return;
-  __shared__ double sh[32][33];
+  __shared__ double sh2[2][32][33];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const size_t nn = (size_t)n * n;
   const int c = J * 32 + tx;
@@ -727,31 +727,44 @@ __device__ __forceinline__ void fock_dev(int n, const int* __restrict__ ao_at,
       acc[s] = H[rc] - 0.5 * S[rc] * (vao[r] + vc);
     }
   }
-  // multipole terms (absent, D == nullptr, for a Hamiltonian without anisotropic electrostatics)
-  for (int k = 0; D != nullptr && k < 9; ++k) {
+  // multipole terms (absent, D == nullptr, for a Hamiltonian without anisotropic electrostatics).  A
+  // small molecule's time is the latency of its loads, so the next matrix is loaded while this one
+  // is used, with one barrier each (67 -> 54 us at 1202 orbitals, 13.6 -> 13.0 at 192)
+  double tile[4], mrc[4];
+  auto load = [&](int k) {
     const double* M = k < 3 ? D + k * nn : Q + (k - 3) * nn;
-    const double* u = k < 3 ? vdp : vqp;
-    const int ku = k < 3 ? k : k - 3, su = k < 3 ? 3 : 6;
-    // stage tile (J, I) of M: sh[a][b] = M[J*32 + a][I*32 + b]
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
-      const int a = ty + 8 * s;
-      const int rr = J * 32 + a, cc = I * 32 + tx;
-      sh[a][tx] = (rr < n && cc < n) ? M[(size_t)rr * n + cc] : 0.0;
+      const int rr = J * 32 + ty + 8 * s, cc = I * 32 + tx;  // tile (J, I) of M
+      tile[s] = (rr < n && cc < n) ? M[(size_t)rr * n + cc] : 0.0;
+      mrc[s] = (rows[s] < n && cin) ? M[(size_t)rows[s] * n + c] : 0.0;
+    }
+  };
+  if (D != nullptr) load(0);
+  for (int k = 0; D != nullptr && k < 9; ++k) {
+    const double* u = k < 3 ? vdp : vqp;
+    const int ku = k < 3 ? k : k - 3, su = k < 3 ? 3 : 6;
+    double(&sh)[32][33] = sh2[k & 1];  // sh[a][b] = M[J*32 + a][I*32 + b]
+    double m[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      sh[ty + 8 * s][tx] = tile[s];
+      m[s] = mrc[s];
     }
     __syncthreads();
+    if (k < 8) load(k + 1);
     const double uc = cin ? u[su * atc + ku] : 0.0;
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
       const int r = rows[s];
       if (r < n && cin) {
-        const double t1 = M[(size_t)r * n + c] * uc;          // M_rc u_A(c)
+        const double t1 = m[s] * uc;                                   // M_rc u_A(c)
         const double t2 = sh[tx][ty + 8 * s] * u[su * ao_at[r] + ku];  // M_cr u_A(r)
         acc[s] -= 0.5 * (r <= c ? (t1 + t2) : (t2 + t1));
       }
     }
-    __syncthreads();
   }
+  double(&sh)[32][33] = sh2[1];  // (the last matrix used the other buffer)
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
     const int r = rows[s];
@@ -794,12 +807,16 @@ void launch_fock(int n, const int* ao_at, const double* H, const double* S, cons
 //   0: sum_r P S, 1-3: sum_r P D_k, 4-9: sum_r P Q_q, 10: sum_r P H
 // ------------------------------------------------------------------------------------
 // rows per chunk: 11 FP64 multiply-adds per row and column, so short chunks spread a molecule
-// over more SMs (68 orbitals: 64 rows 80 us, see the table of kernels for 16)
+// over more SMs (68 orbitals: 64 rows 80 us, 16 rows 21 us)
 // (above 512 orbitals the one-molecule path keeps its order of summation, see tridiag_fixed)
 __host__ __device__ constexpr int mull_rows(int n) { return n <= 512 ? 16 : 64; }
 
 int mulliken_chunks(int n) { return (n + mull_rows(n) - 1) / mull_rows(n); }
 
+// ROWS rows with their loads in flight: four for one molecule, whose few blocks wait for them (21 ->
+// 10 us at 192 orbitals, 207 -> 73 us at 1202), one in a batch, where other blocks fill the time
+// (four take 95 us a launch instead of 65 there)
+template <int ROWS>
 __device__ __forceinline__ void mull_partial_dev(int n, const double* __restrict__ P,
                                                       const double* __restrict__ S,
                                                       const double* __restrict__ H,
@@ -814,6 +831,7 @@ __device__ __forceinline__ void mull_partial_dev(int n, const double* __restrict
 #pragma unroll
   for (int k = 0; k < 11; ++k) acc[k] = 0.0;
   const int r0 = chunk * mull_rows(n), r1 = min(n, r0 + mull_rows(n));
+#pragma unroll ROWS
   for (int r = r0; r < r1; ++r) {
     const size_t rc = (size_t)r * n + c;
     const double pv = P[rc];
@@ -833,7 +851,7 @@ __global__ void __launch_bounds__(128) k_mull_partial(int n, const double* __res
                                                       const double* __restrict__ D,
                                                       const double* __restrict__ Q,
                                                       double* partial) {
-  mull_partial_dev(n, P, S, H, D, Q, partial);
+  mull_partial_dev<4>(n, P, S, H, D, Q, partial);
 }
 
 // 16 threads per atom, one per sum (population, 3 dipole, 6 quadrupole, band energy): reduce the
@@ -1539,7 +1557,7 @@ void launch_fock_b(const BatchLaunch& b) {
 __global__ void __launch_bounds__(128) kb_mull_partial(BARGS) {
   BMOL;
   if ((int)blockIdx.y >= q.mull_chunks) return;
-  mull_partial_dev(q.m.nao, q.P, q.S, q.H, q.D, q.Q, q.mull);
+  mull_partial_dev<1>(q.m.nao, q.P, q.S, q.H, q.D, q.Q, q.mull);
 }
 __global__ void kb_mull_reduce(BARGS) {
   BMOL;
