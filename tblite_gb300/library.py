@@ -287,8 +287,7 @@ def batch_projected() -> int:
 
 
 def set_small_tridiag(full_storage: bool) -> None:
-    """Small batch buckets: one-CTA full-storage tridiagonalisation (default) or the packed
-    lower-triangle kernel."""
+    """Small batch buckets: one CTA per molecule in the tridiagonalisation (default) or a cluster."""
     load().tblite_gb300_set_small_tridiag(1 if full_storage else 0)
 
 
