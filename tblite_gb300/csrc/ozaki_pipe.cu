@@ -1,4 +1,4 @@
-// Pipelined FP64-accurate split GEMM on the BF16 tensor cores for the one-molecule path.
+// Pipelined FP64-accurate split GEMM on the BF16 tensor cores.
 //
 // Two splittings (struct Balanced, struct Magnitude).  Balanced: x = 2^e sum_p d_p 2^(-7 - 8p),
 // p = 0..6, with digits d_p in [-128, 128]: seven slices in BF16, and the 28 slice products d_p d_q
@@ -6,10 +6,10 @@
 // x's sign, 36 products with p + q <= 7.  Balanced radix-256 digits have the same magnitude bound
 // (products <= 2^14, so as many of them sum exactly in FP32) and hold one bit more each, and what
 // is rounded or dropped has no sign bias: 28 products instead of 36 and a smaller error (A A^T of
-// 3072: 8.5e-16 against 1.2e-15).  The batch and tblite_gb300_split_gemm use Balanced.  The
-// one-molecule projection (purify.cu) keeps Magnitude and with it its results: its bias loses
-// 2e-10 electrons of 4000 (500 waters), which the dipole of a cluster far from the origin shows at
-// 5e-10, so the splittings' results differ visibly there although both are within the solver's
+// 3072: 8.5e-16 against 1.2e-15).  The batch, the small products of one molecule (pgemm_pair) and
+// tblite_gb300_split_gemm use Balanced.  The one-molecule projection (purify.cu) keeps Magnitude and
+// with it its results: its bias loses 2e-10 electrons of 4000 (500 waters), which the dipole of a
+// cluster far from the origin shows at 5e-10, so the splittings' results differ visibly there although both are within the solver's
 // tolerance.  The operands are split once per matrix instead of once per tile pair, and the
 // products are grouped so that each tensor-core instruction is wide (figures of Balanced;
 // Magnitude in brackets where they differ):
@@ -24,17 +24,20 @@
 //            slices of a stage lie one after another, so d_p times [d_q0 .. d_q0+3] is a single
 //            M 128 x N 256 x K 16 tcgen05.mma whose four 64-column blocks land in the TMEM
 //            accumulators of the levels p + q0 .. p + q0 + 3 (one accumulator of 64 columns per
-//            level 0..6); 10 [13] MMAs per k step.  Warps 2..9 drain the levels 0..4 [0..5] every
-//            6 [5] chunks (192 [160] values of k): they hold exact integers (at most 5 [6]
-//            products of <= 2^14 each per k: < 2^24) that go into one int64 per element.  The
-//            levels 5..6 [6..7] (weight 2^-40 [2^-42] of the
-//            leading level and a random sum of balanced digits) stay in FP32 over the whole of k
-//            (their rounding is below 2^-53 of the largest possible element) and are read with
+//            level 0..6); 11 [12] MMAs per k step, first those of the levels below 4, then the
+//            others.  Warps 2..9 drain the levels 0..4 [0..5] every 6 [5] chunks (192 [160] values
+//            of k): they hold exact integers (at most 5 [6] products of <= 2^14 each per k: < 2^24)
+//            that go into one int64 per element.  The levels 5..6 [6..7] (weight 2^-40 [2^-42] of
+//            the leading level and a random sum of balanced digits) stay in FP32 over the whole of
+//            k (their rounding is below 2^-53 of the largest possible element) and are read with
 //            the output at the end.
 //
-// Bound by the tensor pipe (896 [1152] cycles per k step of 16) and, at the end of every window, by the
-// conversion of the drained sums (8 cycles per warp and conversion): the drain's loads are issued
-// one level ahead, level 0 (below 2^22) is converted by an FP32 addition instead.
+// Bound by the tensor pipe (896 [1152] cycles per k step of 16) and by what does not run beside it:
+// prologue, last drain and epilogue of a tile (one CTA per SM), and what is left of a window's drain
+// (8 cycles per warp and conversion, about 3000 in all) when the other half's MMAs are done: the lower
+// levels are drained under the window's last upper MMAs, the upper ones under the next window's
+// first lower MMAs (A A^T of 3072 770 -> 697 us, a product of 3000 804 -> 668 us).  The drain's loads
+// are issued one level ahead, level 0 (below 2^22) is converted by an FP32 addition instead.
 //
 // Every wait is bounded; a wait that runs out sets a CTA-wide abort flag, the other roles leave
 // their loops, copies and MMAs still in flight are waited for (bounded), TMEM is freed and the

@@ -297,6 +297,8 @@ __device__ __forceinline__ void aes_scalars(const DevMol& m, const Gfn2Scalars& 
 
 // tab: the pair table of coulomb_table_dev, or nullptr to evaluate the pair terms here.  The sixteen
 // sums over the warp cost as much as the pairs of a molecule of 50 atoms when each is taken alone.
+// 1500 atoms 756 us without the table, 330 with it; 96 atoms 28 and 15 us (energy: 736 and 217, 28
+// and 12 us, the contraction by pairs included).
 __device__ __forceinline__ void coulomb_potential_dev(DevMol m, Gfn2Scalars p,
                           const double* __restrict__ mrad, const double* __restrict__ qsh,
                           const double* __restrict__ qat, const double* __restrict__ dpat,
