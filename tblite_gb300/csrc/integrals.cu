@@ -117,8 +117,8 @@ __device__ __forceinline__ double hscale_of(const DevMol& m, const Gfn2Scalars& 
 // there.
 //
 // H0 gradient and H0 build of a 1024-molecule ensemble, ms of the device: pairs of mixed kinds 36 and
-// 27, by kind 19.2 and 14.6, with the queue 13.5 and 10.8; of an octane cation, us: one lane per pair
-// 761 and 355, eight lanes 133 and 70.
+// 27, by kind 19.2 and 14.6, with the queue 13.5 and 10.8; H0 gradient of an octane cation: one lane
+// per pair 761 us, eight lanes 133 us.
 constexpr int WALK_G = 8;
 constexpr int WALK_THREADS = 128;
 // the form and the rounds for a number of tasks: 8 lanes while that is at most eight warps per
