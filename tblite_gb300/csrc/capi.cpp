@@ -867,6 +867,17 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   // spectral projection (purify.cu): closed shells with whole electron pairs only
   const bool purify = c->density_solver == 1;
   const int nocc = (int)llround(nalp);
+  // large and elongated molecules keep the order of every sum of their SCF (see tridiag_fixed)
+  double extent = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    double lo = mol->xyz[k], hi = lo;
+    for (int i = 1; i < nat; ++i) {
+      lo = std::min(lo, mol->xyz[3 * i + k]);
+      hi = std::max(hi, mol->xyz[3 * i + k]);
+    }
+    extent = std::max(extent, hi - lo);
+  }
+  const bool ordered = n > TRIDIAG_FIXED_MAX || extent > ORDERED_EXTENT;
   if (purify) {
     if (nalp != nbet)
       throw std::runtime_error("the spectral-projection density solver needs a closed shell");
@@ -887,12 +898,12 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   // the table's pair terms are the ones evaluated in place but for their last bits, which a large
   // molecule keeps (see tridiag_fixed); it stays small beside the matrices
   const size_t ctab_words = coulomb_table_words(nsh, nat);
-  const bool ctab = (purify || n <= TRIDIAG_FIXED_MAX) && ctab_words <= COULOMB_TABLE_MAX;
+  const bool ctab = (purify || !ordered) && ctab_words <= COULOMB_TABLE_MAX;
   if (ctab) {
     w.ctab.alloc(ctab_words);
     launch_coulomb_table(m, p, w.mrad.p, w.ctab.p, s);
   }
-  launch_build_h0(m, p, w.se.p, w.S.p, w.H.p, w.D.p, w.Q.p, s);
+  launch_build_h0(m, p, w.se.p, w.S.p, w.H.p, w.D.p, w.Q.p, s, ordered);
   cuda_check(cudaMemsetAsync(w.grad.p, 0, sizeof(double) * 3 * nat, s), "zero");
   cuda_check(cudaMemsetAsync(w.sig_at.p, 0, sizeof(double) * 9 * nat, s), "zero");
   cuda_check(cudaMemsetAsync(w.sigma.p, 0, sizeof(double) * 9, s), "zero");
@@ -910,7 +921,10 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   }
   int chol = 0;
   if (purify) chol = purify_set_overlap(w.pur, w.S.p) < 0 ? 1 : 0;
-  else chol = eigen_set_overlap(w.eig, w.S.p);
+  else {
+    eigen_set_ordered(w.eig, ordered);
+    chol = eigen_set_overlap(w.eig, w.S.p);
+  }
   g_prof.end(s);
   if (c->fault == 1) chol = 1;  // injected: the first pivot is not positive
   if (chol != 0) {
@@ -958,7 +972,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   b.omega = w.b_omega.p;
   b.work = w.b_work.p;
   b.status = w.b_status.p;
-  b.ordered = n > TRIDIAG_FIXED_MAX;
+  b.ordered = ordered;
 
   const double econv = 1.0e-6 * c->accuracy, pconv = 2.0e-5 * c->accuracy;
   const double target_kt = c->etemp;
@@ -1055,7 +1069,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
         throw std::runtime_error("(sygvd) failed to solve eigenvalue problem. info=" +
                                  std::to_string(info));
       launch_fermi(n, w.emo.p, nalp, nbet, kt, w.focc.p, w.scal.p, w.icount.p, s, nev);
-      if (n > TRIDIAG_FIXED_MAX) {  // vectors of the occupied levels only
+      if (ordered) {  // vectors of the occupied levels only
         collect();
         if (more_levels()) fill_more_levels();
         nvec = h_cnt[0];
@@ -1073,7 +1087,8 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
     }
     auto analyse = [&]() {
     g_prof.begin(PH_MULLIKEN, s);
-    launch_mulliken(m, w.P.p, w.S.p, w.H.p, w.D.p, w.Q.p, w.mull.p, mulliken_chunks(n), w.qsh_o.p,
+    launch_mulliken(m, w.P.p, w.S.p, w.H.p, w.D.p, w.Q.p, w.mull.p,
+                    ordered ? (n + 63) / 64 : mulliken_chunks(n), w.qsh_o.p,
                     w.qat_o.p, w.dpat_o.p, w.qpat_o.p, w.eband.p, s);
     launch_pack(m, w.qsh_o.p, w.dpat_o.p, w.qpat_o.p, w.vec_out.p, s, with_mp);
     launch_diff((int)nd, w.vec_out.p, w.b_q.p, w.b_dq.p, w.scal.p + 1, s);  // mixer%diff
@@ -1091,7 +1106,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
     // the Broyden step that began this iteration (its status came with the rest)
     if (iscf > 1 && h_status != 0)
       throw std::runtime_error("Broyden mixing failed to obtain next iteration");
-    if (!purify && n <= TRIDIAG_FIXED_MAX && more_levels()) {  // the density again, all levels
+    if (!purify && !ordered && more_levels()) {  // the density again, all levels
       fill_more_levels();
       nvec = n;
       eigen_vectors(w.eig, nvec, w.C.p);
@@ -1200,7 +1215,7 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   std::vector<double> h_pgrad, h_cn;
   if (c->param_grad) {
     w.ones.upload(std::vector<double>(nsh, 1.0), s);
-    launch_build_h0(m, p, w.ones.p, w.S.p, w.scratch.p, w.D.p, w.Q.p, s);
+    launch_build_h0(m, p, w.ones.p, w.S.p, w.scratch.p, w.D.p, w.Q.p, s, ordered);
     w.pgrad.alloc((size_t)3 * nsh);
     launch_param_grad(m, p, w.P.p, w.scratch.p, w.qsh_o.p, w.pgrad.p, s);
     w.pgrad.download(h_pgrad, (size_t)3 * nsh, s);

@@ -60,6 +60,7 @@ struct EigenSolver {
   int* status = nullptr;  // device
   void* pair = nullptr;   // workspace of the pipelined products up to PAIR_MAX orbitals
   bool pair_on = true;
+  bool ordered = false;  // roundings of the FP64 kernels (eigen_set_ordered)
   int* gstatus = nullptr; // device: 1 once a tensor-core GEMM did not answer
   int* hstatus = nullptr; // pinned
   int coop_blocks = 0;
@@ -592,7 +593,7 @@ __device__ double tri_ladder(int n, const double* __restrict__ d, const double* 
 template <int D>
 __device__ double tri_eigenvalue(int n, const double* __restrict__ d, const double* __restrict__ e2,
                                  const float* __restrict__ fd, const float* __restrict__ fe2,
-                                 int j, bool active, const TriBounds& b) {
+                                 int j, bool active, const TriBounds& b, bool ladder = true) {
   constexpr int G = 1 << D;
   const int sub = threadIdx.x & (G - 1), lead = (threadIdx.x & 31) - sub;
   // 1. FP32 bisection
@@ -631,7 +632,7 @@ __device__ double tri_eigenvalue(int n, const double* __restrict__ d, const doub
     }
   }
   if constexpr (D == 4) {
-    if (n <= TRIDIAG_FIXED_MAX) return tri_ladder(n, d, e2, flo, fhi, j, active, b);
+    if (ladder && n <= TRIDIAG_FIXED_MAX) return tri_ladder(n, d, e2, flo, fhi, j, active, b);
   }
   // 2. widened bracket, checked in FP64
   const double wid = b.tnorm * 0x1p-16;
@@ -758,6 +759,7 @@ __global__ void k_tri_prep(int n, const double* __restrict__ d, const double* __
 // block (the warps of a single molecule spread over as many SMs as possible), 16 lanes per
 // eigenvalue: 2 warps per SM at 600 eigenvalues, so the extra FP32 counts cost no time
 constexpr int EIG_D = 4;
+// fill: bit 0 mark the eigenvalues not computed, bit 1 the order of large molecules (no ladder)
 __global__ void __launch_bounds__(32) k_eigvals(int n, int j0, int j1, int fill,
                                                  const double* __restrict__ d,
                                                  const double* __restrict__ ws,
@@ -766,7 +768,7 @@ __global__ void __launch_bounds__(32) k_eigvals(int n, int j0, int j1, int fill,
   const float* fd = reinterpret_cast<const float*>(ws + n);
   const float* fe2 = fd + n;
   if (j0 + (int)((blockIdx.x * blockDim.x) >> EIG_D) >= j1) {  // a warp of unwanted eigenvalues
-    if (fill && (threadIdx.x & ((1 << EIG_D) - 1)) == 0 && j < n) w[j] = TRI_SENTINEL;
+    if ((fill & 1) && (threadIdx.x & ((1 << EIG_D) - 1)) == 0 && j < n) w[j] = TRI_SENTINEL;
     return;
   }
   TriBounds b;
@@ -775,10 +777,10 @@ __global__ void __launch_bounds__(32) k_eigvals(int n, int j0, int j1, int fill,
   b.hi = scal[3];
   b.pivmin = scal[4];
   const bool active = j < j1;
-  const double v = tri_eigenvalue<EIG_D>(n, d, ws, fd, fe2, j, active, b);
+  const double v = tri_eigenvalue<EIG_D>(n, d, ws, fd, fe2, j, active, b, !(fill & 2));
   if ((threadIdx.x & ((1 << EIG_D) - 1)) != 0) return;
   if (active) w[j] = v;
-  else if (fill && j < n) w[j] = TRI_SENTINEL;
+  else if ((fill & 1) && j < n) w[j] = TRI_SENTINEL;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1327,7 +1329,7 @@ int eigen_set_overlap(EigenSolver* e, const double* S) {
   const int n = e->n;
   // a new geometry: the tensor-core status word starts clear
   ck(cudaMemsetAsync(e->gstatus, 0, sizeof(int), e->stream), "gstatus");
-  if (cholinv_fixed(n, S, e->X, e->status, e->stream)) {
+  if (!e->ordered && cholinv_fixed(n, S, e->X, e->status, e->stream)) {
     ck(cudaMemcpyAsync(e->hstatus, e->status, sizeof(int), cudaMemcpyDeviceToHost, e->stream),
        "Cholesky status");
     stream_wait(e->stream);
@@ -1361,7 +1363,7 @@ int eigen_values(EigenSolver* es, const double* F, double* w_out, int nev) {
   // tridiagonalise
   {
     const int tk = prof_kbegin(s);
-    if (n <= TRIDIAG_FIXED_MAX) {
+    if (n <= TRIDIAG_FIXED_MAX && !es->ordered) {
       tridiag_fixed(n, es->A, es->d, es->e, es->tau, es->xch, s);
     } else {
       int nn = n, blocks = std::min(es->coop_blocks, (n * 32 + 255) / 256);
@@ -1383,7 +1385,8 @@ int eigen_values(EigenSolver* es, const double* F, double* w_out, int nev) {
   g_kernel_launches += 2;
   const int tm = prof_kbegin(s);
   k_tri_prep<<<(n + 255) / 256, 256, 0, s>>>(n, es->d, es->e, es->tw, es->scal);
-  k_eigvals<<<((n << EIG_D) + 31) / 32, 32, 0, s>>>(n, 0, nev, 1, es->d, es->tw, es->scal, es->w);
+  k_eigvals<<<((n << EIG_D) + 31) / 32, 32, 0, s>>>(n, 0, nev, es->ordered ? 3 : 1, es->d,
+                                                             es->tw, es->scal, es->w);
   prof_kend(KS_MULTISECT, tm, s);
   ck(cudaMemcpyAsync(w_out, es->w, sizeof(double) * n, cudaMemcpyDeviceToDevice, s), "w");
   return 0;
@@ -1396,7 +1399,8 @@ void eigen_values_rest(EigenSolver* es, int nev, double* w_out) {
   g_kernel_launches += 2;
   const int tm = prof_kbegin(s);
   k_tri_prep<<<(n + 255) / 256, 256, 0, s>>>(n, es->d, es->e, es->tw, es->scal);
-  k_eigvals<<<(((n - nev) << EIG_D) + 31) / 32, 32, 0, s>>>(n, nev, n, 0, es->d, es->tw, es->scal, es->w);
+  k_eigvals<<<(((n - nev) << EIG_D) + 31) / 32, 32, 0, s>>>(n, nev, n, es->ordered ? 2 : 0,
+                                                                     es->d, es->tw, es->scal, es->w);
   prof_kend(KS_MULTISECT, tm, s);
   ck(cudaMemcpyAsync(w_out + nev, es->w + nev, sizeof(double) * (n - nev), cudaMemcpyDeviceToDevice, s),
      "w");
@@ -1466,7 +1470,10 @@ void density_matrix(int n, int k, const double* C, const double* f, double* P, d
 }
 
 int* eigen_gemm_status(EigenSolver* es) { return es->gstatus; }
-void* eigen_gemm_pair(EigenSolver* es) { return es->pair_on ? es->pair : nullptr; }
+void* eigen_gemm_pair(EigenSolver* es) {
+  return es->pair_on && !es->ordered ? es->pair : nullptr;
+}
+void eigen_set_ordered(EigenSolver* es, bool ordered) { es->ordered = ordered; }
 void eigen_set_pair(EigenSolver* es, bool on) { es->pair_on = on; }
 bool eigen_pair_failed(EigenSolver* es) {
   int h = 0;

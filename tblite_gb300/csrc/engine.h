@@ -187,7 +187,7 @@ void launch_cn_grad(const DevMol& m, const Gfn2Scalars& p, const double* dEdcn, 
 void launch_setup_levels(const DevMol& m, const Gfn2Scalars& p, const double* cn,
                          double* selfenergy, double* mrad, double* dmrdcn, cudaStream_t s);
 void launch_build_h0(const DevMol& m, const Gfn2Scalars& p, const double* selfenergy, double* S,
-                     double* H, double* D, double* Q, cudaStream_t s);
+                     double* H, double* D, double* Q, cudaStream_t s, bool ordered);
 void launch_h0_gradient(const DevMol& m, const Gfn2Scalars& p, const double* selfenergy,
                         const double* P, const double* W, const double* vao, const double* vdp,
                         const double* vqp, double* grad, double* sigma, double* dEdcn,
@@ -268,6 +268,11 @@ void eigen_resize(EigenSolver*, int n);
 // of 1e-16 anywhere in the iteration into 1e-9 of itself, so results comparable to the last digits
 // need the same roundings there
 constexpr int TRIDIAG_FIXED_MAX = 512;
+// the same for elongated molecules: the extent (largest side of the box around the atoms, Bohr) above
+// which a molecule keeps those roundings.  Charges that differ by 1e-13 over alkanes of 25 / 45 / 75
+// carbons (60 / 110 / 180 Bohr) change their dipole by 1e-9 / 3e-9 / 1e-8 of itself; clusters of 64
+// waters (30 Bohr) by 3e-11.
+constexpr double ORDERED_EXTENT = 34.0;
 void tridiag_fixed(int n, double* A, double* d, double* e, double* tau, long long* xch,
                    cudaStream_t s);
 size_t tridiag_exchange_words(int n);
@@ -365,6 +370,7 @@ void density_matrix(int n, int k, const double* C, const double* f, double* P, d
 void ogemm(bool ta, bool tb, int M, int N, int K, const double* A, const double* B, double* C,
            int ld, int kmode, int* ex, int* status, cudaStream_t s);
 // the eigensolver's tensor-core GEMM status word, and its check (synchronises the stream)
+void eigen_set_ordered(EigenSolver*, bool ordered);
 int* eigen_gemm_status(EigenSolver*);
 void* eigen_gemm_pair(EigenSolver*);  // workspace of the small products (pgemm_pair), or null
 void eigen_set_pair(EigenSolver*, bool on);

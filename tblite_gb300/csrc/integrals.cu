@@ -404,13 +404,14 @@ __global__ void __launch_bounds__(WALK_THREADS)
 }
 
 void launch_build_h0(const DevMol& m, const Gfn2Scalars& p, const double* se, double* S,
-                     double* H, double* D, double* Q, cudaStream_t s) {
+                     double* H, double* D, double* Q, cudaStream_t s, bool ordered) {
   const size_t nn = (size_t)m.nao * m.nao;
   cudaMemsetAsync(S, 0, nn * sizeof(double), s);
   cudaMemsetAsync(H, 0, nn * sizeof(double), s);
   cudaMemsetAsync(D, 0, 3 * nn * sizeof(double), s);
   cudaMemsetAsync(Q, 0, 6 * nn * sizeof(double), s);
-  const Walk w = walk_of(h0_padded(m.nsh, m.nsh - m.ns, {1, 1}));
+  Walk w = walk_of(h0_padded(m.nsh, m.nsh - m.ns, {1, 1}));
+  if (ordered) w.lanes = 1;  // the sums over the primitives in their order
   const unsigned blocks = walk_blocks(h0_padded(m.nsh, m.nsh - m.ns, w), w);
   ++g_kernel_launches;
   if (w.lanes == 1)

@@ -832,7 +832,9 @@ __device__ __forceinline__ void mull_partial_dev(int n, const double* __restrict
   double acc[11];
 #pragma unroll
   for (int k = 0; k < 11; ++k) acc[k] = 0.0;
-  const int r0 = chunk * mull_rows(n), r1 = min(n, r0 + mull_rows(n));
+  // (one molecule: the grid's chunks tell its rows, 64 where the order of summation is kept)
+  const int rows = ROWS > 1 ? ((int)gridDim.y == (n + 63) / 64 ? 64 : 16) : mull_rows(n);
+  const int r0 = chunk * rows, r1 = min(n, r0 + rows);
 #pragma unroll ROWS
   for (int r = r0; r < r1; ++r) {
     const size_t rc = (size_t)r * n + c;

@@ -99,6 +99,15 @@ def test_three_body_partners(waters, hydrogens, far):
     _check(_calculator(z, x).singlepoint(), _oracle(z, x))
 
 
+# 28, 30, 33, 35 and 64 Bohr long: from 34 Bohr on the one-molecule path keeps the FP64 kernels' sums
+@pytest.mark.parametrize("carbons", [11, 12, 13, 14, 26])
+def test_elongated_molecules(carbons):
+    from tblite_gb300 import workloads
+
+    z, x = workloads.alkane(carbons, seed=carbons)
+    _check(_calculator(z, x).singlepoint(), _oracle(z, x))
+
+
 def _product(lib, a, b, sym):
     import torch
 
