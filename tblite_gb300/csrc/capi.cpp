@@ -1180,11 +1180,13 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   }
   g_prof.end(s);
   // the result carries every orbital (wavefunction/type.f90 coeff(nao, nao)): the SCF only
-  // needed the occupied ones, the empty ones come from the last tridiagonal form
+  // needed the occupied ones, the empty ones come from the last tridiagonal form.  Vectors of close
+  // levels are made orthogonal within one call only, so all empty levels come from one call, from
+  // the gap on: nvec may lie inside a degenerate pair of empty levels (benzene: 21 of 30)
   if (!purify) {  // the projection has no orbitals
     g_prof.begin(PH_EIGEN, s);
     eigen_values_rest(w.eig, nev, w.emo.p);
-    eigen_vectors_range(w.eig, nvec, (int)n, w.C.p);
+    if (nvec < n) eigen_vectors_range(w.eig, h_cnt[0], (int)n, w.C.p);
     g_prof.end(s);
   }
   // Wiberg/Mayer bond orders (post_processing/wbo.f90:60-115): closed shell from P; restricted
