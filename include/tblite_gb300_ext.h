@@ -187,6 +187,10 @@ void tblite_gb300_get_result_gap(tblite_error error, tblite_result res, double* 
  */
 int tblite_gb300_split_gemm(int m, int n, int k, const double* a, const double* b, double* c,
                             int sym, void* stream);
+/* The slice images of a product (14 bytes per element of A and B) come from a pool of the library
+ * on the current device, which keeps up to 512 MiB between calls.  This gives back what no call in
+ * flight holds; the next product allocates again.  Returns 0, or -2 on a CUDA error. */
+int tblite_gb300_split_gemm_release(void);
 /* products of the spectral-projection solver: 1 (default) pipelined split GEMM from slice
  * images, 0 the per-tile split GEMM */
 void tblite_gb300_set_pipelined_gemm(int enable);

@@ -1428,16 +1428,18 @@ namespace {
 // that calls of any thread on any stream take and return memory in stream order (five cudaMalloc /
 // cudaFree pairs and a pageable copy were 380 of the 468 us of a 1202 x 601 x 777 product).  At
 // most GEMM_POOL_KEEP bytes stay with the pool between calls; what a larger product takes beyond
-// that goes back to the device when its call has synchronised.
+// that goes back to the device when its call has synchronised, and
+// tblite_gb300_split_gemm_release gives back the rest.
 constexpr uint64_t GEMM_POOL_KEEP = 512ull << 20;
 constexpr int GEMM_MAX_DEVICES = 64;
-cudaMemPool_t gemm_pool() {
+// the current device's pool; null: it could not be made, or (make == false) no call has made it yet
+cudaMemPool_t gemm_pool(bool make = true) {
   static std::mutex mutex;
   static cudaMemPool_t pools[GEMM_MAX_DEVICES] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= GEMM_MAX_DEVICES) return nullptr;
   std::lock_guard<std::mutex> lock(mutex);
-  if (!pools[dev]) {
+  if (!pools[dev] && make) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -1516,6 +1518,11 @@ extern "C" int tblite_gb300_split_gemm(int m, int n, int k, const double* a, con
   if (cudaFreeAsync(w, s) != cudaSuccess) rc = -2;
   if (cudaStreamSynchronize(s) != cudaSuccess) rc = -2;
   return rc != 0 ? rc : *(volatile int*)st != 0 ? 1 : 0;
+}
+
+extern "C" int tblite_gb300_split_gemm_release(void) {
+  const cudaMemPool_t pool = tb::gemm_pool(false);
+  return !pool || cudaMemPoolTrimTo(pool, 0) == cudaSuccess ? 0 : -2;
 }
 
 extern "C" void tblite_gb300_set_pipelined_gemm(int enable) { tb::g_pipe_gemm = enable != 0; }

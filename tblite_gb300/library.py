@@ -104,6 +104,7 @@ _SIGNATURES = {
     "tblite_gb300_set_calculator_density_solver": (None, [c_void_p, c_void_p, c_int]),
     "tblite_gb300_split_gemm": (
         c_int, [c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
+    "tblite_gb300_split_gemm_release": (c_int, []),
     "tblite_gb300_set_pipelined_gemm": (None, [c_int]),
     "tblite_gb300_get_result_gap": (None, [c_void_p, c_void_p, _dbl_p]),
     "tblite_gb300_get_result_shell_charges": (None, [c_void_p, c_void_p, _dbl_p]),
