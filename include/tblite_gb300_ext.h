@@ -230,6 +230,8 @@ int tblite_gb300_density_matrix_noalloc(int n, int k, const double* C, const dou
  * calculator report a pivot that is not positive, as a singular overlap (coincident atoms)
  * does: the single point fails with the reference's "(sygvd) failed to solve eigenvalue
  * problem. info=<n+1>", a batch entry leaves the batch and fails the same way (0 clears it).
+ * Kind 2: a single point finds no device memory for the pair table of its electrostatics (up to
+ * 1 GiB) and evaluates the pairs in every iteration instead.
  * tblite_gb300_set_pipeline_wait_limit(polls) sets how often a pipeline wait of the
  * pipelined split GEMM polls before it aborts the tile (0: the default 2^22); a wait that runs
  * out sets the status word (projection single point: an error; batch: the molecule takes the

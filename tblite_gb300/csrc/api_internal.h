@@ -67,6 +67,22 @@ struct DBuf {
     cuda_check(cudaMalloc(&p, sizeof(T) * std::max<size_t>(count, 1)), "cudaMalloc");
     n = count;
   }
+  // false (and empty) where the device has not that much left
+  bool try_alloc(size_t count) {
+    if (count <= n && p) return true;
+    if (p) cudaFree(p);
+    p = nullptr;
+    n = 0;
+    const cudaError_t e = cudaMalloc(&p, sizeof(T) * std::max<size_t>(count, 1));
+    if (e == cudaSuccess) {
+      n = count;
+      return true;
+    }
+    p = nullptr;
+    if (e != cudaErrorMemoryAllocation) cuda_check(e, "cudaMalloc");
+    cudaGetLastError();
+    return false;
+  }
   void upload(const std::vector<T>& h, cudaStream_t s) {
     alloc(h.size());
     if (!h.empty())
@@ -217,7 +233,8 @@ struct _tblite_calculator {
   // density solver: 0 diagonalisation (Fermi filling), 1 spectral projection (purify.cu)
   int density_solver = 0;
   // fault injected on the host for tests: 1 = the overlap factorisation reports a pivot that is
-  // not positive (what a singular overlap, e.g. from coincident atoms, produces)
+  // not positive (what a singular overlap, e.g. from coincident atoms, produces), 2 = the device
+  // has no memory left for the pair table of the electrostatics
   int fault = 0;
   // post-processing of every single point, in order ("bond-orders", "molmom"); an empty list
   // becomes the reference's default (bond orders and molecular moments) at the first single

@@ -896,13 +896,12 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
   launch_cn(m, p, w.cn.p, s);
   launch_setup_levels(m, p, w.cn.p, w.se.p, w.mrad.p, w.dmrdcn.p, s);
   // the table's pair terms are the ones evaluated in place but for their last bits, which a large
-  // molecule keeps (see tridiag_fixed); it stays small beside the matrices
+  // molecule keeps (see tridiag_fixed); it stays small beside the matrices, and where the device has
+  // no room for it the pairs are evaluated in place
   const size_t ctab_words = coulomb_table_words(nsh, nat);
-  const bool ctab = (purify || !ordered) && ctab_words <= COULOMB_TABLE_MAX;
-  if (ctab) {
-    w.ctab.alloc(ctab_words);
-    launch_coulomb_table(m, p, w.mrad.p, w.ctab.p, s);
-  }
+  const bool ctab = (purify || !ordered) && ctab_words <= COULOMB_TABLE_MAX && c->fault != 2 &&
+                    w.ctab.try_alloc(ctab_words);
+  if (ctab) launch_coulomb_table(m, p, w.mrad.p, w.ctab.p, s);
   launch_build_h0(m, p, w.se.p, w.S.p, w.H.p, w.D.p, w.Q.p, s, ordered);
   cuda_check(cudaMemsetAsync(w.grad.p, 0, sizeof(double) * 3 * nat, s), "zero");
   cuda_check(cudaMemsetAsync(w.sig_at.p, 0, sizeof(double) * 9 * nat, s), "zero");
@@ -2310,8 +2309,9 @@ void tblite_gb300_set_calculator_fault(tblite_context ctx, tblite_calculator cal
     ctx->push("Calculator object is missing");
     return;
   }
-  if (kind < 0 || kind > 1) {
-    ctx->push("fault kind must be 0 (none) or 1 (overlap not positive definite)");
+  if (kind < 0 || kind > 2) {
+    ctx->push("fault kind must be 0 (none), 1 (overlap not positive definite) or 2 (no memory for "
+              "the pair table)");
     return;
   }
   calc->fault = kind;
