@@ -267,21 +267,26 @@ void eigen_resize(EigenSolver*, int n);
 // TRIDIAG_FIXED_MAX): d, e, tau and the reflectors below the subdiagonal of A, as dsytrd('L'); xch
 // holds tridiag_exchange_words(n) words.  Larger molecules keep the FP64 reduction, and with it the
 // order of every sum of their SCF: a long chain's dipole (0.06 a.u. over 200 carbons) turns a change
-// of 1e-16 anywhere in the iteration into 1e-9 of itself, so results comparable to the last digits
+// of 1e-13 in its charges into 1e-9 of itself, so results comparable to the last digits
 // need the same roundings there
 constexpr int TRIDIAG_FIXED_MAX = 512;
-// the same for elongated molecules: the extent (largest side of the box around the atoms, Bohr) above
-// which a molecule keeps those roundings.  Charges that differ by 1e-13 over alkanes of 25 / 45 / 75
-// carbons (60 / 110 / 180 Bohr) change their dipole by 1e-9 / 3e-9 / 1e-8 of itself; clusters of 64
-// waters (30 Bohr) by 3e-11.
+// the same for elongated molecules of the one-molecule path: the extent (largest side of the box
+// around the atoms along the coordinate axes, Bohr) above which a molecule keeps those roundings.  This
+// is a matter of last digits and not of accuracy.  Below the line the dipole differs from the FP64
+// kernels' by at most 2.4e-10 of itself (alkanes of 8 to 25 carbons with boxes of 15 to 28 Bohr) and
+// 1.3e-10 (85 waters, 27 Bohr), above it charges and dipoles are theirs bit for bit; an SCF at the
+// default accuracy is off from its own limit by 1e-4 to 3e-3 (chains) and 5e-6 to 2e-5 (waters) of
+// the dipole in either form.  The box follows the axes: 14 of 40 alkanes of 25 carbons with random
+// dihedrals (25 to 50 Bohr) are below the line, and a chain turned onto the diagonal can be.  The
+// batch has no such line: it takes the fixed-point kernels for every molecule it holds.
 constexpr double ORDERED_EXTENT = 34.0;
 void tridiag_fixed(int n, double* A, double* d, double* e, double* tau, long long* xch,
                    cudaStream_t s);
 size_t tridiag_exchange_words(int n);
-// factorise S once per geometry; returns 0 on success, >0 if S is not positive definite
 // X = L^-T of S = L L^T in fixed point (cholinv.cu), n up to TRIDIAG_FIXED_MAX; false: not launched.
 // *status (device) 0: done, 1: outside the fixed-point range, X not written
 bool cholinv_fixed(int n, const double* S, double* X, int* status, cudaStream_t s);
+// factorise S once per geometry; returns 0 on success, >0 if S is not positive definite
 int eigen_set_overlap(EigenSolver*, const double* S);
 // eigenvalues (ascending) of F C = S C e; keeps the tridiagonal form for eigen_vectors.
 // Only the nev lowest are computed (nev <= 0: all); e[nev..n) = 1e300, which the Fermi
@@ -371,12 +376,13 @@ void density_matrix(int n, int k, const double* C, const double* f, double* P, d
 // dimension ld; ex: M + ld ints of device scratch; status set to 1 if it did not complete
 void ogemm(bool ta, bool tb, int M, int N, int K, const double* A, const double* B, double* C,
            int ld, int kmode, int* ex, int* status, cudaStream_t s);
-// the eigensolver's tensor-core GEMM status word, and its check (synchronises the stream)
+// roundings of the FP64 kernels for the next molecule (ORDERED_EXTENT)
 void eigen_set_ordered(EigenSolver*, bool ordered);
-int* eigen_gemm_status(EigenSolver*);
 void* eigen_gemm_pair(EigenSolver*);  // workspace of the small products (pgemm_pair), or null
 void eigen_set_pair(EigenSolver*, bool on);
 bool eigen_pair_failed(EigenSolver*);  // small products are on and one did not complete
+// the eigensolver's tensor-core GEMM status word, and its check (synchronises the stream)
+int* eigen_gemm_status(EigenSolver*);
 bool eigen_gemm_failed(EigenSolver*);
 // wbo[A][B] += scale * sum (PS)_{nu mu} (PS)_{mu nu} over the orbitals of atoms A != B
 void launch_wbo(const DevMol& m, const double* PS, double* wbo, double scale, cudaStream_t s);
