@@ -80,13 +80,25 @@ MOLECULES = {"benzene": benzene, "ethane": ethane, "neopentane": neopentane,
 
 @pytest.mark.parametrize("name", list(MOLECULES))
 def test_orbitals(name):
+    z, x = MOLECULES[name]()
+    if name == "chain16":
+        assert np.ptp(x, axis=0).max() > 34.0
+    _check(z, x)
+
+
+# one CTA, cluster, grid, the FP64 kernels above; products on FP64 tiles and the tensor cores
+@pytest.mark.parametrize("nao", [2, 7, 33, 63, 64, 65, 127, 128, 163, 256, 257, 512, 513])
+def test_orbitals_by_size(nao):
+    from test_gpu_tridiag import _molecule
+
+    _check(*_molecule(nao))
+
+
+def _check(z, x):
     from oracle import gfn2
     from oracle.d4 import D4
     from tblite_gb300.interface import Calculator
 
-    z, x = MOLECULES[name]()
-    if name == "chain16":
-        assert np.ptp(x, axis=0).max() > 34.0
     calc = Calculator("GFN2-xTB", z, x)
     calc.set("accuracy", 1e-3)
     calc.set("save-integrals", True)
