@@ -1086,8 +1086,8 @@ static void singlepoint(_tblite_context* ctx, const _tblite_structure* mol,
     }
     auto analyse = [&]() {
     g_prof.begin(PH_MULLIKEN, s);
-    launch_mulliken(m, w.P.p, w.S.p, w.H.p, w.D.p, w.Q.p, w.mull.p, mulliken_rows(n, ordered),
-                    w.qsh_o.p, w.qat_o.p, w.dpat_o.p, w.qpat_o.p, w.eband.p, s);
+    launch_mulliken(m, w.P.p, w.S.p, w.H.p, w.D.p, w.Q.p, w.mull.p, ordered, w.qsh_o.p,
+                    w.qat_o.p, w.dpat_o.p, w.qpat_o.p, w.eband.p, s);
     launch_pack(m, w.qsh_o.p, w.dpat_o.p, w.qpat_o.p, w.vec_out.p, s, with_mp);
     launch_diff((int)nd, w.vec_out.p, w.b_q.p, w.b_dq.p, w.scal.p + 1, s);  // mixer%diff
     launch_eelec_init(nat, w.scal.p, w.eband.p, w.eelec.p, s);

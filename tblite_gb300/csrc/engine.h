@@ -222,14 +222,13 @@ void launch_vao(const DevMol& m, const double* vsh, const double* vat, double* v
 void launch_fock(int n, const int* ao_at, const double* H, const double* S, const double* D,
                  const double* Q, const double* vao, const double* vdp, const double* vqp,
                  double* F, cudaStream_t s);
-// Mulliken analysis + band energy: column partial sums over chunks of `rows` rows (mulliken_rows),
-// then per-shell/atom reduction; partial holds mulliken_chunks(n) chunks of 11 n
+// Mulliken analysis + band energy: column partial sums over chunks of rows (ordered: 64 rows at any
+// size), then per-shell/atom reduction; partial holds mulliken_chunks(n) chunks of 11 n
 void launch_mulliken(const DevMol& m, const double* P, const double* S, const double* H,
-                     const double* D, const double* Q, double* partial, int rows,
+                     const double* D, const double* Q, double* partial, bool ordered,
                      double* qsh, double* qat, double* dpat, double* qpat, double* eat_band,
                      cudaStream_t s);
-int mulliken_rows(int n, bool ordered);  // rows of a chunk
-int mulliken_chunks(int n);              // the most chunks there are
+int mulliken_chunks(int n);  // the most chunks there are
 
 // Fermi filling of both spin channels; writes focc (alpha+beta), ts (entropy term) to scal[0]
 // nocc_cols[0]: orbitals with non-zero occupation; nocc_cols[1] = 1 when the nev computed

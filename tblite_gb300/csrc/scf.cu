@@ -811,15 +811,16 @@ void launch_fock(int n, const int* ao_at, const double* H, const double* S, cons
 // rows per chunk: 11 FP64 multiply-adds per row and column, so short chunks spread a molecule
 // over more SMs (68 orbitals: 64 rows 80 us, 16 rows 21 us)
 // (64 where a molecule keeps its order of summation, see tridiag_fixed)
-__host__ __device__ constexpr int mull_rows(int n) { return n <= 512 ? 16 : 64; }
+constexpr int MULL_SHORT = 16, MULL_LONG = 64;
+__host__ __device__ constexpr int mull_rows(int n) { return n <= 512 ? MULL_SHORT : MULL_LONG; }
 
-int mulliken_rows(int n, bool ordered) { return ordered ? 64 : mull_rows(n); }
 int mulliken_chunks(int n) { return (n + mull_rows(n) - 1) / mull_rows(n); }
 
-// ROWS rows with their loads in flight: four for one molecule, whose few blocks wait for them (21 ->
-// 10 us at 192 orbitals, 207 -> 73 us at 1202), one in a batch, where other blocks fill the time
-// (four take 95 us a launch instead of 65 there)
-template <int ROWS>
+// FLIGHT rows with their loads in flight: four for one molecule, whose few blocks wait for them (21 ->
+// 10 us at 192 orbitals, 207 -> 73 us at 1202; 245 us where the rows of a chunk are not a constant of
+// the kernel), one in a batch, where other blocks fill the time (four take 95 us a launch instead of
+// 65 there)
+template <int FLIGHT>
 __device__ __forceinline__ void mull_partial_dev(int n, int rows, const double* __restrict__ P,
                                                       const double* __restrict__ S,
                                                       const double* __restrict__ H,
@@ -834,7 +835,7 @@ __device__ __forceinline__ void mull_partial_dev(int n, int rows, const double* 
 #pragma unroll
   for (int k = 0; k < 11; ++k) acc[k] = 0.0;
   const int r0 = chunk * rows, r1 = min(n, r0 + rows);
-#pragma unroll ROWS
+#pragma unroll FLIGHT
   for (int r = r0; r < r1; ++r) {
     const size_t rc = (size_t)r * n + c;
     const double pv = P[rc];
@@ -848,14 +849,14 @@ __device__ __forceinline__ void mull_partial_dev(int n, int rows, const double* 
 #pragma unroll
   for (int k = 0; k < 11; ++k) partial[((size_t)chunk * 11 + k) * n + c] = acc[k];
 }
-__global__ void __launch_bounds__(128) k_mull_partial(int n, int rows,
-                                                      const double* __restrict__ P,
+template <int ROWS>
+__global__ void __launch_bounds__(128) k_mull_partial(int n, const double* __restrict__ P,
                                                       const double* __restrict__ S,
                                                       const double* __restrict__ H,
                                                       const double* __restrict__ D,
                                                       const double* __restrict__ Q,
                                                       double* partial) {
-  mull_partial_dev<4>(n, rows, P, S, H, D, Q, partial);
+  mull_partial_dev<4>(n, ROWS, P, S, H, D, Q, partial);
 }
 
 // 16 threads per atom, one per sum (population, 3 dipole, 6 quadrupole, band energy): reduce the
@@ -895,12 +896,13 @@ __global__ void k_mull_reduce(DevMol m, const double* __restrict__ partial, int 
 }
 
 void launch_mulliken(const DevMol& m, const double* P, const double* S, const double* H,
-                     const double* D, const double* Q, double* partial, int rows, double* qsh,
+                     const double* D, const double* Q, double* partial, bool ordered, double* qsh,
                      double* qat, double* dpat, double* qpat, double* eband, cudaStream_t s) {
-  const int n = m.nao, nchunk = (n + rows - 1) / rows;
+  const int n = m.nao, rows = ordered ? MULL_LONG : mull_rows(n), nchunk = (n + rows - 1) / rows;
+  auto partial_sums = rows == MULL_LONG ? k_mull_partial<MULL_LONG> : k_mull_partial<MULL_SHORT>;
   ++g_kernel_launches;
   const int tk = prof_kbegin(s);
-  k_mull_partial<<<dim3((n + 127) / 128, nchunk), 128, 0, s>>>(n, rows, P, S, H, D, Q, partial);
+  partial_sums<<<dim3((n + 127) / 128, nchunk), 128, 0, s>>>(n, P, S, H, D, Q, partial);
   prof_kend(KS_MULLIKEN, tk, s);
   ++g_kernel_launches;
   k_mull_reduce<<<(m.nat * MULL_LANES + 127) / 128, 128, 0, s>>>(m, partial, nchunk, qsh, qat, dpat,
