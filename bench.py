@@ -59,7 +59,8 @@ SOLVATED = {"h2o1000_alpb"}
 PURIFIED = {"h2o1000_alpb", "c200h402_sp2"}
 LARGE = {"h2o1000_alpb"}  # one oracle evaluation takes tens of minutes: bounded CPU samples
 SPLIT_SLICE_PRODUCTS = 36  # BF16 slice products per FP64 product in the split GEMM
-BATCH_SLICE_PRODUCTS = 28  # the same in the batch (balanced radix-256 digits)
+BATCH_SLICE_PRODUCTS = 28  # the same in the batch and up to 512 orbitals (balanced radix-256 digits)
+FIXED_POINT_MAX = 512  # orbitals up to which one molecule is tridiagonalised in fixed point
 # comparison legs of the ensemble: one seeded random order of the ensemble's molecules; the
 # plain GPU leg takes its first 64, the CPU baseline its first 256 (with the accuracy check of
 # the GPU results), the reference arm consecutive slices of REF_PER_STEP per step
@@ -191,20 +192,26 @@ def _profile_traffic(name):
 def _roofline(kprof, n, ms_step, peaks, peak_kind, fp64_peak, split_flops=None):
     """Roofline of the dominant own kernel (largest summed event time in the step).
 
-    Algorithmic work per launch: Householder tridiagonalisation 4/3 n^3 flop; Fock assembly
+    Algorithmic work per launch: Householder tridiagonalisation 4/3 n^3 flop (above 512 orbitals;
+    the fixed-point form below is bound by integer issue and the chain of its columns, for which
+    there is no measured peak); Fock assembly
     reads H, S, D(3), Q(6) and writes F = 12 n^2 doubles; Mulliken column sums read P, S, H,
     D(3), Q(6) = 12 n^2 doubles; split GEMM (split_flops: FP64 flop of the step's products,
-    counted by the library) 36 BF16 slice products per FP64 product on the tensor cores,
-    against the sustained bf16 peak.  The other slots have data-dependent work and are listed
-    with their times only."""
+    counted by the library) 36 BF16 slice products (28 up to 512 orbitals) per FP64 product on the
+    tensor cores, against the sustained bf16 peak.  The other slots have data-dependent work and
+    are listed with their times only."""
     kernels = {k: {"ms_per_launch": round(t / c, 4) if c else None, "launches": c,
                    "share_of_step": round(t / ms_step, 4) if ms_step else None}
                for k, (t, c) in kprof.items()}
     work = {"tridiag": ("fp64", 4.0 / 3.0 * n ** 3, "tridiag_smem_c200h402.md"),
             "fock": ("hbm", 12.0 * n * n * 8.0, None),
             "mulliken": ("hbm", 12.0 * n * n * 8.0, None)}
+    products = SPLIT_SLICE_PRODUCTS
+    if n <= FIXED_POINT_MAX:
+        del work["tridiag"]
+        products = BATCH_SLICE_PRODUCTS
     if split_flops and kprof.get("gemm", (0, 0))[1]:
-        work["gemm"] = ("tensor", SPLIT_SLICE_PRODUCTS * split_flops / kprof["gemm"][1], None)
+        work["gemm"] = ("tensor", products * split_flops / kprof["gemm"][1], None)
     dom = max(kprof, key=lambda k: kprof[k][0])
     pick = dom if dom in work else max(work, key=lambda k: kprof[k][0])
     t, c = kprof[pick]
@@ -228,8 +235,7 @@ def _roofline(kprof, n, ms_step, peaks, peak_kind, fp64_peak, split_flops=None):
             "peak_source": src, "algorithmic_work_per_launch": units, "ms_per_launch": round(ms, 4),
             "launches_per_step": c}
     if bound == "tensor":
-        roof["fp64_equivalent_tflops"] = round(units / SPLIT_SLICE_PRODUCTS / (ms / 1000.0) / 1e12,
-                                               4)
+        roof["fp64_equivalent_tflops"] = round(units / products / (ms / 1000.0) / 1e12, 4)
     return roof, kernels
 
 
@@ -523,15 +529,17 @@ def run_batch(args):
     timing = ("CUDA events around each launch on its stream, one untimed call with the size "
               "buckets serialised on one stream")
     tri_roof = {"kernel": "tridiag (batched, one block cluster per molecule, 64-bit fixed "
-                          "point: FP64-equivalent flop)", "bound": "fp64",
+                          "point: FP64-equivalent flop)",
+                "bound": "integer multiply-add issue and the chain of the columns",
                 "achieved": round(tri_flops_s / (t_tri / 1000.0) / 1e12, 4) if t_tri else None,
-                "peak": round(fp64_peak, 4), "unit": "TFLOP/s",
-                "frac": round(tri_flops_s / (t_tri / 1000.0) / 1e12 / fp64_peak, 4) if t_tri else None,
-                "timing": timing, "traffic": 17577984,
-                "traffic_note": "dram__bytes_read+write of one launch of the FP64 form (38 molecules, "
-                                "288-384 orbitals; profiles/tridiag_cluster_ensemble512.md): each "
-                                "matrix is read once, n^2 x 8 B per molecule, as now",
-                "peak_source": "measured in this run (cuBLAS DGEMM 4096^3)",
+                "peak": None, "unit": "TFLOP/s", "frac": None,
+                "peak_note": "no measured rate to compare with: the column loop is integer work "
+                             f"(FP64 peak of this run, cuBLAS DGEMM 4096^3: {fp64_peak:.3f})",
+                "timing": timing, "traffic": _profile_traffic("fixed_point_ensemble512.md"),
+                "traffic_note": "dram__bytes_read+write of one captured kb_tri_fixed launch (33 "
+                                "molecules of 72-92 orbitals; "
+                                "profiles/fixed_point_ensemble512.md): each matrix is read once, "
+                                "n^2 x 8 B per molecule",
                 "algorithmic_work_per_call": tri_flops_s, "ms_per_call": round(t_tri, 3),
                 "launches_per_call": c_tri,
                 "ms_per_launch": round(t_tri / c_tri, 4) if c_tri else None}
@@ -542,11 +550,12 @@ def run_batch(args):
                                "kb_opipe_sq and product sites kb_opipe_site)",
                      "bound": "tensor", "achieved": round(ach, 4), "peak": round(bf16, 4),
                      "unit": "TFLOP/s", "frac": round(ach / bf16, 4), "timing": timing,
-                     "traffic": _profile_traffic("pipe_sq_ensemble512.md"),
+                     "traffic": _profile_traffic("pipe_sq_step_ensemble512.md"),
                      "traffic_note": "dram__bytes_read+write of one captured kb_opipe_sq launch "
                                      "(38 molecules of 288-384 orbitals; "
-                                     "profiles/pipe_sq_ensemble512.md): each slice image read "
-                                     "about once from DRAM, the tile re-reads served by L2",
+                                     "profiles/pipe_sq_step_ensemble512.md): each slice "
+                                     "image read about once from DRAM, the tile re-reads "
+                                     "served by L2; the next iterate and its image written",
                      "peak_source": f"{peak_kind} (bf16 sustained)",
                      "algorithmic_work_per_call": BATCH_SLICE_PRODUCTS * pipe_flops_s,
                      "work_note": "28 BF16 slice products per FP64-equivalent flop; FP64-"

@@ -53,9 +53,9 @@ int tblite_gb300_batch_last_projected(void);
 int tblite_gb300_batch_last_modes(int* modes, int nmol);
 /* Autotuner of the batch schedule: coordinate descent over CUDA graphs (kept, or switched off;
  * never switched on against tblite_gb300_set_batch_graphs), the projection threshold (64, 80, 96,
- * 112, 128, 144, 176 orbitals or off), the bucket cut (3/4, 2/3, 4/5 of the largest orbital count), the CTAs
- * per SM of the cluster tridiagonalisation (1, 2), the small-bucket tridiagonalisation (full
- * storage or packed) and the side streams (4, 8, 16), each candidate
+ * 112, 128, 144, 176 orbitals or off), the bucket cut (3/4, 2/3, 4/5 of the largest orbital count), the
+ * two switches of the batched tridiagonalisation (tblite_gb300_set_tridiag_ctas_per_sm,
+ * tblite_gb300_set_small_tridiag) and the side streams (4, 8, 16), each candidate
  * timed as the wall time of a batch call (best of three) on a fixed pseudo-random sample of
  * `sample` of the given molecules (256 if <= 0); a candidate replaces the current choice only
  * when more than 1 % faster.  The fastest schedule stays set.  Returns the
@@ -116,8 +116,9 @@ int tblite_gb300_get_profile(double* phase_ms, int* phase_count, int nphase, dou
  * events around each launch on the engine stream (profiling enabled).  Slots: 0 Householder
  * tridiagonalisation, 1 eigenvalue multisection, 2 inverse iteration, 3 back-transformation,
  * 4 GEMM (all uses outside the pipelined split GEMM), 5 Fock assembly, 6 Mulliken column sums,
- * 7 pipelined split GEMM products of the batch (kb_opipe_sq, kb_opipe_site), 8 their operand
- * preparation (projection steps kb_sp2_step, exponents and slice images of the GEMM sites).
+ * 7 pipelined split GEMM products of the batch (kb_opipe_sq with the next iterate's slice image,
+ * kb_opipe_site), 8 their operand preparation (first iterate kb_sp2_init, exponents and slice
+ * images of the GEMM sites).
  * Returns the slot count. */
 int tblite_gb300_get_kernel_profile(double* kernel_ms, int* kernel_count, int nslot);
 

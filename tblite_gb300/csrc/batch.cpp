@@ -1302,8 +1302,8 @@ int get_tridiag_ctas_per_sm();
 int get_tridiag_small();
 }
 
-// back to the default schedule (CUDA graphs, projection from 96 orbitals, bucket cut 3/4, two
-// CTAs per SM, full-storage small tridiagonalisation, 8 streams)
+// back to the default schedule (CUDA graphs, projection from 96 orbitals, bucket cut 3/4, wider
+// tridiagonalisation clusters in small batches, one CTA where the matrix fits, 8 streams)
 extern "C" void tblite_gb300_batch_reset_schedule(void) {
   g_batch_graphs = true;
   g_sp2_min_nao = SP2_MIN_NAO;
@@ -1315,17 +1315,17 @@ extern "C" void tblite_gb300_batch_reset_schedule(void) {
   g_schedule_note = "defaults";
 }
 
-// The batch schedule: projection threshold, bucket cut, CTAs per SM of the cluster
-// tridiagonalisation and side streams, as a short text for logs and benchmark records.
+// The batch schedule: projection threshold, bucket cut, clusters of the tridiagonalisation and side
+// streams, as a short text for logs and benchmark records.
 extern "C" int tblite_gb300_batch_schedule(char* buf, int n) {
   char tmp[384];
   const int len = std::snprintf(
       tmp, sizeof(tmp),
-      "projection from %d orbitals%s; bucket cut %d/%d; tridiagonalisation %d CTA(s) per SM, "
-      "%s below 157 orbitals; %d streams; %s",
+      "projection from %d orbitals%s; bucket cut %d/%d; tridiagonalisation in %s clusters, "
+      "%s where one holds the matrix; %d streams; %s",
       g_sp2_min_nao, g_batch_sp2 ? "" : " (off)", g_cut_num, g_cut_den,
-      tb::get_tridiag_ctas_per_sm(), tb::get_tridiag_small() ? "full storage" : "packed",
-      g_batch_streams, g_schedule_note.c_str());
+      tb::get_tridiag_ctas_per_sm() == 2 ? "wider" : "the narrowest",
+      tb::get_tridiag_small() ? "one CTA" : "two CTAs", g_batch_streams, g_schedule_note.c_str());
   if (buf && n > 0) {
     std::strncpy(buf, tmp, (size_t)n - 1);
     buf[n - 1] = '\0';
@@ -1334,7 +1334,7 @@ extern "C" int tblite_gb300_batch_schedule(char* buf, int n) {
 }
 
 // Autotuner of the batch schedule (no counterpart in the reference): coordinate descent over
-// CUDA graphs on/off, the projection threshold, the bucket cut, the CTAs per SM of the tridiagonalisation and the side
+// CUDA graphs on/off, the projection threshold, the bucket cut, the clusters of the tridiagonalisation and the side
 // streams, each candidate timed (wall time of the call, best of three) on a seeded sample of the given
 // molecules; the fastest schedule stays set.  Returns the number of timed calls, or -1 if the
 // sample could not be evaluated (the schedule is then left as it was).
